@@ -10,9 +10,9 @@
 //       near   : offsets < 2 per axis, 20-point rule with the weakly singular
 //                pairs replaced by the self / edge / vertex integrals
 //                (nearby_correct.m), overriding medium
-//     Only 21 face pairs are integrated; the other 15 are copies
-//     (cubature_nop.cpp:100-115).  The far loop skips offsets that the medium
-//     loop overwrites.
+//     The reference integrates 21 face pairs per offset and copies the other
+//     15 (cubature_nop.cpp:100-115).  Here the sums are taken from tables that
+//     all offsets, face pairs and components share (k_face_sums).
 //   circulant embedding 2L x 2M x 2N with per-axis parities (circulant_nop.m,
 //     gperiodic_coeff_nop.m) and the 3-D FFT of each of the 6 components.
 //
@@ -25,7 +25,9 @@
 // Gauss-Legendre converges to machine precision; it differs from DIRECTFN at
 // Np_1D = 20 by up to 3.4e-5 (the truncation error of DIRECTFN at that order).
 // singular = 'U' takes the five values from the caller.
+#include <algorithm>
 #include <cmath>
+#include <utility>
 #include <vector>
 
 #include "matvec_launch.cuh"
@@ -113,32 +115,9 @@ __constant__ int c_copy_src[15][2] = {{0, 0}, {1, 3}, {0, 3}, {1, 2}, {0, 2}, {2
 
 struct CubArgs {
   double face_o[6][3], face_a[6][3], face_b[6][3];
-  double P[6][6][6];  // vector_projection.m: P(i,j,k)
-  double2 sing[5];    // ST, EAc, EAo, VAc, VAo
   double ko, dx, scale;  // K: the factor dx^4 / (j k0)^2 / (4 pi) of assembly_kop.m
   int L, M, N;
 };
-
-// vector_projection.m:10-25 with face normals [-x,+x,-y,+y,-z,+z]
-static void make_projection(double P[6][6][6]) {
-  const double nrm[6][3] = {{-1, 0, 0}, {1, 0, 0}, {0, -1, 0}, {0, 1, 0}, {0, 0, -1}, {0, 0, 1}};
-  const int comp[6][2] = {{0, 0}, {0, 1}, {0, 2}, {1, 1}, {1, 2}, {2, 2}};
-  auto cross = [](const double* a, const double* b, double* c) {
-    c[0] = a[1] * b[2] - a[2] * b[1];
-    c[1] = a[2] * b[0] - a[0] * b[2];
-    c[2] = a[0] * b[1] - a[1] * b[0];
-  };
-  for (int i = 0; i < 6; ++i)
-    for (int j = 0; j < 6; ++j)
-      for (int k = 0; k < 6; ++k) {
-        double ea[3] = {0, 0, 0}, eb[3] = {0, 0, 0}, c1[3], c2[3];
-        ea[comp[k][0]] = 1;
-        eb[comp[k][1]] = 1;
-        cross(nrm[i], ea, c1);
-        cross(nrm[j], eb, c2);
-        P[i][j][k] = c1[0] * c2[0] + c1[1] * c2[1] + c1[2] * c2[2];
-      }
-}
 
 // Singular class of face pair (obs face i of the voxel at offset m in {0,1}^3,
 // src face j of the voxel at the origin), derived from the geometry:
@@ -179,133 +158,160 @@ __device__ __forceinline__ void face_points(const CubArgs& A, int f, const doubl
   }
 }
 
-// Sum over Np x Np point pairs of w_p w_q exp(-j ko R)/R for one face pair
-// (points of the observation face P, of the source face Q, both [i][3] in
-// shared memory; the observation voxel is displaced by rm); threads t0,
-// t0 + nt, ... split the pairs.  1/R comes from one reciprocal square root
-// (R = R^2 / R), not a square root and a division: the FP64 pipe is the limit.
-__device__ double2 face_pair_sum(const double* __restrict__ P, const double* __restrict__ Q,
-                                 const double* __restrict__ w, int Np, double ko, const double rm[3], int t0,
-                                 int nt) {
-  double2 acc = mk<double2>(0, 0);
-  const int tot = Np * Np;
-  for (int t = t0; t < tot; t += nt) {
-    const int ip = t / Np, iq = t - ip * Np;
-    const double dx0 = Q[3 * iq] - (P[3 * ip] + rm[0]);
-    const double dx1 = Q[3 * iq + 1] - (P[3 * ip + 1] + rm[1]);
-    const double dx2 = Q[3 * iq + 2] - (P[3 * ip + 2] + rm[2]);
-    const double R2 = dx0 * dx0 + dx1 * dx1 + dx2 * dx2;
-    const double Ri = rsqrt(R2);
-    double s, c;
-    sincos(ko * (R2 * Ri), &s, &c);
-    const double wt = w[ip] * w[iq] * Ri;
-    acc.x += wt * c;
-    acc.y -= wt * s;
-  }
-  return acc;
-}
+// ---------------------------------------------------------------------------
+// Face-pair sums shared by offsets, face pairs and components.
+//
+// With tensor Gauss-Legendre rules on both squares, the quadrature of
+// exp(-j k0 R)/R over two faces depends only on where the faces lie relative to
+// each other (lengths in voxels, u the rule's nodes on [0, 1]):
+//   F(s; b, c)  parallel faces, planes s apart, displaced by b and c in plane:
+//               R^2 = s^2 + (b + u_i - u_k)^2 + (c + u_j - u_l)^2
+//   Q(c; p, q)  crossed faces, planes p and q of the other face's axis:
+//               R^2 = (p - u_i)^2 + (q - u_k)^2 + (c + u_j - u_l)^2
+// (the nodes are symmetric about 1/2, so the sign of an offset and the order of
+// the two faces do not matter).  The nine parallel pairs of an offset are F at
+// s = m - 1, m, m + 1 along the three axes and the twelve crossed pairs are Q
+// at p, q = m, m + 1; neighbouring offsets read the same entries, and on cubic
+// voxels the three axes are permutations of one table.  So F and Q are
+// evaluated once per sorted triple, with the differences u_i - u_k merged by
+// value (9 of the 4-point rule's 16): at most 3*81 + 3*144 evaluations per
+// sorted triple, about 112 per offset of a cubic grid, where one sum per offset
+// and face pair takes 21*256.
+//
+// FP64-pipe bound (an evaluation is about 50 FP64 instructions, most of them
+// sincos and rsqrt): one warp per entry, its lanes over the points of the sum,
+// so that short rows of a small grid fill the pipe as well as long ones.
+// Measured on GB300 for a 96^3 grid: 10.1 ms for the 4-point rule, 0.4 and 0.6
+// ms for the other two, where the sum per offset and face pair took 438, 2.3
+// and 4.0 ms.
+// ---------------------------------------------------------------------------
+constexpr int kRuleMax = 20;                                   // nodes of the largest rule
+constexpr int kDiffMax = kRuleMax * (kRuleMax - 1) / 2 * 2 + 1;  // its differences, before merging less than this
 
-// Mirror, optional near-field correction, projection and scaling of one
-// offset's 21 integrals J21 (already multiplied by nothing); writes G (6 comps).
-__device__ void finish_offset(const CubArgs& A, const double2* J21, int mx, int my, int mz, bool near,
-                              double2* __restrict__ G, long long V, long long off) {
-  double2 J[6][6];
-  for (int i = 0; i < 6; ++i)
-    for (int j = 0; j < 6; ++j) J[i][j] = mk<double2>(0, 0);
-  for (int p = 0; p < 21; ++p) J[c_pair_obs[p]][c_pair_src[p]] = cscale(J21[p], A.dx * A.dx * A.dx * A.dx);
-  for (int c = 0; c < 15; ++c) J[c_copy_dst[c][0]][c_copy_dst[c][1]] = J[c_copy_src[c][0]][c_copy_src[c][1]];
-  if (near) {
-    for (int i = 0; i < 6; ++i)
-      for (int j = 0; j < 6; ++j) {
-        const int cls = near_class(mx, my, mz, i, j);
-        if (cls > 0) J[i][j] = A.sing[cls - 1];
+struct FaceRule {
+  int nu, nd;
+  double u[kRuleMax], wu[kRuleMax];  // nodes on [0, 1], weights
+  double d[kDiffMax], wd[kDiffMax];  // distinct differences u_i - u_k, summed weight products
+};
+
+// Entries of the sorted triples x >= y >= z, x < e0, y < e1, z < e2; table i < 3:
+// F with s at sorted place i, table 3 + i: Q with c at sorted place i.  Each
+// entry is the sum of `split` parts.
+struct FaceTable {
+  const double2* v;
+  int e0, e1, e2, split;
+  __device__ __forceinline__ double2 get(int kind, int s, int b, int c) const {
+    const int hi = b > c ? b : c, lo = b > c ? c : b;
+    int x = hi, y = lo, z = s, place = 2;
+    if (s >= hi) {
+      x = s; y = hi; z = lo; place = 0;
+    } else if (s >= lo) {
+      x = hi; y = s; z = lo; place = 1;
+    }
+    const long long n = (long long)e0 * e1 * e2;
+    const double2* p = v + (3 * kind + place) * n + ((long long)z * e1 + y) * e0 + x;
+    double2 r = p[0];
+    for (int i = 1; i < split; ++i) r = cadd(r, p[6 * n * i]);
+    return r;
+  }
+};
+
+// grid (e1, e2, 6 * split): row (y, z) of one table, the block's warps over x
+__global__ void __launch_bounds__(128) k_face_sums(const FaceRule* __restrict__ rule, double k, int e0, int split,
+                                                   double2* __restrict__ out) {
+  const int y = blockIdx.x, z = blockIdx.y;
+  if (y < z) return;
+  const int e1 = gridDim.x, e2 = gridDim.y;
+  const int table = blockIdx.z % 6, part = blockIdx.z / 6;
+  __shared__ FaceRule r;
+  {
+    const double* src = reinterpret_cast<const double*>(rule);
+    double* dst = reinterpret_cast<double*>(&r);
+    static_assert(sizeof(FaceRule) % sizeof(double) == 0, "rule copied in doubles");
+    for (int i = threadIdx.x; i < (int)(sizeof(FaceRule) / sizeof(double)); i += blockDim.x) dst[i] = src[i];
+  }
+  __syncthreads();
+  const int place = table % 3;
+  const bool crossed = table >= 3;
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const int n1 = crossed ? r.nu : r.nd, n0 = r.nd;
+  const int total = crossed ? n0 * n1 * n1 : n0 * n1;
+  const int chunk = (total + split - 1) / split;
+  const int t0 = part * chunk, t1 = min(total, t0 + chunk);
+  double2* row = out + (long long)part * 6 * e0 * e1 * e2 + (((long long)table * e2 + z) * e1 + y) * e0;
+  for (int x = y + (threadIdx.x >> 5); x < e0; x += warps) {
+    // the special coordinate (F: the plane distance s, Q: c) and the other two
+    const double s = place == 0 ? x : place == 1 ? y : z;
+    const double b = place == 0 ? y : x, c = place == 2 ? y : z;
+    double2 acc = mk<double2>(0, 0);
+    for (int t = t0 + lane; t < t1; t += 32) {
+      const int i0 = t % n0;
+      int i1 = t / n0;
+      double r2, w;
+      if (crossed) {
+        const int i2 = i1 / n1;
+        i1 -= i2 * n1;
+        const double a0 = s + r.d[i0], a1 = b - r.u[i1], a2 = c - r.u[i2];
+        r2 = fma(a0, a0, fma(a1, a1, a2 * a2));
+        w = r.wd[i0] * (r.wu[i1] * r.wu[i2]);
+      } else {
+        const double a0 = b + r.d[i0], a1 = c + r.d[i1];
+        r2 = fma(a0, a0, fma(a1, a1, s * s));
+        w = r.wd[i0] * r.wd[i1];
       }
-  }
-  const double s = 1.0 / (4.0 * M_PI);
-  for (int k = 0; k < 6; ++k) {
-    double2 g = mk<double2>(0, 0);
-    for (int i = 0; i < 6; ++i)
-      for (int j = 0; j < 6; ++j) {
-        const double pp = A.P[i][j][k];
-        if (pp != 0.0) g = cadd(g, cscale(J[i][j], pp));
-      }
-    G[k * V + off] = cscale(g, s);
-  }
-}
-
-// far field: one warp per offset outside the medium region
-__global__ void k_cub_far(CubArgs A, const double* __restrict__ gw, const double* __restrict__ gu,
-                          const double* __restrict__ gv, int Np, int n_medium, double2* __restrict__ G) {
-  __shared__ double w[16], u[16], v[16];
-  __shared__ double X[6][16 * 3];  // quadrature points of the six faces
-  if (threadIdx.x < Np) {
-    w[threadIdx.x] = gw[threadIdx.x];
-    u[threadIdx.x] = gu[threadIdx.x];
-    v[threadIdx.x] = gv[threadIdx.x];
-  }
-  __syncthreads();
-  for (int f = 0; f < 6; ++f) face_points(A, f, u, v, Np, X[f], threadIdx.x, blockDim.x);
-  __syncthreads();
-  const long long V = (long long)A.L * A.M * A.N;
-  const int lane = threadIdx.x & 31;
-  const long long wpb = blockDim.x >> 5;
-  for (long long off = blockIdx.x * wpb + (threadIdx.x >> 5); off < V; off += (long long)gridDim.x * wpb) {
-    const int mx = (int)(off % A.L);
-    const int my = (int)((off / A.L) % A.M);
-    const int mz = (int)(off / ((long long)A.L * A.M));
-    if (mx < n_medium && my < n_medium && mz < n_medium) continue;
-    const double rm[3] = {mx * A.dx, my * A.dx, mz * A.dx};
-    double2 J21[21];
-    for (int p = 0; p < 21; ++p)
-      J21[p] = warp_sum2(face_pair_sum(X[c_pair_obs[p]], X[c_pair_src[p]], w, Np, A.ko, rm, lane, 32));
-    if (lane == 0) finish_offset(A, J21, mx, my, mz, false, G, V, off);
+      const double ri = rsqrt(r2);
+      double sn, cs;
+      sincos(k * (r2 * ri), &sn, &cs);
+      w *= ri;
+      acc.x = fma(w, cs, acc.x);
+      acc.y = fma(-w, sn, acc.y);
+    }
+    acc = warp_sum2(acc);
+    if (lane == 0) row[x] = acc;
   }
 }
 
-// medium / near: one block per (offset, pair); offsets enumerated in [0,nr)^3
-__global__ void k_cub_region(CubArgs A, const double* __restrict__ gw, const double* __restrict__ gu,
-                             const double* __restrict__ gv, int Np, int nr, double2* __restrict__ J21out) {
-  extern __shared__ double sh[];
-  double* w = sh;
-  double* u = sh + Np;
-  double* v = sh + 2 * Np;
-  double* P = sh + 3 * Np;  // points of the observation face, [i][3]
-  double* Q = P + 3 * Np;   // points of the source face
-  for (int i = threadIdx.x; i < Np; i += blockDim.x) {
-    w[i] = gw[i];
-    u[i] = gu[i];
-    v[i] = gv[i];
-  }
-  __syncthreads();
-  const int pair = blockIdx.y;
-  face_points(A, c_pair_obs[pair], u, v, Np, P, threadIdx.x, blockDim.x);
-  face_points(A, c_pair_src[pair], u, v, Np, Q, threadIdx.x, blockDim.x);
-  __syncthreads();
-  const int o = blockIdx.x;
-  const int mx = o % nr, my = (o / nr) % nr, mz = o / (nr * nr);
-  const double rm[3] = {mx * A.dx, my * A.dx, mz * A.dx};
-  double2 acc = face_pair_sum(P, Q, w, Np, A.ko, rm, threadIdx.x, blockDim.x);
-  acc = warp_sum2(acc);
-  __shared__ double2 ws[32];
-  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double2 t = mk<double2>(0, 0);
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t = cadd(t, ws[i]);
-    J21out[(long long)o * 21 + pair] = t;
-  }
-}
+struct NearSums {
+  double2 v[5];  // ST, EAc, EAo, VAc, VAo in the tables' unit (dx^3)
+};
 
-__global__ void k_region_finish(CubArgs A, const double2* __restrict__ J21, int nr, bool near, double2* __restrict__ G) {
-  const long long V = (long long)A.L * A.M * A.N;
-  const int o = blockIdx.x * blockDim.x + threadIdx.x;
-  if (o >= nr * nr * nr) return;
-  const int mx = o % nr, my = (o / nr) % nr, mz = o / (nr * nr);
-  if (mx >= A.L || my >= A.M || mz >= A.N) return;
-  const long long off = mx + (long long)A.L * (my + (long long)A.M * mz);
-  double2 j21[21];
-  for (int p = 0; p < 21; ++p) j21[p] = J21[(long long)o * 21 + p];
-  finish_offset(A, j21, mx, my, mz, near, G, V, off);
+// Toeplitz entries from the tables: tab[0] the 4-point rule, tab[1] the
+// 10-point rule for offsets below 5, tab[2] the 20-point rule for offsets
+// below 2, where the touching faces take the singular integrals
+// (nearby_correct.m).  G_pp sums the second differences of F over the two
+// sides of the faces normal to the other axes, G_pq the mixed differences of Q
+// (vector_projection.m:10-25 with the face normals' signs).
+__global__ void __launch_bounds__(256) k_toeplitz(FaceTable far, FaceTable medium, FaceTable near, NearSums sing,
+                                                  double scale, int L, int M, int N, double2* __restrict__ G) {
+  const long long V = (long long)L * M * N;
+  for (long long off = blockIdx.x * (long long)blockDim.x + threadIdx.x; off < V;
+       off += (long long)gridDim.x * blockDim.x) {
+    const int mx = (int)(off % L), my = (int)((off / L) % M), mz = (int)(off / ((long long)L * M));
+    const int top = max(mx, max(my, mz));
+    const FaceTable& T = top < 2 ? near : top < 5 ? medium : far;
+    auto F = [&](int s, int b, int c) -> double2 {
+      if (top < 2 && s == 0 && b < 2 && c < 2) return sing.v[b + c == 0 ? 0 : b + c == 1 ? 1 : 3];
+      return T.get(0, s, b, c);
+    };
+    auto Q = [&](int c, int p, int q) -> double2 {
+      if (top < 2 && p < 2 && q < 2 && c < 2) return sing.v[c == 0 ? 2 : 4];
+      return T.get(1, c, p, q);
+    };
+    auto second = [&](int s, int b, int c) {
+      const double2 f = F(s, b, c);
+      return csub(cadd(f, f), cadd(F(s + 1, b, c), F(s > 0 ? s - 1 : 1, b, c)));
+    };
+    auto mixed = [&](int c, int p, int q) {
+      return csub(cadd(Q(c, p + 1, q + 1), Q(c, p, q)), cadd(Q(c, p + 1, q), Q(c, p, q + 1)));
+    };
+    const double2 dx = second(mx, my, mz), dy = second(my, mx, mz), dz = second(mz, mx, my);
+    G[off] = cscale(cadd(dy, dz), scale);
+    G[V + off] = cscale(mixed(mz, my, mx), scale);
+    G[2 * V + off] = cscale(mixed(my, mz, mx), scale);
+    G[3 * V + off] = cscale(cadd(dx, dz), scale);
+    G[4 * V + off] = cscale(mixed(mx, mz, my), scale);
+    G[5 * V + off] = cscale(cadd(dx, dy), scale);
+  }
 }
 
 // circulant_nop.m:23-40: index L of each axis stays zero; reflected blocks take
@@ -338,22 +344,41 @@ __global__ void k_circulant(const double2* __restrict__ G, int L, int M, int N, 
   }
 }
 
-// plain in-place forward FFT of contiguous rows of length NL (full input)
-template <int NL>
+// ---------------------------------------------------------------------------
+// FFT of the circulant from the Toeplitz entries.  Every component is even or
+// odd along each axis and zero at index L (circulant_nop.m:23-40), so each
+// 1-D transform takes its L entries, reflects them as it loads them, and keeps
+// the outputs 0 .. L; the others are +- their mirror images.  The three passes
+// then touch an eighth of the padded array and run a quarter of its transforms
+// (FP64-pipe bound, like all FP64 transforms here), and leave the octant that a
+// plan stores; k_expand_octant writes the full array where a caller wants it.
+// Measured for a 96^3 grid: 0.53 + 0.54 + 0.51 ms and 0.26 ms for the full
+// array, where writing the circulant and transforming all of it took 0.45 +
+// 2.2 + 1.9 + 1.9 ms.
+// ---------------------------------------------------------------------------
+// x: rows of L = NL/2 entries to rows of L + 1 outputs; row = (q * rows_q + ...)
+template <int NL, int KIND>
 __global__ void __launch_bounds__(RowCfg<double2, NL>::THREADS)
-k_rows_full(double2* __restrict__ data, long long rows, const double2* __restrict__ tw) {
+k_rows_parity(const double2* __restrict__ in, double2* __restrict__ out, long long rows, long long rows_q,
+              const double2* __restrict__ tw) {
   using V = double2;
   using F = FFT<V, NL, false>;
   constexpr int S = RowCfg<double2, NL>::S;
-  constexpr int ES = S + 1;
+  constexpr int ES = S + 1, L = NL / 2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V* tw_s = reinterpret_cast<V*>(smem_raw);
   V* buf = tw_s + NL;
   const long long row0 = (long long)blockIdx.x * S;
   stage_twiddles(tw_s, tw, NL);
-  for (int i = threadIdx.x; i < S * NL; i += blockDim.x) {
-    const int s = i / NL, x = i - s * NL;
-    buf[x * ES + s] = (row0 + s < rows) ? data[(row0 + s) * NL + x] : mk<V>(0, 0);
+  for (int i = threadIdx.x; i < S * L; i += blockDim.x) {
+    const int s = i / L, x = i - s * L;
+    const long long row = row0 + s;
+    const V v = row < rows ? in[row * L + x] : mk<V>(0, 0);
+    buf[x * ES + s] = v;
+    if (x > 0)
+      buf[(NL - x) * ES + s] = OpKind<KIND>::odd((int)(row / rows_q), 0) ? mk<V>(-v.x, -v.y) : v;
+    else
+      buf[L * ES + s] = mk<V>(0, 0);
   }
   __syncthreads();
   const int s = threadIdx.x % S, t = threadIdx.x / S;
@@ -363,21 +388,71 @@ k_rows_full(double2* __restrict__ data, long long rows, const double2* __restric
   __syncthreads();
   F::store(reg, buf + s, ES, t);
   __syncthreads();
-  for (int i = threadIdx.x; i < S * NL; i += blockDim.x) {
-    const int ss = i / NL, x = i - ss * NL;
-    if (row0 + ss < rows) data[(row0 + ss) * NL + x] = buf[x * ES + ss];
+  for (int i = threadIdx.x; i < S * (L + 1); i += blockDim.x) {
+    const int ss = i / (L + 1), x = i - ss * (L + 1);
+    if (row0 + ss < rows) out[(row0 + ss) * (L + 1) + x] = buf[x * ES + ss];
   }
 }
 
-static cudaError_t rows_full(int NL, double2* data, long long rows, const double2* tw, cudaStream_t st) {
+// y or z (axis): columns in[c + pitch * i + in_w * w], i < NC/2, to
+// out[c + pitch * k + out_w * w], k <= NC/2; component q = w / w_q
+template <int NC, int KIND>
+__global__ void __launch_bounds__(ColS<double>::S * FFT<double2, NC, false>::T)
+k_cols_parity(const double2* __restrict__ in, long long in_w, double2* __restrict__ out, long long out_w,
+              long long pitch, int w_q, int axis, const double2* __restrict__ tw) {
+  using V = double2;
+  using F = FFT<V, NC, false>;
+  constexpr int S = ColS<double>::S;
+  constexpr int ES = S + 1, H = NC / 2;
+  constexpr int E = F::E, R0 = F::R0, RL = F::RL;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  V* tw_s = reinterpret_cast<V*>(smem_raw);
+  V* buf = tw_s + NC;
+  const int s = threadIdx.x % S, t = threadIdx.x / S;
+  const long long c = (long long)blockIdx.x * S + s;
+  const long long w = blockIdx.y;
+  const bool active = c < pitch;
+  const bool odd = OpKind<KIND>::odd((int)(w / w_q), axis);
+  const V* inp = in + w * in_w + c;
+  V* outp = out + w * out_w + c;
+  stage_twiddles(tw_s, tw, NC);
+  V reg[E];
+#pragma unroll
+  for (int b = 0; b < E / R0; ++b)
+#pragma unroll
+    for (int r = 0; r < R0; ++r) {
+      const int p = F::in_pos(t, b, r);
+      V v = mk<V>(0, 0);
+      if (active && p != H) {
+        v = inp[pitch * (p < H ? p : NC - p)];
+        if (odd && p > H) v = mk<V>(-v.x, -v.y);
+      }
+      reg[b * R0 + r] = v;
+    }
+  __syncthreads();  // twiddles staged
+  F::run(reg, buf + s, ES, t, tw_s);
+#pragma unroll
+  for (int b = 0; b < E / RL; ++b)
+#pragma unroll
+    for (int r = 0; r < RL; ++r) {
+      const int k = F::out_pos(t, b, r);
+      if (active && k <= H) outp[pitch * k] = reg[b * RL + r];
+    }
+}
+
+template <int KIND>
+static cudaError_t rows_parity(int NL, const double2* in, double2* out, long long rows_q, const double2* tw,
+                               cudaStream_t st) {
+  const long long rows = OpKind<KIND>::NQ * rows_q;
   switch (NL) {
 #define MARIE_CASE(n_)                                                                                   \
   case n_: {                                                                                             \
-    constexpr int S = RowCfg<double2, n_>::S;                                                                     \
+    constexpr int S = RowCfg<double2, n_>::S;                                                            \
     const size_t smem = (size_t)(n_ + n_ * (S + 1)) * sizeof(double2);                                   \
-    cudaError_t e = opt_in_smem(k_rows_full<n_>, smem);                                                  \
+    cudaError_t e = opt_in_smem(k_rows_parity<n_, KIND>, smem);                                          \
     if (e != cudaSuccess) return e;                                                                      \
-    k_rows_full<n_><<<(unsigned)((rows + S - 1) / S), RowCfg<double2, n_>::THREADS, smem, st>>>(data, rows, tw); \
+    k_rows_parity<n_, KIND><<<(unsigned)((rows + S - 1) / S), RowCfg<double2, n_>::THREADS, smem, st>>>( \
+        in, out, rows, rows_q, tw);                                                                      \
     count_launch();                                                                                      \
     return cudaGetLastError();                                                                           \
   }
@@ -385,6 +460,54 @@ static cudaError_t rows_full(int NL, double2* data, long long rows, const double
 #undef MARIE_CASE
   }
   return cudaErrorInvalidValue;
+}
+
+template <int KIND>
+static cudaError_t cols_parity(int NC, const double2* in, long long in_w, double2* out, long long out_w,
+                               long long pitch, int w_q, int axis, const double2* tw, cudaStream_t st) {
+  switch (NC) {
+#define MARIE_CASE(n_)                                                                                      \
+  case n_: {                                                                                                \
+    constexpr int S = ColS<double>::S;                                                                      \
+    const size_t smem = (size_t)(n_ + n_ * (S + 1)) * sizeof(double2);                                      \
+    cudaError_t e = opt_in_smem(k_cols_parity<n_, KIND>, smem);                                             \
+    if (e != cudaSuccess) return e;                                                                         \
+    const dim3 grid((unsigned)((pitch + S - 1) / S), OpKind<KIND>::NQ * w_q);                               \
+    k_cols_parity<n_, KIND><<<grid, S * FFT<double2, n_, false>::T, smem, st>>>(in, in_w, out, out_w, pitch, \
+                                                                                w_q, axis, tw);             \
+    count_launch();                                                                                         \
+    return cudaGetLastError();                                                                              \
+  }
+    MARIE_FFT_LENGTHS(MARIE_CASE)
+#undef MARIE_CASE
+  }
+  return cudaErrorInvalidValue;
+}
+
+// Octant O (NQ x (N+1) x (M+1) x (L+1), unscaled) of the FFT of the circulant
+// of G (NQ x N x M x L).
+template <int KIND>
+static int octant_spectrum(int L, int M, int N, const double2* G, double2* O, cudaStream_t st) {
+  const int lens[3] = {2 * L, 2 * M, 2 * N};
+  DBuf twb[3], tmp;
+  for (int a = 0; a < 3; ++a) {
+    std::vector<double2> h(lens[a]);
+    for (int k = 0; k < lens[a]; ++k) {
+      const double ang = 2.0 * M_PI * k / lens[a];
+      h[k] = mk<double2>(std::cos(ang), -std::sin(ang));
+    }
+    MARIE_TRY(twb[a].alloc(lens[a] * sizeof(double2), st));
+    MARIE_CUDA_TRY(cudaMemcpyAsync(twb[a].p, h.data(), lens[a] * sizeof(double2), cudaMemcpyHostToDevice, st));
+  }
+  const long long Lo = L + 1, Mo = M + 1, No = N + 1;
+  MARIE_TRY(tmp.alloc((size_t)OpKind<KIND>::NQ * Lo * Mo * N * sizeof(double2), st));
+  double2* T = tmp.as<double2>();
+  // O holds the x pass's result until the z pass overwrites it
+  MARIE_CUDA_TRY(rows_parity<KIND>(2 * L, G, O, (long long)M * N, twb[0].as<double2>(), st));
+  MARIE_CUDA_TRY(cols_parity<KIND>(2 * M, O, M * Lo, T, Mo * Lo, Lo, N, 1, twb[1].as<double2>(), st));
+  MARIE_CUDA_TRY(cols_parity<KIND>(2 * N, T, N * Mo * Lo, O, No * Mo * Lo, Mo * Lo, 1, 2, twb[2].as<double2>(), st));
+  MARIE_CUDA_TRY(cudaStreamSynchronize(st));
+  return MARIE_OK;
 }
 
 // --------------------------------------------------------------------------
@@ -503,94 +626,62 @@ static int converged_integrals(double ko, double dx, int n, double2 out[5], cuda
   return MARIE_OK;
 }
 
+static void face_rule(int n, FaceRule& r) {
+  std::vector<double> x, w;
+  gauss_legendre(n, x, w);
+  r = FaceRule{};
+  r.nu = n;
+  for (int i = 0; i < n; ++i) {
+    r.u[i] = 0.5 * (x[i] + 1.0);
+    r.wu[i] = 0.5 * w[i];
+  }
+  std::vector<std::pair<double, double>> d;
+  for (int i = 0; i < n; ++i)
+    for (int k = 0; k < n; ++k) d.emplace_back(r.u[i] - r.u[k], r.wu[i] * r.wu[k]);
+  std::sort(d.begin(), d.end());
+  for (const auto& p : d) {
+    // the nodes' symmetry makes equal differences meet to the last bits
+    if (r.nd > 0 && p.first - r.d[r.nd - 1] < 1e-13) {
+      r.wd[r.nd - 1] += p.second;
+    } else {
+      r.d[r.nd] = p.first;
+      r.wd[r.nd++] = p.second;
+    }
+  }
+}
+
 // Toeplitz G (L x M x N x 6) on the device.
 static int assemble_toeplitz(int L, int M, int N, double dx, double ko, const double2 sing[5], double2* G,
                              cudaStream_t st) {
-  CubArgs A{};
-  const FaceGeom fg = make_faces(dx);
-  for (int f = 0; f < 6; ++f)
-    for (int c = 0; c < 3; ++c) {
-      A.face_o[f][c] = fg.o[f][c];
-      A.face_a[f][c] = fg.a[f][c];
-      A.face_b[f][c] = fg.b[f][c];
-    }
-  make_projection(A.P);
-  for (int i = 0; i < 5; ++i) A.sing[i] = sing[i];
-  A.ko = ko;
-  A.dx = dx;
-  A.L = L; A.M = M; A.N = N;
-  const int n_medium = 5;
-  struct Rule { DBuf w, u, v; int Np; };
-  Rule rules[3];
+  std::vector<FaceRule> rules(3);
   const int orders[3] = {4, 10, 20};
+  for (int r = 0; r < 3; ++r) face_rule(orders[r], rules[r]);
+  DBuf drules, tables[3];
+  MARIE_TRY(drules.alloc(3 * sizeof(FaceRule), st));
+  MARIE_CUDA_TRY(cudaMemcpyAsync(drules.p, rules.data(), 3 * sizeof(FaceRule), cudaMemcpyHostToDevice, st));
+  int dims[3] = {L, M, N};
+  std::sort(dims, dims + 3, [](int a, int b) { return a > b; });
+  // the reference's loops: medium offsets below 5, near ones below 2.  The few
+  // entries of those rules have long sums: 16 warps share each near entry
+  // (40401 or 80400 points), 2 each medium entry
+  const int ext[3][3] = {{dims[0] + 1, dims[1] + 1, dims[2] + 1}, {6, 6, 6}, {3, 3, 3}};
+  const int split[3] = {1, 2, 16};
+  FaceTable t[3];
   for (int r = 0; r < 3; ++r) {
-    std::vector<double> w, u, v;
-    gauss_2d(orders[r], w, u, v);
-    rules[r].Np = (int)w.size();
-    MARIE_TRY(rules[r].w.alloc(w.size() * sizeof(double), st));
-    MARIE_TRY(rules[r].u.alloc(w.size() * sizeof(double), st));
-    MARIE_TRY(rules[r].v.alloc(w.size() * sizeof(double), st));
-    MARIE_CUDA_TRY(cudaMemcpyAsync(rules[r].w.p, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-    MARIE_CUDA_TRY(cudaMemcpyAsync(rules[r].u.p, u.data(), u.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-    MARIE_CUDA_TRY(cudaMemcpyAsync(rules[r].v.p, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-  }
-  const long long V = (long long)L * M * N;
-  {
-    const int warps = 8;
-    long long blocks = (V + warps - 1) / warps;
-    if (blocks > 152 * 64) blocks = 152 * 64;
-    k_cub_far<<<(unsigned)blocks, 32 * warps, 0, st>>>(A, rules[0].w.as<double>(), rules[0].u.as<double>(),
-                                                       rules[0].v.as<double>(), rules[0].Np, n_medium, G);
+    const int e0 = ext[r][0], e1 = ext[r][1], e2 = ext[r][2];
+    MARIE_TRY(tables[r].alloc((size_t)6 * split[r] * e0 * e1 * e2 * sizeof(double2), st));
+    k_face_sums<<<dim3(e1, e2, 6 * split[r]), 128, 0, st>>>(drules.as<FaceRule>() + r, ko * dx, e0, split[r],
+                                                            tables[r].as<double2>());
     count_launch();
     MARIE_CUDA_TRY(cudaGetLastError());
+    t[r] = FaceTable{tables[r].as<double2>(), e0, e1, e2, split[r]};
   }
-  // medium (10-point) then near (20-point, corrected); MATLAB loops run 1:5 and
-  // 1:2 per axis; offsets beyond the grid are dropped here.
-  for (int pass = 0; pass < 2; ++pass) {
-    const int nr = pass == 0 ? n_medium : 2;
-    Rule& R = rules[pass + 1];
-    const int nO = nr * nr * nr;
-    DBuf J21;
-    MARIE_TRY(J21.alloc((size_t)nO * 21 * sizeof(double2), st));
-    dim3 grid(nO, 21);
-    const size_t smem = 9 * R.Np * sizeof(double);  // w, u, v and the two faces' points
-    if (smem > 48 * 1024)
-      MARIE_CUDA_TRY(cudaFuncSetAttribute(k_cub_region, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_cub_region<<<grid, 256, smem, st>>>(A, R.w.as<double>(), R.u.as<double>(), R.v.as<double>(), R.Np, nr,
-                                          J21.as<double2>());
-    count_launch();
-    MARIE_CUDA_TRY(cudaGetLastError());
-    k_region_finish<<<(nO + 127) / 128, 128, 0, st>>>(A, J21.as<double2>(), nr, pass == 1, G);
-    count_launch();
-    MARIE_CUDA_TRY(cudaGetLastError());
-    MARIE_CUDA_TRY(cudaStreamSynchronize(st));
-  }
-  return MARIE_OK;
-}
-
-// Forward 3-D FFT in place of the nq components of a 2L x 2M x 2N circulant.
-static int fft_operator(double2* C, int Lp, int Mp, int Np, cudaStream_t st, int nq = 6) {
-  std::vector<double2*> tw(3, nullptr);
-  const int lens[3] = {Lp, Mp, Np};
-  std::vector<DBuf> twb(3);
-  for (int a = 0; a < 3; ++a) {
-    std::vector<double2> h(lens[a]);
-    for (int k = 0; k < lens[a]; ++k) {
-      const double ang = 2.0 * M_PI * k / lens[a];
-      h[k] = mk<double2>(std::cos(ang), -std::sin(ang));
-    }
-    MARIE_TRY(twb[a].alloc(lens[a] * sizeof(double2), st));
-    MARIE_CUDA_TRY(cudaMemcpyAsync(twb[a].p, h.data(), lens[a] * sizeof(double2), cudaMemcpyHostToDevice, st));
-    tw[a] = twb[a].as<double2>();
-  }
-  const long long P = (long long)Lp * Mp * Np;
-  MARIE_CUDA_TRY(rows_full(Lp, C, nq * P / Lp, tw[0], st));
-  using ML = MatvecLaunch<double>;
-  // y: columns of S consecutive x, stride Lp, w = (z, q)
-  MARIE_CUDA_TRY(ML::cols(false, Mp, C, (long long)Lp * Mp, 0, Mp, C, (long long)Lp * Mp, 0, Mp, Lp, nq * Np,
-                          tw[1], 1, st));
-  // z: columns over the contiguous (x, y) plane, stride Lp*Mp, w = q
-  MARIE_CUDA_TRY(ML::cols(false, Np, C, P, 0, Np, C, P, 0, Np, Lp * Mp, nq, tw[2], 1, st));
+  NearSums ns;
+  for (int i = 0; i < 5; ++i) ns.v[i] = cscale(sing[i], 1.0 / (dx * dx * dx));
+  k_toeplitz<<<grid_stride_blocks((long long)L * M * N, 8), 256, 0, st>>>(
+      t[0], t[1], t[2], ns, dx * dx * dx / (4.0 * M_PI), L, M, N, G);
+  count_launch();
+  MARIE_CUDA_TRY(cudaGetLastError());
   MARIE_CUDA_TRY(cudaStreamSynchronize(st));
   return MARIE_OK;
 }
@@ -842,23 +933,38 @@ static int assemble_toeplitz_k(int L, int M, int N, double dx, double ko, double
   return MARIE_OK;
 }
 
-int assemble_k_device(int L, int M, int N, double dx, double freq, char type, double2* out, cudaStream_t st) {
-  const double ko = 2.0 * M_PI / 299792458.0 * freq;  // getOPERATORS.m:48
-  const long long V = (long long)L * M * N;
-  if (type == 'T') return assemble_toeplitz_k(L, M, N, dx, ko, out, st);
-  DBuf G;
-  MARIE_TRY(G.alloc(3 * V * sizeof(double2), st));
-  MARIE_TRY(assemble_toeplitz_k(L, M, N, dx, ko, G.as<double2>(), st));
-  const long long P = 8 * V;
-  k_circulant_k<<<(unsigned)std::min<long long>((3 * P + 255) / 256, 152 * 32), 256, 0, st>>>(G.as<double2>(), L, M,
-                                                                                              N, out);
-  count_launch();
-  MARIE_CUDA_TRY(cudaGetLastError());
+// out: the Toeplitz entries ('T'), the circulant ('C'), its FFT ('F', the full
+// array) or that FFT's octant ('O')
+template <int KIND>
+static int finish_operator(int L, int M, int N, const double2* G, char type, double2* out, cudaStream_t st) {
+  const long long Q = OpKind<KIND>::NQ, P = 8LL * L * M * N;
   if (type == 'C') {
+    const unsigned blocks = (unsigned)std::min<long long>((Q * P + 255) / 256, 152 * 32);
+    if (KIND == 0)
+      k_circulant<<<blocks, 256, 0, st>>>(G, L, M, N, out);
+    else
+      k_circulant_k<<<blocks, 256, 0, st>>>(G, L, M, N, out);
+    count_launch();
+    MARIE_CUDA_TRY(cudaGetLastError());
     MARIE_CUDA_TRY(cudaStreamSynchronize(st));
     return MARIE_OK;
   }
-  return fft_operator(out, 2 * L, 2 * M, 2 * N, st, 3);
+  if (type == 'O') return octant_spectrum<KIND>(L, M, N, G, out, st);
+  DBuf O;
+  MARIE_TRY(O.alloc((size_t)Q * (L + 1) * (M + 1) * (N + 1) * sizeof(double2), st));
+  MARIE_TRY(octant_spectrum<KIND>(L, M, N, G, O.as<double2>(), st));
+  MARIE_TRY(expand_octant(O.as<double2>(), L, M, N, KIND, 1.0, out, st));
+  MARIE_CUDA_TRY(cudaStreamSynchronize(st));
+  return MARIE_OK;
+}
+
+int assemble_k_device(int L, int M, int N, double dx, double freq, char type, double2* out, cudaStream_t st) {
+  const double ko = 2.0 * M_PI / 299792458.0 * freq;  // getOPERATORS.m:48
+  if (type == 'T') return assemble_toeplitz_k(L, M, N, dx, ko, out, st);
+  DBuf G;
+  MARIE_TRY(G.alloc((size_t)3 * L * M * N * sizeof(double2), st));
+  MARIE_TRY(assemble_toeplitz_k(L, M, N, dx, ko, G.as<double2>(), st));
+  return finish_operator<1>(L, M, N, G.as<double2>(), type, out, st);
 }
 
 // The reference's Np_1D for the singular integrals (Np_DEMCEM, assembly_nop.m:16).
@@ -897,21 +1003,11 @@ int assemble_operator_device(int L, int M, int N, double dx, double freq, char s
   const double ko = 2.0 * M_PI / 299792458.0 * freq;  // getOPERATORS.m:48
   double2 sing[5];
   MARIE_TRY(get_sing(singular, user_sing, ko, dx, sing, st));
-  const long long V = (long long)L * M * N;
   if (type == 'T') return assemble_toeplitz(L, M, N, dx, ko, sing, out, st);
   DBuf G;
-  MARIE_TRY(G.alloc(6 * V * sizeof(double2), st));
+  MARIE_TRY(G.alloc((size_t)6 * L * M * N * sizeof(double2), st));
   MARIE_TRY(assemble_toeplitz(L, M, N, dx, ko, sing, G.as<double2>(), st));
-  const long long P = 8 * V;
-  k_circulant<<<(unsigned)std::min<long long>((6 * P + 255) / 256, 152 * 32), 256, 0, st>>>(G.as<double2>(), L, M, N,
-                                                                                             out);
-  count_launch();
-  MARIE_CUDA_TRY(cudaGetLastError());
-  if (type == 'C') {
-    MARIE_CUDA_TRY(cudaStreamSynchronize(st));
-    return MARIE_OK;
-  }
-  return fft_operator(out, 2 * L, 2 * M, 2 * N, st);
+  return finish_operator<0>(L, M, N, G.as<double2>(), type, out, st);
 }
 
 }  // namespace marie
@@ -971,21 +1067,23 @@ int marie_plan_assemble(marie_plan* p, double dx, double freq, char singular, co
   if (!p) return set_error(MARIE_EINVAL, "NULL plan");
   if (!(dx > 0) || !(freq > 0)) return set_error(MARIE_EINVAL, "dx and freq must be positive");
   MARIE_TRACE("getOPERATORS N");
-  DBuf F;
-  MARIE_TRY(F.alloc((size_t)48 * p->d.V * sizeof(double2), p->stream));
-  MARIE_TRY(assemble_operator_device(p->d.L, p->d.M, p->d.N, dx, freq, singular, singular_values, 'F',
-                                     F.as<double2>(), p->stream));
-  return install_operator(p, F.as<double2>());
+  const Dims& d = p->d;
+  DBuf O;
+  MARIE_TRY(O.alloc((size_t)6 * (d.L + 1) * (d.M + 1) * (d.N + 1) * sizeof(double2), p->stream));
+  MARIE_TRY(assemble_operator_device(d.L, d.M, d.N, dx, freq, singular, singular_values, 'O', O.as<double2>(),
+                                     p->stream));
+  return install_octant(p, O.as<double2>());
 }
 
 int marie_plan_assemble_k(marie_plan* p, double dx, double freq) {
   if (!p) return set_error(MARIE_EINVAL, "NULL plan");
   if (!(dx > 0) || !(freq > 0)) return set_error(MARIE_EINVAL, "dx and freq must be positive");
   MARIE_TRACE("getOPERATORS K");
-  DBuf F;
-  MARIE_TRY(F.alloc((size_t)24 * p->d.V * sizeof(double2), p->stream));
-  MARIE_TRY(assemble_k_device(p->d.L, p->d.M, p->d.N, dx, freq, 'F', F.as<double2>(), p->stream));
-  return install_operator(p, F.as<double2>(), 1);
+  const Dims& d = p->d;
+  DBuf O;
+  MARIE_TRY(O.alloc((size_t)3 * (d.L + 1) * (d.M + 1) * (d.N + 1) * sizeof(double2), p->stream));
+  MARIE_TRY(assemble_k_device(d.L, d.M, d.N, dx, freq, 'O', O.as<double2>(), p->stream));
+  return install_octant(p, O.as<double2>(), 1);
 }
 
 }  // extern "C"

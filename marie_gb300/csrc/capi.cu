@@ -448,17 +448,25 @@ __global__ void k_extract_octant(const double2* __restrict__ f, int L, int M, in
 
 // the N operator full along x, half along y and z: fx[q][oz][oy][kx] =
 // s * f[q][oz][oy][kx] for oy <= M, oz <= N, in FP32 (the z pass's bulk tile
-// source; the full operator already carries the x-reflection signs)
-__global__ void k_extract_fullx(const double2* __restrict__ f, int L, int M, int N, double s, float2* __restrict__ fx) {
+// source), from the full operator or from its octant (oct; the x reflections
+// are signed here)
+__global__ void k_extract_fullx(const double2* __restrict__ f, int oct, int L, int M, int N, double s,
+                                float2* __restrict__ fx) {
   const long long Lp = 2LL * L, Mp = 2LL * M, Np = 2LL * N, P = Lp * Mp * Np;
-  const long long Mo = M + 1, No = N + 1, X = Lp * Mo * No;
+  const long long Lo = L + 1, Mo = M + 1, No = N + 1, X = Lp * Mo * No;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < 6 * X; t += (long long)gridDim.x * blockDim.x) {
     const int q = (int)(t / X);
     long long r = t - q * X;
     const long long kx = r % Lp;
     r /= Lp;
     const long long oy = r % Mo, oz = r / Mo;
-    const double2 v = f[q * P + kx + Lp * (oy + Mp * oz)];
+    double2 v;
+    if (oct) {
+      v = f[q * Lo * Mo * No + (kx > L ? Lp - kx : kx) + Lo * (oy + Mo * oz)];
+      if (kx > L && comp_odd(0, q, 0)) v = mk<double2>(-v.x, -v.y);
+    } else {
+      v = f[q * P + kx + Lp * (oy + Mp * oz)];
+    }
     fx[t] = mk<float2>((float)(v.x * s), (float)(v.y * s));
   }
 }
@@ -484,10 +492,14 @@ __global__ void k_expand_octant(const double2* __restrict__ o, int L, int M, int
   }
 }
 
-// Installs an operator (full layout, device) into the plan: the octant when it
-// has the circulant's parity symmetry to 1e-12 of its maximum (every operator
-// built by getOPERATORS does), the full array otherwise.  Scaled by 1/(8LMN).
-// kind 0: N (6 components, fN64/fN32), 1: K (3 components, fK64/fK32).
+int expand_octant(const double2* o, int L, int M, int N, int kind, double s, double2* f, cudaStream_t st) {
+  const long long n = (long long)comp_count(kind) * 8 * L * M * N;
+  k_expand_octant<<<grid_for(n), 256, 0, st>>>(o, L, M, N, kind, s, f);
+  count_launch();
+  MARIE_CUDA_TRY(cudaGetLastError());
+  return MARIE_OK;
+}
+
 // cuTensorMapEncodeTiled from the driver (looked up once through the runtime;
 // the library links no driver library)
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -512,7 +524,7 @@ static EncodeTiledFn encode_tiled() {
 // tensor map per box width (8, 4, 2 columns) over (2L, M+1, N+1, 6) 8-byte
 // elements.  Without the driver entry point, or with N + 1 > 256 (beyond the
 // box limit), the plan keeps the per-thread tile copies.
-static int build_zt(marie_plan* p, const double2* fN_dev) {
+static int build_zt(marie_plan* p, const double2* fN_dev, int oct) {
   const Dims& d = p->d;
   cudaFree(p->fN32x);
   p->fN32x = nullptr;
@@ -523,7 +535,7 @@ static int build_zt(marie_plan* p, const double2* fN_dev) {
   const long long X = (long long)d.Lp * (d.M + 1) * (d.N + 1);
   MARIE_CUDA_TRY(cudaMalloc(&p->fN32x, 6 * X * sizeof(float2)));
   const long long P = (long long)d.Lp * d.Mp * d.Np;
-  k_extract_fullx<<<grid_for(6 * X), 256, 0, p->stream>>>(fN_dev, d.L, d.M, d.N, 1.0 / (double)P, p->fN32x);
+  k_extract_fullx<<<grid_for(6 * X), 256, 0, p->stream>>>(fN_dev, oct, d.L, d.M, d.N, 1.0 / (double)P, p->fN32x);
   count_launch();
   MARIE_CUDA_TRY(cudaGetLastError());
   const cuuint64_t gd[4] = {(cuuint64_t)d.Lp, (cuuint64_t)d.M + 1, (cuuint64_t)d.N + 1, 6};
@@ -559,27 +571,18 @@ int check_kernel_status(marie_plan* p) {
   return MARIE_OK;
 }
 
-int install_operator(marie_plan* p, const double2* fN_dev, int kind) {
+// Puts an operator's octant (src_oct) or full array into the plan, scaled by
+// 1/(8LMN); oct: keep the octant.  kind 0: N (6 components, fN64/fN32), 1: K
+// (3 components, fK64/fK32).
+static int store_operator(marie_plan* p, const double2* src, bool src_oct, int oct, int kind) {
   const Dims& d = p->d;
   const long long P = (long long)d.Lp * d.Mp * d.Np;
   const long long O = (long long)(d.L + 1) * (d.M + 1) * (d.N + 1);
   const int NQ = comp_count(kind);
   const bool need64 = p->precision != MARIE_FP32;
   const bool need32 = p->precision != MARIE_FP64;
-  DBuf flags;
-  MARIE_TRY(flags.alloc(2 * sizeof(unsigned long long), p->stream));
-  MARIE_CUDA_TRY(cudaMemsetAsync(flags.p, 0, 2 * sizeof(unsigned long long), p->stream));
-  k_symmetry_check<<<grid_for(NQ * P), 256, 0, p->stream>>>(fN_dev, d.L, d.M, d.N, kind,
-                                                            flags.as<unsigned long long>());
-  count_launch();
-  unsigned long long h[2];
-  MARIE_CUDA_TRY(cudaMemcpyAsync(h, flags.p, sizeof(h), cudaMemcpyDeviceToHost, p->stream));
-  MARIE_CUDA_TRY(cudaStreamSynchronize(p->stream));
-  double dev, mx;
-  memcpy(&dev, &h[0], sizeof(double));
-  memcpy(&mx, &h[1], sizeof(double));
-  const int oct = (dev <= 1e-12 * mx) ? 1 : 0;
   const long long n = oct ? NQ * O : NQ * P;
+  MARIE_CUDA_TRY(cudaStreamSynchronize(p->stream));  // nothing reads the old operator any more
   if (kind == 0) {
     release_cufft_state(p);  // its full copy of fN is stale now
     cudaFree(p->fN32x);
@@ -598,16 +601,16 @@ int install_operator(marie_plan* p, const double2* fN_dev, int kind) {
     p->has_opK = false;
   if (need64) MARIE_CUDA_TRY(cudaMalloc(&f64, n * sizeof(double2)));
   if (need32) MARIE_CUDA_TRY(cudaMalloc(&f32, n * sizeof(float2)));
-  if (oct) {
-    k_extract_octant<<<grid_for(n), 256, 0, p->stream>>>(fN_dev, d.L, d.M, d.N, NQ, 1.0 / (double)P,
+  if (oct && !src_oct) {
+    k_extract_octant<<<grid_for(n), 256, 0, p->stream>>>(src, d.L, d.M, d.N, NQ, 1.0 / (double)P,
                                                          need64 ? f64 : nullptr, need32 ? f32 : nullptr);
   } else {
-    k_scale_convert<<<grid_for(n), 256, 0, p->stream>>>(fN_dev, n, 1.0 / (double)P, need64 ? f64 : nullptr,
+    k_scale_convert<<<grid_for(n), 256, 0, p->stream>>>(src, n, 1.0 / (double)P, need64 ? f64 : nullptr,
                                                          need32 ? f32 : nullptr);
   }
   count_launch();
   MARIE_CUDA_TRY(cudaGetLastError());
-  if (kind == 0 && oct && need32) MARIE_TRY(build_zt(p, fN_dev));
+  if (kind == 0 && oct && need32) MARIE_TRY(build_zt(p, src, src_oct));
   MARIE_CUDA_TRY(cudaStreamSynchronize(p->stream));
   if (kind == 0) {
     p->oct = oct;
@@ -618,6 +621,28 @@ int install_operator(marie_plan* p, const double2* fN_dev, int kind) {
   }
   return MARIE_OK;
 }
+
+// An operator given in full: its octant is kept when it has the circulant's
+// parity symmetry to 1e-12 of its maximum (every operator built by
+// getOPERATORS does), the full array otherwise.
+int install_operator(marie_plan* p, const double2* fN_dev, int kind) {
+  const Dims& d = p->d;
+  const long long n = (long long)comp_count(kind) * d.Lp * d.Mp * d.Np;
+  DBuf flags;
+  MARIE_TRY(flags.alloc(2 * sizeof(unsigned long long), p->stream));
+  MARIE_CUDA_TRY(cudaMemsetAsync(flags.p, 0, 2 * sizeof(unsigned long long), p->stream));
+  k_symmetry_check<<<grid_for(n), 256, 0, p->stream>>>(fN_dev, d.L, d.M, d.N, kind, flags.as<unsigned long long>());
+  count_launch();
+  unsigned long long h[2];
+  MARIE_CUDA_TRY(cudaMemcpyAsync(h, flags.p, sizeof(h), cudaMemcpyDeviceToHost, p->stream));
+  MARIE_CUDA_TRY(cudaStreamSynchronize(p->stream));
+  double dev, mx;
+  memcpy(&dev, &h[0], sizeof(double));
+  memcpy(&mx, &h[1], sizeof(double));
+  return store_operator(p, fN_dev, false, (dev <= 1e-12 * mx) ? 1 : 0, kind);
+}
+
+int install_octant(marie_plan* p, const double2* O_dev, int kind) { return store_operator(p, O_dev, true, 1, kind); }
 
 }  // namespace marie
 

@@ -159,6 +159,11 @@ int run_matvec32(marie_plan* p, const float2* J, long long js, float2* out, long
 // Scale fN by 1/(8LMN) into the plan's FP64/FP32 copies (fN_dev: full layout).
 // kind 0: the N operator (6 components), 1: the K operator (3 components).
 int install_operator(marie_plan* p, const double2* fN_dev, int kind = 0);
+// The same from the octant (L+1)(M+1)(N+1) per component of an operator with
+// the circulant's parities, unscaled.
+int install_octant(marie_plan* p, const double2* O_dev, int kind = 0);
+// Full 2L x 2M x 2N operator from its octant, scaled by s.
+int expand_octant(const double2* o, int L, int M, int N, int kind, double s, double2* f, cudaStream_t st);
 
 // Reads the plan's kernel status word after the plan's stream has finished
 // (a synchronising copy), clears it and returns MARIE_ETIMEOUT if a kernel's
