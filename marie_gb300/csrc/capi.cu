@@ -127,6 +127,17 @@ int DBuf::alloc(size_t bytes, cudaStream_t st) {
   return MARIE_OK;
 }
 
+bool DBuf::try_alloc(size_t bytes, cudaStream_t st) {
+  s = st;
+  cudaMemPool_t pool = device_pool();
+  if (bytes == 0) bytes = 16;
+  const cudaError_t e = pool ? cudaMallocFromPoolAsync(&p, bytes, pool, st) : cudaMallocAsync(&p, bytes, st);
+  if (e == cudaSuccess) return true;
+  p = nullptr;
+  cudaGetLastError();
+  return false;
+}
+
 bool is_device_ptr(const void* ptr) { return ptr && host_kind(ptr) == HostKind::Device; }
 
 int stage_in(const void* user, size_t bytes, cudaStream_t st, DBuf& tmp, const void** dev) {
@@ -524,20 +535,19 @@ static EncodeTiledFn encode_tiled() {
 // tensor map per box width (8, 4, 2 columns) over (2L, M+1, N+1, 6) 8-byte
 // elements.  Without the driver entry point, or with N + 1 > 256 (beyond the
 // box limit), the plan keeps the per-thread tile copies.
-static int build_zt(marie_plan* p, const double2* fN_dev, int oct) {
+size_t fullx_elems(const Dims& d) { return (size_t)6 * d.Lp * (d.M + 1) * (d.N + 1); }
+
+// Fills p->fN32x from the operator (full or octant, scaled by s here) and
+// encodes its tensor maps; false when the driver refuses a map.
+static bool encode_zt(marie_plan* p, const double2* src, int oct, double s) {
   const Dims& d = p->d;
-  cudaFree(p->fN32x);
-  p->fN32x = nullptr;
+  EncodeTiledFn enc = encode_tiled();
   p->zt.ok = 0;
   p->zt.err = p->kerr;
-  EncodeTiledFn enc = encode_tiled();
-  if (!enc || d.N + 1 > 256) return MARIE_OK;
-  const long long X = (long long)d.Lp * (d.M + 1) * (d.N + 1);
-  MARIE_CUDA_TRY(cudaMalloc(&p->fN32x, 6 * X * sizeof(float2)));
-  const long long P = (long long)d.Lp * d.Mp * d.Np;
-  k_extract_fullx<<<grid_for(6 * X), 256, 0, p->stream>>>(fN_dev, oct, d.L, d.M, d.N, 1.0 / (double)P, p->fN32x);
+  if (!enc || d.N + 1 > 256) return false;
+  k_extract_fullx<<<grid_for(fullx_elems(d)), 256, 0, p->stream>>>(src, oct, d.L, d.M, d.N, s, p->fN32x);
   count_launch();
-  MARIE_CUDA_TRY(cudaGetLastError());
+  if (cudaGetLastError() != cudaSuccess) return false;
   const cuuint64_t gd[4] = {(cuuint64_t)d.Lp, (cuuint64_t)d.M + 1, (cuuint64_t)d.N + 1, 6};
   const cuuint64_t gs[3] = {(cuuint64_t)d.Lp * 8, (cuuint64_t)d.Lp * (d.M + 1) * 8,
                             (cuuint64_t)d.Lp * (d.M + 1) * (d.N + 1) * 8};
@@ -548,13 +558,34 @@ static int build_zt(marie_plan* p, const double2* fN_dev, int oct) {
     const CUresult r = enc(&p->zt.map[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, p->fN32x, gd, gs, bd, es,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-      cudaFree(p->fN32x);
-      p->fN32x = nullptr;
-      return MARIE_OK;
-    }
+    if (r != CUDA_SUCCESS) return false;
   }
   p->zt.ok = 1;
+  return true;
+}
+
+static int build_zt(marie_plan* p, const double2* fN_dev, int oct) {
+  const Dims& d = p->d;
+  cudaFree(p->fN32x);
+  p->fN32x = nullptr;
+  p->zt.ok = 0;
+  if (!encode_tiled() || d.N + 1 > 256) return MARIE_OK;
+  MARIE_CUDA_TRY(cudaMalloc(&p->fN32x, fullx_elems(d) * sizeof(float2)));
+  if (!encode_zt(p, fN_dev, oct, 1.0 / ((double)d.Lp * d.Mp * d.Np))) {
+    cudaFree(p->fN32x);
+    p->fN32x = nullptr;
+  }
+  return MARIE_OK;
+}
+
+int store_crop_f32(marie_plan* q, float2* fullx) {
+  const Dims& d = q->d;
+  const long long n = 6LL * (d.L + 1) * (d.M + 1) * (d.N + 1);
+  k_scale_convert<<<grid_for(n), 256, 0, q->stream>>>(q->fN64, n, 1.0, nullptr, q->fN32);
+  count_launch();
+  MARIE_CUDA_TRY(cudaGetLastError());
+  q->fN32x = fullx;
+  if (!encode_zt(q, q->fN64, 1, 1.0)) cudaGetLastError();  // per-thread tile copies instead
   return MARIE_OK;
 }
 
@@ -584,6 +615,8 @@ static int store_operator(marie_plan* p, const double2* src, bool src_oct, int o
   const long long n = oct ? NQ * O : NQ * P;
   MARIE_CUDA_TRY(cudaStreamSynchronize(p->stream));  // nothing reads the old operator any more
   if (kind == 0) {
+    p->crop.reset();
+    p->bnd_crop.reset();
     release_cufft_state(p);  // its full copy of fN is stale now
     cudaFree(p->fN32x);
     p->fN32x = nullptr;
@@ -655,6 +688,9 @@ static void free_bound(marie_plan* p) {
   cudaFree(p->bnd_b);
   cudaFree(p->bnd_af);
   cudaFree(p->bnd_bf);
+  cudaFree(p->bnd_inv_crop);
+  p->bnd_inv_crop = nullptr;
+  p->bnd_crop.reset();
   p->bnd_idx = nullptr;
   p->bnd_inv = nullptr;
   p->bnd_a = p->bnd_b = nullptr;
@@ -670,12 +706,26 @@ __global__ void k_to_f32(const double2* __restrict__ in, long long n, float2* __
 
 namespace marie {
 
+// The plan a bound product runs on, the crop of the bound DOFs where there is
+// one (per-pass timing wants the plan itself), and their map on it.
+static marie_plan* bound_plan(marie_plan* p, const int** inv) {
+  if (p->bnd_crop && !p->profile) {
+    crop_settings(p, p->bnd_crop.get());
+    *inv = p->bnd_inv_crop;
+    return p->bnd_crop.get();
+  }
+  *inv = p->bnd_inv;
+  return p;
+}
+
 int bound_operator(marie_plan* p, long long n, DevOp* op) {
   if (!p->bnd_n) return set_error(MARIE_EINVAL, "NULL operator and no mv_AN bound to the plan (marie_plan_bind_mv_AN)");
   if (p->bnd_n != n) return set_error(MARIE_EINVAL, "vector length %lld differs from the bound mv_AN's %lld DOFs", n,
                                       p->bnd_n);
   const int prec = p->fN64 ? MARIE_FP64 : MARIE_FP32;
   *op = [p, n, prec](const double2* x, double2* y) -> int {
+    const int* inv;
+    marie_plan* q = bound_plan(p, &inv);
     Prologue pro{nullptr, 0};
     Epilogue ep{};
     if (p->bnd_transp == 0) {
@@ -687,7 +737,7 @@ int bound_operator(marie_plan* p, long long n, DevOp* op) {
       ep.a = p->bnd_a;
       ep.conjout = 1;
     }
-    return run_matvec(p, prec, x, y, n, 1, p->bnd_inv, pro, ep);
+    return run_matvec(q, prec, x, y, n, 1, inv, pro, ep);
   };
   return MARIE_OK;
 }
@@ -789,6 +839,18 @@ int marie_plan_bind_mv_AN(marie_plan* p, const double* Mr, const double* Mc, dou
       count_launch(2);
     }
   }
+  if (s == MARIE_OK && crop_possible(p)) {
+    // the products on the smallest grid that holds the DOFs
+    int box[6], origin[3];
+    s = dof_box(p, p->bnd_idx, n, box);
+    if (s == MARIE_OK) p->bnd_crop = crop_plan(p, box, origin);
+    if (p->bnd_crop && cudaMalloc(&p->bnd_inv_crop, 3 * p->bnd_crop->d.V * sizeof(int)) != cudaSuccess) {
+      cudaGetLastError();
+      p->bnd_inv_crop = nullptr;
+      p->bnd_crop.reset();
+    }
+    if (p->bnd_crop) s = build_inverse_box(p, p->bnd_crop.get(), origin, p->bnd_idx, n, p->bnd_inv_crop);
+  }
   if (s == MARIE_OK && cudaStreamSynchronize(p->stream) != cudaSuccess) s = set_error(MARIE_ECUDA, "bind mv_AN failed");
   if (s != MARIE_OK) {
     free_bound(p);
@@ -804,6 +866,7 @@ int marie_plan_destroy(marie_plan* p) {
   if (p->stream) cudaStreamSynchronize(p->stream);
   release_cufft_state(p);
   free_bound(p);
+  p->crop.reset();
   if (p->wsA) cudaFreeAsync(p->wsA, p->stream);
   if (p->wsB) cudaFreeAsync(p->wsB, p->stream);
   if (p->stream) cudaStreamSynchronize(p->stream);
@@ -1106,7 +1169,9 @@ int marie_plan_apply_mv_AN(marie_plan* p, const double* JIn0, double* JOut, int6
     ep.af = p->bnd_af;
     ep.bf = p->bnd_bf;
   }
-  MARIE_TRY(run_matvec(p, precision, (const double2*)J_d, (double2*)out_d, n, (int)nrhs, p->bnd_inv, pro, ep));
+  const int* inv;
+  marie_plan* q = bound_plan(p, &inv);
+  MARIE_TRY(run_matvec(q, precision, (const double2*)J_d, (double2*)out_d, n, (int)nrhs, inv, pro, ep));
   if (out_d != JOut) {
     MARIE_TRY(finish_out(JOut, out_d, n * nrhs * sizeof(double2), p->stream));
     return check_kernel_status(p);

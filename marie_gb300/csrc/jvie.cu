@@ -14,6 +14,7 @@
 // the same way around an FP32-matvec bicgstab / pgmresDR.
 #include <algorithm>
 #include <chrono>
+#include <climits>
 #include <cmath>
 #include <string>
 #include <thread>
@@ -49,11 +50,24 @@ __device__ __forceinline__ bool non_air(const double2* er, long long v) {
   return hypot(e.x - 1.0, e.y) > 1e-12;
 }
 
-__global__ void k_count_nonair(const double2* __restrict__ er, long long V, int* __restrict__ counts) {
+// counts per block; box: the voxels' box, as dof_box gives it
+__global__ void k_count_nonair(const double2* __restrict__ er, int L, int M, long long V, int* __restrict__ counts,
+                               int* __restrict__ box) {
   const long long chunk = (V + gridDim.x - 1) / gridDim.x;
   const long long i0 = blockIdx.x * chunk, i1 = i0 + chunk < V ? i0 + chunk : V;
   int c = 0;
-  for (long long i = i0 + threadIdx.x; i < i1; i += blockDim.x) c += non_air(er, i) ? 1 : 0;
+  int b[6] = {INT_MIN, INT_MIN, INT_MIN, INT_MIN, INT_MIN, INT_MIN};
+  for (long long i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+    if (!non_air(er, i)) continue;
+    ++c;
+    const int v = (int)i;
+    const int x[3] = {v % L, (v / L) % M, v / (L * M)};
+    for (int a = 0; a < 3; ++a) {
+      b[a] = max(b[a], -x[a]);
+      b[3 + a] = max(b[3 + a], x[a]);
+    }
+  }
+  box_reduce(b, box);
   __shared__ int s[32];
   for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
   if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = c;
@@ -196,6 +210,10 @@ __global__ void k_add_b(const double2* __restrict__ d, double2* __restrict__ x, 
 
 struct JvieState {
   long long nS = 0, n = 0;
+  // the grid the products run on: the crop to the body's box, or the plan's
+  // (inv is the DOF map on it)
+  std::shared_ptr<marie_plan> crop;
+  marie_plan* on(marie_plan* p) const { return crop ? crop.get() : p; }
   DBuf idxS, idx3, inv, f, a, b, pa, pb;
   DBuf af, bf, paf, pbf;  // FP32 copies of a, b, pa, pb (plans with an FP32 operator)
 };
@@ -204,11 +222,12 @@ static int jvie_setup(marie_plan* p, const double2* er, double dx, double freq, 
   cudaStream_t st = p->stream;
   const long long V = p->d.V;
   DBuf counts;
-  MARIE_TRY(counts.alloc(CMP_BLOCKS * sizeof(int), st));
-  k_count_nonair<<<CMP_BLOCKS, 256, 0, st>>>(er, V, counts.as<int>());
+  MARIE_TRY(counts.alloc((CMP_BLOCKS + 6) * sizeof(int), st));
+  MARIE_CUDA_TRY(cudaMemsetAsync(counts.as<int>() + CMP_BLOCKS, 0x80, 6 * sizeof(int), st));
+  k_count_nonair<<<CMP_BLOCKS, 256, 0, st>>>(er, p->d.L, p->d.M, V, counts.as<int>(), counts.as<int>() + CMP_BLOCKS);
   count_launch();
-  std::vector<int> hc(CMP_BLOCKS);
-  MARIE_CUDA_TRY(cudaMemcpyAsync(hc.data(), counts.p, CMP_BLOCKS * sizeof(int), cudaMemcpyDeviceToHost, st));
+  std::vector<int> hc(CMP_BLOCKS + 6);
+  MARIE_CUDA_TRY(cudaMemcpyAsync(hc.data(), counts.p, hc.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
   MARIE_CUDA_TRY(cudaStreamSynchronize(st));
   long long tot = 0;
   for (int i = 0; i < CMP_BLOCKS; ++i) {
@@ -231,7 +250,9 @@ static int jvie_setup(marie_plan* p, const double2* er, double dx, double freq, 
   MARIE_TRY(S.b.alloc(n * sizeof(double2), st));
   MARIE_TRY(S.pa.alloc(n * sizeof(double2), st));
   MARIE_TRY(S.pb.alloc(n * sizeof(double2), st));
-  MARIE_TRY(S.inv.alloc(3 * V * sizeof(int), st));
+  int origin[3];
+  S.crop = crop_plan(p, hc.data() + CMP_BLOCKS, origin);
+  MARIE_TRY(S.inv.alloc(3 * S.on(p)->d.V * sizeof(int), st));
   const double Gram = dx * dx * dx;
   const double omega = 2.0 * M_PI * freq;
   k_jvie_coef<<<grid_n(n), 256, 0, st>>>(S.idxS.as<int>(), tot, V, er, Gram, omega * eps0(), form,
@@ -250,8 +271,9 @@ static int jvie_setup(marie_plan* p, const double2* er, double dx, double freq, 
     count_launch();
     MARIE_CUDA_TRY(cudaGetLastError());
   }
-  MARIE_TRY(build_inverse_index(p, S.idx3.as<int64_t>(), n, S.inv.as<int>()));
-  return MARIE_OK;
+  // idx3 is in range and without repeats by construction
+  if (S.crop) return build_inverse_box(p, S.crop.get(), origin, S.idx3.as<int64_t>(), n, S.inv.as<int>());
+  return build_inverse_index(p, S.idx3.as<int64_t>(), n, S.inv.as<int>());
 }
 
 static int any_nonzero(marie_plan* p, const double2* b, long long n, bool* nz) {
@@ -374,11 +396,12 @@ static int jvie_solve_core(marie_plan* p, const double2* E, long long es, int S_
   k_jvie_rhs<<<dim3(grid_n(n), S_exc), 256, 0, st>>>(S.f.as<double2>(), S.idx3.as<int64_t>(), n, E, es,
                                                       rhs->as<double2>());
   count_launch();
+  marie_plan* q = S.on(p);
   if (sa.solver == 'G')
-    MARIE_TRY(solve_systems(p, S, rhs->as<double2>(), S_exc, x->as<double2>(), precond, tol, inner_it, outer_it, out,
+    MARIE_TRY(solve_systems(q, S, rhs->as<double2>(), S_exc, x->as<double2>(), precond, tol, inner_it, outer_it, out,
                             dfr));
   else
-    MARIE_TRY(solve_single(p, S, rhs->as<double2>(), x->as<double2>(), precond, tol, inner_it, outer_it, sa, out));
+    MARIE_TRY(solve_single(q, S, rhs->as<double2>(), x->as<double2>(), precond, tol, inner_it, outer_it, sa, out));
   auto scatter = [p, Sp, x, n, S_exc, Je, js]() -> int {
     k_scatter_dofs<<<dim3(grid_n(n), S_exc), 256, 0, p->stream>>>(x->as<double2>(), Sp->idx3.as<int64_t>(), n, Je,
                                                                    js);
@@ -680,7 +703,8 @@ int jvie_adjoint_core(marie_plan* p, const double2* Einc, const double2* er, dou
   k_jvie_rhs<<<dim3(nb, 1), 256, 0, st>>>(S.f.as<double2>(), S.idx3.as<int64_t>(), n, Einc, 0, rhs.as<double2>());
   count_launch();
   SolveOut fwd, adj;
-  MARIE_TRY(solve_systems(p, S, rhs.as<double2>(), 1, J.as<double2>(), 0, tol, inner_it, outer_it, fwd));
+  marie_plan* on = S.on(p);
+  MARIE_TRY(solve_systems(on, S, rhs.as<double2>(), 1, J.as<double2>(), 0, tol, inner_it, outer_it, fwd));
   k_adj_fields<<<nb, 256, 0, st>>>(J.as<double2>(), S.idx3.as<int64_t>(), n, V, er, omega_eps0, objective, Et,
                                    E.as<double2>(), w.as<double2>(), Fp.as<double>());
   count_launch();
@@ -692,14 +716,14 @@ int jvie_adjoint_core(marie_plan* p, const double2* Einc, const double2* er, dou
   for (double v : hF) Fs += v;
   *F = Fs;
   // adjoint solve A lambda = w (rows divided by eps_c, like the forward form 2)
-  MARIE_TRY(solve_systems(p, S, w.as<double2>(), 1, lam.as<double2>(), 0, tol, inner_it, outer_it, adj));
+  MARIE_TRY(solve_systems(on, S, w.as<double2>(), 1, lam.as<double2>(), 0, tol, inner_it, outer_it, adj));
   // q = (Gram - N) lambda in FP64
   Prologue pro{nullptr, 0};
   Epilogue ep{};
   ep.a_s = mk<double2>(dx * dx * dx, 0.0);
   ep.b_s = mk<double2>(1.0, 0.0);
   const int prec = p->fN64 ? MARIE_FP64 : MARIE_FP32;
-  MARIE_TRY(run_matvec(p, prec, lam.as<double2>(), q.as<double2>(), n, 1, S.inv.as<int>(), pro, ep));
+  MARIE_TRY(run_matvec(on, prec, lam.as<double2>(), q.as<double2>(), n, 1, S.inv.as<int>(), pro, ep));
   k_adj_grad<<<grid_n(S.nS), 256, 0, st>>>(q.as<double2>(), E.as<double2>(), S.idxS.as<int>(), S.nS, er, omega_eps0,
                                            objective, g_eps, g_sig);
   count_launch();
@@ -1045,6 +1069,13 @@ int marie_jvie2solver(marie_plan* p, const int64_t* idx, int64_t n_idx, const do
     MARIE_CUDA_TRY(cudaMemsetAsync(S.pb.p, 0, n * sizeof(double2), st));
     MARIE_TRY(S.inv.alloc(3 * V * sizeof(int), st));
     MARIE_TRY(build_inverse_index(p, S.idx3.as<int64_t>(), n, S.inv.as<int>()));
+    if (crop_possible(p)) {
+      int box[6], origin[3];
+      MARIE_TRY(dof_box(p, S.idx3.as<int64_t>(), n, box));
+      S.crop = crop_plan(p, box, origin);
+      // (the crop's map needs less than the whole grid's)
+      if (S.crop) MARIE_TRY(build_inverse_box(p, S.crop.get(), origin, S.idx3.as<int64_t>(), n, S.inv.as<int>()));
+    }
     MARIE_TRY(build_coefficients(p, S.idx3.as<int64_t>(), n, (const double2*)Mr_d, (const double2*)Mc_d, Gram, 0,
                                  S.a.as<double2>(), S.b.as<double2>()));
     // bicgstab(fVIE, Vrhs, tol, max_it, [], [], Vini) (jvie2solver.m:54-77)
@@ -1053,7 +1084,7 @@ int marie_jvie2solver(marie_plan* p, const int64_t* idx, int64_t n_idx, const do
     sa.max_it = max_it;
     SolveOut so;
     so.r.assign(1, GmresResult());
-    MARIE_TRY(solve_single(p, S, (const double2*)b_d, (double2*)x_d, 0, tol, 50, 200, sa, so,
+    MARIE_TRY(solve_single(S.on(p), S, (const double2*)b_d, (double2*)x_d, 0, tol, 50, 200, sa, so,
                            (const double2*)x0_d));
     if (flag) *flag = so.b.flag;
     if (relres) *relres = so.b.relres;

@@ -2,6 +2,7 @@
 #pragma once
 #include <unistd.h>
 
+#include <climits>
 #include <functional>
 #include <memory>
 #include <thread>
@@ -52,6 +53,12 @@ struct marie_plan {
   double2* tw64[3] = {nullptr, nullptr, nullptr};
   float2* tw32[3] = {nullptr, nullptr, nullptr};
 
+  // The operator on the smallest grid that holds the last body solved for
+  // (crop.cu); dropped when the operator changes.  A crop's own arrays live in
+  // its arena, its stream and status word are the plan's.
+  std::shared_ptr<marie_plan> crop;
+  void* arena = nullptr;
+
   // Spectra workspaces (A: 3 x N x M x 2L, B: 3 x N x 2M x 2L per rhs).
   void* wsA = nullptr;
   void* wsB = nullptr;
@@ -74,6 +81,8 @@ struct marie_plan {
   float2* bnd_bf = nullptr;
   long long bnd_n = 0;
   int bnd_transp = 0;
+  std::shared_ptr<marie_plan> bnd_crop;  // the bound DOFs' crop and their inverse map on it
+  int* bnd_inv_crop = nullptr;
 
   // Pinned host staging for small scalars (reductions, Hessenberg columns).
   double* pinned = nullptr;
@@ -94,6 +103,7 @@ struct DBuf {
   DBuf& operator=(const DBuf&) = delete;
   ~DBuf() { if (p) cudaFreeAsync(p, s); }
   int alloc(size_t bytes, cudaStream_t st);
+  bool try_alloc(size_t bytes, cudaStream_t st);  // for memory the caller can do without
   template <typename T> T* as() const { return reinterpret_cast<T*>(p); }
 };
 
@@ -164,6 +174,31 @@ int install_operator(marie_plan* p, const double2* fN_dev, int kind = 0);
 int install_octant(marie_plan* p, const double2* O_dev, int kind = 0);
 // Full 2L x 2M x 2N operator from its octant, scaled by s.
 int expand_octant(const double2* o, int L, int M, int N, int kind, double s, double2* f, cudaStream_t st);
+
+// Crop of a plan to the box of a body's DOFs (crop.cu).  crop_possible: worth
+// finding the box; dof_box: the box (max of -x -y -z, x y z) of 1-based DOFs;
+// crop_plan: the plan's operator on the box's grid with the plan's settings, or
+// null to stay on the whole grid, origin the box's first voxel; crop_settings:
+// the plan's present settings again; build_inverse_box: DOF map on that grid.
+bool crop_possible(const marie_plan* p);
+int dof_box(marie_plan* p, const int64_t* idx_dev, long long n, int box[6]);
+std::shared_ptr<marie_plan> crop_plan(marie_plan* p, const int box[6], int origin[3]);
+void crop_settings(const marie_plan* p, marie_plan* q);
+int build_inverse_box(marie_plan* p, marie_plan* q, const int origin[3], const int64_t* idx_dev, long long n,
+                      int* inv);
+// elements of the FP32 operator stored full along x; the FP32 copies of a
+// crop's octant (fN32, and fN32x into the given memory)
+size_t fullx_elems(const Dims& d);
+int store_crop_f32(marie_plan* q, float2* fullx);
+
+// Block-wide maxima of b[0..5] into box by atomics.
+__device__ __forceinline__ void box_reduce(int b[6], int* box) {
+#pragma unroll
+  for (int a = 0; a < 6; ++a) {
+    const int v = __reduce_max_sync(0xffffffffu, b[a]);
+    if ((threadIdx.x & 31) == 0 && v > INT_MIN) atomicMax(&box[a], v);
+  }
+}
 
 // Reads the plan's kernel status word after the plan's stream has finished
 // (a synchronising copy), clears it and returns MARIE_ETIMEOUT if a kernel's

@@ -1,5 +1,7 @@
 """The plan-bound mv_AN as the operator of pgmres / pgmresDR / bicgstab (the C
 ABI's NULL operator) against the oracle with the same mv_AN handle."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -88,3 +90,94 @@ def test_apply_bound_mv_AN(cuda, transp):
     assert outd.is_cuda
     np.testing.assert_array_equal(outd.cpu().numpy(), out32[:, 0])
     op.close()
+
+
+def _off_centre_body(shape, lo, size, dx=4e-3, seed=5):
+    """A box of scattered non-air voxels inside a larger grid of air."""
+    rng = np.random.default_rng(seed)
+    r = vo.grid(*shape, dx)
+    er = np.ones(shape, complex)
+    part = er[tuple(slice(a, a + s) for a, s in zip(lo, size))]
+    part[rng.random(size) < 0.7] = 30.0 - 20.0j
+    part[0, 0, 0] = part[-1, -1, -1] = 12.0 - 3.0j
+    return r, np.asfortranarray(er)
+
+
+# grids above the crop's smallest size; boxes at an edge, in the middle and
+# one voxel above a supported size; one, two and three axes shrink
+CROPS = [((48, 32, 40), (0, 3, 20), (17, 8, 20)), ((32, 96, 12), (5, 40, 0), (27, 33, 12)),
+         ((40, 32, 32), (12, 9, 11), (9, 23, 21))]
+
+
+@pytest.mark.parametrize("shape,lo,size", CROPS)
+@pytest.mark.parametrize("transp", ["notransp", "transp"])
+def test_bound_product_on_the_bodys_box(cuda, shape, lo, size, transp):
+    """A body that leaves most of its grid empty: the bound product, run on the
+    smallest grid that holds the body, against the unbound one on the whole
+    grid; 1e-13 of the largest value in FP64 (the smaller spectrum carries a
+    few roundings of its own), the FP32 bar in FP32, two columns."""
+    import marie_gb300 as mg
+
+    r, er = _off_centre_body(shape, lo, size)
+    op = mg.Operator.assemble(*shape, 4e-3, FREQ, precision="mixed", nrhs_max=2)
+    V = er.size
+    idxS = np.flatnonzero(np.abs(er.reshape(-1, order="F") - 1) > 1e-12) + 1
+    idx = np.concatenate([idxS, V + idxS, 2 * V + idxS]).astype(np.int64)
+    Mr, Mc = np.asfortranarray(er / er), np.asfortranarray((er - 1) / er)
+    rng = np.random.default_rng(2)
+    J = np.asfortranarray(rng.standard_normal((idx.size, 2)) + 1j * rng.standard_normal((idx.size, 2)))
+    ref = mg.mv_AN(J, op, Mr, Mc, 4e-3**3, transp, idx)
+    op.bind_mv_AN(Mr, Mc, 4e-3**3, transp, idx)
+    scale = np.max(np.abs(ref))
+    assert np.max(np.abs(op.apply_mv_AN(J, "fp64") - ref)) < 1e-13 * scale
+    assert np.max(np.abs(op.apply_mv_AN(J, "fp32") - ref)) < 1e-5 * scale
+    # another operator in the plan: the bound DOFs follow it
+    other = mg.Operator.assemble(*shape, 4e-3, 0.5 * FREQ)
+    fN = other.to_array()
+    mg._lib.check(op.lib.marie_set_operator(op.plan, C.c_void_p(fN.ctypes.data), *fN.shape[:3]))
+    ref = mg.mv_AN(J, op, Mr, Mc, 4e-3**3, transp, idx)
+    assert np.max(np.abs(op.apply_mv_AN(J, "fp64") - ref)) < 1e-13 * np.max(np.abs(ref))
+    op.close()
+
+
+@pytest.mark.parametrize("shape,lo,size", CROPS[:2])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_solves_on_the_bodys_box(cuda, shape, lo, size, precision):
+    """JVIE_Solver ('G', 'B'), the batch, jvie2solver and the gradient of a body
+    in a mostly empty grid against the same calls on a grid cut around it by
+    hand: the same flags, and fields equal to the solves' tolerance (1e-9,
+    times a condition of up to 1e3); two bodies in turn on one plan."""
+    import marie_gb300 as mg
+    from marie_gb300.autograd import adjoint_gradient
+
+    dx, em = 4e-3, vo.EMconstants(FREQ)
+    small = [mg.supported_size(s) for s in size]
+    cut = tuple(slice(min(a, n - s), min(a, n - s) + s) for a, n, s in zip(lo, shape, small))
+    op = mg.Operator.assemble(*shape, dx, FREQ, precision=precision, nrhs_max=2)
+    ref_op = mg.Operator.assemble(*small, dx, FREQ, precision=precision, nrhs_max=2)
+
+    def calls(op, r, er, E):
+        E2 = np.asfortranarray(np.stack([E, 1j * E[..., ::-1]], axis=4))
+        V = er.size
+        idxS = np.flatnonzero(np.abs(er.reshape(-1, order="F") - 1) > 1e-12) + 1
+        idx = np.concatenate([idxS, V + idxS, 2 * V + idxS]).astype(np.int64)
+        Mr, Mc = np.asfortranarray(er / er), np.asfortranarray((er - 1) / er)
+        yield mg.JVIE_Solver(E, er, r, FREQ, op, tol=1e-9, solver="G")[:2]
+        yield mg.JVIE_Solver(E, er, r, FREQ, op, tol=1e-9, solver="B")[:2]
+        yield mg.JVIE_Solver_batch(E2, er, r, FREQ, op, tol=1e-9)[:2]
+        b = E.reshape(-1, order="F")[idx - 1] * dx**3
+        yield mg.jvie2solver(b, op, idx, Mr, Mc, dx**3, 1e-9)[:2]
+        g = adjoint_gradient(op, E, er, dx, FREQ, "power", tol=1e-9)
+        yield g[1], g[3]
+
+    for k in range(2):
+        r, er = _off_centre_body(shape, lo, [s - 2 * k for s in size], seed=5 + k)
+        E = np.asfortranarray(vo.PlaneWave_Excitation(r, [0, 0, em["ko"]], em["omega_mu"], [1, 0, 0])[0])
+        f = lambda a: np.asfortranarray(a[cut])
+        for (x, fx), (y, fy) in zip(calls(op, r, er, E), calls(ref_op, f(r), f(er), f(E))):
+            assert np.all(np.asarray(fx) == 0) and np.all(np.asarray(fy) == 0)
+            inside = x[cut] if x.ndim > 1 else x
+            assert np.linalg.norm(inside - y) <= 1e-6 * np.linalg.norm(y)
+            assert np.count_nonzero(inside) == np.count_nonzero(x)  # nothing outside the body
+    op.close()
+    ref_op.close()
