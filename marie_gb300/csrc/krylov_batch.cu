@@ -39,6 +39,14 @@ static constexpr int BG = 152 * 2;
 // basis at HBM speed rather than at the FP64 rate, so they want more loads in
 // flight (four blocks per SM)
 static constexpr int BG32 = 152 * 4;
+// Smaller systems take fewer row blocks (counts that depend on the rows alone).
+// The dots: one block per SM and column group up to 4096 rows per block, whose
+// sums within a block stay a small share of its work.  The update: one row per
+// thread, so one round of loads, up to 2 BG blocks.
+static int dot_blocks(long long rows, int most) { return rows <= 4096LL * 152 ? 152 : most; }
+static int update_blocks(long long rows, int most) {
+  return rows <= 512LL * BG ? (int)std::max<long long>(1, (rows + 255) / 256) : most;
+}
 static constexpr int BT = 256;
 
 __device__ __forceinline__ double2 wsum2(double2 v) {
@@ -147,19 +155,6 @@ template <> struct BUnit<float2> {
   __device__ __forceinline__ static U scale(U w, float f) { return make_float4(w.x * f, w.y * f, w.z * f, w.w * f); }
 };
 
-__device__ __forceinline__ float2 wsum2f(float2 v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-  }
-  return v;
-}
-// warp sum of per-lane partial dots: FP64 lanes in FP64; FP32 lanes in FP32
-// (a few more roundings on a 32-term sum), then FP64 across warps and blocks
-__device__ __forceinline__ double2 warp_dot_sum(double2 v) { return wsum2(v); }
-__device__ __forceinline__ double2 warp_dot_sum(float2 v) { return cvt<double2>(wsum2f(v)); }
-
 // cycle start: V_s(:,0) = r_s / beta_s (zeros in the padding rows n..ld)
 template <typename VB>
 __global__ void kb_cycle_init(const double2* __restrict__ r, long long rs, VB* __restrict__ Vb, long long vs,
@@ -178,11 +173,11 @@ __global__ void kb_cycle_init(const double2* __restrict__ r, long long rs, VB* _
 // the reduction over the blocks' partials: the usual fence-then-count
 // pattern, no waiting.  The final sums have a fixed order whichever block
 // runs them.
-__device__ __forceinline__ bool last_block(unsigned* cnt) {
+__device__ __forceinline__ bool last_block(unsigned* cnt, unsigned blocks) {
   __shared__ bool is_last;
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) is_last = atomicAdd(cnt, 1u) == gridDim.x - 1;
+  if (threadIdx.x == 0) is_last = atomicAdd(cnt, 1u) == blocks - 1;
   __syncthreads();
   if (is_last) {
     __threadfence();
@@ -191,16 +186,44 @@ __device__ __forceinline__ bool last_block(unsigned* cnt) {
   return is_last;
 }
 
-// One sweep over NC basis columns c0..c0+NC-1 (units of U, column stride nu):
-// the block's partial sums of conj(V(:,j)) w, reduced in the block (warp sums,
-// then warp partials in warp order by one thread per column: a fixed order).
-// NC is a template argument so that a short last sweep issues no idle work.
+// Warp sums of NV values per lane, NV a power of two up to 16: at each step a
+// lane hands half of its values to its partner and adds the partner's to the
+// rest, so that after log2(NV) steps it holds one value summed over the lanes
+// that differ in those bits; the remaining steps sum that one value.  NV - 1
+// plus 5 - log2(NV) additions instead of 5 NV, in a fixed order.  On return
+// a[0] is value lane >> (5 - log2(NV)).
+template <int NV, typename T> __device__ __forceinline__ void warp_sums(T* a) {
+  const int lane = threadIdx.x & 31;
+  int o = 16;
+#pragma unroll
+  for (int half = NV / 2; half > 0; half /= 2) {
+    const bool upper = lane & o;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const T give = upper ? a[i] : a[i + half];
+      const T keep = upper ? a[i + half] : a[i];
+      a[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+    o >>= 1;
+  }
+#pragma unroll
+  for (int r = 32 / NV; r > 1; r /= 2) {
+    a[0] += __shfl_xor_sync(0xffffffffu, a[0], o);
+    o >>= 1;
+  }
+}
+
+// The block's rows of NC basis columns (units of U, column stride nu): partial
+// sums of conj(V(:,j)) w for j = c0 .. c0 + NC - 1, summed within warps (FP32
+// lanes in FP32, then FP64), then the warps' partials in warp order by one
+// thread per value: a fixed order.
 template <int NC, typename VB>
-__device__ __forceinline__ void kb_dot_sweep(const typename BUnit<VB>::U* __restrict__ V,
-                                             const typename BUnit<VB>::U* __restrict__ w, long long nu,
-                                             long long i0, long long i1, int c0, double2* __restrict__ part_s,
-                                             double2 (*red)[8]) {
+__device__ __forceinline__ void kb_dot_cols(const typename BUnit<VB>::U* __restrict__ V,
+                                            const typename BUnit<VB>::U* __restrict__ w, long long nu, long long i0,
+                                            long long i1, double* __restrict__ part, double (*red)[16]) {
   using BU = BUnit<VB>;
+  using T = decltype(VB::x);
+  constexpr int NV = NC > 4 ? 16 : NC > 2 ? 8 : NC > 1 ? 4 : 2;
   VB acc[NC];
 #pragma unroll
   for (int q = 0; q < NC; ++q) acc[q] = mk<VB>(0, 0);
@@ -208,53 +231,68 @@ __device__ __forceinline__ void kb_dot_sweep(const typename BUnit<VB>::U* __rest
   for (long long i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
     const typename BU::U wv = w[i];
 #pragma unroll
-    for (int q = 0; q < NC; ++q) BU::dot(acc[q], V[(long long)(c0 + q) * nu + i], wv);
+    for (int q = 0; q < NC; ++q) BU::dot(acc[q], V[(long long)q * nu + i], wv);
   }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  T a[NV];
 #pragma unroll
-  for (int q = 0; q < NC; ++q) {
-    const double2 r = warp_dot_sum(acc[q]);
-    if (lane == 0) red[wid][q] = r;
+  for (int q = 0; q < NV / 2; ++q) {
+    a[2 * q] = q < NC ? acc[q].x : (T)0;
+    a[2 * q + 1] = q < NC ? acc[q].y : (T)0;
   }
+  warp_sums<NV>(a);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  constexpr int REP = 32 / NV;
+  if (lane % REP == 0) red[wid][lane / REP] = (double)a[0];
   __syncthreads();
-  if (threadIdx.x < NC) {
-    double2 r = red[0][threadIdx.x];
-    for (int w2 = 1; w2 < BT / 32; ++w2) r = cadd(r, red[w2][threadIdx.x]);
-    part_s[(long long)(c0 + threadIdx.x) * gridDim.x + blockIdx.x] = r;
+  if (threadIdx.x < 2 * NC) {
+    double r = red[0][threadIdx.x];
+    for (int w2 = 1; w2 < BT / 32; ++w2) r += red[w2][threadIdx.x];
+    // part[column][block] as (re, im)
+    part[((long long)(threadIdx.x >> 1) * gridDim.x + blockIdx.x) * 2 + (threadIdx.x & 1)] = r;
   }
-  __syncthreads();  // red is reused by the next sweep
 }
 
 // partial[s][j][b] = sum over block rows of conj(V_s(:,j)) w_s, j < k, w_s = V_s(:,k);
 // h[s][j] = sum_b partial[s][j][b].  ld: column stride in complex elements.
+// grid (row blocks, column groups of at most 8, systems): the groups of a step
+// are as even as k allows and run side by side, so a step's latency is one
+// sweep whatever k.
+//
+// FP64-pipe bound at large n (4 FMAs per element and column; the warp sums add
+// 16 per 8 columns and warp, where five-step sums of each value added 80: 14 %
+// of the work at 4.5 rows per thread).  Measured with
+// the block counts above, kb_dots and kb_update: GMRES with 8 right-hand sides
+// of 64^3 (170k rows each) 172 -> 147 ms, the 64^3 gradient 97.4 -> 87.8 ms, a
+// 32^3 FP64 solve (42k rows) 20.5 -> 18.1 ms.
 template <typename VB>
 __global__ void __launch_bounds__(BT) kb_dots(const VB* __restrict__ Vb, long long vs, long long ld, int k,
-                                              const int* __restrict__ stop, double2* __restrict__ part,
+                                              const int* __restrict__ stop, double2* __restrict__ part, long long ps,
                                               unsigned* __restrict__ cnt, double2* __restrict__ h, int hld) {
   using U = typename BUnit<VB>::U;
-  const int s = blockIdx.y;
+  const int s = blockIdx.z;
   if (skip(stop, s, k)) return;
   const long long nu = ld / BUnit<VB>::W;
-  const U* V = reinterpret_cast<const U*>(Vb + s * vs);
-  const U* w = V + (long long)k * nu;
-  double2* part_s = part + (long long)s * 128 * gridDim.x;
-  __shared__ double2 red[BT / 32][8];
+  const U* w = reinterpret_cast<const U*>(Vb + s * vs) + (long long)k * nu;
+  const int c0 = k * blockIdx.y / gridDim.y, c1 = k * (blockIdx.y + 1) / gridDim.y;
+  const U* V = reinterpret_cast<const U*>(Vb + s * vs) + (long long)c0 * nu;
+  double2* part_s = part + s * ps;
+  double* pd = reinterpret_cast<double*>(part_s + (long long)c0 * gridDim.x);
+  __shared__ double red[BT / 32][16];
   long long i0, i1;
   rows_of(nu, i0, i1);
-  int c0 = 0;
-  for (; c0 + 8 <= k; c0 += 8) kb_dot_sweep<8, VB>(V, w, nu, i0, i1, c0, part_s, red);
-  switch (k - c0) {
-    case 1: kb_dot_sweep<1, VB>(V, w, nu, i0, i1, c0, part_s, red); break;
-    case 2: kb_dot_sweep<2, VB>(V, w, nu, i0, i1, c0, part_s, red); break;
-    case 3: kb_dot_sweep<3, VB>(V, w, nu, i0, i1, c0, part_s, red); break;
-    case 4: kb_dot_sweep<4, VB>(V, w, nu, i0, i1, c0, part_s, red); break;
-    case 5: kb_dot_sweep<5, VB>(V, w, nu, i0, i1, c0, part_s, red); break;
-    case 6: kb_dot_sweep<6, VB>(V, w, nu, i0, i1, c0, part_s, red); break;
-    case 7: kb_dot_sweep<7, VB>(V, w, nu, i0, i1, c0, part_s, red); break;
+  switch (c1 - c0) {
+    case 1: kb_dot_cols<1, VB>(V, w, nu, i0, i1, pd, red); break;
+    case 2: kb_dot_cols<2, VB>(V, w, nu, i0, i1, pd, red); break;
+    case 3: kb_dot_cols<3, VB>(V, w, nu, i0, i1, pd, red); break;
+    case 4: kb_dot_cols<4, VB>(V, w, nu, i0, i1, pd, red); break;
+    case 5: kb_dot_cols<5, VB>(V, w, nu, i0, i1, pd, red); break;
+    case 6: kb_dot_cols<6, VB>(V, w, nu, i0, i1, pd, red); break;
+    case 7: kb_dot_cols<7, VB>(V, w, nu, i0, i1, pd, red); break;
+    case 8: kb_dot_cols<8, VB>(V, w, nu, i0, i1, pd, red); break;
     default: break;
   }
   // h[s][j] = sum_b part[s][j][b] by the last block, one warp per column
-  if (!last_block(cnt + s)) return;
+  if (!last_block(cnt + s, gridDim.x * gridDim.y)) return;
   const int G = gridDim.x, lane = threadIdx.x & 31;
   for (int j = threadIdx.x >> 5; j < k; j += BT / 32) {
     double2 a = mk<double2>(0, 0);
@@ -306,9 +344,13 @@ __device__ void givens_warp(const GState& G, int m, int k, const double2* __rest
   __shared__ double cs_s[128];
   const int kk = k - 1;
   double nn = 0;
+#pragma unroll 4
   for (int b = lane; b < NB; b += 32) nn += __ldcg(npart + (long long)s * NB + b);
   nn = wsum(nn);
-  const double hnv = sqrt(nn);
+  // the norms and the rotation from reciprocal square roots: a step's end is
+  // one thread's chain of FP64 operations, and hypot and division are the
+  // longest of them
+  const double hnv = nn > 0 ? nn * rsqrt(nn) : sqrt(nn);
   for (int i = lane; i < k; i += 32) {
     const double2 v = h[(long long)s * hld + i];
     H[kk * ld + i] = v;
@@ -333,30 +375,32 @@ __device__ void givens_warp(const GState& G, int m, int k, const double2* __rest
       const double c = cs_s[i];
       const double2 sv = sn_s[i];
       col[i] = cadd(cscale(a, c), cmul(sv, b));
-      a = csub(cscale(b, c), cmulc(a, sv));  // -conj(s) a + c b
+      // -conj(s) a + c b, two dependent FMAs per component
+      a = mk<double2>(fma(-a.y, sv.y, fma(-a.x, sv.x, b.x * c)), fma(a.x, sv.y, fma(-a.y, sv.x, b.y * c)));
     }
-    const double aa = hypot(a.x, a.y), bb = hnv;
-    double c;
+    const double a2 = a.x * a.x + a.y * a.y;
+    double c, sa;
     double2 sv;
-    if (aa == 0.0) {
+    if (a2 == 0.0) {
       c = 0.0;
+      sa = 1.0;
       sv = mk<double2>(1.0, 0.0);
-      col[kk] = mk<double2>(bb, 0);
+      col[kk] = mk<double2>(hnv, 0);
     } else {
-      const double rho = hypot(aa, bb);
-      const double2 ph = mk<double2>(a.x / aa, a.y / aa);
-      c = aa / rho;
-      sv = cscale(ph, bb / rho);  // ph * conj(b) / rho, b real
-      col[kk] = cscale(ph, rho);
+      const double ia = rsqrt(a2), rho2 = a2 + nn, ir = rsqrt(rho2);
+      const double2 ph = mk<double2>(a.x * ia, a.y * ia);
+      c = a2 * ia * ir;
+      sa = hnv * ir;
+      sv = cscale(ph, sa);  // ph * conj(b) / rho, b = hnv real
+      col[kk] = cscale(ph, rho2 * ir);
     }
     col[k] = mk<double2>(0, 0);
     cs[kk] = c;
     sn[kk] = sv;
     const double2 gk = g[kk];
     g[kk] = cscale(gk, c);
-    const double2 gn = mk<double2>(-(sv.x * gk.x + sv.y * gk.y), -(sv.x * gk.y - sv.y * gk.x));  // -conj(s) g
-    g[k] = gn;
-    rn = hypot(gn.x, gn.y);
+    g[k] = mk<double2>(-(sv.x * gk.x + sv.y * gk.y), -(sv.x * gk.y - sv.y * gk.x));  // -conj(s) g
+    rn = sa * (k == 1 ? G.beta[s] : G.resv[(long long)s * m + kk - 1]);  // |g(k)| = |s| |g(k-1)|
     G.resv[(long long)s * m + kk] = rn;
     G.hn[s] = hnv;
   }
@@ -409,7 +453,7 @@ __global__ void __launch_bounds__(BT) kb_update(VB* __restrict__ Vb, long long v
   }
   const double2 r = bsum2(mk<double2>((double)a, 0));
   if (threadIdx.x == 0) part[(long long)s * gridDim.x + blockIdx.x] = r.x;
-  if (!last_block(cnt + s)) return;
+  if (!last_block(cnt + s, gridDim.x)) return;
   if (threadIdx.x < 32) givens_warp(G, m, k, h, hld, part, gridDim.x, s, threadIdx.x);
 }
 
@@ -447,6 +491,7 @@ __global__ void kb_combine(const VB* __restrict__ Vb, long long vs, long long n,
   double2* o = out + s * os;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     VB v = mk<VB>(0, 0);
+#pragma unroll 8
     for (int j = 0; j < nc; ++j) {
       const VB b = V[(long long)j * ld + i];
       v.x = fmaT(b.x, cf[j].x, fmaT(-b.y, cf[j].y, v.x));
@@ -529,7 +574,7 @@ struct BatchWork {
   int S = 0, m = 0;
   long long n = 0, ld = 0;  // rows; column stride of the basis
   bool f32 = false;  // FP32 basis (t1f, t2f: FP32 work vectors of the preconditioner chains)
-  int bg = BG;       // row blocks of kb_dots / kb_update
+  int bd = BG, bu = BG;  // row blocks of kb_dots / kb_update
   DBuf V, t1, t2, t1f, t2f, r, part_d, part_n, h, H, R, g, cs, sn, y, res, resv, beta, tol, hn, stop, norms;
   DBuf cnt;  // [2][S] last-block counters of kb_dots and kb_update (zero between launches)
   GState gs{};
@@ -571,9 +616,11 @@ struct BatchWork {
     }
     MARIE_TRY(t1.alloc((size_t)S * n * sizeof(double2), st));
     MARIE_TRY(t2.alloc((size_t)S * n * sizeof(double2), st));
-    bg = f32 ? BG32 : BG;
-    MARIE_TRY(part_d.alloc((size_t)S * 128 * bg * sizeof(double2), st));
-    MARIE_TRY(part_n.alloc((size_t)S * (bg > BG ? bg : BG) * sizeof(double), st));
+    const long long rows = f32 ? ld / 2 : ld;
+    bd = dot_blocks(rows, f32 ? BG32 : BG);
+    bu = update_blocks(rows, f32 ? BG32 : BG);
+    MARIE_TRY(part_d.alloc((size_t)S * 128 * bd * sizeof(double2), st));
+    MARIE_TRY(part_n.alloc((size_t)S * std::max(bu, BG) * sizeof(double), st));
     MARIE_TRY(h.alloc((size_t)S * (m + 1) * sizeof(double2), st));
     MARIE_TRY(H.alloc((size_t)S * (m + 1) * m * sizeof(double2), st));
     MARIE_TRY(R.alloc((size_t)S * (m + 1) * m * sizeof(double2), st));
@@ -673,10 +720,11 @@ static void group_gs(BatchWork& W, int g0, int Sg, int k, cudaStream_t sm) {
   gs.tolabs += g0;
   gs.hn += g0;
   gs.stop += g0;
-  kb_dots<VB><<<dim3(W.bg, Sg), BT, 0, sm>>>(V, vs, ld, k, stop, W.part_d.as<double2>() + (long long)g0 * 128 * W.bg,
-                                             cnt + g0, h, m + 1);
-  kb_update<VB><<<dim3(W.bg, Sg), BT, 0, sm>>>(V, vs, ld, k, h, m + 1, stop,
-                                               W.part_n.as<double>() + (long long)g0 * W.bg, cnt + S + g0, gs, m);
+  const long long ps = 128LL * W.bd;
+  kb_dots<VB><<<dim3(W.bd, (k + 7) / 8, Sg), BT, 0, sm>>>(V, vs, ld, k, stop, W.part_d.as<double2>() + g0 * ps, ps,
+                                                          cnt + g0, h, m + 1);
+  kb_update<VB><<<dim3(W.bu, Sg), BT, 0, sm>>>(V, vs, ld, k, h, m + 1, stop,
+                                               W.part_n.as<double>() + (long long)g0 * W.bu, cnt + S + g0, gs, m);
   kb_scale<VB><<<dim3(gx(ld / BUnit<VB>::W), Sg), 256, 0, sm>>>(V, vs, ld, k, W.hn.as<double>() + g0, stop);
   count_launch(3);
 }
