@@ -11,29 +11,49 @@ namespace marie {
 template <typename T> struct MatvecImpl {
   using V = cplx<T>;
 
-  template <int NL, typename IO>
-  static cudaError_t xfwd_n(const IO* J, long long js, const int* inv, Prologue pro, V* A, long long as,
+  template <int NL, int THR, typename IO>
+  static cudaError_t xfwd_nt(const IO* J, long long js, const int* inv, Prologue pro, V* A, long long as,
                             const Dims& d, const V* tw, int nrhs, cudaStream_t st) {
-    constexpr int S = RowCfg<cplx<T>, NL>::S;
+    constexpr int S = RowCfg<cplx<T>, NL, THR>::S;
     const size_t smem = (size_t)(NL + NL * (S + 1)) * sizeof(V);
-    cudaError_t e = opt_in_smem(k_xfwd<T, NL, IO>, smem);
+    cudaError_t e = opt_in_smem(k_xfwd<T, NL, THR, IO>, smem);
     if (e != cudaSuccess) return e;
     const int rows = d.M * d.N * 3;
     dim3 grid((rows + S - 1) / S, nrhs);
-    k_xfwd<T, NL, IO><<<grid, RowCfg<cplx<T>, NL>::THREADS, smem, st>>>(J, js, inv, pro, A, as, d, tw);
+    k_xfwd<T, NL, THR, IO><<<grid, RowCfg<cplx<T>, NL, THR>::THREADS, smem, st>>>(J, js, inv, pro, A, as, d, tw);
     return cudaGetLastError();
+  }
+  template <int NL, int THR, typename IO>
+  static cudaError_t xinv_nt(const V* A, long long as, const IO* J, long long js, const int* inv, Epilogue ep,
+                            IO* out, long long os, const Dims& d, const V* tw, int nrhs, cudaStream_t st) {
+    constexpr int S = RowCfg<cplx<T>, NL, THR>::S;
+    const size_t smem = (size_t)(NL + NL * (S + 1)) * sizeof(V);
+    cudaError_t e = opt_in_smem(k_xinv<T, NL, THR, IO>, smem);
+    if (e != cudaSuccess) return e;
+    const int rows = d.M * d.N * 3;
+    dim3 grid((rows + S - 1) / S, nrhs);
+    k_xinv<T, NL, THR, IO><<<grid, RowCfg<cplx<T>, NL, THR>::THREADS, smem, st>>>(A, as, J, js, inv, ep, out, os, d, tw);
+    return cudaGetLastError();
+  }
+  // An x pass of 256-thread CTAs is taken when it fills the chip four times over;
+  // below that, CTAs of a quarter the rows spread the work over all SMs.
+  // First and last pass of a 40^3 FP64 grid 46 -> 32 and 51 -> 37 us; of a 12 x 8
+  // x 20 grid, two CTAs before, 34 and 49 us to a tenth.
+  template <int NL> static bool many_rows(const Dims& d, int nrhs) {
+    constexpr int S = RowCfg<cplx<T>, NL>::S;
+    return ((long long)d.M * d.N * 3 + S - 1) / S * nrhs >= 4 * 152;
+  }
+  template <int NL, typename IO>
+  static cudaError_t xfwd_n(const IO* J, long long js, const int* inv, Prologue pro, V* A, long long as,
+                            const Dims& d, const V* tw, int nrhs, cudaStream_t st) {
+    return many_rows<NL>(d, nrhs) ? xfwd_nt<NL, 256, IO>(J, js, inv, pro, A, as, d, tw, nrhs, st)
+                                  : xfwd_nt<NL, 64, IO>(J, js, inv, pro, A, as, d, tw, nrhs, st);
   }
   template <int NL, typename IO>
   static cudaError_t xinv_n(const V* A, long long as, const IO* J, long long js, const int* inv, Epilogue ep,
                             IO* out, long long os, const Dims& d, const V* tw, int nrhs, cudaStream_t st) {
-    constexpr int S = RowCfg<cplx<T>, NL>::S;
-    const size_t smem = (size_t)(NL + NL * (S + 1)) * sizeof(V);
-    cudaError_t e = opt_in_smem(k_xinv<T, NL, IO>, smem);
-    if (e != cudaSuccess) return e;
-    const int rows = d.M * d.N * 3;
-    dim3 grid((rows + S - 1) / S, nrhs);
-    k_xinv<T, NL, IO><<<grid, RowCfg<cplx<T>, NL>::THREADS, smem, st>>>(A, as, J, js, inv, ep, out, os, d, tw);
-    return cudaGetLastError();
+    return many_rows<NL>(d, nrhs) ? xinv_nt<NL, 256, IO>(A, as, J, js, inv, ep, out, os, d, tw, nrhs, st)
+                                  : xinv_nt<NL, 64, IO>(A, as, J, js, inv, ep, out, os, d, tw, nrhs, st);
   }
   template <int NC, bool INV>
   static cudaError_t cols_n(const V* in, long long in_w, long long in_rhs, int n_in, V* out, long long out_w,

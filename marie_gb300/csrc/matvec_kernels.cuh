@@ -101,9 +101,12 @@ __device__ __forceinline__ IO prologue_in(const IO* J, const Prologue& pro, int 
   return jv;
 }
 
-template <typename V, int N> struct RowCfg {
+// Rows per CTA of the x passes, THR the thread count aimed at: 256 where that
+// gives the chip enough CTAs, 64 (at least 32 rows of one thread) otherwise.
+template <typename V, int N, int THR = 256> struct RowCfg {
   static constexpr int T = FFT<V, N, false>::T;
-  static constexpr int S = (256 / T) < 2 ? 2 : (256 / T);
+  static constexpr int AIM = THR / T;
+  static constexpr int S = THR < 256 && T <= 2 ? 32 : (AIM < 2 ? 2 : AIM);
   static constexpr int THREADS = S * T;
 };
 
@@ -116,13 +119,13 @@ __device__ __forceinline__ void stage_twiddles(V* tw_s, const V* __restrict__ tw
 // ---------------------------------------------------------------------------
 // xfwd: gather + forward x transform.  grid.x = ceil(rows / S), grid.y = rhs
 // ---------------------------------------------------------------------------
-template <typename T, int NL, typename IO>
-__global__ void __launch_bounds__(RowCfg<cplx<T>, NL>::THREADS)
+template <typename T, int NL, int THR, typename IO>
+__global__ void __launch_bounds__(RowCfg<cplx<T>, NL, THR>::THREADS)
 k_xfwd(const IO* __restrict__ J, long long j_stride, const int* __restrict__ inv, Prologue pro,
        cplx<T>* __restrict__ A, long long a_stride, Dims d, const cplx<T>* __restrict__ tw) {
   using V = cplx<T>;
   using F = FFT<V, NL, false>;
-  constexpr int S = RowCfg<cplx<T>, NL>::S;
+  constexpr int S = RowCfg<cplx<T>, NL, THR>::S;
   constexpr int ES = S + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V* tw_s = reinterpret_cast<V*>(smem_raw);
@@ -163,14 +166,14 @@ k_xfwd(const IO* __restrict__ J, long long j_stride, const int* __restrict__ inv
 // ---------------------------------------------------------------------------
 // xinv: inverse x transform + crop + epilogue + scatter to DOFs.
 // ---------------------------------------------------------------------------
-template <typename T, int NL, typename IO>
-__global__ void __launch_bounds__(RowCfg<cplx<T>, NL>::THREADS)
+template <typename T, int NL, int THR, typename IO>
+__global__ void __launch_bounds__(RowCfg<cplx<T>, NL, THR>::THREADS)
 k_xinv(const cplx<T>* __restrict__ A, long long a_stride, const IO* __restrict__ J, long long j_stride,
        const int* __restrict__ inv, Epilogue ep, IO* __restrict__ out, long long o_stride, Dims d,
        const cplx<T>* __restrict__ tw) {
   using V = cplx<T>;
   using F = FFT<V, NL, true>;
-  constexpr int S = RowCfg<cplx<T>, NL>::S;
+  constexpr int S = RowCfg<cplx<T>, NL, THR>::S;
   constexpr int ES = S + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V* tw_s = reinterpret_cast<V*>(smem_raw);
@@ -306,9 +309,13 @@ template <> struct OpKind<1> {
 // z-pass variants the autotuner chooses from (FP32, N operator): 0 the
 // default (wide radix schedule where one exists, 8 columns per CTA), 1 the
 // narrow radix schedule, 2 half the columns per CTA.
+// FP64 takes 4 columns, and 8 for the lengths whose 4 threads per transform
+// would fill half a warp per component (96 points, 24 values per thread: the
+// product's three branches ran on half-empty warps).  z pass of a
+// 48^3 FP64 grid: 474 -> 281 us.
 template <typename T, int NZ, int VAR> struct ZVar {
   static constexpr bool W = VAR == 1 ? false : (sizeof(cplx<T>) == 8 && HasWide<NZ>::value);
-  static constexpr int S0 = (sizeof(T) == 4 ? 8 : 4) / (VAR == 2 ? 2 : 1);
+  static constexpr int S0 = (sizeof(T) == 4 || FFT<cplx<T>, NZ, false, W>::T == 4 ? 8 : 4) / (VAR == 2 ? 2 : 1);
 };
 
 template <typename T, int NZ, int KIND = 0, int VAR = 0> struct ZS {
@@ -317,6 +324,9 @@ template <typename T, int NZ, int KIND = 0, int VAR = 0> struct ZS {
   static constexpr int S0 = ZVar<T, NZ, VAR>::S0;            // columns per CTA
   static constexpr int S = (3 * S0 * TT <= 1024) ? S0 : ((3 * (S0 / 2) * TT <= 1024) ? S0 / 2 : S0 / 4);
   static constexpr int THREADS = 3 * S * TT;               // one thread group per component
+  // a component's threads fill whole warps: its row of the product is chosen by
+  // a branch, otherwise by data
+  static constexpr bool UNIFORM = (S * TT) % 32 == 0;
   // rows of 64 B use the half-line swizzle, others one pad element per row
   static constexpr bool HALF = S * (int)sizeof(cplx<T>) == 64;
   static constexpr int ES = HALF ? S : S + 1;
@@ -358,6 +368,11 @@ template <int C> struct ZRow {
 
 template <typename V> __device__ __forceinline__ V neg_if(V v, bool f) { return f ? mk<V>(-v.x, -v.y) : v; }
 
+// a b + c, four FMAs
+template <typename V> __device__ __forceinline__ V cfma(V a, V b, V c) {
+  return mk<V>(fma(-a.y, b.y, fma(a.x, b.x, c.x)), fma(a.y, b.x, fma(a.x, b.y, c.y)));
+}
+
 // Row C of the product at this thread's output positions of the forward
 // transform.  With the octant operator the tile already carries the x and y
 // reflection signs; the z reflection (positions kz > NZ/2) flips the two
@@ -392,7 +407,44 @@ __device__ __forceinline__ void zrow(V* reg, int t, int s, bool active, int oct,
           n2 = fp[RW::q2 * fq + o];
         }
         const int e = ad(kz);
-        y = cadd(cadd(cmul(n0, b0[e]), cmul(n1, b1[e])), cmul(n2, b2[e]));
+        y = cfma(n2, b2[e], cfma(n1, b1[e], cmul(n0, b0[e])));
+      }
+      reg[b * RL + r] = y;
+    }
+}
+
+// The same with the row c as data, for transforms so short that one warp holds
+// threads of several components: three divergent copies of the product would
+// each cost a whole warp's issue slots (FP64: 16 cycles per instruction).
+// z pass of a 40^3 FP64 grid (80 points, with the 8-column tiles): 299 -> 185 us.
+template <typename FF, typename V, int NZ, int S>
+__device__ __forceinline__ void zrow_any(V* reg, int c, int t, int s, bool active, int oct, const V* tile, const V* fp,
+                                         long long fq, long long fplane, const V* b0, const V* b1, const V* b2,
+                                         SAddr ad) {
+  constexpr int NH = NZ / 2, NO = NH + 1, RL = FF::RL;
+  const int q0 = c, q1 = c == 0 ? 1 : c + 2, q2 = c == 0 ? 2 : c + 3;  // ZRow<c>
+#pragma unroll
+  for (int b = 0; b < FF::E / RL; ++b)
+#pragma unroll
+    for (int r = 0; r < RL; ++r) {
+      const int kz = FF::out_pos(t, b, r);
+      V y = mk<V>(0, 0);
+      if (active) {
+        V n0, n1, n2;
+        if (oct) {
+          const bool fz = kz > NH;
+          const int oz = fz ? NZ - kz : kz;
+          n0 = neg_if(tile[(q0 * NO + oz) * S + s], fz && q0 == 2);
+          n1 = neg_if(tile[(q1 * NO + oz) * S + s], fz && q1 == 4);
+          n2 = neg_if(tile[(q2 * NO + oz) * S + s], fz && q2 != 5);
+        } else {
+          const long long o = (long long)kz * fplane;
+          n0 = fp[q0 * fq + o];
+          n1 = fp[q1 * fq + o];
+          n2 = fp[q2 * fq + o];
+        }
+        const int e = ad(kz);
+        y = cfma(n2, b2[e], cfma(n1, b1[e], cmul(n0, b0[e])));
       }
       reg[b * RL + r] = y;
     }
@@ -432,7 +484,7 @@ __device__ __forceinline__ void zrow_k(V* reg, int t, int s, bool active, int oc
           nb = fp[RW::qb * fq + o];
         }
         const int e = ad(kz);
-        y = csub(cmul(na, bc[RW::ia][e]), cmul(nb, bc[RW::ib][e]));
+        y = cfma(mk<V>(-nb.x, -nb.y), bc[RW::ib][e], cmul(na, bc[RW::ia][e]));
       }
       reg[b * RL + r] = y;
     }
@@ -610,8 +662,9 @@ k_zmul(cplx<T>* __restrict__ B, long long b_rhs, const cplx<T>* __restrict__ fN,
   const V* b0 = buf + s;
   const V* b1 = buf + BUF + s;
   const V* b2 = buf + 2 * BUF + s;
-  // c is uniform over whole warps (groups of S * T threads) for the long transforms
-  if constexpr (KIND == 0) {
+  if constexpr (KIND == 0 && !ZC::UNIFORM) {
+    zrow_any<FF, V, NZ, S>(reg, c, t, s, active, oct, tile, fp, fq, fplane, b0, b1, b2, ad);
+  } else if constexpr (KIND == 0) {
     if (c == 0)
       zrow<0, FF, V, NZ, S>(reg, t, s, active, oct, tile, fp, fq, fplane, b0, b1, b2, ad);
     else if (c == 1)
