@@ -460,7 +460,7 @@ __global__ void k_extract_octant(const double2* __restrict__ f, int L, int M, in
 // the N operator full along x, half along y and z: fx[q][oz][oy][kx] =
 // s * f[q][oz][oy][kx] for oy <= M, oz <= N, in FP32 (the z pass's bulk tile
 // source), from the full operator or from its octant (oct; the x reflections
-// are signed here)
+// are signed here); columns kx, kx + 1 (kx even) as {re, re, im, im}
 __global__ void k_extract_fullx(const double2* __restrict__ f, int oct, int L, int M, int N, double s,
                                 float2* __restrict__ fx) {
   const long long Lp = 2LL * L, Mp = 2LL * M, Np = 2LL * N, P = Lp * Mp * Np;
@@ -478,7 +478,9 @@ __global__ void k_extract_fullx(const double2* __restrict__ f, int oct, int L, i
     } else {
       v = f[q * P + kx + Lp * (oy + Mp * oz)];
     }
-    fx[t] = mk<float2>((float)(v.x * s), (float)(v.y * s));
+    float* pair = reinterpret_cast<float*>(fx + (t & ~1LL)) + (t & 1);  // rows of 2L: t and kx have the same parity
+    pair[0] = (float)(v.x * s);
+    pair[2] = (float)(v.y * s);
   }
 }
 

@@ -34,14 +34,10 @@ namespace {
 // Products below this many voxels are bound by launches, not by the padded
 // volume.
 constexpr long long kCropMinVoxels = 30000;
-// Crop when the product's estimated cost falls to this share or less: building
-// the smaller operator costs up to a few FP64 products, and a solve takes tens
-// to hundreds.
+// Crop when the padded volume, to which the passes' time is proportional, falls
+// to this share or less: building the smaller operator costs up to a few FP64
+// products, and a solve takes tens to hundreds.
 constexpr double kCropShare = 0.8;
-// FP32 products without a fused x+y pass for their lengths cost this much more
-// per padded point (measured: see MARIE_FUSED_PAIRS).
-constexpr double kUnfusedCost = 1.3;
-
 // sin(pi m / d), the angle reduced to the first quarter turn as an integer
 __device__ __forceinline__ double sin_ratio(long long m, long long d) {
   m %= 2 * d;
@@ -162,15 +158,6 @@ __global__ void k_inverse_box(const int64_t* __restrict__ idx, long long n, int 
     const int x = v % L - x0, y = (v / L) % M - y0, z = v / (L * M) - z0;
     inv[x + (long long)L2 * (y + (long long)M2 * (z + (long long)N2 * c))] = (int)i;
   }
-}
-
-double product_cost(const marie_plan* p, int L, int M, int N) {
-  Dims d{};
-  d.L = L; d.M = M; d.N = N;
-  d.Lp = 2 * L; d.Mp = 2 * M; d.Np = 2 * N;
-  double c = (double)L * M * N;
-  if (p->precision == MARIE_MIXED && p->fuse && !MatvecLaunch<float>::fused(d)) c *= kUnfusedCost;
-  return c;
 }
 
 }  // namespace
@@ -308,24 +295,11 @@ std::shared_ptr<marie_plan> crop_plan(marie_plan* p, const int box[6], int origi
     need[a] = box[3 + a] + box[a] + 1;
     if (origin[a] < 0 || need[a] < 1 || origin[a] + need[a] > n[a]) return nullptr;
   }
-  std::vector<int> sizes[3];
+  int best[3];
   for (int a = 0; a < 3; ++a)
-    for (int s = need[a]; s <= n[a]; ++s)
-      if (fft_length_supported(2 * s)) sizes[a].push_back(s);
-  int best[3] = {n[0], n[1], n[2]};
-  const double full = product_cost(p, n[0], n[1], n[2]);
-  double cost = full;
-  for (int x : sizes[0])
-    for (int y : sizes[1]) {
-      const double c = product_cost(p, x, y, sizes[2][0]);
-      if (c < cost) {
-        cost = c;
-        best[0] = x;
-        best[1] = y;
-        best[2] = sizes[2][0];
-      }
+    for (best[a] = need[a]; !fft_length_supported(2 * best[a]); ++best[a]) {
     }
-  if (!(cost <= kCropShare * full)) return nullptr;
+  if ((double)best[0] * best[1] * best[2] > kCropShare * (double)p->d.V) return nullptr;
   std::shared_ptr<marie_plan> q = p->crop;
   if (!q || q->d.L != best[0] || q->d.M != best[1] || q->d.N != best[2]) {
     // the last one stays with the plan: its size depends on the body's box only

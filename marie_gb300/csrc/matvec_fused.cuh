@@ -258,101 +258,17 @@ k_yxinv(const cplx<T>* __restrict__ B, long long bs, const IO* __restrict__ J, l
     // rows delivered: arrive (release) now and wait (acquire) once the first
     // sweep's epilogue indices are in flight
     cluster_arrive();
-    int kk[E <= 16 ? E : 1];
-    if constexpr (E <= 16) load_epi_idx(kk, 0);
+    int kk[E];
+    load_epi_idx(kk, 0);
     cluster_wait();
     for (int row0 = 0; row0 < C::RYP; row0 += C::SX) {
       const int yl = row0 + s;
-      const bool valid = yl < C::RY;
-      const int y = q * C::RY + yl;
       V* base = rows + yl * C::ROWP;
       V reg[E];
       FXI::load(reg, base, rowa, t, NL);
       FXI::run(reg, base, rowa, t, twx_s);
-      if constexpr (E <= 16)
-        if (row0 > 0) load_epi_idx(kk, row0);
-      if (valid) {
-        const int* invr = inv + (long long)L * (y + (long long)M * plane);
-        if constexpr (E <= 16) {
-          // index loads (above), then the per-DOF loads, then the epilogue arithmetic
-          // per-DOF loads in groups of EPI (bounded registers)
-          constexpr int EPI = 2;
-          // FP64 vectors with FP32 coefficient copies (the matvec of the
-          // mixed-precision inner solves): the whole epilogue in FP32, the
-          // transforms' precision, with one conversion in and one out
-          constexpr bool MIX = std::is_same<IO, double2>::value && std::is_same<V, float2>::value;
-          const bool f32epi = MIX && ep.af != nullptr;
-#pragma unroll
-          for (int i0 = 0; i0 < E; i0 += EPI) {
-            IO jv[EPI], ak[EPI], bk[EPI];
-            float2 af[EPI], bf[EPI];
-#pragma unroll
-            for (int j = 0; j < EPI; ++j) {
-              const int k = kk[i0 + j];
-              if (k < 0) continue;
-              jv[j] = Jr[k];
-              if (f32epi) {
-                af[j] = ep.af[k];
-                bf[j] = ep.bf[k];
-              } else {
-                ak[j] = EpiIO<IO>::a(ep, k);
-                bk[j] = EpiIO<IO>::b(ep, k);
-              }
-            }
-#pragma unroll
-            for (int j = 0; j < EPI; ++j) {
-              const int k = kk[i0 + j];
-              if (k < 0) continue;
-              if constexpr (MIX) {
-                if (f32epi) {
-                  const float2 v = reg[i0 + j];
-                  float2 r32 = cmul(af[j], cvt<float2>(jv[j]));
-                  if (ep.conjout) {
-                    r32.x -= v.x;
-                    r32.y += v.y;
-                  } else {
-                    r32 = csub(r32, cmul(bf[j], v));
-                  }
-                  outr[k] = cvt<IO>(r32);
-                  continue;
-                }
-              }
-              // the diagonal Gram*Mr*J term in the vectors' precision; the
-              // circulant term in the transform's precision
-              IO res = cmul(ak[j], jv[j]);
-              if (ep.conjout) {
-                const IO v = cvt<IO>(reg[i0 + j]);
-                res.x -= v.x;
-                res.y += v.y;
-              } else {
-                res = csub(res, cvt<IO>(cmul(cvt<V>(bk[j]), reg[i0 + j])));
-              }
-              outr[k] = res;
-            }
-          }
-        } else {
-          // wide register sets (E = 20, 24): one DOF at a time
-#pragma unroll
-          for (int b = 0; b < E / RL; ++b)
-#pragma unroll
-            for (int r = 0; r < RL; ++r) {
-              const int x = FXI::out_pos(t, b, r);
-              if (x >= L) continue;
-              const int k = invr[x];
-              if (k < 0) continue;
-              const IO jv = Jr[k];
-              IO res = cmul(EpiIO<IO>::a(ep, k), jv);
-              if (ep.conjout) {
-                const IO v = cvt<IO>(reg[b * RL + r]);
-                res.x -= v.x;
-                res.y += v.y;
-              } else {
-                res = csub(res, cvt<IO>(cmul(cvt<V>(EpiIO<IO>::b(ep, k)), reg[b * RL + r])));
-              }
-              outr[k] = res;
-            }
-        }
-      }
+      if (row0 > 0) load_epi_idx(kk, row0);
+      epilogue_dofs<IO, V, E, 2, true>(reg, kk, Jr, ep, outr);
     }
   }
 }

@@ -5,8 +5,26 @@
 
 #include "matvec_fused.cuh"
 #include "matvec_launch.cuh"
+#include "matvec_zpack.cuh"
 
 namespace marie {
+
+// Launches a pass as a programmatic dependent of the kernel before it (the
+// passes wait before they read anything that kernel writes).
+template <typename... P, typename... A>
+static cudaError_t launch_pass(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
 
 template <typename T> struct MatvecImpl {
   using V = cplx<T>;
@@ -14,31 +32,49 @@ template <typename T> struct MatvecImpl {
   template <int NL, int THR, typename IO>
   static cudaError_t xfwd_nt(const IO* J, long long js, const int* inv, Prologue pro, V* A, long long as,
                             const Dims& d, const V* tw, int nrhs, cudaStream_t st) {
+    if constexpr (sizeof(T) == 4) {
+      using X = XRow<NL, THR>;
+      cudaError_t e = opt_in_smem(k_xfwd_rows<NL, THR, IO>, X::bytes);
+      if (e != cudaSuccess) return e;
+      dim3 grid((d.M * d.N * 3 + X::S - 1) / X::S, nrhs);
+      return launch_pass(k_xfwd_rows<NL, THR, IO>, grid, RowCfg<V, NL, THR>::THREADS, X::bytes, st, J, js, inv, pro, A,
+                         as, d, tw);
+    } else {
     constexpr int S = RowCfg<cplx<T>, NL, THR>::S;
     const size_t smem = (size_t)(NL + NL * (S + 1)) * sizeof(V);
     cudaError_t e = opt_in_smem(k_xfwd<T, NL, THR, IO>, smem);
     if (e != cudaSuccess) return e;
     const int rows = d.M * d.N * 3;
     dim3 grid((rows + S - 1) / S, nrhs);
-    k_xfwd<T, NL, THR, IO><<<grid, RowCfg<cplx<T>, NL, THR>::THREADS, smem, st>>>(J, js, inv, pro, A, as, d, tw);
-    return cudaGetLastError();
+    return launch_pass(k_xfwd<T, NL, THR, IO>, grid, RowCfg<cplx<T>, NL, THR>::THREADS, smem, st, J, js, inv, pro, A, as,
+                       d, tw);
+    }
   }
   template <int NL, int THR, typename IO>
   static cudaError_t xinv_nt(const V* A, long long as, const IO* J, long long js, const int* inv, Epilogue ep,
                             IO* out, long long os, const Dims& d, const V* tw, int nrhs, cudaStream_t st) {
+    if constexpr (sizeof(T) == 4) {
+      using X = XRow<NL, THR>;
+      cudaError_t e = opt_in_smem(k_xinv_rows<NL, THR, IO>, X::bytes);
+      if (e != cudaSuccess) return e;
+      dim3 grid((d.M * d.N * 3 + X::S - 1) / X::S, nrhs);
+      return launch_pass(k_xinv_rows<NL, THR, IO>, grid, RowCfg<V, NL, THR>::THREADS, X::bytes, st, A, as, J, js, inv,
+                         ep, out, os, d, tw);
+    } else {
     constexpr int S = RowCfg<cplx<T>, NL, THR>::S;
     const size_t smem = (size_t)(NL + NL * (S + 1)) * sizeof(V);
     cudaError_t e = opt_in_smem(k_xinv<T, NL, THR, IO>, smem);
     if (e != cudaSuccess) return e;
     const int rows = d.M * d.N * 3;
     dim3 grid((rows + S - 1) / S, nrhs);
-    k_xinv<T, NL, THR, IO><<<grid, RowCfg<cplx<T>, NL, THR>::THREADS, smem, st>>>(A, as, J, js, inv, ep, out, os, d, tw);
-    return cudaGetLastError();
+    return launch_pass(k_xinv<T, NL, THR, IO>, grid, RowCfg<cplx<T>, NL, THR>::THREADS, smem, st, A, as, J, js, inv, ep,
+                       out, os, d, tw);
+    }
   }
   // An x pass of 256-thread CTAs is taken when it fills the chip four times over;
   // below that, CTAs of a quarter the rows spread the work over all SMs.
   // First and last pass of a 40^3 FP64 grid 46 -> 32 and 51 -> 37 us; of a 12 x 8
-  // x 20 grid, two CTAs before, 34 and 49 us to a tenth.
+  // x 20 grid, two CTAs before, 34 -> 15 and 47 -> 18 us.
   template <int NL> static bool many_rows(const Dims& d, int nrhs) {
     constexpr int S = RowCfg<cplx<T>, NL>::S;
     return ((long long)d.M * d.N * 3 + S - 1) / S * nrhs >= 4 * 152;
@@ -64,9 +100,8 @@ template <typename T> struct MatvecImpl {
     cudaError_t e = opt_in_smem(k_cols<T, NC, INV>, smem);
     if (e != cudaSuccess) return e;
     dim3 grid((Lp + S - 1) / S, nw, nrhs);
-    k_cols<T, NC, INV><<<grid, S * FFT<V, NC, INV>::T, smem, st>>>(in, in_w, in_rhs, n_in, out, out_w, out_rhs,
-                                                                  n_out, Lp, tw, stop, step);
-    return cudaGetLastError();
+    return launch_pass(k_cols<T, NC, INV>, grid, S * FFT<V, NC, INV>::T, smem, st, in, in_w, in_rhs, n_in, out, out_w,
+                       out_rhs, n_out, Lp, tw, stop, step);
   }
   template <int NZ, int KIND, int VAR>
   static cudaError_t zmul_nk(V* B, long long bs, const V* fN, int oct, const Dims& d, const V* tw, int nrhs,
@@ -84,18 +119,19 @@ template <typename T> struct MatvecImpl {
     const size_t smem = (size_t)ZC::bytes(S);  // S columns, 3 component buffers, operator tile
     cudaError_t e = opt_in_smem(k_zmul<T, NZ, KIND, VAR>, smem);
     if (e != cudaSuccess) return e;
-    // the pass waits (griddepcontrol) before reading the previous pass's output
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((d.Lp + S - 1) / S, d.Mp, nrhs);
-    cfg.blockDim = dim3(ZC::THREADS, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_zmul<T, NZ, KIND, VAR>, B, bs, fN, oct, d, tw, tmap, tma, err);
+    return launch_pass(k_zmul<T, NZ, KIND, VAR>, dim3((d.Lp + S - 1) / S, d.Mp, nrhs), ZC::THREADS, smem, st, B, bs, fN,
+                       oct, d, tw, tmap, tma, err);
+  }
+  // the z pass on column pairs (FP32, a tile by bulk copy)
+  template <int NZ>
+  static cudaError_t zmul_pairs(float2* B, long long bs, const Dims& d, const float2* tw, int nrhs, cudaStream_t st,
+                                const ZTile* zt) {
+    using Z = ZP<NZ>;
+    const int tma = take_tile_timeout_injection() ? 2 : 1;  // 2: a test, a wait that runs out
+    cudaError_t e = opt_in_smem(k_zmul_pairs<NZ>, Z::bytes);
+    if (e != cudaSuccess) return e;
+    return launch_pass(k_zmul_pairs<NZ>, dim3(d.Lp / Z::S, d.Mp, nrhs), Z::THREADS, Z::bytes, st, B, bs, d, tw, zt->map[0],
+                       tma, zt->err);
   }
   template <int NZ>
   static cudaError_t zmul_n(V* B, long long bs, const V* fN, int oct, const Dims& d, const V* tw, int nrhs,
@@ -105,6 +141,8 @@ template <typename T> struct MatvecImpl {
       if constexpr (HasWide<NZ>::value)
         if (var == 1) return zmul_nk<NZ, 0, 1>(B, bs, fN, oct, d, tw, nrhs, st, zt);
       if (var == 2) return zmul_nk<NZ, 0, 2>(B, bs, fN, oct, d, tw, nrhs, st, zt);
+      if constexpr (ZP<NZ>::ok)
+        if (oct && zt && zt->ok) return zmul_pairs<NZ>(B, bs, d, tw, nrhs, st, zt);
     }
     return zmul_nk<NZ, 0, 0>(B, bs, fN, oct, d, tw, nrhs, st, zt);
   }
@@ -161,8 +199,11 @@ template <typename T> struct MatvecImpl {
 };
 
 
-// (2L, 2M, cluster size) of the grids with fused x+y passes
-#define MARIE_FUSED_PAIRS(X) X(64, 64, 2) X(96, 96, 2) X(128, 128, 4) X(192, 192, 4) X(256, 256, 8) X(512, 384, 8)
+// (2L, 2M, cluster size) of the grids with fused x+y passes.  Only the smallest
+// of them gains (64 x 64: three launches of 37.6 us against five of 40.5 us in
+// all); the separate passes are faster from 96 x 96 on (96^3 grid: 318 us
+// against 429 us; 128^3 with every voxel a DOF 593 against 607 us).
+#define MARIE_FUSED_PAIRS(X) X(64, 64, 2)
 
 template <typename T> struct FusedImpl {
   using V = cplx<T>;

@@ -40,8 +40,8 @@ __device__ __forceinline__ bool rhs_skipped(const Dims& d, int rhs) { return d.s
 // finishes.  It loads only what that kernel cannot have written (the plan's
 // operator tile and twiddles), then waits for it to complete (pdl_wait; a
 // no-op when launched without the attribute) before reading anything else.
-// The skip mask read at the top of the z and y+x passes is written by the
-// Givens step at least two kernels earlier.  A pass signals with pdl_trigger,
+// The skip mask read at the top of the passes after the first is written by
+// the Givens step at least two kernels earlier, and the first pass has waited.  A pass signals with pdl_trigger,
 // in its last phase, that the next one may start.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -121,7 +121,7 @@ __device__ __forceinline__ void stage_twiddles(V* tw_s, const V* __restrict__ tw
 // ---------------------------------------------------------------------------
 template <typename T, int NL, int THR, typename IO>
 __global__ void __launch_bounds__(RowCfg<cplx<T>, NL, THR>::THREADS)
-k_xfwd(const IO* __restrict__ J, long long j_stride, const int* __restrict__ inv, Prologue pro,
+k_xfwd(const IO* J, long long j_stride, const int* inv, Prologue pro,
        cplx<T>* __restrict__ A, long long a_stride, Dims d, const cplx<T>* __restrict__ tw) {
   using V = cplx<T>;
   using F = FFT<V, NL, false>;
@@ -130,11 +130,15 @@ k_xfwd(const IO* __restrict__ J, long long j_stride, const int* __restrict__ inv
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V* tw_s = reinterpret_cast<V*>(smem_raw);
   V* buf = tw_s + NL;
-  if (rhs_skipped(d, blockIdx.y)) return;
   const int rows = d.M * d.N * 3;
   const int row0 = blockIdx.x * S;
-  const IO* Jr = J + blockIdx.y * j_stride;
   stage_twiddles(tw_s, tw, NL);
+  // the kernel before may have written the skip mask, the map, the factors and J
+  pdl_wait();
+  if (rhs_skipped(d, blockIdx.y)) return;
+  inv = after_wait(inv);
+  pro.pre = after_wait(pro.pre);
+  const IO* Jr = after_wait(J) + blockIdx.y * j_stride;
   // gather: x fastest across threads
   for (int i = threadIdx.x; i < S * d.L; i += blockDim.x) {
     const int s = i / d.L, x = i - s * d.L;
@@ -155,6 +159,7 @@ k_xfwd(const IO* __restrict__ J, long long j_stride, const int* __restrict__ inv
   __syncthreads();
   F::store(reg, buf + s, ES, t);
   __syncthreads();
+  pdl_trigger();
   V* Ar = A + blockIdx.y * a_stride;
   for (int i = threadIdx.x; i < S * NL; i += blockDim.x) {
     const int ss = i / NL, kx = i - ss * NL;
@@ -168,7 +173,7 @@ k_xfwd(const IO* __restrict__ J, long long j_stride, const int* __restrict__ inv
 // ---------------------------------------------------------------------------
 template <typename T, int NL, int THR, typename IO>
 __global__ void __launch_bounds__(RowCfg<cplx<T>, NL, THR>::THREADS)
-k_xinv(const cplx<T>* __restrict__ A, long long a_stride, const IO* __restrict__ J, long long j_stride,
+k_xinv(const cplx<T>* A, long long a_stride, const IO* __restrict__ J, long long j_stride,
        const int* __restrict__ inv, Epilogue ep, IO* __restrict__ out, long long o_stride, Dims d,
        const cplx<T>* __restrict__ tw) {
   using V = cplx<T>;
@@ -181,8 +186,9 @@ k_xinv(const cplx<T>* __restrict__ A, long long a_stride, const IO* __restrict__
   if (rhs_skipped(d, blockIdx.y)) return;
   const int rows = d.M * d.N * 3;
   const int row0 = blockIdx.x * S;
-  const V* Ar = A + blockIdx.y * a_stride;
   stage_twiddles(tw_s, tw, NL);
+  pdl_wait();  // A is the previous pass's output
+  const V* Ar = after_wait(A) + blockIdx.y * a_stride;
   for (int i = threadIdx.x; i < S * NL; i += blockDim.x) {
     const int s = i / NL, kx = i - s * NL;
     const int row = row0 + s;
@@ -218,6 +224,163 @@ k_xinv(const cplx<T>* __restrict__ A, long long a_stride, const IO* __restrict__
   }
 }
 
+// out[kk] = A J - B v of one row sweep: reg[i] is the circulant term at DOF
+// kk[i] (-1: none).  Per-DOF loads in groups of EPI (bounded registers).  FP64
+// vectors with FP32 coefficient copies (the matvec of the mixed-precision
+// inner solves and of FP32 products of a bound operator) run the whole epilogue
+// in FP32, the transforms' precision, with one conversion in and one out.
+// NARROW: the product B v in the transforms' precision, otherwise in the
+// vectors'.
+template <typename IO, typename V, int E, int EPI, bool NARROW>
+__device__ __forceinline__ void epilogue_dofs(const V* reg, const int* kk, const IO* Jr, const Epilogue& ep, IO* outr) {
+  constexpr bool MIX = std::is_same<IO, double2>::value && std::is_same<V, float2>::value;
+  const bool f32epi = MIX && ep.af != nullptr;
+#pragma unroll
+  for (int i0 = 0; i0 < E; i0 += EPI) {
+    IO jv[EPI], ak[EPI], bk[EPI];
+    float2 af[EPI], bf[EPI];
+#pragma unroll
+    for (int j = 0; j < EPI; ++j) {
+      const int k = kk[i0 + j];
+      if (k < 0) continue;
+      jv[j] = Jr[k];
+      if (f32epi) {
+        af[j] = ep.af[k];
+        bf[j] = ep.bf ? ep.bf[k] : mk<float2>(0, 0);
+      } else {
+        ak[j] = EpiIO<IO>::a(ep, k);
+        bk[j] = EpiIO<IO>::b(ep, k);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < EPI; ++j) {
+      const int k = kk[i0 + j];
+      if (k < 0) continue;
+      if constexpr (MIX) {
+        if (f32epi) {
+          const float2 v = reg[i0 + j];
+          float2 r32 = cmul(af[j], cvt<float2>(jv[j]));
+          if (ep.conjout) {
+            r32.x -= v.x;
+            r32.y += v.y;
+          } else {
+            r32 = csub(r32, cmul(bf[j], v));
+          }
+          outr[k] = cvt<IO>(r32);
+          continue;
+        }
+      }
+      // the diagonal Gram*Mr*J term in the vectors' precision
+      IO res = cmul(ak[j], jv[j]);
+      const IO v = cvt<IO>(reg[i0 + j]);
+      if (ep.conjout) {
+        res.x -= v.x;
+        res.y += v.y;
+      } else if constexpr (NARROW) {
+        res = csub(res, cvt<IO>(cmul(cvt<V>(bk[j]), reg[i0 + j])));
+      } else {
+        res = csub(res, cmul(bk[j], v));
+      }
+      outr[k] = res;
+    }
+  }
+}
+
+// The FP32 x passes: lanes run along a row, so the index map, the DOFs and the
+// spectrum go straight between global memory and the transform's registers
+// (16-value schedules: whole 128-byte segments per access); only the exchange
+// between its passes uses shared memory.  Staging the rows through shared
+// memory first, as the FP64 passes do (whose time is the FP64 pipe's), cost
+// two more shared round trips and three barriers per row.  Measured with every
+// voxel a DOF: first pass of a 64^3 grid 21 -> 13 us, of 96^3 60 -> 38 us; of
+// 128^3, where the vectors' own 20 bytes per DOF bound it, 96 -> 93 us.
+template <int NL, int THR> struct XRow {
+  static constexpr int T = FFT<float2, NL, false>::T;
+  static constexpr int S = RowCfg<float2, NL, THR>::S;
+  static constexpr int ROWP = NL + NL / 16;
+  static constexpr size_t bytes = (size_t)(NL + S * ROWP) * sizeof(float2);
+};
+
+template <int NL, int THR, typename IO>
+__global__ void __launch_bounds__(RowCfg<float2, NL, THR>::THREADS)
+k_xfwd_rows(const IO* J, long long j_stride, const int* inv, Prologue pro,
+            float2* __restrict__ A, long long a_stride, Dims d, const float2* __restrict__ tw) {
+  using F = FFT<float2, NL, false>;
+  using X = XRow<NL, THR>;
+  constexpr int L = NL / 2, E = F::E, R0 = F::R0, RL = F::RL;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float2* tw_s = reinterpret_cast<float2*>(smem_raw);
+  const int t = threadIdx.x % X::T, s = threadIdx.x / X::T;
+  float2* xb = tw_s + NL + s * X::ROWP;
+  const int row = blockIdx.x * X::S + s;
+  const bool valid = row < d.M * d.N * 3;
+  stage_twiddles(tw_s, tw, NL);
+  // the kernel before may have written the skip mask, the map, the factors and J
+  pdl_wait();
+  if (rhs_skipped(d, blockIdx.y)) return;
+  const int* invr = after_wait(inv) + (long long)row * L;
+  const IO* Jr = after_wait(J) + blockIdx.y * j_stride;
+  pro.pre = after_wait(pro.pre);
+  int kk[E];
+#pragma unroll
+  for (int b = 0; b < E / R0; ++b)
+#pragma unroll
+    for (int r = 0; r < R0; ++r) {
+      const int p = F::in_pos(t, b, r);
+      kk[b * R0 + r] = (valid && r < R0 / 2 && p < L) ? invr[p] : -1;
+    }
+  float2 reg[E];
+#pragma unroll
+  for (int i = 0; i < E; ++i) reg[i] = kk[i] >= 0 ? cvt<float2>(prologue_in(Jr, pro, kk[i])) : mk<float2>(0, 0);
+  __syncthreads();  // twiddles staged
+  F::run_half(reg, xb, SAddr(1, true), t, tw_s);
+  pdl_trigger();
+  if (!valid) return;
+  float2* Ar = A + blockIdx.y * a_stride + (long long)row * NL;
+#pragma unroll
+  for (int b = 0; b < E / RL; ++b)
+#pragma unroll
+    for (int r = 0; r < RL; ++r) Ar[F::out_pos(t, b, r)] = reg[b * RL + r];
+}
+
+template <int NL, int THR, typename IO>
+__global__ void __launch_bounds__(RowCfg<float2, NL, THR>::THREADS)
+k_xinv_rows(const float2* A, long long a_stride, const IO* __restrict__ J, long long j_stride,
+            const int* __restrict__ inv, Epilogue ep, IO* __restrict__ out, long long o_stride, Dims d,
+            const float2* __restrict__ tw) {
+  using F = FFT<float2, NL, true>;
+  using X = XRow<NL, THR>;
+  constexpr int L = NL / 2, E = F::E, R0 = F::R0, RL = F::RL;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float2* tw_s = reinterpret_cast<float2*>(smem_raw);
+  if (rhs_skipped(d, blockIdx.y)) return;
+  const int t = threadIdx.x % X::T, s = threadIdx.x / X::T;
+  float2* xb = tw_s + NL + s * X::ROWP;
+  const int row = blockIdx.x * X::S + s;
+  const bool valid = row < d.M * d.N * 3;
+  stage_twiddles(tw_s, tw, NL);
+  pdl_wait();  // A is the previous pass's output
+  const float2* Ar = after_wait(A) + blockIdx.y * a_stride + (long long)row * NL;
+  float2 reg[E];
+#pragma unroll
+  for (int b = 0; b < E / R0; ++b)
+#pragma unroll
+    for (int r = 0; r < R0; ++r) reg[b * R0 + r] = valid ? Ar[F::in_pos(t, b, r)] : mk<float2>(0, 0);
+  __syncthreads();  // twiddles staged
+  // the DOF indices arrive while the transform runs
+  const int* invr = inv + (long long)row * L;
+  int kk[E];
+#pragma unroll
+  for (int b = 0; b < E / RL; ++b)
+#pragma unroll
+    for (int r = 0; r < RL; ++r) {
+      const int x = F::out_pos(t, b, r);
+      kk[b * RL + r] = (valid && x < L) ? invr[x] : -1;
+    }
+  F::run(reg, xb, SAddr(1, true), t, tw_s);
+  epilogue_dofs<IO, float2, E, 2, false>(reg, kk, J + blockIdx.y * j_stride, ep, out + blockIdx.y * o_stride);
+}
+
 // ---------------------------------------------------------------------------
 // cols: transform along the middle (y) axis for S consecutive kx columns.
 //   in [kx + Lp*y + in_w*w], y < n_in      out [kx + Lp*y + out_w*w], y < n_out
@@ -231,7 +394,7 @@ template <typename T> struct ColS { static constexpr int S = 128 / (int)sizeof(c
 // exchanges go through shared memory only.
 template <typename T, int NC, bool INV>
 __global__ void __launch_bounds__(ColS<T>::S * FFT<cplx<T>, NC, INV>::T)
-k_cols(const cplx<T>* __restrict__ in, long long in_w, long long in_rhs, int n_in,
+k_cols(const cplx<T>* in, long long in_w, long long in_rhs, int n_in,
        cplx<T>* __restrict__ out, long long out_w, long long out_rhs, int n_out, int Lp,
        const cplx<T>* __restrict__ tw, const int* __restrict__ stop, int step) {
   if (stop && stop[blockIdx.z] < step) return;
@@ -245,9 +408,10 @@ k_cols(const cplx<T>* __restrict__ in, long long in_w, long long in_rhs, int n_i
   V* buf = tw_s + NC;
   const int kx0 = blockIdx.x * S;
   const long long w = blockIdx.y;
-  const V* inp = in + blockIdx.z * in_rhs + w * in_w + kx0;
   V* outp = out + blockIdx.z * out_rhs + w * out_w + kx0;
   stage_twiddles(tw_s, tw, NC);
+  pdl_wait();  // the input is the previous pass's output (its skip mask is older)
+  const V* inp = after_wait(in) + blockIdx.z * in_rhs + w * in_w + kx0;
   const int s = threadIdx.x % S, t = threadIdx.x / S;
   const bool active = kx0 + s < Lp;
   const bool half = !INV && 2 * n_in <= NC;
@@ -269,6 +433,7 @@ k_cols(const cplx<T>* __restrict__ in, long long in_w, long long in_rhs, int n_i
   } else {
     F::run(reg, buf + s, ES, t, tw_s);
   }
+  pdl_trigger();
 #pragma unroll
   for (int b = 0; b < E / RL; ++b)
 #pragma unroll
@@ -373,13 +538,25 @@ template <typename V> __device__ __forceinline__ V cfma(V a, V b, V c) {
   return mk<V>(fma(-a.y, b.y, fma(a.x, b.x, c.x)), fma(a.y, b.x, fma(a.x, b.y, c.y)));
 }
 
+// Column s of a tile row: as it stands, or (pairs, the bulk copy's FP32 tile)
+// from {re, re, im, im} of the column and its neighbour.
+template <typename V> __device__ __forceinline__ V tile_at(const V* tile, int row, int s, bool pairs) {
+  if constexpr (sizeof(V) == 8) {
+    if (pairs) {
+      const float* p = reinterpret_cast<const float*>(tile + row + (s & ~1)) + (s & 1);
+      return mk<V>(p[0], p[2]);
+    }
+  }
+  return tile[row + s];
+}
+
 // Row C of the product at this thread's output positions of the forward
 // transform.  With the octant operator the tile already carries the x and y
 // reflection signs; the z reflection (positions kz > NZ/2) flips the two
 // z-odd components.  Without it the full operator is read from global memory.
 template <int C, typename FF, typename V, int NZ, int S>
-__device__ __forceinline__ void zrow(V* reg, int t, int s, bool active, int oct, const V* tile, const V* fp,
-                                     long long fq, long long fplane, const V* b0, const V* b1, const V* b2,
+__device__ __forceinline__ void zrow(V* reg, int t, int s, bool active, int oct, bool pairs, const V* tile,
+                                     const V* fp, long long fq, long long fplane, const V* b0, const V* b1, const V* b2,
                                      SAddr ad) {
   using RW = ZRow<C>;
   constexpr int NH = NZ / 2, NO = NH + 1, RL = FF::RL;
@@ -394,9 +571,9 @@ __device__ __forceinline__ void zrow(V* reg, int t, int s, bool active, int oct,
         if (oct) {
           const bool fz = kz > NH;
           const int oz = fz ? NZ - kz : kz;
-          n0 = tile[(RW::q0 * NO + oz) * S + s];
-          n1 = tile[(RW::q1 * NO + oz) * S + s];
-          n2 = tile[(RW::q2 * NO + oz) * S + s];
+          n0 = tile_at(tile, (RW::q0 * NO + oz) * S, s, pairs);
+          n1 = tile_at(tile, (RW::q1 * NO + oz) * S, s, pairs);
+          n2 = tile_at(tile, (RW::q2 * NO + oz) * S, s, pairs);
           if constexpr (odd_z(RW::q0)) n0 = neg_if(n0, fz);
           if constexpr (odd_z(RW::q1)) n1 = neg_if(n1, fz);
           if constexpr (odd_z(RW::q2)) n2 = neg_if(n2, fz);
@@ -418,8 +595,8 @@ __device__ __forceinline__ void zrow(V* reg, int t, int s, bool active, int oct,
 // each cost a whole warp's issue slots (FP64: 16 cycles per instruction).
 // z pass of a 40^3 FP64 grid (80 points, with the 8-column tiles): 299 -> 185 us.
 template <typename FF, typename V, int NZ, int S>
-__device__ __forceinline__ void zrow_any(V* reg, int c, int t, int s, bool active, int oct, const V* tile, const V* fp,
-                                         long long fq, long long fplane, const V* b0, const V* b1, const V* b2,
+__device__ __forceinline__ void zrow_any(V* reg, int c, int t, int s, bool active, int oct, bool pairs,
+                                         const V* tile, const V* fp, long long fq, long long fplane, const V* b0, const V* b1, const V* b2,
                                          SAddr ad) {
   constexpr int NH = NZ / 2, NO = NH + 1, RL = FF::RL;
   const int q0 = c, q1 = c == 0 ? 1 : c + 2, q2 = c == 0 ? 2 : c + 3;  // ZRow<c>
@@ -434,9 +611,9 @@ __device__ __forceinline__ void zrow_any(V* reg, int c, int t, int s, bool activ
         if (oct) {
           const bool fz = kz > NH;
           const int oz = fz ? NZ - kz : kz;
-          n0 = neg_if(tile[(q0 * NO + oz) * S + s], fz && q0 == 2);
-          n1 = neg_if(tile[(q1 * NO + oz) * S + s], fz && q1 == 4);
-          n2 = neg_if(tile[(q2 * NO + oz) * S + s], fz && q2 != 5);
+          n0 = neg_if(tile_at(tile, (q0 * NO + oz) * S, s, pairs), fz && q0 == 2);
+          n1 = neg_if(tile_at(tile, (q1 * NO + oz) * S, s, pairs), fz && q1 == 4);
+          n2 = neg_if(tile_at(tile, (q2 * NO + oz) * S, s, pairs), fz && q2 != 5);
         } else {
           const long long o = (long long)kz * fplane;
           n0 = fp[q0 * fq + o];
@@ -663,14 +840,14 @@ k_zmul(cplx<T>* __restrict__ B, long long b_rhs, const cplx<T>* __restrict__ fN,
   const V* b1 = buf + BUF + s;
   const V* b2 = buf + 2 * BUF + s;
   if constexpr (KIND == 0 && !ZC::UNIFORM) {
-    zrow_any<FF, V, NZ, S>(reg, c, t, s, active, oct, tile, fp, fq, fplane, b0, b1, b2, ad);
+    zrow_any<FF, V, NZ, S>(reg, c, t, s, active, oct, bulk, tile, fp, fq, fplane, b0, b1, b2, ad);
   } else if constexpr (KIND == 0) {
     if (c == 0)
-      zrow<0, FF, V, NZ, S>(reg, t, s, active, oct, tile, fp, fq, fplane, b0, b1, b2, ad);
+      zrow<0, FF, V, NZ, S>(reg, t, s, active, oct, bulk, tile, fp, fq, fplane, b0, b1, b2, ad);
     else if (c == 1)
-      zrow<1, FF, V, NZ, S>(reg, t, s, active, oct, tile, fp, fq, fplane, b0, b1, b2, ad);
+      zrow<1, FF, V, NZ, S>(reg, t, s, active, oct, bulk, tile, fp, fq, fplane, b0, b1, b2, ad);
     else
-      zrow<2, FF, V, NZ, S>(reg, t, s, active, oct, tile, fp, fq, fplane, b0, b1, b2, ad);
+      zrow<2, FF, V, NZ, S>(reg, t, s, active, oct, bulk, tile, fp, fq, fplane, b0, b1, b2, ad);
   } else {
     const V* bc[3] = {b0, b1, b2};
     if (c == 0)
