@@ -253,19 +253,17 @@ __global__ void k_tune_fill(double2* __restrict__ J, int* __restrict__ inv, long
 int build_inverse_index(marie_plan* p, const int64_t* idx_dev, long long n, int* inv) {
   const long long n3V = 3 * p->d.V;
   if (n < 0 || n > n3V) return set_error(MARIE_EINVAL, "n_idx = %lld outside [0, 3*L*M*N = %lld]", n, n3V);
-  DBuf err;
-  MARIE_TRY(err.alloc(sizeof(int), p->stream));
-  MARIE_CUDA_TRY(cudaMemsetAsync(err.p, 0, sizeof(int), p->stream));
-  k_fill_int<<<grid_for(n3V), 256, 0, p->stream>>>(inv, n3V, -1);
-  count_launch();
+  int* err = p->kerr + 1;
+  MARIE_CUDA_TRY(cudaMemsetAsync(inv, 0xff, n3V * sizeof(int), p->stream));
   if (n > 0) {
-    k_scatter_inverse<<<grid_for(n), 256, 0, p->stream>>>(idx_dev, n, n3V, inv, err.as<int>());
+    k_scatter_inverse<<<grid_for(n), 256, 0, p->stream>>>(idx_dev, n, n3V, inv, err);
     count_launch();
   }
   MARIE_CUDA_TRY(cudaGetLastError());
   int herr = 0;
-  MARIE_CUDA_TRY(cudaMemcpyAsync(&herr, err.p, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
+  MARIE_CUDA_TRY(cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
   MARIE_CUDA_TRY(cudaStreamSynchronize(p->stream));
+  if (herr) MARIE_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), p->stream));
   if (herr & 1) return set_error(MARIE_EINVAL, "idx entry outside [1, 3*L*M*N]");
   if (herr & 2) return set_error(MARIE_EINVAL, "idx has repeated entries");
   return MARIE_OK;
@@ -783,7 +781,8 @@ int marie_plan_create(int64_t L, int64_t M, int64_t N, int precision, int64_t nr
     }
     p->own_stream = true;
   }
-  if (cudaMalloc(&p->kerr, sizeof(int)) != cudaSuccess || cudaMemset(p->kerr, 0, sizeof(int)) != cudaSuccess) {
+  if (cudaMalloc(&p->kerr, 2 * sizeof(int)) != cudaSuccess ||
+      cudaMemset(p->kerr, 0, 2 * sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
     marie_plan_destroy(p);
     return set_error(MARIE_ENOMEM, "plan status word allocation failed");
@@ -1141,8 +1140,7 @@ int marie_mv_AN(marie_plan* p, const double* JIn0, const double* Mr, const doubl
   if (n > 0)
     MARIE_TRY(run_matvec(p, precision, (const double2*)J_d, (double2*)out_d, n, (int)nrhs, inv.as<int>(), pro, ep));
   MARIE_TRY(finish_out(JOut, out_d, n * nrhs * sizeof(double2), p->stream));
-  MARIE_CUDA_TRY(cudaStreamSynchronize(p->stream));
-  return check_kernel_status(p);
+  return check_kernel_status(p);  // (synchronises)
 }
 
 int marie_plan_apply_mv_AN(marie_plan* p, const double* JIn0, double* JOut, int64_t nrhs, int precision) {
@@ -1204,8 +1202,7 @@ int marie_mv_L(marie_plan* p, const double* JIn0, double Gram, const int64_t* id
   if (n > 0)
     MARIE_TRY(run_matvec(p, precision, (const double2*)J_d, (double2*)out_d, n, (int)nrhs, inv.as<int>(), pro, ep));
   MARIE_TRY(finish_out(JOut, out_d, n * nrhs * sizeof(double2), p->stream));
-  MARIE_CUDA_TRY(cudaStreamSynchronize(p->stream));
-  return check_kernel_status(p);
+  return check_kernel_status(p);  // (synchronises)
 }
 
 int marie_mv_K(marie_plan* p, const double* JIn0, const int64_t* idx, int64_t n_idx, double* JOut, int64_t nrhs,

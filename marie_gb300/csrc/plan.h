@@ -39,8 +39,9 @@ struct marie_plan {
   // circulant parity symmetry and N + 1 <= 256.
   float2* fN32x = nullptr;
   marie::ZTile zt{};
-  // Device status word of the kernels' bounded waits (1: a tile copy did not
-  // arrive in time); read and cleared by check_kernel_status.
+  // Device status words: the kernels' bounded waits (1: a tile copy did not
+  // arrive in time), read and cleared by check_kernel_status, and the entries
+  // that build_inverse_index rejected, read and cleared by it.
   int* kerr = nullptr;
 
   // K operator (mv_K, H_field_Kop), same scaling and layouts with 3 components.

@@ -78,6 +78,12 @@ def _colmajor_cuda(t, dtype):
     t = t.to(dtype)
     if t.dim() <= 1:
         return t.contiguous()
+    step, ordered = 1, True
+    for n, st in zip(t.shape, t.stride()):
+        ordered = ordered and (n == 1 or st == step)
+        step *= n
+    if ordered:
+        return t
     rev = list(range(t.dim() - 1, -1, -1))
     return t.permute(*rev).contiguous().permute(*rev)
 
@@ -100,6 +106,11 @@ def _out(shape, like_cuda: bool, dtype=np.complex128):
         return C.c_void_p(t.data_ptr()), t
     arr = np.empty(shape, dtype=dtype, order="F")
     return C.c_void_p(arr.ctypes.data), arr
+
+
+def _any_nonzero(a) -> bool:
+    """np.any(a), where a lives: a CUDA tensor is not brought to the host."""
+    return bool(a.ne(0).any()) if _is_cuda(a) else bool(np.any(np.asarray(a)))
 
 
 def release_cached_memory():
@@ -427,7 +438,7 @@ def H_field_Kop(J, fK, Gram, Hinc=None, GPU_flag=1, precision="fp64"):
     """H_field_Kop.m:46-77: Htot = Hinc + mv_K(J) / Gram."""
     opr, tmp = _k_operator_for(fK, "fp64")
     try:
-        if Hinc is not None and not np.any(np.asarray(J.cpu() if _is_cuda(J) else J)):
+        if Hinc is not None and not _any_nonzero(J):
             return Hinc
         jp, jk = _in(J)
         hp, hk = _in(Hinc) if Hinc is not None else (None, None)
@@ -443,7 +454,7 @@ def E_field_Nop(J, fN, Gram, freq, Einc=None, GPU_flag=1, precision="fp64"):
     """E_field_Nop.m:59-84: Etot = Einc + (N J - Gram J)/(Gram j omega eps0)."""
     opr, tmp = _operator_for(fN, "fp64")
     try:
-        if Einc is not None and not np.any(np.asarray(J.cpu() if _is_cuda(J) else J)):
+        if Einc is not None and not _any_nonzero(J):
             return Einc
         jp, jk = _in(J)
         if Einc is not None:
