@@ -60,6 +60,13 @@ __device__ __forceinline__ double bi_wsum(double v) {
   return v;
 }
 
+// the eight warps' sums in three dependent additions (an FP64 addition that
+// waits for another costs some hundred cycles)
+static_assert(BI_THREADS == 256, "eight warps");
+__device__ __forceinline__ double bi_sum8(const double* w) {
+  return ((w[0] + w[1]) + (w[2] + w[3])) + ((w[4] + w[5]) + (w[6] + w[7]));
+}
+
 // conj(a) * b accumulated into (re, im)
 __device__ __forceinline__ void dotc(double2 a, double2 b, double& re, double& im) {
   re = fma(a.x, b.x, fma(a.y, b.y, re));
@@ -133,9 +140,7 @@ __global__ void __launch_bounds__(BI_THREADS) k_bi(BiVec a, double* __restrict__
     }
     __syncthreads();
     if (threadIdx.x < NQ) {
-      double s = 0;
-      for (int w = 0; w < BI_THREADS / 32; ++w) s += ws[threadIdx.x][w];
-      part[(long long)threadIdx.x * gridDim.x + blockIdx.x] = s;
+      part[(long long)threadIdx.x * gridDim.x + blockIdx.x] = bi_sum8(ws[threadIdx.x]);
     }
   }
 }
@@ -149,11 +154,7 @@ __global__ void k_bi_fin(const double* __restrict__ part, int G, double* __restr
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (lane == 0) ws[wid] = s;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += ws[w];
-    out[blockIdx.x] = t;
-  }
+  if (threadIdx.x == 0) out[blockIdx.x] = bi_sum8(ws);
 }
 
 namespace {

@@ -39,15 +39,14 @@ static constexpr int BG = 152 * 2;
 // basis at HBM speed rather than at the FP64 rate, so they want more loads in
 // flight (four blocks per SM)
 static constexpr int BG32 = 152 * 4;
-// Smaller systems take fewer row blocks (counts that depend on the rows alone).
-// The dots: one block per SM and column group up to 4096 rows per block, whose
-// sums within a block stay a small share of its work.  The update: one row per
-// thread, so one round of loads, up to 2 BG blocks.
+// The dots of smaller systems: one block per SM and column group up to 4096 rows
+// per block (a count that depends on the rows alone), whose sums within a block
+// stay a small share of its work.  The update keeps its blocks, two per SM at
+// any size: fewer would leave some SMs' FP64 pipe twice the work of others.
 static int dot_blocks(long long rows, int most) { return rows <= 4096LL * 152 ? 152 : most; }
-static int update_blocks(long long rows, int most) {
-  return rows <= 512LL * BG ? (int)std::max<long long>(1, (rows + 255) / 256) : most;
-}
 static constexpr int BT = 256;
+// partials per lane loaded at once by a last block: BG blocks, 152 blocks in one round
+static constexpr int TAIL = 10, DTAIL = 5;
 
 __device__ __forceinline__ double2 wsum2(double2 v) {
 #pragma unroll
@@ -62,20 +61,27 @@ __device__ __forceinline__ double wsum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-// block sum, valid in thread 0
-__device__ double2 bsum2(double2 v) {
-  __shared__ double2 ws[32];
-  v = wsum2(v);
+// Sum of N values by halves: log2 N dependent additions.  An FP64 addition that
+// waits for the one before it costs some hundred cycles here (the pipe is two
+// lanes wide), so the short sums that end a step are trees, not chains.
+template <int N, typename V> __device__ __forceinline__ V tree_sum(const V* v) {
+  if constexpr (N == 1) {
+    return v[0];
+  } else {
+    const V a = tree_sum<N / 2>(v), b = tree_sum<N - N / 2>(v + N / 2);
+    if constexpr (std::is_same<V, double>::value) return a + b;
+    else return cadd(a, b);
+  }
+}
+// block sum of BT threads, valid in thread 0
+__device__ double bsum(double v) {
+  __shared__ double ws[BT / 32];
+  v = wsum(v);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   __syncthreads();
   if (lane == 0) ws[wid] = v;
   __syncthreads();
-  double2 r = mk<double2>(0, 0);
-  if (wid == 0) {
-    r = lane < (int)(blockDim.x >> 5) ? ws[lane] : mk<double2>(0, 0);
-    r = wsum2(r);
-  }
-  return r;
+  return threadIdx.x == 0 ? tree_sum<BT / 32>(ws) : 0.0;
 }
 __device__ __forceinline__ void rows_of(long long n, long long& i0, long long& i1) {
   const long long chunk = (n + gridDim.x - 1) / gridDim.x;
@@ -99,8 +105,8 @@ __global__ void __launch_bounds__(BT) kb_norm_part(const double2* __restrict__ X
     const double2 v = x[i];
     a = fma(v.x, v.x, fma(v.y, v.y, a));
   }
-  const double2 r = bsum2(mk<double2>(a, 0));
-  if (threadIdx.x == 0) part[(long long)s * gridDim.x + blockIdx.x] = r.x;
+  const double r = bsum(a);
+  if (threadIdx.x == 0) part[(long long)s * gridDim.x + blockIdx.x] = r;
 }
 
 // norm[s] = sqrt(sum of partials), fixed order
@@ -109,7 +115,15 @@ __global__ void kb_norm_fin(const double* __restrict__ part, int G, const int* _
   const int s = blockIdx.x;
   if (stop && skip(stop, s, step)) return;
   double a = 0;
-  for (int b = threadIdx.x; b < G; b += 32) a += part[(long long)s * G + b];
+  for (int b0 = 0; b0 < G; b0 += 32 * TAIL) {
+    double v[TAIL];
+#pragma unroll
+    for (int i = 0; i < TAIL; ++i) {
+      const int b = b0 + threadIdx.x + 32 * i;
+      v[i] = b < G ? part[(long long)s * G + b] : 0.0;
+    }
+    a += tree_sum<TAIL>(v);
+  }
   a = wsum(a);
   if (threadIdx.x == 0) out[s] = sqrt(a);
 }
@@ -215,8 +229,8 @@ template <int NV, typename T> __device__ __forceinline__ void warp_sums(T* a) {
 
 // The block's rows of NC basis columns (units of U, column stride nu): partial
 // sums of conj(V(:,j)) w for j = c0 .. c0 + NC - 1, summed within warps (FP32
-// lanes in FP32, then FP64), then the warps' partials in warp order by one
-// thread per value: a fixed order.
+// lanes in FP32, then FP64), then the warps' partials by one thread per value:
+// a fixed order.
 template <int NC, typename VB>
 __device__ __forceinline__ void kb_dot_cols(const typename BUnit<VB>::U* __restrict__ V,
                                             const typename BUnit<VB>::U* __restrict__ w, long long nu, long long i0,
@@ -245,8 +259,10 @@ __device__ __forceinline__ void kb_dot_cols(const typename BUnit<VB>::U* __restr
   if (lane % REP == 0) red[wid][lane / REP] = (double)a[0];
   __syncthreads();
   if (threadIdx.x < 2 * NC) {
-    double r = red[0][threadIdx.x];
-    for (int w2 = 1; w2 < BT / 32; ++w2) r += red[w2][threadIdx.x];
+    double v[BT / 32];
+#pragma unroll
+    for (int w2 = 0; w2 < BT / 32; ++w2) v[w2] = red[w2][threadIdx.x];
+    const double r = tree_sum<BT / 32>(v);
     // part[column][block] as (re, im)
     part[((long long)(threadIdx.x >> 1) * gridDim.x + blockIdx.x) * 2 + (threadIdx.x & 1)] = r;
   }
@@ -293,12 +309,27 @@ __global__ void __launch_bounds__(BT) kb_dots(const VB* __restrict__ Vb, long lo
   }
   // h[s][j] = sum_b part[s][j][b] by the last block, one warp per column
   if (!last_block(cnt + s, gridDim.x * gridDim.y)) return;
+  // (two columns per warp at once, all of a lane's loads in flight together)
   const int G = gridDim.x, lane = threadIdx.x & 31;
-  for (int j = threadIdx.x >> 5; j < k; j += BT / 32) {
-    double2 a = mk<double2>(0, 0);
-    for (int b = lane; b < G; b += 32) a = cadd(a, __ldcg(part_s + (long long)j * G + b));
-    a = wsum2(a);
-    if (lane == 0) h[(long long)s * hld + j] = a;
+  for (int j0 = 2 * (threadIdx.x >> 5); j0 < k; j0 += 2 * (BT / 32)) {
+    const double2* p0 = part_s + (long long)j0 * G;
+    const double2* p1 = j0 + 1 < k ? p0 + G : p0;
+    double2 sum0 = mk<double2>(0, 0), sum1 = sum0;
+    for (int b0 = lane; b0 < G; b0 += 32 * DTAIL) {
+      double2 v0[DTAIL], v1[DTAIL];
+#pragma unroll
+      for (int i = 0; i < DTAIL; ++i) {
+        const bool in = b0 + 32 * i < G;
+        v0[i] = in ? __ldcg(p0 + b0 + 32 * i) : mk<double2>(0, 0);
+        v1[i] = in ? __ldcg(p1 + b0 + 32 * i) : mk<double2>(0, 0);
+      }
+      sum0 = cadd(sum0, tree_sum<DTAIL>(v0));
+      sum1 = cadd(sum1, tree_sum<DTAIL>(v1));
+    }
+    double a[4] = {sum0.x, sum0.y, sum1.x, sum1.y};
+    warp_sums<4>(a);
+    const int j = j0 + (lane >> 4);
+    if ((lane & 7) == 0 && j < k) reinterpret_cast<double*>(h + (long long)s * hld + j)[(lane >> 3) & 1] = a[0];
   }
 }
 
@@ -343,41 +374,70 @@ __device__ void givens_warp(const GState& G, int m, int k, const double2* __rest
   __shared__ double2 col_s[128], sn_s[128];
   __shared__ double cs_s[128];
   const int kk = k - 1;
+  // every load of the step at once: the partial norms, the previous step's
+  // residual (|g(k-1)|), the tolerance, then the column and the rotations
+  const double before = k == 1 ? G.beta[s] : G.resv[(long long)s * m + kk - 1];
+  const double tolabs = G.tolabs[s];
+  const double2 gk0 = k == 1 ? mk<double2>(G.beta[s], 0) : g[kk];
   double nn = 0;
-#pragma unroll 4
-  for (int b = lane; b < NB; b += 32) nn += __ldcg(npart + (long long)s * NB + b);
+  for (int b0 = 0; b0 < NB; b0 += 32 * TAIL) {
+    double v[TAIL];
+#pragma unroll
+    for (int i = 0; i < TAIL; ++i) {
+      const int b = b0 + lane + 32 * i;
+      v[i] = b < NB ? __ldcg(npart + (long long)s * NB + b) : 0.0;
+    }
+    if (b0 == 0) {
+      for (int i = lane; i < k; i += 32) {
+        const double2 hv = h[(long long)s * hld + i];
+        H[kk * ld + i] = hv;
+        col_s[i] = hv;
+      }
+      for (int i = lane; i < kk; i += 32) {
+        cs_s[i] = cs[i];
+        sn_s[i] = sn[i];
+      }
+    }
+    nn += tree_sum<TAIL>(v);
+  }
   nn = wsum(nn);
   // the norms and the rotation from reciprocal square roots: a step's end is
   // one thread's chain of FP64 operations, and hypot and division are the
   // longest of them
   const double hnv = nn > 0 ? nn * rsqrt(nn) : sqrt(nn);
-  for (int i = lane; i < k; i += 32) {
-    const double2 v = h[(long long)s * hld + i];
-    H[kk * ld + i] = v;
-    col_s[i] = v;
-  }
-  for (int i = lane; i < kk; i += 32) {
-    cs_s[i] = cs[i];
-    sn_s[i] = sn[i];
-  }
-  if (lane == 0) {
-    H[kk * ld + k] = mk<double2>(hnv, 0);
-    if (k == 1) g[0] = mk<double2>(G.beta[s], 0);
-  }
+  if (lane == 0) H[kk * ld + k] = mk<double2>(hnv, 0);
   __syncwarp();
+  // The previous rotations: a(i+1) = -conj(s_i) a(i) + c_i b_i with b_i the
+  // column's entry i + 1, and the rotated entry i is c_i a(i) + s_i b_i.  The
+  // recurrence is a chain of affine maps, composed over the lanes in five steps
+  // (32 maps a round) instead of one after the other (a chain of two dependent
+  // FMAs per rotation took 0.35 us each).
+  double2* col = R + kk * ld;
+  double2 a = col_s[0];
+  for (int i0 = 0; i0 < kk; i0 += 32) {
+    const int i = i0 + lane;
+    const bool on = i < kk;
+    const double c = on ? cs_s[i] : 0.0;
+    const double2 sv = on ? sn_s[i] : mk<double2>(0, 0), b = on ? col_s[i + 1] : mk<double2>(0, 0);
+    double2 A = on ? mk<double2>(-sv.x, sv.y) : mk<double2>(1.0, 0.0);  // x -> A x + B
+    double2 B = cscale(b, c);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double2 Ap = mk<double2>(__shfl_up_sync(0xffffffffu, A.x, o), __shfl_up_sync(0xffffffffu, A.y, o));
+      const double2 Bp = mk<double2>(__shfl_up_sync(0xffffffffu, B.x, o), __shfl_up_sync(0xffffffffu, B.y, o));
+      if (lane >= o) {
+        B = cfma(A, Bp, B);
+        A = cmul(A, Ap);
+      }
+    }
+    const double2 after = cfma(A, a, B);  // a(i + 1)
+    double2 here = mk<double2>(__shfl_up_sync(0xffffffffu, after.x, 1), __shfl_up_sync(0xffffffffu, after.y, 1));
+    if (lane == 0) here = a;
+    if (on) col[i] = cfma(sv, b, cscale(here, c));
+    a = mk<double2>(__shfl_sync(0xffffffffu, after.x, 31), __shfl_sync(0xffffffffu, after.y, 31));
+  }
   double rn = 0;
   if (lane == 0) {
-    double2* col = R + kk * ld;
-    // the rotated entry i+1 is carried in a register along the chain
-    double2 a = col_s[0];
-    for (int i = 0; i < kk; ++i) {
-      const double2 b = col_s[i + 1];
-      const double c = cs_s[i];
-      const double2 sv = sn_s[i];
-      col[i] = cadd(cscale(a, c), cmul(sv, b));
-      // -conj(s) a + c b, two dependent FMAs per component
-      a = mk<double2>(fma(-a.y, sv.y, fma(-a.x, sv.x, b.x * c)), fma(a.x, sv.y, fma(-a.y, sv.x, b.y * c)));
-    }
     const double a2 = a.x * a.x + a.y * a.y;
     double c, sa;
     double2 sv;
@@ -397,36 +457,68 @@ __device__ void givens_warp(const GState& G, int m, int k, const double2* __rest
     col[k] = mk<double2>(0, 0);
     cs[kk] = c;
     sn[kk] = sv;
-    const double2 gk = g[kk];
+    const double2 gk = gk0;
     g[kk] = cscale(gk, c);
     g[k] = mk<double2>(-(sv.x * gk.x + sv.y * gk.y), -(sv.x * gk.y - sv.y * gk.x));  // -conj(s) g
-    rn = sa * (k == 1 ? G.beta[s] : G.resv[(long long)s * m + kk - 1]);  // |g(k)| = |s| |g(k-1)|
+    rn = sa * before;  // |g(k)| = |s| |g(k-1)|
     G.resv[(long long)s * m + kk] = rn;
     G.hn[s] = hnv;
   }
   rn = __shfl_sync(0xffffffffu, rn, 0);
-  if (!(rn < G.tolabs[s] || k == m)) return;
+  if (!(rn < tolabs || k == m)) return;
   __syncwarp();
-  // back-substitution y = R(0:k,0:k) \ g(0:k)
-  for (int i = k - 1; i >= 0; --i) {
-    double2 p = mk<double2>(0, 0);
-    for (int j = i + 1 + lane; j < k; j += 32) p = cadd(p, cmul(R[j * ld + i], y[j]));
-    p = wsum2(p);
-    if (lane == 0) y[i] = cdiv(csub(g[i], p), R[i * ld + i]);
-    __syncwarp();
+  // back-substitution y = R(0:k,0:k) \ g(0:k): a lane holds the right-hand
+  // sides of rows lane, lane + 32, ...; each solved entry is broadcast and taken
+  // off the rows above it
+  double2 gl[4], yl[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int i = lane + 32 * q;
+    gl[q] = i < k ? g[i] : mk<double2>(0, 0);
+    yl[q] = i < k ? R[i * ld + i] : mk<double2>(1.0, 0.0);
+    yl[q] = cdiv(mk<double2>(1.0, 0.0), yl[q]);  // 1 / R(i, i) until the entry is solved
   }
+  for (int i = k - 1; i >= 0; --i) {
+    const int q = i >> 5, src = i & 31;
+    double2 v = mk<double2>(0, 0);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (u == q) {
+        v = cmul(gl[u], yl[u]);
+        if (lane == src) yl[u] = v;
+      }
+    v = mk<double2>(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+    if (lane == 0) y[i] = v;
+    const double2* Ri = R + (long long)i * ld;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int r = lane + 32 * u;
+      if (r < i) gl[u] = csub(gl[u], cmul(Ri[r], v));
+    }
+  }
+  __syncwarp();
   // res = rhs - Hc y with rhs = [beta; 0], Hc = H(0:k+1, 0:k)
   for (int i = lane; i <= k; i += 32) {
-    double2 v = i == 0 ? mk<double2>(G.beta[s], 0) : mk<double2>(0, 0);
-    for (int j = (i > 0 ? i - 1 : 0); j < k; ++j) v = csub(v, cmul(H[j * ld + i], y[j]));
-    res[i] = v;
+    double2 v[4] = {i == 0 ? mk<double2>(G.beta[s], 0) : mk<double2>(0, 0), mk<double2>(0, 0), mk<double2>(0, 0),
+                    mk<double2>(0, 0)};
+    for (int j0 = i > 0 ? i - 1 : 0; j0 < k; j0 += 4) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (j0 + u < k) v[u] = csub(v[u], cmul(H[(j0 + u) * ld + i], y[j0 + u]));
+    }
+    res[i] = tree_sum<4>(v);
   }
   if (lane == 0) G.stop[s] = k;
 }
 // w_s -= V_s(:,0:k) h_s with w_s = V_s(:,k) ; partial norms of the new w_s,
 // then the Givens step of the system (givens_warp) by the last block
+// FP64-pipe bound at large n (4 FMAs per element and column); at 40k to 170k
+// rows the step's end counts as much, hence givens_warp's short chains: 42k
+// rows and 19 columns 25.8 -> 18.6 us, 170k rows and 40 columns 84 -> 68 us.
+// Five blocks per SM: the end's registers would otherwise leave three, which
+// batches feel (1.5 %).
 template <typename VB>
-__global__ void __launch_bounds__(BT) kb_update(VB* __restrict__ Vb, long long vs, long long ld, int k,
+__global__ void __launch_bounds__(BT, 5) kb_update(VB* __restrict__ Vb, long long vs, long long ld, int k,
                                                 const double2* __restrict__ h, int hld,
                                                 const int* __restrict__ stop, double* __restrict__ part,
                                                 unsigned* __restrict__ cnt, GState G, int m) {
@@ -451,8 +543,8 @@ __global__ void __launch_bounds__(BT) kb_update(VB* __restrict__ Vb, long long v
     w[i] = v;
     a = BU::norm2(v, a);
   }
-  const double2 r = bsum2(mk<double2>((double)a, 0));
-  if (threadIdx.x == 0) part[(long long)s * gridDim.x + blockIdx.x] = r.x;
+  const double r = bsum((double)a);
+  if (threadIdx.x == 0) part[(long long)s * gridDim.x + blockIdx.x] = r;
   if (!last_block(cnt + s, gridDim.x)) return;
   if (threadIdx.x < 32) givens_warp(G, m, k, h, hld, part, gridDim.x, s, threadIdx.x);
 }
@@ -618,7 +710,7 @@ struct BatchWork {
     MARIE_TRY(t2.alloc((size_t)S * n * sizeof(double2), st));
     const long long rows = f32 ? ld / 2 : ld;
     bd = dot_blocks(rows, f32 ? BG32 : BG);
-    bu = update_blocks(rows, f32 ? BG32 : BG);
+    bu = f32 ? BG32 : BG;
     MARIE_TRY(part_d.alloc((size_t)S * 128 * bd * sizeof(double2), st));
     MARIE_TRY(part_n.alloc((size_t)S * std::max(bu, BG) * sizeof(double), st));
     MARIE_TRY(h.alloc((size_t)S * (m + 1) * sizeof(double2), st));

@@ -81,6 +81,29 @@ def test_jvie_solver_matches_oracle(form, precond):
     assert np.max(np.abs(out[0] - ref[0])) < 1e-8 * np.max(np.abs(ref[0]))
 
 
+@pytest.mark.parametrize("restart", [31, 33, 65, 127])
+def test_rotations_and_back_substitution_past_a_warp(restart):
+    """The Givens step composes the previous rotations over 32 lanes a round
+    and the back-substitution holds up to four rows a lane: restarts around and
+    past 32 and 64 against the oracle, on a sphere that takes over 65 steps and
+    is far from exhausting its Krylov space (an operator perturbed by 2e-15
+    moves the oracle's residuals by at most 8e-11 and its fields by 2e-13:
+    1e-8 and 1e-10 here, and the last estimate equals the true residual to the
+    same digits)."""
+    import marie_gb300 as mg
+
+    L, dx = 12, 5e-3
+    r, er, E = sphere_problem(L, dx, 0.028, eps_r=3000.0, sigma=0.02)
+    fN = vo.getOPERATORS(r, FREQ)
+    kw = dict(tol=1e-6, inner_it=restart, solver="G")
+    ref = vo.JVIE_Solver(E, er, r, FREQ, fN, **kw)
+    out = mg.JVIE_Solver(E, er, r, FREQ, mg.Operator.from_array(fN), **kw)
+    assert out[1] == ref[1] == 0 and out[3] == ref[3] and len(ref[4]) > 65
+    np.testing.assert_allclose(out[4], ref[4], rtol=1e-8)
+    assert abs(out[4][-1] / out[2] - 1) < 1e-8
+    assert np.max(np.abs(out[0] - ref[0])) < 1e-10 * np.max(np.abs(ref[0]))
+
+
 def test_restart_cycles_run_in_one_graph_launch():
     """After the first restart cycle, the remaining cycles of a GMRES call run
     in one graph launch (a conditional WHILE node whose body is one cycle and
