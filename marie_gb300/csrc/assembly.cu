@@ -178,12 +178,10 @@ __device__ __forceinline__ void face_points(const CubArgs& A, int f, const doubl
 // sorted triple, about 112 per offset of a cubic grid, where one sum per offset
 // and face pair takes 21*256.
 //
-// FP64-pipe bound (an evaluation is about 50 FP64 instructions, most of them
-// sincos and rsqrt): one warp per entry, its lanes over the points of the sum,
-// so that short rows of a small grid fill the pipe as well as long ones.
-// Measured on GB300 for a 96^3 grid: 10.1 ms for the 4-point rule, 0.4 and 0.6
-// ms for the other two, where the sum per offset and face pair took 438, 2.3
-// and 4.0 ms.
+// FP64-pipe bound: an evaluation is 22 FP64 instructions with the phase's
+// series, about 50 with sincos.  Measured on GB300 for a 96^3 grid: 4.6 ms for
+// the 4-point rule (a warp per entry and sincos: 10.1), 0.28 and 0.37 ms for the
+// other two, where the sum per offset and face pair took 438, 2.3 and 4.0 ms.
 // ---------------------------------------------------------------------------
 constexpr int kRuleMax = 20;                                   // nodes of the largest rule
 constexpr int kDiffMax = kRuleMax * (kRuleMax - 1) / 2 * 2 + 1;  // its differences, before merging less than this
@@ -216,9 +214,97 @@ struct FaceTable {
   }
 };
 
+// The phase factor of the sums.  SMALL: the phase of a point against the entry's
+// centre is at most sqrt(2) k (k per voxel), small enough for the series; the
+// sum is taken relative to the centre's phase and turned by it once at the end
+// (R - R0 is as exact as R).
+template <bool SMALL>
+struct FacePhase {
+  SmallPhase series;
+  double k;
+  explicit FacePhase(double k_) : series(k_), k(k_) {}
+  // distance of the centres (crossed faces: node 1/2 on both)
+  __device__ __forceinline__ double centre(bool crossed, double s, double b, double c) const {
+    if (!SMALL) return 0.0;
+    if (crossed) b -= 0.5, c -= 0.5;
+    return sqrt(fma(s, s, fma(b, b, c * c)));
+  }
+  // acc += w exp(-j k (R - R0)) / R
+  __device__ __forceinline__ void add(double r2, double R0, double w, double2& acc) const {
+    const double ri = rsqrt(r2);
+    double sn, cs;
+    if (SMALL)
+      series.sincos(fma(r2, ri, -R0), sn, cs);
+    else
+      sincos(k * (r2 * ri), &sn, &cs);
+    w *= ri;
+    acc.x = fma(w, cs, acc.x);
+    acc.y = fma(-w, sn, acc.y);
+  }
+  __device__ __forceinline__ double2 turn(double2 acc, double R0) const {
+    if (!SMALL) return acc;
+    double sn, cs;
+    sincos(k * R0, &sn, &cs);
+    return cmul(acc, mk<double2>(cs, -sn));
+  }
+};
+
+// A lane per entry needs this many of them to fill the chip: with 17^3 (tables of
+// a 16^3 grid) the assembly takes 3.97 ms against 3.90 with a warp per entry,
+// with 65 x 21 x 13 it takes 4.34 against 4.68, with 97^3 10.2 against 14.5.
+constexpr long long kLanePerEntry = 16000;
+
+// One lane per entry of the 4-point rule's tables: lanes over the (x, y) of one
+// z, x >= y >= z, row y and the row as far from the other end side by side
+// (together always 2 e0 - z - e1 + 1 long).  No padded point, no reduction, and
+// the entry's sqrt and sincos shared by no lane that idles.
+// grid (blocks over the (x, y), e2, 6)
+template <bool SMALL>
+__global__ void __launch_bounds__(128) k_face_entries(const FaceRule* __restrict__ rule, FacePhase<SMALL> ph, int e0,
+                                                      int e1, double2* __restrict__ out) {
+  const int z = blockIdx.y, e2 = gridDim.y, table = blockIdx.z, place = table % 3;
+  const bool crossed = table >= 3;
+  __shared__ double u[kRuleMax], wu[kRuleMax], d[kDiffMax], wd[kDiffMax];
+  const int nu = rule->nu, nd = rule->nd;
+  for (int i = threadIdx.x; i < nd; i += blockDim.x) d[i] = rule->d[i], wd[i] = rule->wd[i];
+  for (int i = threadIdx.x; i < nu; i += blockDim.x) u[i] = rule->u[i], wu[i] = rule->wu[i];
+  __syncthreads();
+  const int rows = e1 - z, width = 2 * e0 - z - e1 + 1;
+  const int at = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = at / width, j = at - i * width, first = e0 - z - i;
+  const int y = j < first ? z + i : e1 - 1 - i, x = j < first ? y + j : y + (j - first);
+  if (2 * i >= rows || (j >= first && y == z + i)) return;
+  const double s = place == 0 ? x : place == 1 ? y : z;
+  const double b = place == 0 ? y : x, c = place == 2 ? y : z;
+  const double R0 = ph.centre(crossed, s, b, c);
+  double2 acc = mk<double2>(0, 0);
+  if (crossed) {
+    for (int i1 = 0; i1 < nu; ++i1)
+      for (int i2 = 0; i2 < nu; ++i2) {
+        const double a1 = b - u[i1], a2 = c - u[i2], base = fma(a1, a1, a2 * a2), w = wu[i1] * wu[i2];
+        for (int i0 = 0; i0 < nd; ++i0) {
+          const double a0 = s + d[i0];
+          ph.add(fma(a0, a0, base), R0, w * wd[i0], acc);
+        }
+      }
+  } else {
+    for (int i1 = 0; i1 < nd; ++i1) {
+      const double a1 = c + d[i1], base = fma(a1, a1, s * s), w = wd[i1];
+      for (int i0 = 0; i0 < nd; ++i0) {
+        const double a0 = b + d[i0];
+        ph.add(fma(a0, a0, base), R0, w * wd[i0], acc);
+      }
+    }
+  }
+  out[(((long long)table * e2 + z) * e1 + y) * e0 + x] = ph.turn(acc, R0);
+}
+
+// One warp per entry, its lanes over the points, for the few entries of the
+// other two rules, whose sums are 50 to 500 times as long.
 // grid (e1, e2, 6 * split): row (y, z) of one table, the block's warps over x
-__global__ void __launch_bounds__(128) k_face_sums(const FaceRule* __restrict__ rule, double k, int e0, int split,
-                                                   double2* __restrict__ out) {
+template <bool SMALL>
+__global__ void __launch_bounds__(128) k_face_sums(const FaceRule* __restrict__ rule, FacePhase<SMALL> ph, int e0,
+                                                   int split, double2* __restrict__ out) {
   const int y = blockIdx.x, z = blockIdx.y;
   if (y < z) return;
   const int e1 = gridDim.x, e2 = gridDim.y;
@@ -243,31 +329,23 @@ __global__ void __launch_bounds__(128) k_face_sums(const FaceRule* __restrict__ 
     // the special coordinate (F: the plane distance s, Q: c) and the other two
     const double s = place == 0 ? x : place == 1 ? y : z;
     const double b = place == 0 ? y : x, c = place == 2 ? y : z;
+    const double R0 = ph.centre(crossed, s, b, c);
     double2 acc = mk<double2>(0, 0);
     for (int t = t0 + lane; t < t1; t += 32) {
       const int i0 = t % n0;
       int i1 = t / n0;
-      double r2, w;
       if (crossed) {
         const int i2 = i1 / n1;
         i1 -= i2 * n1;
         const double a0 = s + r.d[i0], a1 = b - r.u[i1], a2 = c - r.u[i2];
-        r2 = fma(a0, a0, fma(a1, a1, a2 * a2));
-        w = r.wd[i0] * (r.wu[i1] * r.wu[i2]);
+        ph.add(fma(a0, a0, fma(a1, a1, a2 * a2)), R0, r.wd[i0] * (r.wu[i1] * r.wu[i2]), acc);
       } else {
         const double a0 = b + r.d[i0], a1 = c + r.d[i1];
-        r2 = fma(a0, a0, fma(a1, a1, s * s));
-        w = r.wd[i0] * r.wd[i1];
+        ph.add(fma(a0, a0, fma(a1, a1, s * s)), R0, r.wd[i0] * r.wd[i1], acc);
       }
-      const double ri = rsqrt(r2);
-      double sn, cs;
-      sincos(k * (r2 * ri), &sn, &cs);
-      w *= ri;
-      acc.x = fma(w, cs, acc.x);
-      acc.y = fma(-w, sn, acc.y);
     }
     acc = warp_sum2(acc);
-    if (lane == 0) row[x] = acc;
+    if (lane == 0) row[x] = ph.turn(acc, R0);
   }
 }
 
@@ -670,8 +748,19 @@ static int assemble_toeplitz(int L, int M, int N, double dx, double ko, const do
   for (int r = 0; r < 3; ++r) {
     const int e0 = ext[r][0], e1 = ext[r][1], e2 = ext[r][2];
     MARIE_TRY(tables[r].alloc((size_t)6 * split[r] * e0 * e1 * e2 * sizeof(double2), st));
-    k_face_sums<<<dim3(e1, e2, 6 * split[r]), 128, 0, st>>>(drules.as<FaceRule>() + r, ko * dx, e0, split[r],
-                                                            tables[r].as<double2>());
+    auto launch = [&](auto phase, auto entries, auto sums) {
+      const FaceRule* rule = drules.as<FaceRule>() + r;
+      const int halves = (e1 + 1) / 2, width = 2 * e0 - e1 + 1;
+      if (r == 0 && (long long)e0 * e1 * e2 >= kLanePerEntry)
+        entries<<<dim3((halves * width + 127) / 128, e2, 6), 128, 0, st>>>(rule, phase, e0, e1, tables[r].as<double2>());
+      else
+        sums<<<dim3(e1, e2, 6 * split[r]), 128, 0, st>>>(rule, phase, e0, split[r], tables[r].as<double2>());
+    };
+    const double k = ko * dx;
+    if (std::sqrt(2.0) * std::fabs(k) <= kSmallPhase)
+      launch(FacePhase<true>(k), k_face_entries<true>, k_face_sums<true>);
+    else
+      launch(FacePhase<false>(k), k_face_entries<false>, k_face_sums<false>);
     count_launch();
     MARIE_CUDA_TRY(cudaGetLastError());
     t[r] = FaceTable{tables[r].as<double2>(), e0, e1, e2, split[r]};

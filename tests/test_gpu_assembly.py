@@ -89,6 +89,20 @@ def test_shared_face_sums_at_region_edges(shape):
     assert relerr(mg.getOPERATORS(r, FREQ, "N", "T"), ref) < 1e-12
 
 
+@pytest.mark.parametrize("dx", [4e-3, 2e-2])
+@pytest.mark.parametrize("shape", [(40, 20, 18), (19, 19, 41)])
+def test_face_sums_of_large_tables(shape, dx):
+    """The tables that take one lane per entry, sorted and unsorted, with the
+    phase's series (4 mm) and beyond its range (20 mm): 1e-12 of the largest
+    entry, as above."""
+    import marie_gb300 as mg
+
+    r = vo.grid(*shape, dx)
+    sv = mg.singular_integrals(2 * np.pi * FREQ / 299792458.0, dx)
+    ref = vo.getOPERATORS(r, FREQ, typ="T", sing=sv)
+    assert relerr(mg.getOPERATORS(r, FREQ, "N", "T"), ref) < 1e-12
+
+
 @pytest.mark.parametrize("shape", [(4, 12, 8), (20, 8, 4)])
 def test_octant_transforms_match_full_fft(shape):
     """fN and fK from the reflected octant transforms, through getOPERATORS and
