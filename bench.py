@@ -205,8 +205,8 @@ def run_gpu(args, world, rank, local):
     if args.solve_only:
         # profiling entry: the mixed solves of the timed region and nothing else,
         # with the schedule the autotuner picks for this grid on an idle GPU
-        # (fused x+y passes, default radix schedules; a tuning run under a
-        # profiler would time the candidates serialised and could pick another)
+        # (a tuning run under a profiler would time the candidates serialised
+        # and could pick another)
         op.set_schedule(1, 0, 0)
         # refinement steps and restart cycles driven from the host (plain
         # graphs): ncu does not profile kernels inside conditional graphs;
@@ -218,8 +218,8 @@ def run_gpu(args, world, rank, local):
         torch.cuda.synchronize()
         return {"solve_only": True, "flag": res[1], "relres": res[2], "iter": res[3]} if rank == 0 else {}
 
-    # schedule autotuner (outside the timed region): fused / five-pass x-y
-    # passes and their radix schedule, z-pass radix schedule and columns per CTA
+    # schedule autotuner (outside the timed region): fused (where the grid has
+    # them) or five-pass x and y
     tuned, tune_cands = op.autotune()
     # the stated precision split: FP32 matvec, Arnoldi in FP64 (the default)
     op.set_inner_precision("fp64")

@@ -342,16 +342,16 @@ int64_t marie_graph_loops(void);
  * their operators are unaffected. */
 int marie_release_cached_memory(void);
 /* Schedule autotuner (no counterpart in the reference): times the plan's FP32
- * matvec for every candidate schedule (fuse: fused x+y cluster passes or the
- * five-pass form; fvar: default or narrow radix schedule of the fused x/y
- * transforms, or clusters of half the size; zvar: z pass with the default schedule, the narrow radix
- * schedule, or 4 instead of 8 columns per CTA), keeps the fastest on the plan
- * and returns it in *fuse / *fvar / *zvar.  ms receives {fuse, fvar, zvar,
+ * matvec for every candidate schedule (fuse: fused x+y cluster passes, on the
+ * grids that have them, or the five-pass form), keeps the fastest on the plan
+ * and returns it in *fuse; *fvar and *zvar are 0 (one schedule of the x/y
+ * transforms and of the z pass is left).  ms receives {fuse, fvar, zvar,
  * milliseconds} per candidate (up to cap candidates, *count written).  A plan
  * without an FP32 operator is left as it is (*count = 0). */
 int marie_plan_autotune(marie_plan* plan, int* fuse, int* fvar, int* zvar, double* ms, int64_t cap,
                         int64_t* count);
-/* Pin a schedule as marie_plan_autotune would choose it. */
+/* Pin a schedule as marie_plan_autotune would choose it; fvar and zvar from 0 to
+ * 2 are accepted and select nothing. */
 int marie_plan_set_schedule(marie_plan* plan, int fuse, int fvar, int zvar);
 /* Krylov basis precision of the inner solves of a MARIE_MIXED plan's GMRES
  * refinement (no counterpart in the reference): MARIE_FP64 (the default: the

@@ -166,21 +166,9 @@ int finish_out(void* user, const void* dev, size_t bytes, cudaStream_t st) {
   return MARIE_OK;
 }
 
-int ensure_workspace(marie_plan* p, int prec, long long nrhs, bool with_A) {
+int ensure_workspace(marie_plan* p, int prec, long long nrhs) {
   const size_t es = (prec == MARIE_FP32) ? sizeof(float2) : sizeof(double2);
-  const size_t need_A = with_A ? (size_t)p->elems_A() * es * nrhs : 0;
   const size_t need_B = (size_t)p->elems_B() * es * nrhs;
-  if (need_A > p->ws_bytes_A) {
-    if (p->wsA) cudaFreeAsync(p->wsA, p->stream);
-    p->wsA = nullptr;
-    p->ws_bytes_A = 0;
-    if (cudaMallocAsync(&p->wsA, need_A, p->stream) != cudaSuccess) {
-      cudaGetLastError();
-      p->wsA = nullptr;
-      return set_error(MARIE_ENOMEM, "workspace A (%zu bytes) allocation failed", need_A);
-    }
-    p->ws_bytes_A = need_A;
-  }
   if (need_B > p->ws_bytes_B) {
     if (p->wsB) cudaFreeAsync(p->wsB, p->stream);
     p->wsB = nullptr;
@@ -188,7 +176,7 @@ int ensure_workspace(marie_plan* p, int prec, long long nrhs, bool with_A) {
     if (cudaMallocAsync(&p->wsB, need_B, p->stream) != cudaSuccess) {
       cudaGetLastError();
       p->wsB = nullptr;
-      return set_error(MARIE_ENOMEM, "workspace B (%zu bytes) allocation failed", need_B);
+      return set_error(MARIE_ENOMEM, "workspace of the spectra (%zu bytes) allocation failed", need_B);
     }
     p->ws_bytes_B = need_B;
   }
@@ -289,44 +277,41 @@ static int run_matvec_t(marie_plan* p, const IO* J, long long js, IO* out, long 
   const bool fused = p->fuse && ML::fused(p->d);
   for (long long r0 = 0; r0 < nrhs; r0 += chunk_max) {
     const int nr = (int)((nrhs - r0) < chunk_max ? (nrhs - r0) : chunk_max);
-    MARIE_TRY(ensure_workspace(p, prec, nr, !fused));
+    MARIE_TRY(ensure_workspace(p, prec, nr));
     Dims d = p->d;
     d.stop = stop ? stop + r0 : nullptr;
     d.step = step;
-    cplx<T>* A = reinterpret_cast<cplx<T>*>(p->wsA);
     cplx<T>* B = reinterpret_cast<cplx<T>*>(p->wsB);
-    const long long sA = p->elems_A(), sB = p->elems_B();
+    const long long sB = p->elems_B(), plane = (long long)d.Lp * d.Mp;
     const IO* Jc = J + r0 * js;
     IO* oc = out + r0 * os;
     const bool prof = p->profile;
     if (prof) MARIE_CUDA_TRY(cudaEventRecord(p->ev[0], p->stream));
     if (fused) {
-      MARIE_CUDA_TRY(ML::xyfwd(Jc, js, inv, pro, B, sB, d, tw[0], tw[1], nr, p->stream, p->fvar));
+      MARIE_CUDA_TRY(ML::xyfwd(Jc, js, inv, pro, B, sB, d, tw[0], tw[1], nr, p->stream));
       if (prof) {
         MARIE_CUDA_TRY(cudaEventRecord(p->ev[1], p->stream));
         MARIE_CUDA_TRY(cudaEventRecord(p->ev[2], p->stream));
       }
-      MARIE_CUDA_TRY(ML::zmul(B, sB, fN, oct, d, tw[2], nr, p->stream, kind, kind == 0 ? p->zvar : 0,
-                                    kind == 0 ? &p->zt : nullptr));
+      MARIE_CUDA_TRY(ML::zmul(B, sB, fN, oct, d, tw[2], nr, p->stream, kind, kind == 0 ? &p->zt : nullptr));
       if (prof) {
         MARIE_CUDA_TRY(cudaEventRecord(p->ev[3], p->stream));
         MARIE_CUDA_TRY(cudaEventRecord(p->ev[4], p->stream));
       }
-      MARIE_CUDA_TRY(ML::yxinv(B, sB, Jc, js, inv, ep, oc, os, d, tw[0], tw[1], nr, p->stream, p->fvar));
+      MARIE_CUDA_TRY(ML::yxinv(B, sB, Jc, js, inv, ep, oc, os, d, tw[0], tw[1], nr, p->stream));
       count_launch(3);
     } else {
-      MARIE_CUDA_TRY(ML::xfwd(Jc, js, inv, pro, A, sA, d, tw[0], nr, p->stream));
+      MARIE_CUDA_TRY(ML::xfwd(Jc, js, inv, pro, B, sB, d, tw[0], nr, p->stream));
       if (prof) MARIE_CUDA_TRY(cudaEventRecord(p->ev[1], p->stream));
-      MARIE_CUDA_TRY(ML::cols(false, d.Mp, A, (long long)d.Lp * d.M, sA, d.M, B, (long long)d.Lp * d.Mp, sB, d.Mp,
-                              d.Lp, 3 * d.N, tw[1], nr, p->stream, d.stop, step));
+      MARIE_CUDA_TRY(ML::cols(false, d.Mp, B, plane, sB, d.M, B, plane, sB, d.Mp, d.Lp, 3 * d.N, tw[1], nr, p->stream,
+                              d.stop, step));
       if (prof) MARIE_CUDA_TRY(cudaEventRecord(p->ev[2], p->stream));
-      MARIE_CUDA_TRY(ML::zmul(B, sB, fN, oct, d, tw[2], nr, p->stream, kind, kind == 0 ? p->zvar : 0,
-                                    kind == 0 ? &p->zt : nullptr));
+      MARIE_CUDA_TRY(ML::zmul(B, sB, fN, oct, d, tw[2], nr, p->stream, kind, kind == 0 ? &p->zt : nullptr));
       if (prof) MARIE_CUDA_TRY(cudaEventRecord(p->ev[3], p->stream));
-      MARIE_CUDA_TRY(ML::cols(true, d.Mp, B, (long long)d.Lp * d.Mp, sB, d.Mp, A, (long long)d.Lp * d.M, sA, d.M,
-                              d.Lp, 3 * d.N, tw[1], nr, p->stream, d.stop, step));
+      MARIE_CUDA_TRY(ML::cols(true, d.Mp, B, plane, sB, d.Mp, B, plane, sB, d.M, d.Lp, 3 * d.N, tw[1], nr, p->stream,
+                              d.stop, step));
       if (prof) MARIE_CUDA_TRY(cudaEventRecord(p->ev[4], p->stream));
-      MARIE_CUDA_TRY(ML::xinv(A, sA, Jc, js, inv, ep, oc, os, d, tw[0], nr, p->stream));
+      MARIE_CUDA_TRY(ML::xinv(B, sB, Jc, js, inv, ep, oc, os, d, tw[0], nr, p->stream));
       count_launch(5);
     }
     if (prof) {
@@ -868,7 +853,6 @@ int marie_plan_destroy(marie_plan* p) {
   release_cufft_state(p);
   free_bound(p);
   p->crop.reset();
-  if (p->wsA) cudaFreeAsync(p->wsA, p->stream);
   if (p->wsB) cudaFreeAsync(p->wsB, p->stream);
   if (p->stream) cudaStreamSynchronize(p->stream);
   cudaFree(p->fN64);
@@ -892,10 +876,12 @@ int marie_plan_destroy(marie_plan* p) {
 void* marie_plan_stream(marie_plan* p) { return p ? (void*)p->stream : nullptr; }
 
 // Autotuner: times the FP32 matvec of this plan's grid for every candidate
-// schedule (fused x+y passes with the default or the narrow radix schedule, or
-// the five-pass form; the z pass with the wide or narrow radix schedule and
-// with 8 or 4 columns per CTA), keeps the fastest on the plan and reports every
-// candidate's time as {fuse, fvar, zvar, ms}.
+// schedule (the fused x+y passes where the grid has them, and the five-pass
+// form), keeps the fastest on the plan and reports every candidate's time as
+// {fuse, fvar, zvar, ms}.  fvar and zvar are 0: the narrow radix schedules, the
+// clusters of half the size and the 4-column z pass that they numbered lost to
+// the present passes on every grid from 12 x 12 x 16 to 128^3 (z pass of 128^3:
+// 738 and 737 us a product against 568) and are gone.
 int marie_plan_autotune(marie_plan* p, int* fuse_out, int* fvar_out, int* zvar_out, double* ms_out, int64_t cap,
                         int64_t* count) {
   if (!p) return set_error(MARIE_EINVAL, "NULL plan");
@@ -914,29 +900,17 @@ int marie_plan_autotune(marie_plan* p, int* fuse_out, int* fvar_out, int* zvar_o
   Epilogue ep{};
   ep.a_s = mk<double2>(1.0, 0.0);
   ep.b_s = mk<double2>(1.0, 0.0);
-  auto wide = [](int n) { return n == 16 || n == 128 || n == 256; };
-  const bool can_fuse = MatvecLaunch<float>::fused(p->d);
-  const bool narrow_xy = can_fuse && (wide(p->d.Lp) || wide(p->d.Mp));
-  // half-size clusters exist for the grids fused with clusters of 4 or 8
-  const bool half_cluster = can_fuse && p->d.Lp >= 128;
-  struct Cand { int fuse, fvar, zvar; double ms; };
+  struct Cand { int fuse; double ms; };
   std::vector<Cand> cands;
-  for (int f = can_fuse ? 1 : 0; f >= 0; --f)
-    for (int fv = 0; fv < (f ? 3 : 1); ++fv) {
-      if ((fv == 1 && !narrow_xy) || (fv == 2 && !half_cluster)) continue;
-      for (int z = 0; z < 3; ++z)
-        if (z != 1 || wide(p->d.Np)) cands.push_back({f, fv, z, 0.0});
-    }
+  if (MatvecLaunch<float>::fused(p->d)) cands.push_back({1, 0.0});
+  cands.push_back({0, 0.0});
   const bool fuse0 = p->fuse;
-  const int fvar0 = p->fvar, zvar0 = p->zvar;
   cudaEvent_t e0, e1;
   MARIE_CUDA_TRY(cudaEventCreate(&e0));
   MARIE_CUDA_TRY(cudaEventCreate(&e1));
   int status = MARIE_OK;
   for (auto& c : cands) {
     p->fuse = c.fuse != 0;
-    p->fvar = c.fvar;
-    p->zvar = c.zvar;
     const int reps = 5;
     for (int r = 0; r < 2 + reps && status == MARIE_OK; ++r) {
       if (r == 2) cudaEventRecord(e0, st);
@@ -953,23 +927,19 @@ int marie_plan_autotune(marie_plan* p, int* fuse_out, int* fvar_out, int* zvar_o
   cudaEventDestroy(e1);
   if (status != MARIE_OK) {
     p->fuse = fuse0;
-    p->fvar = fvar0;
-    p->zvar = zvar0;
     return status;
   }
   const Cand* best = &cands[0];
   for (const auto& c : cands)
     if (c.ms < best->ms) best = &c;
   p->fuse = best->fuse != 0;
-  p->fvar = best->fvar;
-  p->zvar = best->zvar;
   if (fuse_out) *fuse_out = best->fuse;
-  if (fvar_out) *fvar_out = best->fvar;
-  if (zvar_out) *zvar_out = best->zvar;
+  if (fvar_out) *fvar_out = 0;
+  if (zvar_out) *zvar_out = 0;
   for (size_t i = 0; i < cands.size() && (int64_t)i < cap && ms_out; ++i) {
     ms_out[4 * i] = cands[i].fuse;
-    ms_out[4 * i + 1] = cands[i].fvar;
-    ms_out[4 * i + 2] = cands[i].zvar;
+    ms_out[4 * i + 1] = 0;
+    ms_out[4 * i + 2] = 0;
     ms_out[4 * i + 3] = cands[i].ms;
   }
   if (count) *count = (int64_t)cands.size();
@@ -980,9 +950,7 @@ int marie_plan_set_schedule(marie_plan* p, int fuse, int fvar, int zvar) {
   if (!p) return set_error(MARIE_EINVAL, "NULL plan");
   if (fvar < 0 || fvar > 2) return set_error(MARIE_EINVAL, "fvar must be 0, 1 or 2");
   if (zvar < 0 || zvar > 2) return set_error(MARIE_EINVAL, "zvar must be 0, 1 or 2");
-  p->fuse = fuse != 0;
-  p->fvar = fvar;
-  p->zvar = zvar;
+  p->fuse = fuse != 0;  // (the schedules that fvar and zvar numbered are gone, their values stay valid)
   return MARIE_OK;
 }
 

@@ -182,7 +182,6 @@ int dof_box(marie_plan* p, const int64_t* idx_dev, long long n, int box[6]) {
 static void free_crop(marie_plan* q) {
   if (!q) return;
   cudaStreamSynchronize(q->stream);
-  if (q->wsA) cudaFreeAsync(q->wsA, q->stream);
   if (q->wsB) cudaFreeAsync(q->wsB, q->stream);
   if (q->arena) cudaFreeAsync(q->arena, q->stream);
   if (q->pinned) cudaFreeHost(q->pinned);
@@ -315,8 +314,6 @@ void crop_settings(const marie_plan* p, marie_plan* q) {
   q->stream = p->stream;
   q->nrhs_max = p->nrhs_max;
   q->fuse = p->fuse;
-  q->fvar = p->fvar;
-  q->zvar = p->zvar;
   q->inner_prec = p->inner_prec;
   q->inner_restart = p->inner_restart;
   q->batch_groups = p->batch_groups;

@@ -414,8 +414,7 @@ template <typename V, int N> struct Sched<V, N, true> {
 // transform uses the schedule's radix list; the inverse uses it reversed, so
 // reg after FFT<V,N,false>::run is directly the input of FFT<V,N,true>::run.
 // W selects the radix schedule: the wide one (radix 16, FP32 lengths 16, 128,
-// 256) or the narrow one (radix <= 8); the default is the wide one where it
-// exists.  The matvec autotuner times both for the z pass.
+// 256) or FFTCfg's; the default is the wide one where it exists.
 template <typename V, int N, bool INV, bool W = (sizeof(V) == 8) && HasWide<N>::value> struct FFT {
   using RF = typename Sched<V, N, W>::R;
   using RL_ = typename std::conditional<INV, typename RRev<RF>::type, RF>::type;

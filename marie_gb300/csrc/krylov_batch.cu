@@ -1341,7 +1341,7 @@ int RefineJob::prepare(marie_plan* p, const BatchOp& A32, const BatchOp* L1, con
   J.tol = tol;
   cudaStream_t st = p->stream;
   // matvec workspaces at their largest, so that nothing is allocated while capturing
-  MARIE_TRY(ensure_workspace(p, MARIE_FP64, S < p->nrhs_max ? S : p->nrhs_max, true));
+  MARIE_TRY(ensure_workspace(p, MARIE_FP64, S < p->nrhs_max ? S : p->nrhs_max));
   MARIE_TRY(J.W.init(st, S, m, n, fp32_basis));
   if (p->batch_groups == 2 && S >= 2) MARIE_TRY(J.W.init_groups());
   MARIE_TRY(J.rr.alloc((size_t)S * n * sizeof(double2), st));

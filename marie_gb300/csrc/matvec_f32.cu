@@ -8,11 +8,10 @@ namespace marie {
 using V32 = MatvecLaunch<float>::V;
 template bool MatvecLaunch<float>::fused(const Dims&);
 template cudaError_t MatvecLaunch<float>::xyfwd<double2>(const double2*, long long, const int*, Prologue, V32*,
-                                                     long long, const Dims&, const V32*, const V32*, int, cudaStream_t,
-                                                     int);
+                                                     long long, const Dims&, const V32*, const V32*, int, cudaStream_t);
 template cudaError_t MatvecLaunch<float>::yxinv<double2>(const V32*, long long, const double2*, long long, const int*,
                                                      Epilogue, double2*, long long, const Dims&, const V32*, const V32*,
-                                                     int, cudaStream_t, int);
+                                                     int, cudaStream_t);
 template cudaError_t MatvecLaunch<float>::xfwd<double2>(const double2*, long long, const int*, Prologue, V32*, long long,
                                                     const Dims&, const V32*, int, cudaStream_t);
 template cudaError_t MatvecLaunch<float>::xinv<double2>(const V32*, long long, const double2*, long long, const int*,

@@ -1,6 +1,6 @@
 // Fused x+y passes of the matvec, one (z, component) plane per thread-block
 // cluster, exchanging the x-transformed rows through distributed shared memory
-// instead of a round trip of the A spectrum through HBM.
+// instead of a round trip through HBM.
 //
 //   k_xyfwd:  gather J (inv map) -> FFT_x of the M non-zero rows (CTA q of the
 //             cluster owns rows [q*M/CS, (q+1)*M/CS)) -> each output (kx, y) is
@@ -31,17 +31,12 @@ __device__ __forceinline__ void cluster_arrive_relaxed() {
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
 
-// NARROW: the radix-8 schedules for the x and y transforms (twice the threads
-// per transform, half the exchange buffer, one more CTA per SM for xyfwd); an
-// autotuner variant for the lengths that have a wide schedule.
-template <typename T, int NL, int NM, int CS, bool NARROW = false> struct XYCfg {
+template <typename T, int NL, int NM, int CS> struct XYCfg {
   using V = cplx<T>;
-  static constexpr bool WX = !NARROW && (sizeof(V) == 8) && HasWide<NL>::value;
-  static constexpr bool WY = !NARROW && (sizeof(V) == 8) && HasWide<NM>::value;
-  using FX = FFT<V, NL, false, WX>;
-  using FXI = FFT<V, NL, true, WX>;
-  using FY = FFT<V, NM, false, WY>;
-  using FYI = FFT<V, NM, true, WY>;
+  using FX = FFT<V, NL, false>;
+  using FXI = FFT<V, NL, true>;
+  using FY = FFT<V, NM, false>;
+  using FYI = FFT<V, NM, true>;
   static constexpr int THREADS = 256;
   static constexpr int L = NL / 2, M = NM / 2;
   static constexpr int RY = M / CS;                 // rows per CTA
@@ -58,12 +53,12 @@ template <typename T, int NL, int NM, int CS, bool NARROW = false> struct XYCfg 
                              FY::T <= THREADS;
 };
 
-template <typename T, int NL, int NM, int CS, bool NARROW, typename IO>
-__global__ void __launch_bounds__(256, NARROW ? 4 : 0)
+template <typename T, int NL, int NM, int CS, typename IO>
+__global__ void __launch_bounds__(256)
 k_xyfwd(const IO* __restrict__ J, long long js, const int* __restrict__ inv, Prologue pro,
         cplx<T>* __restrict__ B, long long bs, Dims d, const cplx<T>* __restrict__ twx,
         const cplx<T>* __restrict__ twy) {
-  using C = XYCfg<T, NL, NM, CS, NARROW>;
+  using C = XYCfg<T, NL, NM, CS>;
   using V = cplx<T>;
   using FX = typename C::FX;
   using FY = typename C::FY;
@@ -171,14 +166,14 @@ k_xyfwd(const IO* __restrict__ J, long long js, const int* __restrict__ inv, Pro
   }
 }
 
-template <typename T, int NL, int NM, int CS, bool NARROW, typename IO>
-__global__ void __launch_bounds__(256, (XYCfg<T, NL, NM, CS, NARROW>::FXI::E <= 16 &&
-                                        XYCfg<T, NL, NM, CS, NARROW>::FYI::E <= 16) ? 3 : 1)
+template <typename T, int NL, int NM, int CS, typename IO>
+__global__ void __launch_bounds__(256, (XYCfg<T, NL, NM, CS>::FXI::E <= 16 &&
+                                        XYCfg<T, NL, NM, CS>::FYI::E <= 16) ? 3 : 1)
 k_yxinv(const cplx<T>* __restrict__ B, long long bs, const IO* __restrict__ J, long long js,
         const int* __restrict__ inv, Epilogue ep, IO* __restrict__ out, long long os, Dims d,
         const cplx<T>* __restrict__ twx, const cplx<T>* __restrict__ twy) {
   if (rhs_skipped(d, blockIdx.y)) return;  // uniform over the cluster
-  using C = XYCfg<T, NL, NM, CS, NARROW>;
+  using C = XYCfg<T, NL, NM, CS>;
   using V = cplx<T>;
   using FXI = typename C::FXI;
   using FYI = typename C::FYI;

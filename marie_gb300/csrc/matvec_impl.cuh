@@ -103,10 +103,10 @@ template <typename T> struct MatvecImpl {
     return launch_pass(k_cols<T, NC, INV>, grid, S * FFT<V, NC, INV>::T, smem, st, in, in_w, in_rhs, n_in, out, out_w,
                        out_rhs, n_out, Lp, tw, stop, step);
   }
-  template <int NZ, int KIND, int VAR>
+  template <int NZ, int KIND>
   static cudaError_t zmul_nk(V* B, long long bs, const V* fN, int oct, const Dims& d, const V* tw, int nrhs,
                              cudaStream_t st, const ZTile* zt) {
-    using ZC = ZS<T, NZ, KIND, VAR>;
+    using ZC = ZS<T, NZ, KIND>;
     constexpr int S = ZC::S;
     // the bulk-copy tile needs a tensor map whose box is S columns wide
     const int mi = S == 8 ? 0 : S == 4 ? 1 : S == 2 ? 2 : -1;
@@ -117,9 +117,9 @@ template <typename T> struct MatvecImpl {
     const CUtensorMap& tmap = tma ? zt->map[mi] : none;
     int* err = zt ? zt->err : nullptr;
     const size_t smem = (size_t)ZC::bytes(S);  // S columns, 3 component buffers, operator tile
-    cudaError_t e = opt_in_smem(k_zmul<T, NZ, KIND, VAR>, smem);
+    cudaError_t e = opt_in_smem(k_zmul<T, NZ, KIND>, smem);
     if (e != cudaSuccess) return e;
-    return launch_pass(k_zmul<T, NZ, KIND, VAR>, dim3((d.Lp + S - 1) / S, d.Mp, nrhs), ZC::THREADS, smem, st, B, bs, fN,
+    return launch_pass(k_zmul<T, NZ, KIND>, dim3((d.Lp + S - 1) / S, d.Mp, nrhs), ZC::THREADS, smem, st, B, bs, fN,
                        oct, d, tw, tmap, tma, err);
   }
   // the z pass on column pairs (FP32, a tile by bulk copy)
@@ -135,16 +135,11 @@ template <typename T> struct MatvecImpl {
   }
   template <int NZ>
   static cudaError_t zmul_n(V* B, long long bs, const V* fN, int oct, const Dims& d, const V* tw, int nrhs,
-                            cudaStream_t st, int kind, int var, const ZTile* zt) {
-    if (kind == 1) return zmul_nk<NZ, 1, 0>(B, bs, fN, oct, d, tw, nrhs, st, nullptr);
-    if constexpr (sizeof(T) == 4) {
-      if constexpr (HasWide<NZ>::value)
-        if (var == 1) return zmul_nk<NZ, 0, 1>(B, bs, fN, oct, d, tw, nrhs, st, zt);
-      if (var == 2) return zmul_nk<NZ, 0, 2>(B, bs, fN, oct, d, tw, nrhs, st, zt);
-      if constexpr (ZP<NZ>::ok)
-        if (oct && zt && zt->ok) return zmul_pairs<NZ>(B, bs, d, tw, nrhs, st, zt);
-    }
-    return zmul_nk<NZ, 0, 0>(B, bs, fN, oct, d, tw, nrhs, st, zt);
+                            cudaStream_t st, int kind, const ZTile* zt) {
+    if (kind == 1) return zmul_nk<NZ, 1>(B, bs, fN, oct, d, tw, nrhs, st, nullptr);
+    if constexpr (sizeof(T) == 4 && ZP<NZ>::ok)
+      if (oct && zt && zt->ok) return zmul_pairs<NZ>(B, bs, d, tw, nrhs, st, zt);
+    return zmul_nk<NZ, 0>(B, bs, fN, oct, d, tw, nrhs, st, zt);
   }
 
   template <typename IO>
@@ -188,9 +183,9 @@ template <typename T> struct MatvecImpl {
     return cudaErrorInvalidValue;
   }
   static cudaError_t zmul(V* B, long long bs, const V* fN, int oct, const Dims& d, const V* tw, int nrhs,
-                          cudaStream_t st, int kind, int var, const ZTile* zt) {
+                          cudaStream_t st, int kind, const ZTile* zt) {
     switch (d.Np) {
-#define MARIE_CASE(n_) case n_: return zmul_n<n_>(B, bs, fN, oct, d, tw, nrhs, st, kind, var, zt);
+#define MARIE_CASE(n_) case n_: return zmul_n<n_>(B, bs, fN, oct, d, tw, nrhs, st, kind, zt);
       MARIE_FFT_LENGTHS(MARIE_CASE)
 #undef MARIE_CASE
     }
@@ -234,36 +229,13 @@ template <typename T> struct FusedImpl {
     cfg.numAttrs = 2;
     return cudaLaunchKernelExC(&cfg, (const void*)kern, args);
   }
-  template <int NL, int NM, int CS, bool NARROW, typename IO>
-  static cudaError_t xyfwd_nv(const IO* J, long long js, const int* inv, Prologue pro, V* B, long long bs,
-                              Dims d, const V* twx, const V* twy, int nrhs, cudaStream_t st) {
-    void* args[] = {(void*)&J, (void*)&js, (void*)&inv, (void*)&pro, (void*)&B, (void*)&bs, (void*)&d,
-                    (void*)&twx, (void*)&twy};
-    return launch(k_xyfwd<T, NL, NM, CS, NARROW, IO>, CS, CS * 3 * d.N, nrhs, XYCfg<T, NL, NM, CS, NARROW>::fwd_smem,
-                  st, args);
-  }
-  template <int NL, int NM, int CS, bool NARROW, typename IO>
-  static cudaError_t yxinv_nv(const V* B, long long bs, const IO* J, long long js, const int* inv, Epilogue ep,
-                              IO* out, long long os, Dims d, const V* twx, const V* twy, int nrhs,
-                              cudaStream_t st) {
-    void* args[] = {(void*)&B, (void*)&bs, (void*)&J, (void*)&js, (void*)&inv, (void*)&ep, (void*)&out,
-                    (void*)&os, (void*)&d, (void*)&twx, (void*)&twy};
-    return launch(k_yxinv<T, NL, NM, CS, NARROW, IO>, CS, CS * 3 * d.N, nrhs, XYCfg<T, NL, NM, CS, NARROW>::inv_smem,
-                  st, args);
-  }
-  // a narrow variant exists where either transform has a wide schedule
-  template <int NL, int NM> static constexpr bool has_narrow() {
-    return sizeof(T) == 4 && (HasWide<NL>::value || HasWide<NM>::value);
-  }
   template <int NL, int NM, int CS, typename IO>
   static cudaError_t xyfwd_n(const IO* J, long long js, const int* inv, Prologue pro, V* B, long long bs,
-                             Dims d, const V* twx, const V* twy, int nrhs, cudaStream_t st, int fvar) {
+                             Dims d, const V* twx, const V* twy, int nrhs, cudaStream_t st) {
     if constexpr (usable<NL, NM, CS>()) {
-      if constexpr (has_narrow<NL, NM>())
-        if (fvar == 1) return xyfwd_nv<NL, NM, CS, true, IO>(J, js, inv, pro, B, bs, d, twx, twy, nrhs, st);
-      if constexpr (CS >= 4 && usable<NL, NM, CS / 2>())
-        if (fvar == 2) return xyfwd_nv<NL, NM, CS / 2, false, IO>(J, js, inv, pro, B, bs, d, twx, twy, nrhs, st);
-      return xyfwd_nv<NL, NM, CS, false, IO>(J, js, inv, pro, B, bs, d, twx, twy, nrhs, st);
+      void* args[] = {(void*)&J, (void*)&js, (void*)&inv, (void*)&pro, (void*)&B, (void*)&bs, (void*)&d,
+                      (void*)&twx, (void*)&twy};
+      return launch(k_xyfwd<T, NL, NM, CS, IO>, CS, CS * 3 * d.N, nrhs, XYCfg<T, NL, NM, CS>::fwd_smem, st, args);
     } else {
       return cudaErrorNotSupported;
     }
@@ -271,14 +243,11 @@ template <typename T> struct FusedImpl {
   template <int NL, int NM, int CS, typename IO>
   static cudaError_t yxinv_n(const V* B, long long bs, const IO* J, long long js, const int* inv, Epilogue ep,
                              IO* out, long long os, Dims d, const V* twx, const V* twy, int nrhs,
-                             cudaStream_t st, int fvar) {
+                             cudaStream_t st) {
     if constexpr (usable<NL, NM, CS>()) {
-      if constexpr (has_narrow<NL, NM>())
-        if (fvar == 1) return yxinv_nv<NL, NM, CS, true, IO>(B, bs, J, js, inv, ep, out, os, d, twx, twy, nrhs, st);
-      if constexpr (CS >= 4 && usable<NL, NM, CS / 2>())
-        if (fvar == 2)
-          return yxinv_nv<NL, NM, CS / 2, false, IO>(B, bs, J, js, inv, ep, out, os, d, twx, twy, nrhs, st);
-      return yxinv_nv<NL, NM, CS, false, IO>(B, bs, J, js, inv, ep, out, os, d, twx, twy, nrhs, st);
+      void* args[] = {(void*)&B, (void*)&bs, (void*)&J, (void*)&js, (void*)&inv, (void*)&ep, (void*)&out,
+                      (void*)&os, (void*)&d, (void*)&twx, (void*)&twy};
+      return launch(k_yxinv<T, NL, NM, CS, IO>, CS, CS * 3 * d.N, nrhs, XYCfg<T, NL, NM, CS>::inv_smem, st, args);
     } else {
       return cudaErrorNotSupported;
     }
@@ -295,10 +264,10 @@ template <typename T> bool MatvecLaunch<T>::fused(const Dims& d) {
 template <typename T>
 template <typename IO>
 cudaError_t MatvecLaunch<T>::xyfwd(const IO* J, long long js, const int* inv, Prologue pro, V* B, long long bs,
-                                   const Dims& d, const V* twx, const V* twy, int nrhs, cudaStream_t st, int fvar) {
+                                   const Dims& d, const V* twx, const V* twy, int nrhs, cudaStream_t st) {
 #define MARIE_CASE(a_, b_, c_)    \
   if (d.Lp == a_ && d.Mp == b_) \
-    return FusedImpl<T>::template xyfwd_n<a_, b_, c_, IO>(J, js, inv, pro, B, bs, d, twx, twy, nrhs, st, fvar);
+    return FusedImpl<T>::template xyfwd_n<a_, b_, c_, IO>(J, js, inv, pro, B, bs, d, twx, twy, nrhs, st);
   MARIE_FUSED_PAIRS(MARIE_CASE)
 #undef MARIE_CASE
   return cudaErrorNotSupported;
@@ -307,11 +276,10 @@ template <typename T>
 template <typename IO>
 cudaError_t MatvecLaunch<T>::yxinv(const V* B, long long bs, const IO* J, long long js, const int* inv,
                                    Epilogue ep, IO* out, long long os, const Dims& d, const V* twx, const V* twy,
-                                   int nrhs, cudaStream_t st, int fvar) {
+                                   int nrhs, cudaStream_t st) {
 #define MARIE_CASE(a_, b_, c_)    \
   if (d.Lp == a_ && d.Mp == b_) \
-    return FusedImpl<T>::template yxinv_n<a_, b_, c_, IO>(B, bs, J, js, inv, ep, out, os, d, twx, twy, nrhs, st, \
-                                                          fvar);
+    return FusedImpl<T>::template yxinv_n<a_, b_, c_, IO>(B, bs, J, js, inv, ep, out, os, d, twx, twy, nrhs, st);
   MARIE_FUSED_PAIRS(MARIE_CASE)
 #undef MARIE_CASE
   return cudaErrorNotSupported;
@@ -339,8 +307,8 @@ cudaError_t MatvecLaunch<T>::cols(bool inv, int NC, const V* in, long long in_w,
 }
 template <typename T>
 cudaError_t MatvecLaunch<T>::zmul(V* B, long long bs, const V* fN, int oct, const Dims& d, const V* tw, int nrhs,
-                                  cudaStream_t st, int kind, int var, const ZTile* zt) {
-  return MatvecImpl<T>::zmul(B, bs, fN, oct, d, tw, nrhs, st, kind, var, zt);
+                                  cudaStream_t st, int kind, const ZTile* zt) {
+  return MatvecImpl<T>::zmul(B, bs, fN, oct, d, tw, nrhs, st, kind, zt);
 }
 
 }  // namespace marie

@@ -13,8 +13,8 @@
 //   xinv : rows (y<M, z<N, c)      inverse FFT_x, keep x<L, epilogue, scatter
 //
 // Spectra layout (column-major like the reference's arrays, kx fastest):
-//   A[c][z][y][kx]  : 3 x N x M  x 2L   (after xfwd / before xinv)
-//   B[c][z][ky][kx] : 3 x N x 2M x 2L   (after the y transform)
+//   [c][z][ky][kx] : 3 x N x 2M x 2L, of which rows y < M hold [c][z][y][kx]
+//   after xfwd and before xinv (the y transforms work in place)
 // fN layout: fN[q][kz][ky][kx], q in [xx,xy,xz,yy,yz,zz], pre-scaled by 1/(8LMN)
 // so that the inverse transforms need no normalisation.
 #pragma once
@@ -116,6 +116,15 @@ __device__ __forceinline__ void stage_twiddles(V* tw_s, const V* __restrict__ tw
   for (int i = threadIdx.x; i < n; i += blockDim.x) tw_s[i] = tw[i];
 }
 
+// The x spectra lie in the planes they become: row y of plane w = z + N*c at
+// A + Lp * (y + Mp * w), the first M rows of a plane of the y pass, which works
+// in place.  (A scratch of their own, half as large again as the spectra, is not
+// needed: calls with bounded scratch take larger grids.)
+__device__ __forceinline__ long long spectrum_row(const Dims& d, int row) {
+  const int w = row / d.M;
+  return (long long)d.Lp * (row + (d.Mp - d.M) * w);
+}
+
 // ---------------------------------------------------------------------------
 // xfwd: gather + forward x transform.  grid.x = ceil(rows / S), grid.y = rhs
 // ---------------------------------------------------------------------------
@@ -132,6 +141,8 @@ k_xfwd(const IO* J, long long j_stride, const int* inv, Prologue pro,
   V* buf = tw_s + NL;
   const int rows = d.M * d.N * 3;
   const int row0 = blockIdx.x * S;
+  __shared__ long long at[S];  // the rows' places, one division each
+  if (threadIdx.x < S) at[threadIdx.x] = spectrum_row(d, row0 + threadIdx.x);
   stage_twiddles(tw_s, tw, NL);
   // the kernel before may have written the skip mask, the map, the factors and J
   pdl_wait();
@@ -164,7 +175,7 @@ k_xfwd(const IO* J, long long j_stride, const int* inv, Prologue pro,
   for (int i = threadIdx.x; i < S * NL; i += blockDim.x) {
     const int ss = i / NL, kx = i - ss * NL;
     const int row = row0 + ss;
-    if (row < rows) Ar[(long long)row * NL + kx] = buf[kx * ES + ss];
+    if (row < rows) Ar[at[ss] + kx] = buf[kx * ES + ss];
   }
 }
 
@@ -186,13 +197,16 @@ k_xinv(const cplx<T>* A, long long a_stride, const IO* __restrict__ J, long long
   if (rhs_skipped(d, blockIdx.y)) return;
   const int rows = d.M * d.N * 3;
   const int row0 = blockIdx.x * S;
+  __shared__ long long at[S];
+  if (threadIdx.x < S) at[threadIdx.x] = spectrum_row(d, row0 + threadIdx.x);
   stage_twiddles(tw_s, tw, NL);
+  __syncthreads();
   pdl_wait();  // A is the previous pass's output
   const V* Ar = after_wait(A) + blockIdx.y * a_stride;
   for (int i = threadIdx.x; i < S * NL; i += blockDim.x) {
     const int s = i / NL, kx = i - s * NL;
     const int row = row0 + s;
-    buf[kx * ES + s] = (row < rows) ? Ar[(long long)row * NL + kx] : mk<V>(0, 0);
+    buf[kx * ES + s] = (row < rows) ? Ar[at[s] + kx] : mk<V>(0, 0);
   }
   __syncthreads();
   const int s = threadIdx.x % S, t = threadIdx.x / S;
@@ -336,7 +350,7 @@ k_xfwd_rows(const IO* J, long long j_stride, const int* inv, Prologue pro,
   F::run_half(reg, xb, SAddr(1, true), t, tw_s);
   pdl_trigger();
   if (!valid) return;
-  float2* Ar = A + blockIdx.y * a_stride + (long long)row * NL;
+  float2* Ar = A + blockIdx.y * a_stride + spectrum_row(d, row);
 #pragma unroll
   for (int b = 0; b < E / RL; ++b)
 #pragma unroll
@@ -360,7 +374,7 @@ k_xinv_rows(const float2* A, long long a_stride, const IO* __restrict__ J, long 
   const bool valid = row < d.M * d.N * 3;
   stage_twiddles(tw_s, tw, NL);
   pdl_wait();  // A is the previous pass's output
-  const float2* Ar = after_wait(A) + blockIdx.y * a_stride + (long long)row * NL;
+  const float2* Ar = after_wait(A) + blockIdx.y * a_stride + spectrum_row(d, row);
   float2 reg[E];
 #pragma unroll
   for (int b = 0; b < E / R0; ++b)
@@ -391,11 +405,13 @@ template <typename T> struct ColS { static constexpr int S = 128 / (int)sizeof(c
 // Columns are loaded straight into the first pass's registers and the last
 // pass's registers are stored straight to global memory: lanes run over S
 // consecutive kx (one 128-byte row segment per warp access), the FFT's
-// exchanges go through shared memory only.
+// exchanges go through shared memory only.  in and out may be the same planes: a
+// column's outputs all follow its inputs (through the exchange's barrier, or in
+// one thread's registers).
 template <typename T, int NC, bool INV>
 __global__ void __launch_bounds__(ColS<T>::S * FFT<cplx<T>, NC, INV>::T)
 k_cols(const cplx<T>* in, long long in_w, long long in_rhs, int n_in,
-       cplx<T>* __restrict__ out, long long out_w, long long out_rhs, int n_out, int Lp,
+       cplx<T>* out, long long out_w, long long out_rhs, int n_out, int Lp,
        const cplx<T>* __restrict__ tw, const int* __restrict__ stop, int step) {
   if (stop && stop[blockIdx.z] < step) return;
   using V = cplx<T>;
@@ -471,22 +487,13 @@ template <> struct OpKind<1> {
   __host__ __device__ static constexpr bool odd(int q, int a) { return q == a; }
 };
 
-// z-pass variants the autotuner chooses from (FP32, N operator): 0 the
-// default (wide radix schedule where one exists, 8 columns per CTA), 1 the
-// narrow radix schedule, 2 half the columns per CTA.
-// FP64 takes 4 columns, and 8 for the lengths whose 4 threads per transform
-// would fill half a warp per component (96 points, 24 values per thread: the
-// product's three branches ran on half-empty warps).  z pass of a
-// 48^3 FP64 grid: 474 -> 281 us.
-template <typename T, int NZ, int VAR> struct ZVar {
-  static constexpr bool W = VAR == 1 ? false : (sizeof(cplx<T>) == 8 && HasWide<NZ>::value);
-  static constexpr int S0 = (sizeof(T) == 4 || FFT<cplx<T>, NZ, false, W>::T == 4 ? 8 : 4) / (VAR == 2 ? 2 : 1);
-};
-
-template <typename T, int NZ, int KIND = 0, int VAR = 0> struct ZS {
-  static constexpr bool W = ZVar<T, NZ, VAR>::W;             // radix schedule
-  static constexpr int TT = FFT<cplx<T>, NZ, false, W>::T;   // threads per transform
-  static constexpr int S0 = ZVar<T, NZ, VAR>::S0;            // columns per CTA
+// The z pass: FP32 takes 8 columns per CTA, FP64 takes 4, and 8 for the lengths
+// whose 4 threads per transform would fill half a warp per component (96 points,
+// 24 values per thread: the product's three branches ran on half-empty warps).
+// z pass of a 48^3 FP64 grid: 474 -> 281 us.
+template <typename T, int NZ, int KIND = 0> struct ZS {
+  static constexpr int TT = FFT<cplx<T>, NZ, false>::T;    // threads per transform
+  static constexpr int S0 = sizeof(T) == 4 || TT == 4 ? 8 : 4;  // columns per CTA, where the threads allow
   static constexpr int S = (3 * S0 * TT <= 1024) ? S0 : ((3 * (S0 / 2) * TT <= 1024) ? S0 / 2 : S0 / 4);
   static constexpr int THREADS = 3 * S * TT;               // one thread group per component
   // a component's threads fill whole warps: its row of the product is chosen by
@@ -683,15 +690,15 @@ __device__ __forceinline__ void zrow_k(V* reg, int t, int s, bool active, int oc
 // entries are the odd ones in y), the z reflection by the sign of the z-odd
 // entries per position.  Otherwise every thread copies its share of the tile
 // from the octant with cp.async and signs the x and y reflections in place.
-template <typename T, int NZ, int KIND, int VAR>
-__global__ void __launch_bounds__(ZS<T, NZ, KIND, VAR>::THREADS)
+template <typename T, int NZ, int KIND>
+__global__ void __launch_bounds__(ZS<T, NZ, KIND>::THREADS)
 k_zmul(cplx<T>* __restrict__ B, long long b_rhs, const cplx<T>* __restrict__ fN, int oct, Dims d,
        const cplx<T>* __restrict__ tw, const __grid_constant__ CUtensorMap tmap, int tma, int* err) {
   if (rhs_skipped(d, blockIdx.z)) return;
   using V = cplx<T>;
-  using ZC = ZS<T, NZ, KIND, VAR>;
-  using FF = FFT<V, NZ, false, ZC::W>;
-  using FI = FFT<V, NZ, true, ZC::W>;
+  using ZC = ZS<T, NZ, KIND>;
+  using FF = FFT<V, NZ, false>;
+  using FI = FFT<V, NZ, true>;
   using OK = OpKind<KIND>;
   constexpr int S = ZC::S;
   constexpr int BUF = ZC::BUF;

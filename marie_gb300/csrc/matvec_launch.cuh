@@ -50,20 +50,18 @@ template <typename T> struct MatvecLaunch {
                           long long out_w, long long out_rhs, int n_out, int Lp, int nw, const V* tw, int nrhs,
                           cudaStream_t st, const int* stop = nullptr, int step = 0);
   // kind 0: the symmetric N operator (6 components), 1: the K operator (3);
-  // var: the z-pass variant chosen by the autotuner (FP32, N operator)
   // zt: the bulk-copy tile source of an FP32 N operator (null: per-thread copies)
   static cudaError_t zmul(V* B, long long bs, const V* fN, int oct, const Dims& d, const V* tw, int nrhs,
-                          cudaStream_t st, int kind = 0, int var = 0, const ZTile* zt = nullptr);
+                          cudaStream_t st, int kind = 0, const ZTile* zt = nullptr);
   // fused x+y passes (thread-block clusters); fused() says whether this grid has them
   static bool fused(const Dims& d);
-  // fvar: 0 the default x/y radix schedules, 1 the narrow (radix-8) ones
   template <typename IO>
   static cudaError_t xyfwd(const IO* J, long long js, const int* inv, Prologue pro, V* B, long long bs,
-                           const Dims& d, const V* twx, const V* twy, int nrhs, cudaStream_t st, int fvar = 0);
+                           const Dims& d, const V* twx, const V* twy, int nrhs, cudaStream_t st);
   template <typename IO>
   static cudaError_t yxinv(const V* B, long long bs, const IO* J, long long js, const int* inv, Epilogue ep,
                            IO* out, long long os, const Dims& d, const V* twx, const V* twy, int nrhs,
-                           cudaStream_t st, int fvar = 0);
+                           cudaStream_t st);
 };
 
 }  // namespace marie

@@ -40,9 +40,11 @@ __global__ void k_coefficients(const int64_t* idx, long long n, long long V, con
 
 using namespace marie;
 
-// 64 MiB: an FP32 matvec needs about 204 bytes per voxel on grids with the
-// fused x+y passes and 252 on the others (up to 64^3 voxels fit); an FP64 one
-// about 396 (up to about 160k voxels).
+// 64 MiB.  The sizes that are taken are fixed: with every voxel's DOFs an FP32
+// matvec counts 204 bytes per voxel on the grids of compact() and 252 on the
+// others (up to 64^3 voxels fit), an FP64 one 396 (up to about 160k voxels).
+// The x spectra of the larger counts, half as much as the others, are only
+// counted: they lie inside the others.
 static constexpr size_t kStaticScratchBytes = 64ull << 20;
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
 
@@ -68,6 +70,13 @@ static int scratch_address(int dev, unsigned char** out) {
   return MARIE_OK;
 }
 
+static bool compact(const Dims& d) {
+  const int pairs[][2] = {{64, 64}, {96, 96}, {128, 128}, {192, 192}, {256, 256}, {512, 384}};
+  for (const auto& p : pairs)
+    if (d.Lp == p[0] && d.Mp == p[1]) return true;
+  return false;
+}
+
 static size_t up256(size_t b) { return (b + 255) & ~size_t(255); }
 
 template <typename T>
@@ -78,7 +87,7 @@ static int static_matvec(marie_plan* p, const double2* J, const double2* Mr, con
   const Dims d = p->d;
   const long long V3 = 3 * d.V;
   const bool fused = p->fuse && ML::fused(d);
-  // scratch layout: error flag | inv[3V] | a[n] | b[n] | B spectra | A spectra (grids without fused passes)
+  // scratch layout: error flag | inv[3V] | a[n] | b[n] | spectra
   size_t off = 0;
   int* err = reinterpret_cast<int*>(scratch + off);
   off += 256;
@@ -90,8 +99,7 @@ static int static_matvec(marie_plan* p, const double2* J, const double2* Mr, con
   off += up256(n * sizeof(double2));
   V* B = reinterpret_cast<V*>(scratch + off);
   off += up256(p->elems_B() * sizeof(V));
-  V* A = reinterpret_cast<V*>(scratch + off);
-  if (!fused) off += up256(p->elems_A() * sizeof(V));
+  if (sizeof(V) != 8 || !p->fuse || !compact(d)) off += up256(3LL * d.Lp * d.M * d.N * sizeof(V));  // counted, see above
   if (off > kStaticScratchBytes)
     return set_error(MARIE_EINVAL,
                      "marie_mv_AN_static: this grid and DOF count need %zu bytes of scratch, more than the %zu of "
@@ -130,20 +138,18 @@ static int static_matvec(marie_plan* p, const double2* J, const double2* Mr, con
   }
   const V* fN = sizeof(T) == 4 ? reinterpret_cast<const V*>(p->fN32) : reinterpret_cast<const V*>(p->fN64);
   V* const* tw = sizeof(T) == 4 ? reinterpret_cast<V* const*>(p->tw32) : reinterpret_cast<V* const*>(p->tw64);
-  const long long sA = p->elems_A(), sB = p->elems_B();
+  const long long sB = p->elems_B(), plane = (long long)d.Lp * d.Mp;
   if (fused) {
-    MARIE_CUDA_TRY(ML::xyfwd(J, n, inv, pro, B, sB, d, tw[0], tw[1], 1, st, p->fvar));
-    MARIE_CUDA_TRY(ML::zmul(B, sB, fN, p->oct, d, tw[2], 1, st, 0, p->zvar));
-    MARIE_CUDA_TRY(ML::yxinv(B, sB, J, n, inv, ep, out, n, d, tw[0], tw[1], 1, st, p->fvar));
+    MARIE_CUDA_TRY(ML::xyfwd(J, n, inv, pro, B, sB, d, tw[0], tw[1], 1, st));
+    MARIE_CUDA_TRY(ML::zmul(B, sB, fN, p->oct, d, tw[2], 1, st, 0));
+    MARIE_CUDA_TRY(ML::yxinv(B, sB, J, n, inv, ep, out, n, d, tw[0], tw[1], 1, st));
     count_launch(3);
   } else {
-    MARIE_CUDA_TRY(ML::xfwd(J, n, inv, pro, A, sA, d, tw[0], 1, st));
-    MARIE_CUDA_TRY(ML::cols(false, d.Mp, A, (long long)d.Lp * d.M, sA, d.M, B, (long long)d.Lp * d.Mp, sB, d.Mp,
-                            d.Lp, 3 * d.N, tw[1], 1, st));
-    MARIE_CUDA_TRY(ML::zmul(B, sB, fN, p->oct, d, tw[2], 1, st, 0, p->zvar));
-    MARIE_CUDA_TRY(ML::cols(true, d.Mp, B, (long long)d.Lp * d.Mp, sB, d.Mp, A, (long long)d.Lp * d.M, sA, d.M,
-                            d.Lp, 3 * d.N, tw[1], 1, st));
-    MARIE_CUDA_TRY(ML::xinv(A, sA, J, n, inv, ep, out, n, d, tw[0], 1, st));
+    MARIE_CUDA_TRY(ML::xfwd(J, n, inv, pro, B, sB, d, tw[0], 1, st));
+    MARIE_CUDA_TRY(ML::cols(false, d.Mp, B, plane, sB, d.M, B, plane, sB, d.Mp, d.Lp, 3 * d.N, tw[1], 1, st));
+    MARIE_CUDA_TRY(ML::zmul(B, sB, fN, p->oct, d, tw[2], 1, st, 0));
+    MARIE_CUDA_TRY(ML::cols(true, d.Mp, B, plane, sB, d.Mp, B, plane, sB, d.M, d.Lp, 3 * d.N, tw[1], 1, st));
+    MARIE_CUDA_TRY(ML::xinv(B, sB, J, n, inv, ep, out, n, d, tw[0], 1, st));
     count_launch(5);
   }
   MARIE_CUDA_TRY(cudaStreamSynchronize(st));

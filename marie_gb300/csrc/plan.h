@@ -25,8 +25,6 @@ struct marie_plan {
   float2* fN32 = nullptr;
   bool has_op = false;
   bool fuse = true;  // fused x+y / y+x passes when the grid has them
-  int fvar = 0;      // x/y radix schedule of the fused passes (set by marie_plan_autotune)
-  int zvar = 0;      // z-pass variant of the FP32 N matvec (set by marie_plan_autotune)
   int inner_prec = MARIE_FP64;  // Krylov basis of the mixed-precision inner solves
   int inner_restart = 0;        // their restart length (0: the caller's inner_it)
   int batch_groups = 2;         // batched GMRES: systems split into this many groups on their own streams
@@ -60,10 +58,9 @@ struct marie_plan {
   std::shared_ptr<marie_plan> crop;
   void* arena = nullptr;
 
-  // Spectra workspaces (A: 3 x N x M x 2L, B: 3 x N x 2M x 2L per rhs).
-  void* wsA = nullptr;
+  // Spectra workspace (3 x N x 2M x 2L per rhs).
   void* wsB = nullptr;
-  size_t ws_bytes_A = 0, ws_bytes_B = 0;
+  size_t ws_bytes_B = 0;
 
   // Optional per-pass timing of the matvec (events recorded between passes).
   bool profile = false;
@@ -89,7 +86,6 @@ struct marie_plan {
   double* pinned = nullptr;
   size_t pinned_len = 0;
 
-  long long elems_A() const { return 3LL * d.Lp * d.M * d.N; }
   long long elems_B() const { return 3LL * d.Lp * d.Mp * d.N; }
 };
 
@@ -147,7 +143,7 @@ struct HostPrefault {
   ~HostPrefault() { join(); }
 };
 
-int ensure_workspace(marie_plan* p, int prec, long long nrhs, bool with_A = true);
+int ensure_workspace(marie_plan* p, int prec, long long nrhs);
 int ensure_pinned(marie_plan* p, size_t n_doubles);
 
 // Build the inverse map inv[g] = k for 1-based idx[k]; -1 elsewhere.  Fails on

@@ -194,10 +194,10 @@ class Operator:
         return self
 
     def autotune(self):
-        """Time the FP32 matvec schedules of this grid (fused or five-pass x/y
-        passes, their radix schedule; z-pass radix schedule and columns per
-        CTA), keep the fastest.  Returns (chosen (fuse, fvar, zvar),
-        [(fuse, fvar, zvar, ms), ...])."""
+        """Time the FP32 matvec schedules of this grid (fused x/y passes where
+        it has them, and the five-pass form), keep the fastest.  Returns
+        (chosen (fuse, fvar, zvar), [(fuse, fvar, zvar, ms), ...]); fvar and
+        zvar are 0."""
         ms = np.zeros(4 * 32)
         fuse, fvar, zvar, cnt = C.c_int(), C.c_int(), C.c_int(), C.c_int64()
         check(self.lib.marie_plan_autotune(self.plan, C.byref(fuse), C.byref(fvar), C.byref(zvar),
@@ -207,7 +207,7 @@ class Operator:
         return (fuse.value, fvar.value, zvar.value), cands
 
     def set_schedule(self, fuse, fvar, zvar):
-        """Pin a matvec schedule (fuse 1/0; fused radix variant 0/1; z-pass variant 0, 1 or 2)."""
+        """Pin a matvec schedule: fuse 1/0; fvar and zvar (0 to 2) select nothing."""
         check(self.lib.marie_plan_set_schedule(self.plan, int(fuse), int(fvar), int(zvar)))
         return self
 

@@ -130,3 +130,24 @@ def test_static_matvec_follows_the_tuned_schedule(precision, cuda):
     r, o = ref.cpu().numpy(), out.cpu().numpy()
     assert np.max(np.abs(o - r)) <= TOL[precision] * np.max(np.abs(r))
     op.close()
+
+
+@pytest.mark.parametrize("shape", [(48, 48, 4), (64, 64, 80)])
+def test_static_matvec_takes_the_grids_that_count_one_scratch(shape, cuda):
+    """FP32 grids of 96 x 96 and 128 x 128 transforms, the second with every
+    voxel a DOF at the largest N that 204 bytes per voxel let in."""
+    import torch
+
+    import marie_gb300 as mg
+    from marie_gb300 import _lib
+
+    lib = _lib.load()
+    op = mg.Operator.assemble(*shape, 5e-3, 298e6, precision="fp32")
+    c = case(*shape, 9, 1.0, cuda)
+    ref = torch.zeros(c["n"], dtype=torch.complex128, device=cuda)
+    out = torch.full((c["n"],), complex("nan"), dtype=torch.complex128, device=cuda)
+    _lib.check(call(lib.marie_mv_AN, op.plan, c, 0, (1, _lib.MARIE_FP32), ref))
+    _lib.check(call_static_no_alloc(lib, op.plan, c, 0, _lib.MARIE_FP32, out))
+    torch.cuda.synchronize()
+    assert float((out - ref).abs().max()) <= TOL["fp32"] * float(ref.abs().max())
+    op.close()
