@@ -279,6 +279,10 @@ static int run_matvec_t(marie_plan* p, const IO* J, long long js, IO* out, long 
     const int nr = (int)((nrhs - r0) < chunk_max ? (nrhs - r0) : chunk_max);
     MARIE_TRY(ensure_workspace(p, prec, nr));
     Dims d = p->d;
+    if (pro.M) {
+      d.M = pro.M;
+      d.N = pro.N;
+    }
     d.stop = stop ? stop + r0 : nullptr;
     d.step = step;
     cplx<T>* B = reinterpret_cast<cplx<T>*>(p->wsB);
@@ -693,10 +697,12 @@ namespace marie {
 
 // The plan a bound product runs on, the crop of the bound DOFs where there is
 // one (per-pass timing wants the plan itself), and their map on it.
-static marie_plan* bound_plan(marie_plan* p, const int** inv) {
+static marie_plan* bound_plan(marie_plan* p, const int** inv, Prologue* pro) {
   if (p->bnd_crop && !p->profile) {
     crop_settings(p, p->bnd_crop.get());
     *inv = p->bnd_inv_crop;
+    pro->M = p->bnd_ext.M;
+    pro->N = p->bnd_ext.N;
     return p->bnd_crop.get();
   }
   *inv = p->bnd_inv;
@@ -710,8 +716,8 @@ int bound_operator(marie_plan* p, long long n, DevOp* op) {
   const int prec = p->fN64 ? MARIE_FP64 : MARIE_FP32;
   *op = [p, n, prec](const double2* x, double2* y) -> int {
     const int* inv;
-    marie_plan* q = bound_plan(p, &inv);
     Prologue pro{nullptr, 0};
+    marie_plan* q = bound_plan(p, &inv, &pro);
     Epilogue ep{};
     if (p->bnd_transp == 0) {
       ep.a = p->bnd_a;
@@ -835,7 +841,10 @@ int marie_plan_bind_mv_AN(marie_plan* p, const double* Mr, const double* Mc, dou
       p->bnd_inv_crop = nullptr;
       p->bnd_crop.reset();
     }
-    if (p->bnd_crop) s = build_inverse_box(p, p->bnd_crop.get(), origin, p->bnd_idx, n, p->bnd_inv_crop);
+    if (p->bnd_crop) {
+      p->bnd_ext = box_extent(p->bnd_crop.get(), box);
+      s = build_inverse_box(p, p->bnd_crop.get(), origin, p->bnd_ext, p->bnd_idx, n, p->bnd_inv_crop);
+    }
   }
   if (s == MARIE_OK && cudaStreamSynchronize(p->stream) != cudaSuccess) s = set_error(MARIE_ECUDA, "bind mv_AN failed");
   if (s != MARIE_OK) {
@@ -1138,7 +1147,7 @@ int marie_plan_apply_mv_AN(marie_plan* p, const double* JIn0, double* JOut, int6
     ep.bf = p->bnd_bf;
   }
   const int* inv;
-  marie_plan* q = bound_plan(p, &inv);
+  marie_plan* q = bound_plan(p, &inv, &pro);
   MARIE_TRY(run_matvec(q, precision, (const double2*)J_d, (double2*)out_d, n, (int)nrhs, inv, pro, ep));
   if (out_d != JOut) {
     MARIE_TRY(finish_out(JOut, out_d, n * nrhs * sizeof(double2), p->stream));

@@ -214,9 +214,17 @@ struct JvieState {
   // (inv is the DOF map on it)
   std::shared_ptr<marie_plan> crop;
   marie_plan* on(marie_plan* p) const { return crop ? crop.get() : p; }
+  Extent ext;
   DBuf idxS, idx3, inv, f, a, b, pa, pb;
   DBuf af, bf, paf, pbf;  // FP32 copies of a, b, pa, pb (plans with an FP32 operator)
 };
+
+// A map on the whole grid starts at the box's rows and planes, x keeps its place.
+static void whole_grid_origin(const int box[6], int origin[3]) {
+  origin[0] = 0;
+  origin[1] = -box[1];
+  origin[2] = -box[2];
+}
 
 static int jvie_setup(marie_plan* p, const double2* er, double dx, double freq, int form, JvieState& S) {
   cudaStream_t st = p->stream;
@@ -252,6 +260,7 @@ static int jvie_setup(marie_plan* p, const double2* er, double dx, double freq, 
   MARIE_TRY(S.pb.alloc(n * sizeof(double2), st));
   int origin[3];
   S.crop = crop_plan(p, hc.data() + CMP_BLOCKS, origin);
+  if (!S.crop) whole_grid_origin(hc.data() + CMP_BLOCKS, origin);
   MARIE_TRY(S.inv.alloc(3 * S.on(p)->d.V * sizeof(int), st));
   const double Gram = dx * dx * dx;
   const double omega = 2.0 * M_PI * freq;
@@ -272,8 +281,8 @@ static int jvie_setup(marie_plan* p, const double2* er, double dx, double freq, 
     MARIE_CUDA_TRY(cudaGetLastError());
   }
   // idx3 is in range and without repeats by construction
-  if (S.crop) return build_inverse_box(p, S.crop.get(), origin, S.idx3.as<int64_t>(), n, S.inv.as<int>());
-  return build_inverse_index(p, S.idx3.as<int64_t>(), n, S.inv.as<int>());
+  S.ext = box_extent(S.on(p), hc.data() + CMP_BLOCKS);
+  return build_inverse_box(p, S.on(p), origin, S.ext, S.idx3.as<int64_t>(), n, S.inv.as<int>());
 }
 
 static int any_nonzero(marie_plan* p, const double2* b, long long n, bool* nz) {
@@ -296,9 +305,10 @@ static BatchOp make_bop(marie_plan* p, int prec, const JvieState& S, const doubl
                         bool diag_only, const float2* af = nullptr, const float2* bf = nullptr) {
   const long long n = S.n;
   const int* inv = S.inv.as<int>();
+  const Extent ext = S.ext;
   BatchOp op;
   if (prec == MARIE_FP32 && af && bf) {
-    op.apply32 = [p, n, inv, af, bf, diag_only](const float2* in, long long is, float2* out, long long os, int ns,
+    op.apply32 = [p, n, inv, ext, af, bf, diag_only](const float2* in, long long is, float2* out, long long os, int ns,
                                                 const int* stop, int step) -> int {
       if (diag_only) {
         k_diag_b32<<<dim3(grid_n(n), ns), 256, 0, p->stream>>>(af, in, is, out, os, n, stop, step);
@@ -306,7 +316,7 @@ static BatchOp make_bop(marie_plan* p, int prec, const JvieState& S, const doubl
         MARIE_CUDA_TRY(cudaGetLastError());
         return MARIE_OK;
       }
-      Prologue pro{nullptr, 0};
+      Prologue pro{nullptr, 0, ext.M, ext.N};
       Epilogue ep{};
       ep.af = af;
       ep.bf = bf;
@@ -317,7 +327,7 @@ static BatchOp make_bop(marie_plan* p, int prec, const JvieState& S, const doubl
   // epilogue in FP32 with the coefficient copies af, bf, when given
   const float2* af_epi = prec == MARIE_FP32 ? af : nullptr;
   const float2* bf_epi = prec == MARIE_FP32 ? bf : nullptr;
-  op.apply = [p, prec, n, inv, a, b, af_epi, bf_epi, diag_only](const double2* in, long long is, double2* out,
+  op.apply = [p, prec, n, inv, ext, a, b, af_epi, bf_epi, diag_only](const double2* in, long long is, double2* out,
                                                                 long long os, int ns, const int* stop,
                                                                 int step) -> int {
     if (diag_only) {
@@ -326,7 +336,7 @@ static BatchOp make_bop(marie_plan* p, int prec, const JvieState& S, const doubl
       MARIE_CUDA_TRY(cudaGetLastError());
       return MARIE_OK;
     }
-    Prologue pro{nullptr, 0};
+    Prologue pro{nullptr, 0, ext.M, ext.N};
     Epilogue ep{};
     ep.a = a;
     ep.b = b;
@@ -769,7 +779,7 @@ int jvie_adjoint_core(marie_plan* p, const double2* Einc, const double2* er, dou
   // adjoint solve A lambda = w (rows divided by eps_c, like the forward form 2)
   MARIE_TRY(solve_systems(on, S, w.as<double2>(), 1, lam.as<double2>(), 0, tol, inner_it, outer_it, adj));
   // q = (Gram - N) lambda in FP64
-  Prologue pro{nullptr, 0};
+  Prologue pro{nullptr, 0, S.ext.M, S.ext.N};
   Epilogue ep{};
   ep.a_s = mk<double2>(dx * dx * dx, 0.0);
   ep.b_s = mk<double2>(1.0, 0.0);
@@ -1125,7 +1135,9 @@ int marie_jvie2solver(marie_plan* p, const int64_t* idx, int64_t n_idx, const do
       MARIE_TRY(dof_box(p, S.idx3.as<int64_t>(), n, box));
       S.crop = crop_plan(p, box, origin);
       // (the crop's map needs less than the whole grid's)
-      if (S.crop) MARIE_TRY(build_inverse_box(p, S.crop.get(), origin, S.idx3.as<int64_t>(), n, S.inv.as<int>()));
+      if (!S.crop) whole_grid_origin(box, origin);
+      S.ext = box_extent(S.on(p), box);
+      MARIE_TRY(build_inverse_box(p, S.on(p), origin, S.ext, S.idx3.as<int64_t>(), n, S.inv.as<int>()));
     }
     MARIE_TRY(build_coefficients(p, S.idx3.as<int64_t>(), n, (const double2*)Mr_d, (const double2*)Mc_d, Gram, 0,
                                  S.a.as<double2>(), S.b.as<double2>()));

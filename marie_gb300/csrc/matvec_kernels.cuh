@@ -24,6 +24,10 @@
 
 namespace marie {
 
+// The passes take the rows and planes from M and N, the transform lengths (and
+// the operator, stored for Lp/2 x Mp/2 x Np/2) from Lp, Mp and Np: with a
+// smaller M or N (an Extent) the rows and planes beyond are zero and are neither
+// read, transformed nor written.
 struct Dims {
   int L, M, N, Lp, Mp, Np;
   long long V;  // L*M*N
@@ -71,9 +75,16 @@ struct Epilogue {
   const float2* bf;
 };
 // Prologue: x_in[k] = (pre ? pre[k] : 1) * (conjin ? conj(J[k]) : J[k])
+// Rows (y) and planes (z) of a DOF map that starts at its body's box, 0: the
+// whole grid's.
+struct Extent {
+  int M = 0, N = 0;
+};
+
 struct Prologue {
   const double2* pre;
   int conjin;
+  int M = 0, N = 0;  // the map's rows and planes (Extent), 0: the plan's
 };
 
 // The matvec's input and output vectors are FP64 (IO = double2) or, for the
@@ -714,9 +725,9 @@ k_zmul(cplx<T>* __restrict__ B, long long b_rhs, const cplx<T>* __restrict__ fN,
   // read the same operator tile (ky and its y reflection 2M - ky) run one
   // grid row apart, so the second copy finds the tile in L2
   const int gy = blockIdx.y;
-  const int ky = gy == 0 ? 0 : gy == 1 ? d.M : (gy & 1) ? d.Mp - (gy >> 1) : (gy >> 1);
+  const int ky = gy == 0 ? 0 : gy == 1 ? d.Mp / 2 : (gy & 1) ? d.Mp - (gy >> 1) : (gy >> 1);
   const long long plane = (long long)d.Lp * d.Mp;  // one z-plane of B
-  const long long comp = plane * NH;                // one component of B
+  const long long comp = plane * d.N;               // one component of B
   const int c = threadIdx.x / (S * FF::T);
   const int rem = threadIdx.x - c * S * FF::T;
   const int s = rem % S, t = rem / S;
@@ -725,10 +736,10 @@ k_zmul(cplx<T>* __restrict__ B, long long b_rhs, const cplx<T>* __restrict__ fN,
   tile = reinterpret_cast<V*>(reinterpret_cast<char*>(tile) +
                               ((128u - ((unsigned)__cvta_generic_to_shared(tile) & 127u)) & 127u));
   const bool active = kx0 + s < d.Lp;
-  const bool fy = oct && ky > d.M;
+  const bool fy = oct && ky > d.Mp / 2;
   const int oy = fy ? d.Mp - ky : ky;
-  const long long fq = oct ? (long long)(d.L + 1) * (d.M + 1) * NO : (long long)d.Lp * d.Mp * d.Np;
-  const long long fplane = oct ? (long long)(d.L + 1) * (d.M + 1) : plane;
+  const long long fq = oct ? (long long)(d.L + 1) * (d.Mp / 2 + 1) * NO : (long long)d.Lp * d.Mp * d.Np;
+  const long long fplane = oct ? (long long)(d.L + 1) * (d.Mp / 2 + 1) : plane;
   const long long frow = oct ? (long long)(d.L + 1) : d.Lp;
   // Tile rows (q, oz) of S columns: this thread copies column s of rows
   // row0, row0 + STEP, ... (THREADS is a multiple of S).
@@ -780,7 +791,7 @@ k_zmul(cplx<T>* __restrict__ B, long long b_rhs, const cplx<T>* __restrict__ fN,
 #pragma unroll
     for (int r = 0; r < R0; ++r) {
       const int p = FF::in_pos(t, b, r);
-      reg[b * R0 + r] = (active && r < R0 / 2 && p < NH) ? __ldcg(Bp + p * plane + s) : mk<V>(0, 0);
+      reg[b * R0 + r] = (active && r < R0 / 2 && p < d.N) ? __ldcg(Bp + p * plane + s) : mk<V>(0, 0);
     }
   __syncthreads();  // twiddles staged
   V* my = buf + c * BUF + s;
@@ -875,7 +886,7 @@ k_zmul(cplx<T>* __restrict__ B, long long b_rhs, const cplx<T>* __restrict__ fN,
 #pragma unroll
     for (int r = 0; r < RLI; ++r) {
       const int z = FI::out_pos(t, b, r);
-      if (active && z < NH) Bp[z * plane + s] = reg[b * RLI + r];
+      if (active && z < d.N) Bp[z * plane + s] = reg[b * RLI + r];
     }
 }
 

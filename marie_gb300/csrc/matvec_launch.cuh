@@ -20,7 +20,8 @@ inline bool fft_length_supported(int n) {
 bool smem_opted_in(const void* kernel, size_t bytes);
 void smem_mark_opted_in(const void* kernel, size_t bytes);
 template <typename K> inline cudaError_t opt_in_smem(K kernel, size_t bytes) {
-  if (bytes <= 48 * 1024 || smem_opted_in((const void*)kernel, bytes)) return cudaSuccess;
+  // 48 KB without it, the kernel's static arrays (up to 2 KB) included
+  if (bytes <= 46 * 1024 || smem_opted_in((const void*)kernel, bytes)) return cudaSuccess;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (e == cudaSuccess) smem_mark_opted_in((const void*)kernel, bytes);
   return e;

@@ -93,8 +93,8 @@ k_zmul_pairs(float2* __restrict__ B, long long b_rhs, Dims d, const float2* __re
   const int kx0 = blockIdx.x * Z::S;
   // rows in the order 0, M, 1, 2M-1, 2, ...: the two that share a tile adjacent
   const int gy = blockIdx.y;
-  const int ky = gy == 0 ? 0 : gy == 1 ? d.M : (gy & 1) ? d.Mp - (gy >> 1) : (gy >> 1);
-  const bool fy = ky > d.M;
+  const int ky = gy == 0 ? 0 : gy == 1 ? d.Mp / 2 : (gy & 1) ? d.Mp - (gy >> 1) : (gy >> 1);
+  const bool fy = ky > d.Mp / 2;
   const int oy = fy ? d.Mp - ky : ky;
   const long long plane = (long long)d.Lp * d.Mp;
   const int c = threadIdx.x / (P * FF::T);
@@ -120,7 +120,7 @@ k_zmul_pairs(float2* __restrict__ B, long long b_rhs, Dims d, const float2* __re
     tw_s[i] = cpk{pk(w.x), pk(w.y)};
   }
   pdl_wait();  // the spectrum B is the previous pass's output
-  float2* Bp = after_wait(B) + blockIdx.z * b_rhs + c * plane * NH + (long long)ky * d.Lp + kx0 + 2 * s;
+  float2* Bp = after_wait(B) + blockIdx.z * b_rhs + c * plane * d.N + (long long)ky * d.Lp + kx0 + 2 * s;
   float4 in[E / R0 * (R0 / 2)];
 #pragma unroll
   for (int b = 0; b < E / R0; ++b)
@@ -128,7 +128,7 @@ k_zmul_pairs(float2* __restrict__ B, long long b_rhs, Dims d, const float2* __re
     for (int r = 0; r < R0 / 2; ++r) {
       const int p = FF::in_pos(t, b, r);
       in[b * (R0 / 2) + r] =
-          p < NH ? __ldcg(reinterpret_cast<const float4*>(Bp + p * plane)) : make_float4(0.f, 0.f, 0.f, 0.f);
+          p < d.N ? __ldcg(reinterpret_cast<const float4*>(Bp + p * plane)) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
   __syncthreads();  // twiddles staged, barrier initialised
   cpk reg[E];
@@ -185,7 +185,7 @@ k_zmul_pairs(float2* __restrict__ B, long long b_rhs, Dims d, const float2* __re
 #pragma unroll
     for (int r = 0; r < RLI; ++r) {
       const int z = FI::out_pos(t, b, r);
-      if (z < NH) *reinterpret_cast<float4*>(Bp + z * plane) = unpack2(reg[b * RLI + r]);
+      if (z < d.N) *reinterpret_cast<float4*>(Bp + z * plane) = unpack2(reg[b * RLI + r]);
     }
 }
 

@@ -81,6 +81,7 @@ struct marie_plan {
   int bnd_transp = 0;
   std::shared_ptr<marie_plan> bnd_crop;  // the bound DOFs' crop and their inverse map on it
   int* bnd_inv_crop = nullptr;
+  marie::Extent bnd_ext;
 
   // Pinned host staging for small scalars (reductions, Hessenberg columns).
   double* pinned = nullptr;
@@ -176,13 +177,15 @@ int expand_octant(const double2* o, int L, int M, int N, int kind, double s, dou
 // finding the box; dof_box: the box (max of -x -y -z, x y z) of 1-based DOFs;
 // crop_plan: the plan's operator on the box's grid with the plan's settings, or
 // null to stay on the whole grid, origin the box's first voxel; crop_settings:
-// the plan's present settings again; build_inverse_box: DOF map on that grid.
+// the plan's present settings again; box_extent: the box's rows and planes on a
+// plan; build_inverse_box: DOF map on the plan q (a crop, or p itself).
 bool crop_possible(const marie_plan* p);
 int dof_box(marie_plan* p, const int64_t* idx_dev, long long n, int box[6]);
 std::shared_ptr<marie_plan> crop_plan(marie_plan* p, const int box[6], int origin[3]);
 void crop_settings(const marie_plan* p, marie_plan* q);
-int build_inverse_box(marie_plan* p, marie_plan* q, const int origin[3], const int64_t* idx_dev, long long n,
-                      int* inv);
+Extent box_extent(const marie_plan* q, const int box[6]);
+int build_inverse_box(marie_plan* p, marie_plan* q, const int origin[3], const Extent& ext, const int64_t* idx_dev,
+                      long long n, int* inv);
 // elements of the FP32 operator stored full along x; the FP32 copies of a
 // crop's octant (fN32, and fN32x into the given memory)
 size_t fullx_elems(const Dims& d);

@@ -181,3 +181,37 @@ def test_solves_on_the_bodys_box(cuda, shape, lo, size, precision):
             assert np.count_nonzero(inside) == np.count_nonzero(x)  # nothing outside the body
     op.close()
     ref_op.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("shape,lo,size", [((12, 12, 20), (2, 4, 5), (8, 8, 12)), ((40, 24, 40), (0, 3, 0), (40, 20, 40)),
+                                           ((40, 40, 24), (0, 0, 4), (40, 40, 20)),
+                                           ((32, 32, 48), (0, 0, 3), (32, 32, 40))])
+def test_solves_on_the_bodys_rows_and_planes(cuda, shape, lo, size, precision):
+    """Grids that are not cut to the body's box (small, or filled to more than
+    0.8): the passes run over the box's rows and planes of the whole grid, the
+    last shape with the fused x+y passes in FP32.  Against a grid that is the
+    box, as above."""
+    import marie_gb300 as mg
+
+    dx, em = 4e-3, vo.EMconstants(FREQ)
+    cut = tuple(slice(a, a + s) for a, s in zip(lo, size))
+    r, er = _off_centre_body(shape, lo, size)
+    E = np.asfortranarray(vo.PlaneWave_Excitation(r, [0, 0, em["ko"]], em["omega_mu"], [1, 0, 0])[0])
+    out = []
+    for grid, c in ((shape, (slice(None),) * 3), (size, cut)):
+        op = mg.Operator.assemble(*grid, dx, FREQ, precision=precision)
+        ec, Ec, rc = (np.asfortranarray(a[c]) for a in (er, E, r))
+        J, flag = mg.JVIE_Solver(Ec, ec, rc, FREQ, op, tol=1e-9, solver="G")[:2]
+        V = ec.size
+        idxS = np.flatnonzero(np.abs(ec.reshape(-1, order="F") - 1) > 1e-12) + 1
+        idx = np.concatenate([idxS, V + idxS, 2 * V + idxS]).astype(np.int64)
+        b = Ec.reshape(-1, order="F")[idx - 1] * dx**3
+        x, flag2 = mg.jvie2solver(b, op, idx, np.asfortranarray(ec / ec), np.asfortranarray((ec - 1) / ec), dx**3, 1e-9)[:2]
+        assert flag == 0 and flag2 == 0
+        out.append((J if grid == size else J[cut], x, np.count_nonzero(J)))
+        op.close()
+    (J, x, nz), (Jr, xr, nzr) = out
+    assert nz == nzr
+    assert np.linalg.norm(J - Jr) <= 1e-6 * np.linalg.norm(Jr)
+    assert np.linalg.norm(x - xr) <= 1e-6 * np.linalg.norm(xr)
