@@ -66,9 +66,9 @@ def headline_config(er, world):
 # restatement takes the same iterations by parity); used only to scale the CPU
 # arm's per-iteration time to solves/s.
 FP64_ITERATIONS_C2 = 220
-# DRAM traffic of one z-pass launch (k_zmul<float,256>) at this workload, read
-# from the committed ncu summary of that kernel.
-ZMUL_PROFILE = ROOT / "profiles" / "k_zmul_f32_128cube.md"
+# DRAM traffic of one z-pass launch (k_zmul_pairs<256>, every voxel a DOF) at this
+# workload, read from the committed ncu summary of that kernel.
+ZMUL_PROFILE = ROOT / "profiles" / "k_zmul_pairs_f32_128cube.md"
 
 
 def zmul_traffic():
@@ -352,7 +352,7 @@ def run_gpu(args, world, rank, local):
                           "fp32_bound": mv["fp32_bound_ms"], "fp64_bound": mv["fp64_bound_ms"],
                           "note": "fp32/fp64: marie_mv_AN per call, which rebuilds the DOF map and coefficients; "
                                   "*_bound: marie_plan_apply_mv_AN, the solver's matvec (map and coefficients "
-                                  "bound once; FP32 epilogue in FP32)"},
+                                  "bound once, on the body's box; FP32 epilogue in FP32)"},
             "assembly_s": round(t_asm, 3),
             "autotune": {"chosen": {"fused_xy": tuned[0], "xy_variant": tuned[1], "z_variant": tuned[2]},
                          "candidates_ms": [{"fused_xy": f, "xy_variant": fv, "z_variant": z, "ms": round(ms, 4)}
@@ -363,8 +363,9 @@ def run_gpu(args, world, rank, local):
                          "peak_kind": kind, "alg_bytes_per_launch": dom["bytes"]},
             "matvec_roofline": {"alg_bytes": mv["alg_bytes"], "gbs": round(mv["alg_bytes"] / (mv["fp32_ms"] / 1e3) / 1e9, 1),
                                 "frac": round(mv["alg_bytes"] / (mv["fp32_ms"] / 1e3) / 1e9 / hbm, 4),
-                                "bound_gbs": round(mv["alg_bytes"] / (mv["fp32_bound_ms"] / 1e3) / 1e9, 1),
-                                "bound_frac": round(mv["alg_bytes"] / (mv["fp32_bound_ms"] / 1e3) / 1e9 / hbm, 4)},
+                                "bound_alg_bytes": mv["bound_alg_bytes"],
+                                "bound_gbs": round(mv["bound_alg_bytes"] / (mv["fp32_bound_ms"] / 1e3) / 1e9, 1),
+                                "bound_frac": round(mv["bound_alg_bytes"] / (mv["fp32_bound_ms"] / 1e3) / 1e9 / hbm, 4)},
             "e2e": {"value": round(world / t_e2e, 4), "unit": "solves/s", "h2d_bytes_per_step": 4 * V * 16,
                     "d2h_bytes_per_step": 3 * V * 16, "per_solve_ms": e2e_ms, "library_ms": e2e_lib_ms,
                     "clocks": clk_e2e.summary()},
@@ -464,6 +465,15 @@ def matvec_times(mg, op, op64, er, lib):
     res["dominant"] = {"name": names[k], "bytes": pass_bytes[k],
                        "gbs": pass_bytes[k] / (res["fp32_passes"][k] / 1e3) / 1e9}
     res["alg_bytes"] = S * 56 * V + fN_oct
+    # the bound product runs on the smallest transform grid that holds the body,
+    # over the body's rows and planes: 12 + 24 + 12 complex64 of spectra and 8 of
+    # vectors per voxel of it
+    nz = np.nonzero(np.abs(er - 1) > 1e-12)
+    need = [int(a.max() - a.min()) + 1 for a in nz]
+    Lb, Mb, Nb = (mg.supported_size(a) for a in need)
+    if Lb * Mb * Nb > 0.8 * V:
+        Lb, Mb, Nb, need = L, M, N, [L, M, N]
+    res["bound_alg_bytes"] = S * 56 * Lb * need[1] * need[2] + 6 * (Lb + 1) * (Mb + 1) * (Nb + 1) * S
     return res
 
 

@@ -321,7 +321,7 @@ void crop_settings(const marie_plan* p, marie_plan* q) {
   q->graph_refine = p->graph_refine;
 }
 
-// The body seldom fills its transform grid either (122 x 72 x 98 voxels of 128 x
+// The body seldom fills its transform grid either (98 x 72 x 122 voxels of 128 x
 // 80 x 128): the passes run over its rows and planes only.  Measured with
 // ellipsoid phantoms: FP64 product of a 96 x 80 x 64 grid 538 -> 519 us, FP32
 // product of 128^3 335 -> 322, of 256 x 192 x 160 341 -> 332, mixed solve of

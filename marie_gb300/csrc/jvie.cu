@@ -29,7 +29,7 @@ namespace marie {
 // per basis vector per step at 128^3 on the FP64 pipe, so shorter cycles win
 // although they take more matvecs: measured on the 128^3 phantom, restart
 // 12 / 20 / 30 / 50 gave 224 / 224 / 241 / 262 ms per solve (303 / 273 / 261 /
-// 236 matvecs).  With the FP32 basis the time is flat in the restart and the
+// 236 matvecs) with products of 0.455 ms (0.25 ms since; 20 takes 156 ms).  With the FP32 basis the time is flat in the restart and the
 // caller's inner_it is kept.
 constexpr int kInnerRestart64 = 20;
 
