@@ -520,14 +520,13 @@ static EncodeTiledFn encode_tiled() {
   return fn;
 }
 
-// The z pass's bulk tile source of an FP32 octant N operator: fN32x and one
-// tensor map per box width (8, 4, 2 columns) over (2L, M+1, N+1, 6) 8-byte
-// elements.  Without the driver entry point, or with N + 1 > 256 (beyond the
+// The z pass's bulk tile source of an FP32 octant N operator: fN32x and its
+// tensor map (boxes of 8 columns) over (2L, M+1, N+1, 6) 8-byte elements.  Without the driver entry point, or with N + 1 > 256 (beyond the
 // box limit), the plan keeps the per-thread tile copies.
 size_t fullx_elems(const Dims& d) { return (size_t)6 * d.Lp * (d.M + 1) * (d.N + 1); }
 
 // Fills p->fN32x from the operator (full or octant, scaled by s here) and
-// encodes its tensor maps; false when the driver refuses a map.
+// encodes its tensor map; false when the driver refuses it.
 static bool encode_zt(marie_plan* p, const double2* src, int oct, double s) {
   const Dims& d = p->d;
   EncodeTiledFn enc = encode_tiled();
@@ -541,14 +540,11 @@ static bool encode_zt(marie_plan* p, const double2* src, int oct, double s) {
   const cuuint64_t gs[3] = {(cuuint64_t)d.Lp * 8, (cuuint64_t)d.Lp * (d.M + 1) * 8,
                             (cuuint64_t)d.Lp * (d.M + 1) * (d.N + 1) * 8};
   const cuuint32_t es[4] = {1, 1, 1, 1};
-  const int widths[3] = {8, 4, 2};
-  for (int i = 0; i < 3; ++i) {
-    const cuuint32_t bd[4] = {(cuuint32_t)widths[i], 1, (cuuint32_t)d.N + 1, 6};
-    const CUresult r = enc(&p->zt.map[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, p->fN32x, gd, gs, bd, es,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return false;
-  }
+  const cuuint32_t bd[4] = {8, 1, (cuuint32_t)d.N + 1, 6};
+  const CUresult r = enc(&p->zt.map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, p->fN32x, gd, gs, bd, es,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return false;
   p->zt.ok = 1;
   return true;
 }

@@ -105,22 +105,13 @@ template <typename T> struct MatvecImpl {
   }
   template <int NZ, int KIND>
   static cudaError_t zmul_nk(V* B, long long bs, const V* fN, int oct, const Dims& d, const V* tw, int nrhs,
-                             cudaStream_t st, const ZTile* zt) {
+                             cudaStream_t st) {
     using ZC = ZS<T, NZ, KIND>;
-    constexpr int S = ZC::S;
-    // the bulk-copy tile needs a tensor map whose box is S columns wide
-    const int mi = S == 8 ? 0 : S == 4 ? 1 : S == 2 ? 2 : -1;
-    int tma = (ZC::TMA && zt && zt->ok && oct && mi >= 0) ? 1 : 0;
-    if (tma && take_tile_timeout_injection()) tma = 2;  // test: a wait that runs out
-    CUtensorMap none;
-    memset(&none, 0, sizeof(none));
-    const CUtensorMap& tmap = tma ? zt->map[mi] : none;
-    int* err = zt ? zt->err : nullptr;
-    const size_t smem = (size_t)ZC::bytes(S);  // S columns, 3 component buffers, operator tile
-    cudaError_t e = opt_in_smem(k_zmul<T, NZ, KIND>, smem);
+    constexpr int S = ZC::S;  // S columns, 3 component buffers, operator tile
+    cudaError_t e = opt_in_smem(k_zmul<T, NZ, KIND>, ZC::bytes);
     if (e != cudaSuccess) return e;
-    return launch_pass(k_zmul<T, NZ, KIND>, dim3((d.Lp + S - 1) / S, d.Mp, nrhs), ZC::THREADS, smem, st, B, bs, fN,
-                       oct, d, tw, tmap, tma, err);
+    return launch_pass(k_zmul<T, NZ, KIND>, dim3((d.Lp + S - 1) / S, d.Mp, nrhs), ZC::THREADS, ZC::bytes, st, B, bs,
+                       fN, oct, d, tw);
   }
   // the z pass on column pairs (FP32, a tile by bulk copy)
   template <int NZ>
@@ -130,16 +121,16 @@ template <typename T> struct MatvecImpl {
     const int tma = take_tile_timeout_injection() ? 2 : 1;  // 2: a test, a wait that runs out
     cudaError_t e = opt_in_smem(k_zmul_pairs<NZ>, Z::bytes);
     if (e != cudaSuccess) return e;
-    return launch_pass(k_zmul_pairs<NZ>, dim3(d.Lp / Z::S, d.Mp, nrhs), Z::THREADS, Z::bytes, st, B, bs, d, tw, zt->map[0],
+    return launch_pass(k_zmul_pairs<NZ>, dim3(d.Lp / Z::S, d.Mp, nrhs), Z::THREADS, Z::bytes, st, B, bs, d, tw, zt->map,
                        tma, zt->err);
   }
   template <int NZ>
   static cudaError_t zmul_n(V* B, long long bs, const V* fN, int oct, const Dims& d, const V* tw, int nrhs,
                             cudaStream_t st, int kind, const ZTile* zt) {
-    if (kind == 1) return zmul_nk<NZ, 1>(B, bs, fN, oct, d, tw, nrhs, st, nullptr);
+    if (kind == 1) return zmul_nk<NZ, 1>(B, bs, fN, oct, d, tw, nrhs, st);
     if constexpr (sizeof(T) == 4 && ZP<NZ>::ok)
       if (oct && zt && zt->ok) return zmul_pairs<NZ>(B, bs, d, tw, nrhs, st, zt);
-    return zmul_nk<NZ, 0>(B, bs, fN, oct, d, tw, nrhs, st, zt);
+    return zmul_nk<NZ, 0>(B, bs, fN, oct, d, tw, nrhs, st);
   }
 
   template <typename IO>

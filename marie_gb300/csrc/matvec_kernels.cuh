@@ -516,13 +516,7 @@ template <typename T, int NZ, int KIND = 0> struct ZS {
   static constexpr int BUF = NZ * ES + (HALF ? (NZ / 16 + 1) * S : 0);  // one component's exchange buffer
   // octant operator tile of the CTA's columns: NQ components x (N+1) planes x S
   static constexpr int TILE = OpKind<KIND>::NQ * (NZ / 2 + 1) * S;
-  // + 128 bytes so that the tile can start on a 128-byte boundary (bulk tensor copies)
-  static constexpr long long bytes(int) { return (long long)(NZ + 3 * BUF + TILE) * sizeof(cplx<T>) + 128; }
-  // The tile arrives by one bulk tensor copy (cp.async.bulk.tensor) from the
-  // FP32 N operator stored full along x: needs FP32 values, the N operator, an
-  // even column count (the box starts on a 16-byte boundary) and at most 256
-  // octant planes (the box limit).
-  static constexpr bool TMA = sizeof(T) == 4 && KIND == 0 && S % 2 == 0 && NZ / 2 + 1 <= 256;
+  static constexpr size_t bytes = (size_t)(NZ + 3 * BUF + TILE) * sizeof(cplx<T>);
   __device__ static SAddr addr() { return SAddr(ES, false, HALF ? S : 0); }
 };
 
@@ -556,25 +550,13 @@ template <typename V> __device__ __forceinline__ V cfma(V a, V b, V c) {
   return mk<V>(fma(-a.y, b.y, fma(a.x, b.x, c.x)), fma(a.y, b.x, fma(a.x, b.y, c.y)));
 }
 
-// Column s of a tile row: as it stands, or (pairs, the bulk copy's FP32 tile)
-// from {re, re, im, im} of the column and its neighbour.
-template <typename V> __device__ __forceinline__ V tile_at(const V* tile, int row, int s, bool pairs) {
-  if constexpr (sizeof(V) == 8) {
-    if (pairs) {
-      const float* p = reinterpret_cast<const float*>(tile + row + (s & ~1)) + (s & 1);
-      return mk<V>(p[0], p[2]);
-    }
-  }
-  return tile[row + s];
-}
-
 // Row C of the product at this thread's output positions of the forward
 // transform.  With the octant operator the tile already carries the x and y
 // reflection signs; the z reflection (positions kz > NZ/2) flips the two
 // z-odd components.  Without it the full operator is read from global memory.
 template <int C, typename FF, typename V, int NZ, int S>
-__device__ __forceinline__ void zrow(V* reg, int t, int s, bool active, int oct, bool pairs, const V* tile,
-                                     const V* fp, long long fq, long long fplane, const V* b0, const V* b1, const V* b2,
+__device__ __forceinline__ void zrow(V* reg, int t, int s, bool active, int oct, const V* tile, const V* fp,
+                                     long long fq, long long fplane, const V* b0, const V* b1, const V* b2,
                                      SAddr ad) {
   using RW = ZRow<C>;
   constexpr int NH = NZ / 2, NO = NH + 1, RL = FF::RL;
@@ -589,9 +571,9 @@ __device__ __forceinline__ void zrow(V* reg, int t, int s, bool active, int oct,
         if (oct) {
           const bool fz = kz > NH;
           const int oz = fz ? NZ - kz : kz;
-          n0 = tile_at(tile, (RW::q0 * NO + oz) * S, s, pairs);
-          n1 = tile_at(tile, (RW::q1 * NO + oz) * S, s, pairs);
-          n2 = tile_at(tile, (RW::q2 * NO + oz) * S, s, pairs);
+          n0 = tile[(RW::q0 * NO + oz) * S + s];
+          n1 = tile[(RW::q1 * NO + oz) * S + s];
+          n2 = tile[(RW::q2 * NO + oz) * S + s];
           if constexpr (odd_z(RW::q0)) n0 = neg_if(n0, fz);
           if constexpr (odd_z(RW::q1)) n1 = neg_if(n1, fz);
           if constexpr (odd_z(RW::q2)) n2 = neg_if(n2, fz);
@@ -613,7 +595,7 @@ __device__ __forceinline__ void zrow(V* reg, int t, int s, bool active, int oct,
 // each cost a whole warp's issue slots (FP64: 16 cycles per instruction).
 // z pass of a 40^3 FP64 grid (80 points, with the 8-column tiles): 299 -> 185 us.
 template <typename FF, typename V, int NZ, int S>
-__device__ __forceinline__ void zrow_any(V* reg, int c, int t, int s, bool active, int oct, bool pairs,
+__device__ __forceinline__ void zrow_any(V* reg, int c, int t, int s, bool active, int oct,
                                          const V* tile, const V* fp, long long fq, long long fplane, const V* b0, const V* b1, const V* b2,
                                          SAddr ad) {
   constexpr int NH = NZ / 2, NO = NH + 1, RL = FF::RL;
@@ -629,9 +611,9 @@ __device__ __forceinline__ void zrow_any(V* reg, int c, int t, int s, bool activ
         if (oct) {
           const bool fz = kz > NH;
           const int oz = fz ? NZ - kz : kz;
-          n0 = neg_if(tile_at(tile, (q0 * NO + oz) * S, s, pairs), fz && q0 == 2);
-          n1 = neg_if(tile_at(tile, (q1 * NO + oz) * S, s, pairs), fz && q1 == 4);
-          n2 = neg_if(tile_at(tile, (q2 * NO + oz) * S, s, pairs), fz && q2 != 5);
+          n0 = neg_if(tile[(q0 * NO + oz) * S + s], fz && q0 == 2);
+          n1 = neg_if(tile[(q1 * NO + oz) * S + s], fz && q1 == 4);
+          n2 = neg_if(tile[(q2 * NO + oz) * S + s], fz && q2 != 5);
         } else {
           const long long o = (long long)kz * fplane;
           n0 = fp[q0 * fq + o];
@@ -690,21 +672,13 @@ __device__ __forceinline__ void zrow_k(V* reg, int t, int s, bool active, int oc
 // forms row c of the symmetric product and runs its inverse transform from
 // the registers (the inverse radix order starts where the forward ended).
 //
-// Operator tile (octant operators, oct = 1): with tma = 1 (FP32 N operator)
-// one thread issues a single bulk tensor copy of the S columns x (N+1) planes
-// x 6 components from the copy of the operator stored full along x (x
-// reflections already carry their signs there) and every thread waits on the
-// copy's mbarrier, with a time limit after which err is set and the pass goes
-// on (tma = 2: a test of that path, the barrier armed for more bytes than the
-// copy delivers); the y reflection is applied as N -> D N D with D = diag(1, -1, 1) on the
-// y component's spectrum and product row (the symmetric tensor's xy and yz
-// entries are the odd ones in y), the z reflection by the sign of the z-odd
-// entries per position.  Otherwise every thread copies its share of the tile
-// from the octant with cp.async and signs the x and y reflections in place.
+// Operator tile (octant operators, oct = 1): every thread copies its share of
+// the tile from the octant with cp.async and signs the x and y reflections in
+// place.
 template <typename T, int NZ, int KIND>
 __global__ void __launch_bounds__(ZS<T, NZ, KIND>::THREADS)
 k_zmul(cplx<T>* __restrict__ B, long long b_rhs, const cplx<T>* __restrict__ fN, int oct, Dims d,
-       const cplx<T>* __restrict__ tw, const __grid_constant__ CUtensorMap tmap, int tma, int* err) {
+       const cplx<T>* __restrict__ tw) {
   if (rhs_skipped(d, blockIdx.z)) return;
   using V = cplx<T>;
   using ZC = ZS<T, NZ, KIND>;
@@ -732,9 +706,7 @@ k_zmul(cplx<T>* __restrict__ B, long long b_rhs, const cplx<T>* __restrict__ fN,
   const int rem = threadIdx.x - c * S * FF::T;
   const int s = rem % S, t = rem / S;
   V* Bp = B + blockIdx.z * b_rhs + c * comp + (long long)ky * d.Lp + kx0;
-  V* tile = buf + 3 * BUF;  // operator tile of the CTA's columns, [q][oz][s], 128-byte aligned
-  tile = reinterpret_cast<V*>(reinterpret_cast<char*>(tile) +
-                              ((128u - ((unsigned)__cvta_generic_to_shared(tile) & 127u)) & 127u));
+  V* tile = buf + 3 * BUF;  // operator tile of the CTA's columns, [q][oz][s]
   const bool active = kx0 + s < d.Lp;
   const bool fy = oct && ky > d.Mp / 2;
   const int oy = fy ? d.Mp - ky : ky;
@@ -745,27 +717,7 @@ k_zmul(cplx<T>* __restrict__ B, long long b_rhs, const cplx<T>* __restrict__ fN,
   // row0, row0 + STEP, ... (THREADS is a multiple of S).
   constexpr int ROWS = OK::NQ * NO, STEP = ZC::THREADS / S;
   const int row0 = threadIdx.x / S;
-  const bool bulk = ZC::TMA && tma && oct;
-  __shared__ __align__(8) unsigned long long tile_bar;
-  const unsigned bar = (unsigned)__cvta_generic_to_shared(&tile_bar);
-  if (bulk) {
-    if (threadIdx.x == 0) {
-      // box origin (kx0, oy, 0, 0): kx0 is a multiple of the even S, so the
-      // copy starts on a 16-byte boundary; the box (S x 1 x NO x 6) lies
-      // inside the (Lp, M+1, N+1, 6) tensor
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      // tma == 2 (a test of the bounded wait): armed for 16 bytes more than
-      // the copy delivers, so the barrier never completes
-      const unsigned bytes = (unsigned)(OK::NQ * NO * S * sizeof(V)) + (tma == 2 ? 16u : 0u);
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-      asm volatile(
-          "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
-          "%5}], [%6];" ::"r"((unsigned)__cvta_generic_to_shared(tile)),
-          "l"(reinterpret_cast<unsigned long long>(&tmap)), "r"(kx0), "r"(oy), "r"(0), "r"(0), "r"(bar)
-          : "memory");
-    }
-  } else if (oct && active) {
+  if (oct && active) {
     // the operator tile streams into shared memory while the forward
     // transforms run (its latency was the z pass's main stall)
     const int kx = kx0 + s;
@@ -796,38 +748,9 @@ k_zmul(cplx<T>* __restrict__ B, long long b_rhs, const cplx<T>* __restrict__ fN,
   __syncthreads();  // twiddles staged
   V* my = buf + c * BUF + s;
   FF::run_half(reg, my, ad, t, tw_s);
-  // D N D with D = diag(1, -1, 1) for a y-reflected column (bulk tile only)
-  const bool neg_y = bulk && c == 1 && fy;
-  if (neg_y) {
-#pragma unroll
-    for (int i = 0; i < E; ++i) reg[i] = mk<V>(-reg[i].x, -reg[i].y);
-  }
   __syncthreads();
   FF::store(reg, my, ad, t);
-  if (bulk) {
-    // wait for the tile, at most ~2 s of global time (5 ms in the test of
-    // this path); then flag it and go on (the values are wrong, the status
-    // word tells the host)
-    const unsigned long long limit = tma == 2 ? 5000000ull : 2000000000ull;
-    unsigned long long t_start;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_start));
-    for (;;) {
-      unsigned done;
-      asm volatile(
-          "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
-          "selp.u32 %0, 1, 0, p;\n\t}"
-          : "=r"(done)
-          : "r"(bar)
-          : "memory");
-      if (done) break;
-      unsigned long long t_now;
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_now));
-      if (t_now - t_start > limit) {
-        if (err) atomicExch(err, 1);
-        break;
-      }
-    }
-  } else if (oct && active) {
+  if (oct && active) {
     // each thread signs the tile entries it copied: reflections in x and y
     // flip the components odd along that axis
     cp_async_wait_all();
@@ -858,14 +781,14 @@ k_zmul(cplx<T>* __restrict__ B, long long b_rhs, const cplx<T>* __restrict__ fN,
   const V* b1 = buf + BUF + s;
   const V* b2 = buf + 2 * BUF + s;
   if constexpr (KIND == 0 && !ZC::UNIFORM) {
-    zrow_any<FF, V, NZ, S>(reg, c, t, s, active, oct, bulk, tile, fp, fq, fplane, b0, b1, b2, ad);
+    zrow_any<FF, V, NZ, S>(reg, c, t, s, active, oct, tile, fp, fq, fplane, b0, b1, b2, ad);
   } else if constexpr (KIND == 0) {
     if (c == 0)
-      zrow<0, FF, V, NZ, S>(reg, t, s, active, oct, bulk, tile, fp, fq, fplane, b0, b1, b2, ad);
+      zrow<0, FF, V, NZ, S>(reg, t, s, active, oct, tile, fp, fq, fplane, b0, b1, b2, ad);
     else if (c == 1)
-      zrow<1, FF, V, NZ, S>(reg, t, s, active, oct, bulk, tile, fp, fq, fplane, b0, b1, b2, ad);
+      zrow<1, FF, V, NZ, S>(reg, t, s, active, oct, tile, fp, fq, fplane, b0, b1, b2, ad);
     else
-      zrow<2, FF, V, NZ, S>(reg, t, s, active, oct, bulk, tile, fp, fq, fplane, b0, b1, b2, ad);
+      zrow<2, FF, V, NZ, S>(reg, t, s, active, oct, tile, fp, fq, fplane, b0, b1, b2, ad);
   } else {
     const V* bc[3] = {b0, b1, b2};
     if (c == 0)
@@ -874,10 +797,6 @@ k_zmul(cplx<T>* __restrict__ B, long long b_rhs, const cplx<T>* __restrict__ fN,
       zrow_k<1, FF, V, NZ, S>(reg, t, s, active, oct, tile, fp, fq, fplane, bc, ad);
     else
       zrow_k<2, FF, V, NZ, S>(reg, t, s, active, oct, tile, fp, fq, fplane, bc, ad);
-  }
-  if (neg_y) {
-#pragma unroll
-    for (int i = 0; i < E; ++i) reg[i] = mk<V>(-reg[i].x, -reg[i].y);
   }
   pdl_trigger();
   FI::run(reg, my, ad, t, tw_s);

@@ -27,12 +27,12 @@ template <typename K> inline cudaError_t opt_in_smem(K kernel, size_t bytes) {
   return e;
 }
 
-// The z pass's operator tile by bulk tensor copy (FP32 N operator): tensor
-// maps over the plan's copy of the operator stored full along x,
-// fN32x[q][oz][oy][kx] (2L x (M+1) x (N+1) x 6), one per box width of 8, 4
-// and 2 columns, and the device word a pass sets when a copy does not arrive.
+// The z pass's operator tile by bulk tensor copy (FP32 N operator): the tensor
+// map over the plan's copy of the operator stored full along x,
+// fN32x[q][oz][oy][kx] (2L x (M+1) x (N+1) x 6), the box 8 columns wide, and the
+// device word a pass sets when a copy does not arrive.
 struct ZTile {
-  CUtensorMap map[3];
+  CUtensorMap map;
   int ok = 0;
   int* err = nullptr;
 };

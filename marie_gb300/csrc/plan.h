@@ -33,7 +33,7 @@ struct marie_plan {
 
   // The FP32 N operator stored full along x for the z pass's bulk tile copy
   // (fN32x[q][oz][oy][kx], 2L x (M+1) x (N+1) x 6, x reflections signed in),
-  // with its tensor maps; built beside the octant when the operator has the
+  // with its tensor map; built beside the octant when the operator has the
   // circulant parity symmetry and N + 1 <= 256.
   float2* fN32x = nullptr;
   marie::ZTile zt{};
