@@ -261,7 +261,13 @@ int marie_jvie_adjoint_grad(marie_plan* plan, const double* Einc, const double* 
  * all-zero Vrhs is returned as the solution.  idx: 1-based DOF indices into
  * 3LMN (n_idx of them); Mr, Mc: L x M x N complex; Vrhs, Vini, Vsol: n_idx
  * complex, host or device.  A MARIE_MIXED plan refines FP32-matvec solves
- * with FP64 residuals.  flag / relres / iter (half steps) as bicgstab. */
+ * with FP64 residuals.  flag and iter (half steps) are BiCGSTAB's.  Beyond the
+ * reference, a converged solve may end with one GMRES cycle of up to eight steps
+ * from BiCGSTAB's iterate, which lowers the solution's error where the tolerance
+ * leaves it to chance: its products (not in iter) stay within a quarter of
+ * BiCGSTAB's and within the 2 max_it that max_it allows, none below 16 products.
+ * Its vector is returned if its residual is the smaller one; relres is the true
+ * relative residual of the vector that is returned. */
 int marie_jvie2solver(marie_plan* plan, const int64_t* idx, int64_t n_idx, const double* Mr, const double* Mc,
                       double Gram, const double* Vrhs, double tol, int max_it, const double* Vini, double* Vsol,
                       int* flag, double* relres, double* iter, double* solvert);

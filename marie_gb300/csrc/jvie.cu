@@ -677,40 +677,49 @@ static int solve_single(marie_plan* p, const JvieState& S, const double2* Bv, do
   return MARIE_OK;
 }
 
-// Steps of the minimal-residual cycle that ends a converged inner solve.
-constexpr int kClosingSteps = 8;
+// Steps of the minimal-residual cycle that ends an inner solve of `iter` BiCGSTAB
+// iterations, two products each.  With the cycle's residuals (at most three) they
+// stay within a quarter of those products and within what max_it leaves, so a
+// solve that starts near its solution, or at its limit, ends as BiCGSTAB ends it.
+constexpr int kClosingSteps = 8, kClosingResiduals = 3;
+static int closing_steps(double iter, int max_it) {
+  const long long spent = (long long)(2 * iter);
+  const long long room = std::min(spent / 4, 2LL * max_it - spent) - kClosingResiduals;
+  return (int)std::max(0LL, std::min<long long>(room, kClosingSteps));
+}
 
 // One short GMRES cycle from the iterate at which BiCGSTAB met its tolerance.
 // That iterate's residual is one sample of an erratic sequence, anywhere from a
 // tenth of the tolerance to all of it, and which one depends on the rounding of
 // the products: on twenty bodies the error of the solution varied five-fold
-// between roundings.  Eight minimal-residual steps (3 % of a solve's products)
-// bring it to the low end of that range and hold it there; the result is taken
-// only if its FP64 residual is smaller.  relres becomes the new residual's.
-static int close_inner_solve(marie_plan* p, const JvieState& S, const double2* b, double2* x, double& relres) {
+// between roundings.  Eight minimal-residual steps (6 % of a solve's products at
+// 80 iterations, 3 % at 160) bring it to the low end of that range and hold it
+// there.  The vector is taken only if its true residual (FP64, or FP32 products
+// on a plan of that precision alone) is smaller, and relres is then that residual's; if
+// the cycle fails, for want of memory or otherwise, the solve's own result stands.
+static void close_inner_solve(marie_plan* p, const JvieState& S, const double2* b, int steps, double2* x,
+                              double& relres) {
+  if (steps < 1) return;
   cudaStream_t st = p->stream;
   const long long n = S.n;
   const int prec_main = (p->precision == MARIE_FP32) ? MARIE_FP32 : MARIE_FP64;
   const DevOp A = single(make_bop(p, prec_main, S, S.a.as<double2>(), S.b.as<double2>(), false), n);
   DBuf xb, rb, one;
-  if (!xb.try_alloc((size_t)n * sizeof(double2), st)) return MARIE_OK;
+  if (!xb.try_alloc((size_t)n * sizeof(double2), st)) return;
   double2* x2 = xb.as<double2>();
   GmresResult g;
-  if (p->precision != MARIE_MIXED) {
-    const int s = gmres(p, A, nullptr, nullptr, nullptr, nullptr, b, n, kClosingSteps, 0.0, 1, x, x2, g);
-    if (s == MARIE_ENOMEM) return MARIE_OK;  // the solve's own result stands
-    MARIE_TRY(s);
-  } else {
+  auto refined = [&]() -> int {
+    if (p->precision != MARIE_MIXED)
+      return gmres(p, A, nullptr, nullptr, nullptr, nullptr, b, n, steps, 0.0, 1, x, x2, g);
     // the correction with the FP32 product, the residuals in FP64
     const DevOp A32 = single(make_bop(p, MARIE_FP32, S, S.a.as<double2>(), S.b.as<double2>(), false), n);
-    if (!rb.try_alloc((size_t)n * sizeof(double2), st) || !one.try_alloc(sizeof(int), st)) return MARIE_OK;
+    MARIE_TRY(rb.alloc((size_t)n * sizeof(double2), st));
+    MARIE_TRY(one.alloc(sizeof(int), st));
     double2* r = rb.as<double2>();
     MARIE_CUDA_TRY(cudaMemsetAsync(one.p, 1, sizeof(int), st));
     MARIE_TRY(A(x, r));
     k_sub_b<<<dim3(grid_n(n), 1), 256, 0, st>>>(b, r, n, one.as<int>());
-    const int s = gmres(p, A32, nullptr, nullptr, nullptr, nullptr, r, n, kClosingSteps, 0.0, 1, nullptr, x2, g);
-    if (s == MARIE_ENOMEM) return MARIE_OK;
-    MARIE_TRY(s);
+    MARIE_TRY(gmres(p, A32, nullptr, nullptr, nullptr, nullptr, r, n, steps, 0.0, 1, nullptr, x2, g));
     k_add_b<<<dim3(grid_n(n), 1), 256, 0, st>>>(x, x2, n, one.as<int>());
     MARIE_TRY(A(x2, r));
     k_sub_b<<<dim3(grid_n(n), 1), 256, 0, st>>>(b, r, n, one.as<int>());
@@ -720,12 +729,11 @@ static int close_inner_solve(marie_plan* p, const JvieState& S, const double2* b
     MARIE_TRY(dev_norm2(p, r, n, &rn));
     MARIE_TRY(dev_norm2(p, b, n, &bn));
     g.relres = rn / bn;
-  }
-  if (g.relres < relres) {
-    MARIE_CUDA_TRY(cudaMemcpyAsync(x, x2, (size_t)n * sizeof(double2), cudaMemcpyDeviceToDevice, st));
+    return MARIE_OK;
+  };
+  if (refined() != MARIE_OK || !(g.relres < relres)) return;
+  if (cudaMemcpyAsync(x, x2, (size_t)n * sizeof(double2), cudaMemcpyDeviceToDevice, st) == cudaSuccess)
     relres = g.relres;
-  }
-  return MARIE_OK;
 }
 
 // adjoint-gradient kernels (adjoint.cu)
@@ -1149,8 +1157,8 @@ int marie_jvie2solver(marie_plan* p, const int64_t* idx, int64_t n_idx, const do
     so.r.assign(1, GmresResult());
     MARIE_TRY(solve_single(S.on(p), S, (const double2*)b_d, (double2*)x_d, 0, tol, 50, 200, sa, so,
                            (const double2*)x0_d));
-    if (so.b.flag == 0 && so.b.iter > 0)
-      MARIE_TRY(close_inner_solve(S.on(p), S, (const double2*)b_d, (double2*)x_d, so.b.relres));
+    if (so.b.flag == 0)
+      close_inner_solve(S.on(p), S, (const double2*)b_d, closing_steps(so.b.iter, max_it), (double2*)x_d, so.b.relres);
     if (flag) *flag = so.b.flag;
     if (relres) *relres = so.b.relres;
     if (iter) *iter = so.b.iter;

@@ -839,7 +839,10 @@ def jvie2solver(Vrhs, fN, idx, Mr, Mc, Gram, tol, Vini=None, max_it=1000):
     """jvie2solver.m:1-79: BiCGSTAB (max_it iterations, no preconditioner, x0 =
     Vini) on mv_AN(J, fN, Mr, Mc, Gram, 'notransp', idx); an all-zero Vrhs is
     returned unchanged.  fN: an Operator (or a 2L x 2M x 2N x 6 array).  Returns
-    (Vsol, flag, relres, iter, solvert); iter counts half steps."""
+    (Vsol, flag, relres, iter, solvert); flag and iter (half steps) are
+    BiCGSTAB's.  A converged solve of eight iterations or more may end with up to
+    eight GMRES steps (at most a quarter of its products, within 2 max_it, not in
+    iter); relres is the true residual of the vector that is returned."""
     opr, tmp = _operator_for(fN, "fp64")
     try:
         n = int(np.asarray(idx).size) if not _is_cuda(idx) else int(idx.numel())

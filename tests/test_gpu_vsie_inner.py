@@ -84,3 +84,113 @@ def test_jvie2solver_initial_guess_and_zero_rhs(cuda):
     bd = torch.from_numpy(b).to(cuda)
     xd = solver(bd, 1e-9)
     assert xd.is_cuda and np.linalg.norm(xd.cpu().numpy() - rx) <= 1e-6 * np.linalg.norm(rx)
+
+
+def scattered(L, dx, precision, seed=3, keep=0.5):
+    """jvie2solver's arguments for scattered lossy voxels on an L^3 grid."""
+    import marie_gb300 as mg
+
+    rng = np.random.default_rng(seed)
+    er = np.ones((L, L, L), complex)
+    er[rng.random(er.shape) < keep] = 40.0 - 25.0j
+    er = np.asfortranarray(er)
+    idxS = np.flatnonzero(np.abs(er.reshape(-1, order="F") - 1) > 1e-12) + 1
+    idx = np.concatenate([idxS, er.size + idxS, 2 * er.size + idxS]).astype(np.int64)
+    b = (rng.standard_normal(idx.size) + 1j * rng.standard_normal(idx.size)) * dx**3
+    op = mg.Operator.assemble(L, L, L, dx, FREQ, precision=precision)
+    return op, idx, np.asfortranarray(er / er), np.asfortranarray((er - 1) / er), dx**3, b, rng
+
+
+def products_of(op, call):
+    """call() and the products the plan ran in it."""
+    import ctypes as C
+
+    ms, n = (C.c_double * 5)(), C.c_int64()
+    op.lib.marie_plan_profile(op.plan, 1, ms, C.byref(n))
+    try:
+        out = call()
+    finally:
+        op.lib.marie_plan_profile(op.plan, 0, ms, C.byref(n))
+    return out, n.value
+
+
+def test_jvie2solver_products_stay_in_proportion_and_within_max_it(cuda):
+    """A solve that starts near the solution takes a few products, not the
+    closing cycle's ten as well, and max_it bounds the products.  BiCGSTAB takes
+    two per iteration, one for the start's residual and up to five
+    confirmations; the closing cycle at most a quarter of the iterations'."""
+    import marie_gb300 as mg
+
+    op, idx, Mr, Mc, Gram, b, rng = scattered(12, 5e-3, "fp64")
+    solve = lambda tol, **k: mg.jvie2solver(b, op, idx, Mr, Mc, Gram, tol, **k)
+    x = solve(1e-12)[0]
+    near = x + 1e-6 * np.linalg.norm(x) / np.sqrt(x.size) * (rng.standard_normal(x.size) + 1j * rng.standard_normal(x.size))
+    (_, flag, relres, it, _), n = products_of(op, lambda: solve(2e-7, Vini=near))
+    assert flag == 0 and relres <= 2e-7 and 0 < it <= 6, (it, relres)
+    assert n <= 2.5 * it + 6, (n, it)
+    (_, flag, _, it, _), n = products_of(op, lambda: solve(1e-6))
+    assert flag == 0 and n <= 2.5 * it + 6, (n, it)
+    most = int(np.ceil(it))
+    (_, flag, _, it, _), n = products_of(op, lambda: solve(1e-6, max_it=most))
+    assert flag == 0 and it <= most and n <= 2 * most + 6, (n, it)
+    op.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("tol", [1e-2, 1e-4, 1e-7])
+def test_jvie2solver_relres_is_the_returned_vectors(precision, tol, cuda):
+    """relres is ||b - A x|| / ||b|| of the vector that is returned, cold and
+    from a start near the solution; the two products' roundings move it by 1e-13
+    at most."""
+    import marie_gb300 as mg
+
+    op, idx, Mr, Mc, Gram, b, rng = scattered(12, 5e-3, precision)
+    cold = mg.jvie2solver(b, op, idx, Mr, Mc, Gram, tol)
+    x0 = cold[0] * (1 + 30 * tol * rng.standard_normal(b.size))
+    for x, flag, relres, it, _ in (cold, mg.jvie2solver(b, op, idx, Mr, Mc, Gram, tol, Vini=x0)):
+        res = np.linalg.norm(b - mg.mv_AN(x, op, Mr, Mc, Gram, "notransp", idx)) / np.linalg.norm(b)
+        assert flag == 0 and relres <= tol
+        assert abs(relres - res) <= 1e-13
+    op.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("voxels", [1, 2])
+def test_jvie2solver_of_a_few_dofs(precision, voxels, cuda):
+    """Three and six unknowns: the Krylov space is exhausted before any closing
+    step, and the result stands."""
+    import marie_gb300 as mg
+
+    op, idx, Mr, Mc, Gram, b, _ = scattered(8, 5e-3, precision)
+    part = np.concatenate([idx[c * len(idx) // 3:][:voxels] for c in range(3)])
+    rhs = b[:part.size]
+    x, flag, relres, it, _ = mg.jvie2solver(rhs, op, part, Mr, Mc, Gram, 1e-10)
+    res = np.linalg.norm(rhs - mg.mv_AN(x, op, Mr, Mc, Gram, "notransp", part)) / np.linalg.norm(rhs)
+    assert flag == 0 and relres <= 1e-10 and res <= 1.01e-10
+    op.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_jvie2solver_allocation_failures_leave_a_converged_result(precision, cuda):
+    """An allocation that fails in the solve is MARIE_ENOMEM; one that fails in
+    the closing cycle leaves BiCGSTAB's result."""
+    import marie_gb300 as mg
+
+    op, idx, Mr, Mc, Gram, b, _ = scattered(12, 5e-3, precision)
+    solve = lambda: mg.jvie2solver(b, op, idx, Mr, Mc, Gram, 1e-6)
+    ref = solve()
+    lib, stood, past = mg.load(), 0, 0
+    for nth in range(1, 80):
+        lib.marie_inject_alloc_failure(nth)
+        try:
+            x, flag, relres, it, _ = solve()
+        except mg.MarieError as e:
+            assert e.code == -2
+            continue
+        finally:
+            lib.marie_inject_alloc_failure(0)
+        assert flag == 0 and relres <= 1e-6 and it == ref[3]
+        same = np.array_equal(x, ref[0])
+        stood, past = stood + (not same), past + same
+    assert stood > 0 and past > 0  # some fell into the closing cycle, some came after the last allocation
+    op.close()
