@@ -129,11 +129,12 @@ int marie_mv_AN(marie_plan* plan, const double* JIn0, const double* Mr, const do
  * another allocator, such as MATLAB's gpuArray pool or a serving runtime's
  * fixed arena, or a loop that must not block in cudaMalloc).  Its scratch is a
  * 64 MiB static device array that every GPU loading this library holds until
- * exit; grids needing more (about 204-252 bytes per voxel in FP32, 396 in FP64)
- * are rejected with MARIE_EINVAL.  Device pointers only.  The call runs on the
- * plan's device and stream (the caller's current device is restored) with the
- * plan's matvec schedule and blocks the host until that stream is done (it
- * reads the kernels' error flag), so it cannot be captured into a CUDA graph.
+ * exit; grids needing more (per voxel 108 bytes and 32 per DOF in FP32, so 204
+ * with every voxel a DOF, and 300 in FP64) are rejected with MARIE_EINVAL.
+ * Device pointers only.  The call runs on the plan's device and stream (the
+ * caller's current device is restored) with the plan's matvec schedule and
+ * blocks the host until that stream is done (it reads the kernels' error
+ * flag), so it cannot be captured into a CUDA graph.
  * Calls share the array, so calls that overlap on the GPU race. */
 int marie_mv_AN_static(marie_plan* plan, const double* JIn0, const double* Mr,
                        const double* Mc, double Gram, int transp, const int64_t* idx,

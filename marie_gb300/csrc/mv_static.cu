@@ -40,11 +40,11 @@ __global__ void k_coefficients(const int64_t* idx, long long n, long long V, con
 
 using namespace marie;
 
-// 64 MiB.  The sizes that are taken are fixed: with every voxel's DOFs an FP32
-// matvec counts 204 bytes per voxel on the grids of compact() and 252 on the
-// others (up to 64^3 voxels fit), an FP64 one 396 (up to about 160k voxels).
-// The x spectra of the larger counts, half as much as the others, are only
-// counted: they lie inside the others.
+// 64 MiB: the flag, the DOF map (12 bytes per voxel), the coefficients and the
+// spectra (96 bytes per voxel in FP32, 192 in FP64).  FP32 coefficients take 32
+// bytes per DOF given, so 64^3 voxels fit with any body; FP64 ones are laid out
+// for every voxel's DOFs (96 bytes per voxel), so an FP64 grid is taken, up to
+// about 220k voxels, or refused whatever body it holds.
 static constexpr size_t kStaticScratchBytes = 64ull << 20;
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
 
@@ -70,13 +70,6 @@ static int scratch_address(int dev, unsigned char** out) {
   return MARIE_OK;
 }
 
-static bool compact(const Dims& d) {
-  const int pairs[][2] = {{64, 64}, {96, 96}, {128, 128}, {192, 192}, {256, 256}, {512, 384}};
-  for (const auto& p : pairs)
-    if (d.Lp == p[0] && d.Mp == p[1]) return true;
-  return false;
-}
-
 static size_t up256(size_t b) { return (b + 255) & ~size_t(255); }
 
 template <typename T>
@@ -87,19 +80,19 @@ static int static_matvec(marie_plan* p, const double2* J, const double2* Mr, con
   const Dims d = p->d;
   const long long V3 = 3 * d.V;
   const bool fused = p->fuse && ML::fused(d);
-  // scratch layout: error flag | inv[3V] | a[n] | b[n] | spectra
+  // scratch layout: error flag | inv[3V] | a | b | spectra
+  const long long coefs = sizeof(V) == sizeof(float2) ? n : V3;
   size_t off = 0;
   int* err = reinterpret_cast<int*>(scratch + off);
   off += 256;
   int* inv = reinterpret_cast<int*>(scratch + off);
   off += up256(V3 * sizeof(int));
   double2* ca = reinterpret_cast<double2*>(scratch + off);
-  off += up256(n * sizeof(double2));
+  off += up256(coefs * sizeof(double2));
   double2* cb = reinterpret_cast<double2*>(scratch + off);
-  off += up256(n * sizeof(double2));
+  off += up256(coefs * sizeof(double2));
   V* B = reinterpret_cast<V*>(scratch + off);
   off += up256(p->elems_B() * sizeof(V));
-  if (sizeof(V) != 8 || !p->fuse || !compact(d)) off += up256(3LL * d.Lp * d.M * d.N * sizeof(V));  // counted, see above
   if (off > kStaticScratchBytes)
     return set_error(MARIE_EINVAL,
                      "marie_mv_AN_static: this grid and DOF count need %zu bytes of scratch, more than the %zu of "

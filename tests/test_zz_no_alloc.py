@@ -151,3 +151,54 @@ def test_static_matvec_takes_the_grids_that_count_one_scratch(shape, cuda):
     torch.cuda.synchronize()
     assert float((out - ref).abs().max()) <= TOL["fp32"] * float(ref.abs().max())
     op.close()
+
+
+@pytest.mark.parametrize("shape,precision", [((80, 80, 48), "fp32"), ((64, 64, 48), "fp64")])
+def test_static_matvec_takes_what_its_array_holds(shape, precision, cuda):
+    """Grids with every voxel a DOF whose map, coefficients and spectra (204
+    bytes per voxel in FP32, 300 in FP64) fit the 64 MiB array."""
+    import torch
+
+    import marie_gb300 as mg
+    from marie_gb300 import _lib
+
+    lib = _lib.load()
+    p = _lib.MARIE_FP64 if precision == "fp64" else _lib.MARIE_FP32
+    op = mg.Operator.assemble(*shape, 5e-3, 298e6, precision=precision)
+    c = case(*shape, 10, 1.1, cuda)
+    assert c["n"] == 3 * np.prod(shape)
+    ref = torch.zeros(c["n"], dtype=torch.complex128, device=cuda)
+    out = torch.full((c["n"],), complex("nan"), dtype=torch.complex128, device=cuda)
+    _lib.check(call(lib.marie_mv_AN, op.plan, c, 0, (1, p), ref))
+    _lib.check(call_static_no_alloc(lib, op.plan, c, 0, p, out))
+    torch.cuda.synchronize()
+    assert float((out - ref).abs().max()) <= TOL[precision] * float(ref.abs().max())
+    op.close()
+
+
+def test_static_matvec_runs_the_pinned_passes(cuda):
+    """64 x 64 transforms are the ones with a choice of schedule: pinned to five
+    passes the static FP32 product launches two kernels more than with the fused
+    three, and both match marie_mv_AN."""
+    import torch
+
+    import marie_gb300 as mg
+    from marie_gb300 import _lib
+
+    lib = _lib.load()
+    shape = (32, 32, 16)
+    op = mg.Operator.from_array(operator(*shape, seed=11), precision="mixed")
+    c = case(*shape, 12, 0.6, cuda)
+    launches = []
+    for fuse in (1, 0):
+        op.set_schedule(fuse, 0, 0)
+        ref = torch.zeros(c["n"], dtype=torch.complex128, device=cuda)
+        out = torch.full((c["n"],), complex("nan"), dtype=torch.complex128, device=cuda)
+        _lib.check(call(lib.marie_mv_AN, op.plan, c, 0, (1, _lib.MARIE_FP32), ref))
+        n0 = lib.marie_launch_count()
+        _lib.check(call_static_no_alloc(lib, op.plan, c, 0, _lib.MARIE_FP32, out))
+        launches.append(lib.marie_launch_count() - n0)
+        torch.cuda.synchronize()
+        assert float((out - ref).abs().max()) <= TOL["fp32"] * float(ref.abs().max())
+    assert launches[1] == launches[0] + 2
+    op.close()
