@@ -352,7 +352,7 @@ def run_gpu(args, world, rank, local):
                           "fp32_bound": mv["fp32_bound_ms"], "fp64_bound": mv["fp64_bound_ms"],
                           "note": "fp32/fp64: marie_mv_AN per call, which rebuilds the DOF map and coefficients; "
                                   "*_bound: marie_plan_apply_mv_AN, the solver's matvec (map and coefficients "
-                                  "bound once, on the body's box; FP32 epilogue in FP32)"},
+                                  "bound once, on the body's box)"},
             "assembly_s": round(t_asm, 3),
             "autotune": {"chosen": {"fused_xy": tuned[0], "xy_variant": tuned[1], "z_variant": tuned[2]},
                          "candidates_ms": [{"fused_xy": f, "xy_variant": fv, "z_variant": z, "ms": round(ms, 4)}
@@ -425,8 +425,7 @@ def matvec_times(mg, op, op64, er, lib):
         res[name + "_ms"] = round(e0.elapsed_time(e1) / reps, 4)
         res[name + "_passes"] = passes
         # the same product with the DOF map and coefficients bound to the plan
-        # once (marie_plan_apply_mv_AN: the solver's matvec, no per-call set-up;
-        # FP32 with its epilogue in FP32 as in the inner solves)
+        # once (marie_plan_apply_mv_AN: the solver's matvec, no per-call set-up)
         opr.bind_mv_AN(Mr, Mc, 8e-9, "notransp", idx_d)
 
         def apply():

@@ -162,9 +162,9 @@ int marie_plan_bind_mv_AN(marie_plan* plan, const double* Mr, const double* Mc, 
 /* JOut = mv_AN(JIn0) with the mv_AN bound to the plan (one call of the handle
  * fA of JVIE_Solver.m:211-297): no DOF map or coefficients are rebuilt per
  * call, unlike marie_mv_AN.  JIn0, JOut: n_idx x nrhs complex, host or device.
- * precision MARIE_FP32 runs the whole product in FP32 (transforms and the
- * epilogue Gram*Mr*J - Mc*(N J), the matvec of the mixed-precision inner
- * solves); MARIE_FP64 in FP64.  With device output the call returns without
+ * precision MARIE_FP32 runs the circulant part in FP32 and Gram*Mr*J -
+ * Mc*(N J) in FP64 (the matvec of the mixed-precision inner solves);
+ * MARIE_FP64 all of it in FP64.  With device output the call returns without
  * waiting for the plan's stream (a bounded-wait timeout is then reported by
  * the next call that synchronises the plan); with host output it returns
  * after the copy. */

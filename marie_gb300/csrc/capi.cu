@@ -671,22 +671,13 @@ static void free_bound(marie_plan* p) {
   cudaFree(p->bnd_inv);
   cudaFree(p->bnd_a);
   cudaFree(p->bnd_b);
-  cudaFree(p->bnd_af);
-  cudaFree(p->bnd_bf);
   cudaFree(p->bnd_inv_crop);
   p->bnd_inv_crop = nullptr;
   p->bnd_crop.reset();
   p->bnd_idx = nullptr;
   p->bnd_inv = nullptr;
   p->bnd_a = p->bnd_b = nullptr;
-  p->bnd_af = p->bnd_bf = nullptr;
   p->bnd_n = 0;
-}
-
-// out[k] = (float2) in[k]
-__global__ void k_to_f32(const double2* __restrict__ in, long long n, float2* __restrict__ out) {
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x)
-    out[k] = make_float2((float)in[k].x, (float)in[k].y);
 }
 
 namespace marie {
@@ -815,18 +806,6 @@ int marie_plan_bind_mv_AN(marie_plan* p, const double* Mr, const double* Mc, dou
   if (s == MARIE_OK)
     s = build_coefficients(p, p->bnd_idx, n, (const double2*)Mr_d, (const double2*)Mc_d, Gram, transp, p->bnd_a,
                            p->bnd_b);
-  if (s == MARIE_OK && p->fN32) {
-    // FP32 copies for the FP32 applications, whose epilogue runs in FP32
-    if (cudaMalloc(&p->bnd_af, n * sizeof(float2)) != cudaSuccess ||
-        cudaMalloc(&p->bnd_bf, n * sizeof(float2)) != cudaSuccess) {
-      cudaGetLastError();
-      s = set_error(MARIE_ENOMEM, "bound mv_AN: device allocation failed");
-    } else {
-      k_to_f32<<<grid_stride_blocks(n, 8), 256, 0, p->stream>>>(p->bnd_a, n, p->bnd_af);
-      k_to_f32<<<grid_stride_blocks(n, 8), 256, 0, p->stream>>>(p->bnd_b, n, p->bnd_bf);
-      count_launch(2);
-    }
-  }
   if (s == MARIE_OK && crop_possible(p)) {
     // the products on the smallest grid that holds the DOFs
     int box[6], origin[3];
@@ -1136,11 +1115,6 @@ int marie_plan_apply_mv_AN(marie_plan* p, const double* JIn0, double* JOut, int6
     pro.pre = p->bnd_b;
     pro.conjin = 1;
     ep.conjout = 1;
-  }
-  if (precision == MARIE_FP32) {
-    // the FP32 operator's epilogue in FP32, as in the solver's inner matvecs
-    ep.af = p->bnd_af;
-    ep.bf = p->bnd_bf;
   }
   const int* inv;
   marie_plan* q = bound_plan(p, &inv, &pro);

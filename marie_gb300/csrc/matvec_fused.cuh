@@ -263,7 +263,7 @@ k_yxinv(const cplx<T>* __restrict__ B, long long bs, const IO* __restrict__ J, l
       FXI::load(reg, base, rowa, t, NL);
       FXI::run(reg, base, rowa, t, twx_s);
       if (row0 > 0) load_epi_idx(kk, row0);
-      epilogue_dofs<IO, V, E, 2, true>(reg, kk, Jr, ep, outr);
+      epilogue_dofs<IO, V, E, 2>(reg, kk, Jr, ep, outr);
     }
   }
 }

@@ -249,62 +249,43 @@ k_xinv(const cplx<T>* A, long long a_stride, const IO* __restrict__ J, long long
   }
 }
 
+// a b + c, four FMAs
+template <typename V> __device__ __forceinline__ V cfma(V a, V b, V c) {
+  return mk<V>(fma(-a.y, b.y, fma(a.x, b.x, c.x)), fma(a.y, b.x, fma(a.x, b.y, c.y)));
+}
+
 // out[kk] = A J - B v of one row sweep: reg[i] is the circulant term at DOF
-// kk[i] (-1: none).  Per-DOF loads in groups of EPI (bounded registers).  FP64
-// vectors with FP32 coefficient copies (the matvec of the mixed-precision
-// inner solves and of FP32 products of a bound operator) run the whole epilogue
-// in FP32, the transforms' precision, with one conversion in and one out.
-// NARROW: the product B v in the transforms' precision, otherwise in the
-// vectors'.
-template <typename IO, typename V, int E, int EPI, bool NARROW>
+// kk[i] (-1: none).  In the vectors' precision: the diagonal term of FP64 vectors
+// is FP64's whatever the transforms' is (for bodies of low contrast it is most of
+// the result: with a relative permittivity of 1.2 the FP32 product of 96 x 80 x
+// 64 is off by 2e-8, with an FP32 epilogue by 6e-8).  Its ten FP64 instructions
+// per DOF cost 22 us of a 128^3 product's 344 (322 with an FP32 epilogue).
+// Per-DOF loads in groups of EPI (bounded registers): groups of 4 took 345 us
+// where groups of 2 took 348.
+template <typename IO, typename V, int E, int EPI>
 __device__ __forceinline__ void epilogue_dofs(const V* reg, const int* kk, const IO* Jr, const Epilogue& ep, IO* outr) {
-  constexpr bool MIX = std::is_same<IO, double2>::value && std::is_same<V, float2>::value;
-  const bool f32epi = MIX && ep.af != nullptr;
 #pragma unroll
   for (int i0 = 0; i0 < E; i0 += EPI) {
     IO jv[EPI], ak[EPI], bk[EPI];
-    float2 af[EPI], bf[EPI];
 #pragma unroll
     for (int j = 0; j < EPI; ++j) {
       const int k = kk[i0 + j];
       if (k < 0) continue;
       jv[j] = Jr[k];
-      if (f32epi) {
-        af[j] = ep.af[k];
-        bf[j] = ep.bf ? ep.bf[k] : mk<float2>(0, 0);
-      } else {
-        ak[j] = EpiIO<IO>::a(ep, k);
-        bk[j] = EpiIO<IO>::b(ep, k);
-      }
+      ak[j] = EpiIO<IO>::a(ep, k);
+      if (!ep.conjout) bk[j] = EpiIO<IO>::b(ep, k);
     }
 #pragma unroll
     for (int j = 0; j < EPI; ++j) {
       const int k = kk[i0 + j];
       if (k < 0) continue;
-      if constexpr (MIX) {
-        if (f32epi) {
-          const float2 v = reg[i0 + j];
-          float2 r32 = cmul(af[j], cvt<float2>(jv[j]));
-          if (ep.conjout) {
-            r32.x -= v.x;
-            r32.y += v.y;
-          } else {
-            r32 = csub(r32, cmul(bf[j], v));
-          }
-          outr[k] = cvt<IO>(r32);
-          continue;
-        }
-      }
-      // the diagonal Gram*Mr*J term in the vectors' precision
       IO res = cmul(ak[j], jv[j]);
       const IO v = cvt<IO>(reg[i0 + j]);
       if (ep.conjout) {
         res.x -= v.x;
         res.y += v.y;
-      } else if constexpr (NARROW) {
-        res = csub(res, cvt<IO>(cmul(cvt<V>(bk[j]), reg[i0 + j])));
       } else {
-        res = csub(res, cmul(bk[j], v));
+        res = cfma(mk<IO>(-bk[j].x, -bk[j].y), v, res);
       }
       outr[k] = res;
     }
@@ -403,7 +384,7 @@ k_xinv_rows(const float2* A, long long a_stride, const IO* __restrict__ J, long 
       kk[b * RL + r] = (valid && x < L) ? invr[x] : -1;
     }
   F::run(reg, xb, SAddr(1, true), t, tw_s);
-  epilogue_dofs<IO, float2, E, 2, false>(reg, kk, J + blockIdx.y * j_stride, ep, out + blockIdx.y * o_stride);
+  epilogue_dofs<IO, float2, E, 4>(reg, kk, J + blockIdx.y * j_stride, ep, out + blockIdx.y * o_stride);
 }
 
 // ---------------------------------------------------------------------------
@@ -544,11 +525,6 @@ template <int C> struct ZRow {
 };
 
 template <typename V> __device__ __forceinline__ V neg_if(V v, bool f) { return f ? mk<V>(-v.x, -v.y) : v; }
-
-// a b + c, four FMAs
-template <typename V> __device__ __forceinline__ V cfma(V a, V b, V c) {
-  return mk<V>(fma(-a.y, b.y, fma(a.x, b.x, c.x)), fma(a.y, b.x, fma(a.x, b.y, c.y)));
-}
 
 // Row C of the product at this thread's output positions of the forward
 // transform.  With the octant operator the tile already carries the x and y

@@ -233,7 +233,7 @@ class Operator:
     def apply_mv_AN(self, J, precision="fp64"):
         """mv_AN bound with bind_mv_AN applied to J (n or n x nrhs; numpy or a
         CUDA torch tensor), without rebuilding the DOF map per call.
-        precision 'fp32' runs the product in FP32 throughout."""
+        precision 'fp32' runs its circulant part in FP32."""
         cuda = _is_cuda(J)
         nrhs = 1 if J.ndim == 1 else J.shape[1]
         jp, jk = _in(J)

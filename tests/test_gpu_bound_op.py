@@ -215,3 +215,35 @@ def test_solves_on_the_bodys_rows_and_planes(cuda, shape, lo, size, precision):
     assert nz == nzr
     assert np.linalg.norm(J - Jr) <= 1e-6 * np.linalg.norm(Jr)
     assert np.linalg.norm(x - xr) <= 1e-6 * np.linalg.norm(xr)
+
+
+def _bound_operator(shape, precision, dx=4e-3, seed=5, keep=0.6, box=None, cls_args=()):
+    import marie_gb300 as mg
+
+    lo, size = box or ((0, 0, 0), shape)
+    er = np.ones(shape, complex, order="F")
+    part = er[tuple(slice(a, a + s) for a, s in zip(lo, size))]
+    part[np.random.default_rng(seed).random(size) < keep] = 30.0 - 20.0j
+    part[0, 0, 0] = part[-1, -1, -1] = 12.0 - 3.0j
+    idxS = np.flatnonzero(np.abs(er.reshape(-1, order="F") - 1) > 1e-12) + 1
+    idx = np.concatenate([idxS, er.size + idxS, 2 * er.size + idxS]).astype(np.int64)
+    op = mg.Operator.assemble(*shape, dx, FREQ, precision=precision, nrhs_max=2)
+    return op, er, idx
+
+
+@pytest.mark.parametrize("shape", [(8, 12, 16), (20, 20, 8), (48, 48, 4), (64, 64, 8), (16, 96, 8)])
+@pytest.mark.parametrize("transp", ["notransp", "transp"])
+def test_fp32_products_keep_the_diagonal_term_in_fp64(cuda, shape, transp):
+    """Grids without fused passes: FP32 arithmetic is the circulant's, the
+    diagonal Gram Mr J of FP64 vectors is FP64's.  With Mc = 0 it is all there
+    is: one complex product, three roundings (Gram Mr: one more)."""
+    op, er, idx = _bound_operator(shape, "mixed")
+    rng = np.random.default_rng(1)
+    J = rng.standard_normal(idx.size) + 1j * rng.standard_normal(idx.size)
+    Mr = np.asfortranarray(1 + 40 * rng.random(shape) - 20j * rng.random(shape))
+    op.bind_mv_AN(Mr, np.zeros(shape, complex, order="F"), 0.37, transp, idx)
+    m = Mr.reshape(-1, order="F")[(idx - 1) % Mr.size]
+    ref = 0.37 * (m if transp == "notransp" else np.conj(m)) * J
+    out = op.apply_mv_AN(J, "fp32")
+    assert np.max(np.abs(out - ref) / np.abs(ref)) <= 1e-15
+    op.close()
