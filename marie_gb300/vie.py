@@ -109,8 +109,14 @@ def _out(shape, like_cuda: bool, dtype=np.complex128):
 
 
 def _any_nonzero(a) -> bool:
-    """np.any(a), where a lives: a CUDA tensor is not brought to the host."""
-    return bool(a.ne(0).any()) if _is_cuda(a) else bool(np.any(np.asarray(a)))
+    """np.any(a), where a lives: a CUDA tensor is not brought to the host, but what
+    numpy refuses (one that requires grad, whose graph the call would end, or of a
+    type it does not have) is refused here too, by an empty stand-in (25 us)."""
+    if not _is_cuda(a):
+        return bool(np.any(np.asarray(a)))
+    if a.requires_grad or a.dtype not in (torch.complex128, torch.complex64, torch.float64, torch.float32):
+        np.asarray(torch.empty(0, dtype=a.dtype, requires_grad=a.requires_grad))
+    return bool(a.ne(0).any())
 
 
 def release_cached_memory():

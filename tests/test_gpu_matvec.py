@@ -246,3 +246,23 @@ def test_transpose_is_Mc_similarity_on_device(precision):
         sim = mg.mv_AN(mc * x, op, Mr, Mc, gram, "notransp", idx, precision=precision) / mc
         assert relerr(sim, ATx) < tol
         op.close()
+
+
+def test_field_wrappers_refuse_a_current_that_requires_grad(cuda):
+    """With an incident field a CUDA current that requires grad raises, as numpy
+    does: the result would carry no graph."""
+    import torch
+
+    import marie_gb300 as mg
+
+    shape = (8, 8, 8)
+    op = mg.Operator.assemble(*shape, 5e-3, 298e6).assemble_k(5e-3, 298e6)
+    col = lambda s: torch.randn(*reversed(s), dtype=torch.complex128, device=cuda).permute(*reversed(range(len(s))))
+    J, F = col((*shape, 3)), col((*shape, 3))
+    calls = (lambda j: mg.E_field_Nop(j, op, 1.25e-7, 298e6, F), lambda j: mg.H_field_Kop(j, op, 1.25e-7, F))
+    for f in calls:
+        assert f(J).shape == J.shape
+        with pytest.raises(RuntimeError):
+            f(J.clone().requires_grad_())
+        assert f(torch.zeros_like(J)) is F
+    op.close()
