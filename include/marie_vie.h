@@ -357,8 +357,9 @@ int marie_release_cached_memory(void);
  * without an FP32 operator is left as it is (*count = 0). */
 int marie_plan_autotune(marie_plan* plan, int* fuse, int* fvar, int* zvar, double* ms, int64_t cap,
                         int64_t* count);
-/* Pin a schedule as marie_plan_autotune would choose it; fvar and zvar from 0 to
- * 2 are accepted and select nothing. */
+/* Pin a schedule as marie_plan_autotune would choose it: fuse on the grids that
+ * have fused passes (elsewhere it selects nothing); fvar and zvar from 0 to 2 are
+ * accepted and select nothing. */
 int marie_plan_set_schedule(marie_plan* plan, int fuse, int fvar, int zvar);
 /* Krylov basis precision of the inner solves of a MARIE_MIXED plan's GMRES
  * refinement (no counterpart in the reference): MARIE_FP64 (the default: the

@@ -859,6 +859,13 @@ int marie_plan_destroy(marie_plan* p) {
 
 void* marie_plan_stream(marie_plan* p) { return p ? (void*)p->stream : nullptr; }
 
+// A schedule is a choice on the grids that have fused passes.  Elsewhere there is
+// none to make, and the box that a product is cut to, which may have them where
+// the plan's grid does not, keeps the default.
+static void pin_schedule(marie_plan* p, bool fuse) {
+  if (MatvecLaunch<float>::fused(p->d)) p->fuse = fuse;
+}
+
 // Autotuner: times the FP32 matvec of this plan's grid for every candidate
 // schedule (the fused x+y passes where the grid has them, and the five-pass
 // form), keeps the fastest on the plan and reports every candidate's time as
@@ -909,14 +916,12 @@ int marie_plan_autotune(marie_plan* p, int* fuse_out, int* fvar_out, int* zvar_o
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  if (status != MARIE_OK) {
-    p->fuse = fuse0;
-    return status;
-  }
+  p->fuse = fuse0;
+  if (status != MARIE_OK) return status;
   const Cand* best = &cands[0];
   for (const auto& c : cands)
     if (c.ms < best->ms) best = &c;
-  p->fuse = best->fuse != 0;
+  pin_schedule(p, best->fuse != 0);
   if (fuse_out) *fuse_out = best->fuse;
   if (fvar_out) *fvar_out = 0;
   if (zvar_out) *zvar_out = 0;
@@ -934,7 +939,7 @@ int marie_plan_set_schedule(marie_plan* p, int fuse, int fvar, int zvar) {
   if (!p) return set_error(MARIE_EINVAL, "NULL plan");
   if (fvar < 0 || fvar > 2) return set_error(MARIE_EINVAL, "fvar must be 0, 1 or 2");
   if (zvar < 0 || zvar > 2) return set_error(MARIE_EINVAL, "zvar must be 0, 1 or 2");
-  p->fuse = fuse != 0;  // (the schedules that fvar and zvar numbered are gone, their values stay valid)
+  pin_schedule(p, fuse != 0);  // (the schedules that fvar and zvar numbered are gone, their values stay valid)
   return MARIE_OK;
 }
 

@@ -213,7 +213,8 @@ class Operator:
         return (fuse.value, fvar.value, zvar.value), cands
 
     def set_schedule(self, fuse, fvar, zvar):
-        """Pin a matvec schedule: fuse 1/0; fvar and zvar (0 to 2) select nothing."""
+        """Pin a matvec schedule: fuse 1/0 on grids with fused passes (64 x 64
+        transforms along x and y); fvar and zvar (0 to 2) select nothing."""
         check(self.lib.marie_plan_set_schedule(self.plan, int(fuse), int(fvar), int(zvar)))
         return self
 

@@ -247,3 +247,51 @@ def test_fp32_products_keep_the_diagonal_term_in_fp64(cuda, shape, transp):
     out = op.apply_mv_AN(J, "fp32")
     assert np.max(np.abs(out - ref) / np.abs(ref)) <= 1e-15
     op.close()
+
+
+def _launches(op, call):
+    import torch
+
+    torch.cuda.synchronize()
+    n0 = op.lib.marie_launch_count()
+    out = call()
+    torch.cuda.synchronize()
+    return out, op.lib.marie_launch_count() - n0
+
+
+@pytest.mark.parametrize("how", ["autotune", "schedule"])
+def test_a_schedule_without_choice_leaves_the_box_its_fused_passes(cuda, how):
+    """A 48 x 48 grid has no fused x+y passes, so tuning it chooses nothing; the
+    64 x 64 transforms of a 32 x 32 body in it keep theirs: three passes a
+    product, before and after."""
+    shape = (48, 48, 16)
+    op, er, idx = _bound_operator(shape, "mixed", box=((5, 9, 0), (32, 32, 16)))
+    op.bind_mv_AN(np.asfortranarray(er / er), np.asfortranarray((er - 1) / er), 4e-3**3, "notransp", idx)
+    rng = np.random.default_rng(4)
+    J = rng.standard_normal(idx.size) + 1j * rng.standard_normal(idx.size)
+    op.apply_mv_AN(J, "fp32")
+    ref, before = _launches(op, lambda: op.apply_mv_AN(J, "fp32"))
+    if how == "autotune":
+        chosen, cands = op.autotune()
+        assert chosen == (0, 0, 0) and len(cands) == 1
+    else:
+        op.set_schedule(0, 0, 0)
+    out, after = _launches(op, lambda: op.apply_mv_AN(J, "fp32"))
+    assert before == after == 3
+    np.testing.assert_array_equal(out, ref)
+    op.close()
+
+
+def test_schedule_of_a_grid_with_fused_passes_holds_on_its_box(cuda):
+    """On a grid that has fused passes the schedule is a choice, for the box cut
+    from it along z as well; the products agree to the FP32 bar."""
+    op, er, idx = _bound_operator((32, 32, 48), "mixed", box=((0, 0, 3), (32, 32, 20)))
+    op.bind_mv_AN(np.asfortranarray(er / er), np.asfortranarray((er - 1) / er), 4e-3**3, "notransp", idx)
+    rng = np.random.default_rng(4)
+    J = rng.standard_normal(idx.size) + 1j * rng.standard_normal(idx.size)
+    ref = op.apply_mv_AN(J, "fp64")
+    for fuse, passes in ((1, 3), (0, 5), (1, 3)):
+        op.set_schedule(fuse, 0, 0)
+        out, n = _launches(op, lambda: op.apply_mv_AN(J, "fp32"))
+        assert n == passes and np.max(np.abs(out - ref)) < 1e-5 * np.max(np.abs(ref))
+    op.close()
