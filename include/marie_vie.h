@@ -222,7 +222,13 @@ int marie_bicgstab(marie_plan* plan, marie_op_fn A, void* A_ctx, const double* b
  * refined by FP64 true residuals until relres <= tol.  Je: L x M x N x 3.
  * iter: 2 doubles, {inner, outer} for 'G' and 'D', {iterations, 0} for 'B'
  * (half steps count 0.5).  resvec as the solver returns it: relative for 'G'
- * and 'D', absolute for 'B'. */
+ * and 'D', absolute for 'B'.
+ * On a grid of 30000 voxels or more the products of a solve, and those of a
+ * bound mv_AN, run on the smallest transform grid that holds the body's box, if
+ * that is at most 0.8 of the plan's.  The plan keeps that operator (FP64 plans or
+ * MARIE_MIXED ones, at most 0.8 of its own) for the next body of the same box,
+ * until its own changes, one of its calls finds no memory (the call then runs on
+ * the whole grid) or marie_plan_destroy. */
 int marie_jvie_solve(marie_plan* plan, const double* Einc, const double* e_r, double dx,
                      double freq, double tol, int form, char solver, char precond, int max_it,
                      int inner_it, int outer_it, int ritz, double* Je, int* flag, double* relres,

@@ -114,9 +114,10 @@ extern "C" int marie_jvie_adjoint_grad(marie_plan* p, const double* Einc, const 
   if (E_target) MARIE_TRY(stage_in(E_target, 3 * V * sizeof(double2), st, tEt, &Et_d));
   MARIE_TRY(stage_out(dF_deps, V * sizeof(double), st, tge, &ge_d));
   MARIE_TRY(stage_out(dF_dsigma, V * sizeof(double), st, tgs, &gs_d));
-  MARIE_TRY(jvie_adjoint_core(p, (const double2*)E_d, (const double2*)er_d, dx, freq, objective,
-                              (const double2*)Et_d, tol, inner_it, outer_it, F, (double*)ge_d, (double*)gs_d, flags,
-                              iters));
+  MARIE_TRY(on_box_or_whole_grid(p, [&]() {
+    return jvie_adjoint_core(p, (const double2*)E_d, (const double2*)er_d, dx, freq, objective, (const double2*)Et_d,
+                             tol, inner_it, outer_it, F, (double*)ge_d, (double*)gs_d, flags, iters);
+  }));
   MARIE_TRY(finish_out(dF_deps, ge_d, V * sizeof(double), st));
   MARIE_TRY(finish_out(dF_dsigma, gs_d, V * sizeof(double), st));
   MARIE_CUDA_TRY(cudaStreamSynchronize(st));

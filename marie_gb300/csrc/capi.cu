@@ -99,13 +99,24 @@ static cudaMemPool_t device_pool() {
   return pool;
 }
 
-int DBuf::alloc(size_t bytes, cudaStream_t st) {
-  s = st;
-  if (bytes == 0) bytes = 16;
+// counts an allocation; true for the one that is to fail
+static bool allocation_injected() {
   long long left = g_fail_alloc_in.load();
   while (left > 0 && !g_fail_alloc_in.compare_exchange_weak(left, left - 1)) {
   }
-  if (left == 1) {
+  return left == 1;
+}
+
+void trim_pool(cudaStream_t st) {
+  cudaStreamSynchronize(st);
+  if (cudaMemPool_t pool = device_pool()) cudaMemPoolTrimTo(pool, 0);
+  cudaGetLastError();
+}
+
+int DBuf::alloc(size_t bytes, cudaStream_t st) {
+  s = st;
+  if (bytes == 0) bytes = 16;
+  if (allocation_injected()) {
     p = nullptr;
     return set_error(MARIE_ENOMEM, "device allocation of %zu bytes failed (injected)", bytes);
   }
@@ -115,8 +126,7 @@ int DBuf::alloc(size_t bytes, cudaStream_t st) {
     // blocks cached in the pool may be the wrong sizes: hand them back to the
     // device once and retry before reporting the failure
     cudaGetLastError();
-    cudaStreamSynchronize(st);
-    cudaMemPoolTrimTo(pool, 0);
+    trim_pool(st);
     e = cudaMallocFromPoolAsync(&p, bytes, pool, st);
   }
   if (e != cudaSuccess) {
@@ -129,6 +139,10 @@ int DBuf::alloc(size_t bytes, cudaStream_t st) {
 
 bool DBuf::try_alloc(size_t bytes, cudaStream_t st) {
   s = st;
+  if (allocation_injected()) {
+    p = nullptr;
+    return false;
+  }
   cudaMemPool_t pool = device_pool();
   if (bytes == 0) bytes = 16;
   const cudaError_t e = pool ? cudaMallocFromPoolAsync(&p, bytes, pool, st) : cudaMallocAsync(&p, bytes, st);
@@ -173,7 +187,9 @@ int ensure_workspace(marie_plan* p, int prec, long long nrhs) {
     if (p->wsB) cudaFreeAsync(p->wsB, p->stream);
     p->wsB = nullptr;
     p->ws_bytes_B = 0;
-    if (cudaMallocAsync(&p->wsB, need_B, p->stream) != cudaSuccess) {
+    cudaError_t e = cudaMallocAsync(&p->wsB, need_B, p->stream);
+    if (e != cudaSuccess && give_crop_back(p)) e = cudaMallocAsync(&p->wsB, need_B, p->stream);
+    if (e != cudaSuccess) {
       cudaGetLastError();
       p->wsB = nullptr;
       return set_error(MARIE_ENOMEM, "workspace of the spectra (%zu bytes) allocation failed", need_B);
@@ -617,8 +633,12 @@ static int store_operator(marie_plan* p, const double2* src, bool src_oct, int o
     p->has_op = false;
   else
     p->has_opK = false;
-  if (need64) MARIE_CUDA_TRY(cudaMalloc(&f64, n * sizeof(double2)));
-  if (need32) MARIE_CUDA_TRY(cudaMalloc(&f32, n * sizeof(float2)));
+  auto room = [&](auto** out, size_t bytes) {
+    const cudaError_t e = cudaMalloc(out, bytes);
+    return e != cudaSuccess && give_crop_back(p) ? cudaMalloc(out, bytes) : e;
+  };
+  if (need64) MARIE_CUDA_TRY(room(&f64, n * sizeof(double2)));
+  if (need32) MARIE_CUDA_TRY(room(&f32, n * sizeof(float2)));
   if (oct && !src_oct) {
     k_extract_octant<<<grid_for(n), 256, 0, p->stream>>>(src, d.L, d.M, d.N, NQ, 1.0 / (double)P,
                                                          need64 ? f64 : nullptr, need32 ? f32 : nullptr);
@@ -779,11 +799,19 @@ int marie_plan_create(int64_t L, int64_t M, int64_t N, int precision, int64_t nr
   return MARIE_OK;
 }
 
+static int bind_mv_AN(marie_plan* p, const double* Mr, const double* Mc, double Gram, int transp, const int64_t* idx,
+                      int64_t n_idx);
+
 int marie_plan_bind_mv_AN(marie_plan* p, const double* Mr, const double* Mc, double Gram, int transp,
                           const int64_t* idx, int64_t n_idx) {
   if (!p || !Mr || !Mc || !idx || n_idx < 1) return set_error(MARIE_EINVAL, "NULL argument or n_idx < 1");
   if (transp != 0 && transp != 1) return set_error(MARIE_EINVAL, "transp must be 0 ('notransp') or 1 ('transp')");
   if (!p->has_op) return set_error(MARIE_ENOOP, "plan has no operator");
+  return on_box_or_whole_grid(p, [&]() { return bind_mv_AN(p, Mr, Mc, Gram, transp, idx, n_idx); });
+}
+
+static int bind_mv_AN(marie_plan* p, const double* Mr, const double* Mc, double Gram, int transp, const int64_t* idx,
+                      int64_t n_idx) {
   MARIE_CUDA_TRY(cudaStreamSynchronize(p->stream));
   free_bound(p);
   const long long V = p->d.V, n = n_idx;

@@ -165,7 +165,7 @@ __global__ void k_inverse_box(const int64_t* __restrict__ idx, long long n, int 
 
 bool crop_possible(const marie_plan* p) {
   // the smaller operator is derived from the FP64 octant
-  return p->has_op && p->oct && p->fN64 && !p->profile && p->d.V >= kCropMinVoxels;
+  return p->has_op && p->oct && p->fN64 && !p->profile && !p->whole_grid && p->d.V >= kCropMinVoxels;
 }
 
 int dof_box(marie_plan* p, const int64_t* idx_dev, long long n, int box[6]) {
@@ -319,6 +319,13 @@ void crop_settings(const marie_plan* p, marie_plan* q) {
   q->inner_restart = p->inner_restart;
   q->batch_groups = p->batch_groups;
   q->graph_refine = p->graph_refine;
+}
+
+bool give_crop_back(marie_plan* p) {
+  if (!p->crop) return false;
+  p->crop.reset();
+  trim_pool(p->stream);
+  return true;
 }
 
 // The body seldom fills its transform grid either (98 x 72 x 122 voxels of 128 x

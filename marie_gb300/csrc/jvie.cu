@@ -372,9 +372,9 @@ static int solve_single(marie_plan* p, const JvieState& S, const double2* Bv, do
 // Solves the S excitations E (3V x S, column stride es) of one body.
 // With dfr, a mixed-precision 'G' solve leaves its refinement to dfr's
 // shared graph launch and the DOF scatter to dfr's steps after it.
-static int jvie_solve_core(marie_plan* p, const double2* E, long long es, int S_exc, const double2* er, double dx,
+static int jvie_solve_once(marie_plan* p, const double2* E, long long es, int S_exc, const double2* er, double dx,
                            double freq, int form, char precond, double tol, int inner_it, int outer_it, double2* Je,
-                           long long js, SolveOut& out, const SolverArgs& sa = SolverArgs(), Deferred* dfr = nullptr) {
+                           long long js, SolveOut& out, const SolverArgs& sa, Deferred* dfr) {
   cudaStream_t st = p->stream;
   const long long V = p->d.V;
   auto Sp = std::make_shared<JvieState>();
@@ -418,6 +418,14 @@ static int jvie_solve_core(marie_plan* p, const double2* E, long long es, int S_
   dfr->keep.push_back(x);
   dfr->after.push_back(scatter);
   return MARIE_OK;
+}
+
+static int jvie_solve_core(marie_plan* p, const double2* E, long long es, int S_exc, const double2* er, double dx,
+                           double freq, int form, char precond, double tol, int inner_it, int outer_it, double2* Je,
+                           long long js, SolveOut& out, const SolverArgs& sa = SolverArgs(), Deferred* dfr = nullptr) {
+  return on_box_or_whole_grid(p, [&]() {
+    return jvie_solve_once(p, E, es, S_exc, er, dx, freq, form, precond, tol, inner_it, outer_it, Je, js, out, sa, dfr);
+  });
 }
 
 // Solves A2 x_e = B_e (form-2 J-VIE operator of the state S) for S_exc
@@ -727,6 +735,43 @@ static void close_inner_solve(marie_plan* p, const JvieState& S, const double2* 
   if (refined() != MARIE_OK || !(g.relres < relres)) return;
   if (cudaMemcpyAsync(x, x2, (size_t)n * sizeof(double2), cudaMemcpyDeviceToDevice, st) == cudaSuccess)
     relres = g.relres;
+}
+
+// jvie2solver on the mv_AN('notransp') operator of the DOFs idx (its fVIE):
+// a = Gram Mr(idx), b = Mc(idx).
+static int jvie2_solve(marie_plan* p, const int64_t* idx, long long n, const double2* Mr, const double2* Mc, double Gram,
+                       const double2* b, double tol, int max_it, const double2* x0, double2* x, SolveOut& so) {
+  cudaStream_t st = p->stream;
+  JvieState S;
+  S.n = n;
+  MARIE_TRY(S.idx3.alloc(n * sizeof(int64_t), st));
+  MARIE_CUDA_TRY(cudaMemcpyAsync(S.idx3.p, idx, n * sizeof(int64_t), cudaMemcpyDeviceToDevice, st));
+  MARIE_TRY(S.a.alloc(n * sizeof(double2), st));
+  MARIE_TRY(S.b.alloc(n * sizeof(double2), st));
+  MARIE_TRY(S.pa.alloc(n * sizeof(double2), st));  // no preconditioner: pa, pb unused (pb = 0)
+  MARIE_TRY(S.pb.alloc(n * sizeof(double2), st));
+  MARIE_CUDA_TRY(cudaMemsetAsync(S.pa.p, 0, n * sizeof(double2), st));
+  MARIE_CUDA_TRY(cudaMemsetAsync(S.pb.p, 0, n * sizeof(double2), st));
+  MARIE_TRY(S.inv.alloc(3 * p->d.V * sizeof(int), st));
+  MARIE_TRY(build_inverse_index(p, S.idx3.as<int64_t>(), n, S.inv.as<int>()));
+  if (crop_possible(p)) {
+    int box[6], origin[3];
+    MARIE_TRY(dof_box(p, S.idx3.as<int64_t>(), n, box));
+    S.crop = crop_plan(p, box, origin);
+    // (the crop's map needs less than the whole grid's)
+    if (!S.crop) whole_grid_origin(box, origin);
+    S.ext = box_extent(S.on(p), box);
+    MARIE_TRY(build_inverse_box(p, S.on(p), origin, S.ext, S.idx3.as<int64_t>(), n, S.inv.as<int>()));
+  }
+  MARIE_TRY(build_coefficients(p, S.idx3.as<int64_t>(), n, Mr, Mc, Gram, 0, S.a.as<double2>(), S.b.as<double2>()));
+  // bicgstab(fVIE, Vrhs, tol, max_it, [], [], Vini) (jvie2solver.m:54-77)
+  SolverArgs sa;
+  sa.solver = 'B';
+  sa.max_it = max_it;
+  so.r.assign(1, GmresResult());
+  MARIE_TRY(solve_single(S.on(p), S, b, x, 0, tol, 50, 200, sa, so, x0));
+  if (so.b.flag == 0) close_inner_solve(S.on(p), S, b, closing_steps(so.b.iter, max_it), x, so.b.relres);
+  return MARIE_OK;
 }
 
 // adjoint-gradient kernels (adjoint.cu)
@@ -1118,40 +1163,11 @@ int marie_jvie2solver(marie_plan* p, const int64_t* idx, int64_t n_idx, const do
   if (!nz) {
     MARIE_CUDA_TRY(cudaMemcpyAsync(x_d, b_d, n * sizeof(double2), cudaMemcpyDeviceToDevice, st));
   } else {
-    // the mv_AN('notransp') operator on the DOFs idx (jvie2solver's fVIE): a = Gram Mr(idx), b = Mc(idx)
-    JvieState S;
-    S.n = n;
-    MARIE_TRY(S.idx3.alloc(n * sizeof(int64_t), st));
-    MARIE_CUDA_TRY(cudaMemcpyAsync(S.idx3.p, idx_d, n * sizeof(int64_t), cudaMemcpyDeviceToDevice, st));
-    MARIE_TRY(S.a.alloc(n * sizeof(double2), st));
-    MARIE_TRY(S.b.alloc(n * sizeof(double2), st));
-    MARIE_TRY(S.pa.alloc(n * sizeof(double2), st));  // no preconditioner: pa, pb unused (pb = 0)
-    MARIE_TRY(S.pb.alloc(n * sizeof(double2), st));
-    MARIE_CUDA_TRY(cudaMemsetAsync(S.pa.p, 0, n * sizeof(double2), st));
-    MARIE_CUDA_TRY(cudaMemsetAsync(S.pb.p, 0, n * sizeof(double2), st));
-    MARIE_TRY(S.inv.alloc(3 * V * sizeof(int), st));
-    MARIE_TRY(build_inverse_index(p, S.idx3.as<int64_t>(), n, S.inv.as<int>()));
-    if (crop_possible(p)) {
-      int box[6], origin[3];
-      MARIE_TRY(dof_box(p, S.idx3.as<int64_t>(), n, box));
-      S.crop = crop_plan(p, box, origin);
-      // (the crop's map needs less than the whole grid's)
-      if (!S.crop) whole_grid_origin(box, origin);
-      S.ext = box_extent(S.on(p), box);
-      MARIE_TRY(build_inverse_box(p, S.on(p), origin, S.ext, S.idx3.as<int64_t>(), n, S.inv.as<int>()));
-    }
-    MARIE_TRY(build_coefficients(p, S.idx3.as<int64_t>(), n, (const double2*)Mr_d, (const double2*)Mc_d, Gram, 0,
-                                 S.a.as<double2>(), S.b.as<double2>()));
-    // bicgstab(fVIE, Vrhs, tol, max_it, [], [], Vini) (jvie2solver.m:54-77)
-    SolverArgs sa;
-    sa.solver = 'B';
-    sa.max_it = max_it;
     SolveOut so;
-    so.r.assign(1, GmresResult());
-    MARIE_TRY(solve_single(S.on(p), S, (const double2*)b_d, (double2*)x_d, 0, tol, 50, 200, sa, so,
-                           (const double2*)x0_d));
-    if (so.b.flag == 0)
-      close_inner_solve(S.on(p), S, (const double2*)b_d, closing_steps(so.b.iter, max_it), (double2*)x_d, so.b.relres);
+    MARIE_TRY(on_box_or_whole_grid(p, [&]() {
+      return jvie2_solve(p, (const int64_t*)idx_d, n, (const double2*)Mr_d, (const double2*)Mc_d, Gram,
+                         (const double2*)b_d, tol, max_it, (const double2*)x0_d, (double2*)x_d, so);
+    }));
     if (flag) *flag = so.b.flag;
     if (relres) *relres = so.b.relres;
     if (iter) *iter = so.b.iter;

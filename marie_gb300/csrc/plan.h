@@ -57,6 +57,7 @@ struct marie_plan {
   // its arena, its stream and status word are the plan's.
   std::shared_ptr<marie_plan> crop;
   void* arena = nullptr;
+  bool whole_grid = false;  // no crop is made (a solve that ran out of memory beside one)
 
   // Spectra workspace (3 x N x 2M x 2L per rhs).
   void* wsB = nullptr;
@@ -143,6 +144,8 @@ struct HostPrefault {
 };
 
 int ensure_workspace(marie_plan* p, int prec, long long nrhs);
+// Waits for the stream and hands the pool's cached blocks to the device.
+void trim_pool(cudaStream_t st);
 int ensure_pinned(marie_plan* p, size_t n_doubles);
 
 // Build the inverse map inv[g] = k for 1-based idx[k]; -1 elsewhere.  Fails on
@@ -181,6 +184,19 @@ bool crop_possible(const marie_plan* p);
 int dof_box(marie_plan* p, const int64_t* idx_dev, long long n, int box[6]);
 std::shared_ptr<marie_plan> crop_plan(marie_plan* p, const int box[6], int origin[3]);
 void crop_settings(const marie_plan* p, marie_plan* q);
+// For a call that finds no memory: gives the plan's crop and the pool's cached
+// blocks back.  False when the plan holds no crop.
+bool give_crop_back(marie_plan* p);
+// Runs call(); when it finds no memory while the plan holds a crop, gives that
+// back and runs it again on the whole grid, as if no crop had been made.
+template <typename F> int on_box_or_whole_grid(marie_plan* p, F&& call) {
+  int s = call();
+  if (s != MARIE_ENOMEM || !give_crop_back(p)) return s;
+  p->whole_grid = true;
+  s = call();
+  p->whole_grid = false;
+  return s;
+}
 Extent box_extent(const marie_plan* q, const int box[6]);
 int build_inverse_box(marie_plan* p, marie_plan* q, const int origin[3], const Extent& ext, const int64_t* idx_dev,
                       long long n, int* inv);

@@ -295,3 +295,76 @@ def test_schedule_of_a_grid_with_fused_passes_holds_on_its_box(cuda):
         out, n = _launches(op, lambda: op.apply_mv_AN(J, "fp32"))
         assert n == passes and np.max(np.abs(out - ref)) < 1e-5 * np.max(np.abs(ref))
     op.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_solves_without_memory_for_the_box(cuda, precision):
+    """Whatever allocation of a solve fails once the caller's buffers are there,
+    the box's operator or one beside it, the solve takes the whole grid."""
+    import torch
+
+    import marie_gb300 as mg
+    from marie_gb300.autograd import adjoint_gradient
+
+    shape, lo, size = CROPS[0]
+    r, er = _off_centre_body(shape, lo, size)
+    em = vo.EMconstants(FREQ)
+    E = vo.PlaneWave_Excitation(r, [0, 0, em["ko"]], em["omega_mu"], [1, 0, 0])[0]
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a.transpose())).to(cuda).permute(*reversed(range(a.ndim)))
+    Ed, erd = dev(E), dev(er)
+    op = mg.Operator.assemble(*shape, 4e-3, FREQ, precision=precision)
+    idxS = torch.nonzero((erd.permute(2, 1, 0).reshape(-1) - 1).abs() > 1e-12)[:, 0] + 1
+    idx = torch.cat([idxS + c * erd.numel() for c in range(3)])
+    b = Ed.permute(3, 2, 1, 0).reshape(-1)[idx - 1] * 4e-3**3
+    Mr, Mc = erd / erd, (erd - 1) / erd
+    torch.cuda.synchronize()
+
+    def gradient():
+        F, g, _, flags, _ = adjoint_gradient(op, Ed, erd, 4e-3, FREQ, "power", tol=1e-8)
+        return g, max(flags)
+
+    for solve in (lambda: mg.JVIE_Solver(Ed, erd, r, FREQ, op, tol=1e-8, solver="G")[:2],
+                  lambda: mg.JVIE_Solver(Ed, erd, r, FREQ, op, tol=1e-8, solver="B")[:2],
+                  lambda: mg.jvie2solver(b, op, idx, Mr, Mc, 4e-3**3, 1e-8)[:2], gradient):
+        ref, _ = solve()
+        torch.cuda.synchronize()
+        for nth in (2, 3, 6, 9, 12, 16, 22, 30):
+            solve()
+            op.lib.marie_inject_alloc_failure(nth)
+            try:
+                x, flag = solve()
+            finally:
+                op.lib.marie_inject_alloc_failure(0)
+            assert flag == 0
+            assert float((x - ref).norm()) <= 1e-5 * float(ref.norm())
+            torch.cuda.synchronize()
+    op.close()
+
+
+@pytest.mark.parametrize("nth", [1, 2, 3, 4, 5])
+def test_binding_and_first_solve_without_memory_for_the_box(cuda, nth):
+    """On a fresh plan the nth allocation from the bind on fails: the bind falls
+    back to the whole grid or reports MARIE_ENOMEM, and the products are right."""
+    import torch
+
+    import marie_gb300 as mg
+
+    shape, lo, size = CROPS[0]
+    op, er, idx = _bound_operator(shape, "mixed", box=(lo, size))
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a.transpose())).to(cuda).permute(*reversed(range(a.ndim)))
+    Mr, Mc, idx_d = dev(er / er), dev((er - 1) / er), torch.from_numpy(idx).to(cuda)
+    rng = np.random.default_rng(3)
+    J = torch.from_numpy(rng.standard_normal(idx.size) + 1j * rng.standard_normal(idx.size)).to(cuda)
+    torch.cuda.synchronize()
+    ref = mg.mv_AN(J, op, Mr, Mc, 4e-3**3, "notransp", idx_d)
+    op.lib.marie_inject_alloc_failure(nth)
+    try:
+        op.bind_mv_AN(Mr, Mc, 4e-3**3, "notransp", idx_d)
+    except mg.MarieError as e:
+        assert e.code == -2
+        op.lib.marie_inject_alloc_failure(0)
+        op.bind_mv_AN(Mr, Mc, 4e-3**3, "notransp", idx_d)
+    finally:
+        op.lib.marie_inject_alloc_failure(0)
+    assert float((op.apply_mv_AN(J, "fp64") - ref).abs().max()) < 1e-13 * float(ref.abs().max())
+    op.close()
