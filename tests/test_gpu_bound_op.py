@@ -368,3 +368,26 @@ def test_binding_and_first_solve_without_memory_for_the_box(cuda, nth):
         op.lib.marie_inject_alloc_failure(0)
     assert float((op.apply_mv_AN(J, "fp64") - ref).abs().max()) < 1e-13 * float(ref.abs().max())
     op.close()
+
+
+def test_bodies_on_their_boxes_in_one_launch(cuda):
+    """Two bodies on grids that are cut to their boxes, solved in one graph
+    launch, give bit for bit their own batches."""
+    import marie_gb300 as mg
+
+    em = vo.EMconstants(FREQ)
+    bodies = []
+    for shape, lo, size in CROPS[:2]:
+        r, er = _off_centre_body(shape, lo, size)
+        E = vo.PlaneWave_Excitation(r, [0, 0, em["ko"]], em["omega_mu"], [1, 0, 0])[0]
+        op = mg.Operator.assemble(*shape, 4e-3, FREQ, precision="mixed", nrhs_max=2)
+        bodies.append((np.asfortranarray(np.stack([E, 1j * E[..., ::-1]], axis=4)), er, r, op))
+    alone = [mg.JVIE_Solver_batch(E, er, r, FREQ, op, tol=1e-7) for E, er, r, op in bodies]
+    n0 = bodies[0][3].lib.marie_graph_loops()
+    res, _ = mg.JVIE_Solver_bodies(bodies, FREQ, tol=1e-7)
+    assert bodies[0][3].lib.marie_graph_loops() == n0 + 1
+    for (J, flag, relres, it), ref in zip(res, alone):
+        np.testing.assert_array_equal(J, ref[0])
+        assert list(flag) == [0, 0] and np.all(relres <= 1e-7)
+    for b in bodies:
+        b[3].close()
