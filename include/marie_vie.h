@@ -342,7 +342,9 @@ int marie_mv_AN_cufft(marie_plan* plan, const double* JIn0, const double* Mr, co
  * times of the matvec.  marie_plan_profile(plan, enable, pass_ms, count)
  * returns the mean milliseconds of the five matvec passes (x forward, y
  * forward, z multiply, y inverse, x inverse) over the matvecs run since the
- * previous call, then resets and switches recording on or off. */
+ * previous call, then resets and switches recording on or off.  While it is on,
+ * solves run their products one by one, outside graphs and on the whole grid;
+ * the results agree to rounding (to the bit where the whole grid is used anyway). */
 int64_t marie_launch_count(void);
 /* Number of device-driven GMRES calls (the solvers' restart cycles) whose
  * cycles after the first ran as one graph launch: a conditional WHILE node

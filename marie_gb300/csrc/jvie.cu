@@ -538,7 +538,7 @@ static int solve_systems(marie_plan* p, const JvieState& S, const double2* Bv, i
       }
       return MARIE_OK;
     };
-    if (p->graph_refine) {
+    if (p->graph_refine && !p->profile) {  // (a capture cannot hold timed products)
       // the whole refinement in one graph launch
       RefineOps ops;
       ops.add = [p, n, S_exc](const double2* D, double2* Xv, const int* fl) -> int {
@@ -1229,7 +1229,7 @@ int marie_jvie_solve_bodies(int nbody, marie_plan* const* plans, const double* c
   bool one_launch = nbody >= 2;
   for (int b = 0; b < nbody && one_launch; ++b)
     one_launch = plans[b]->device == plans[0]->device && plans[b]->graph_refine &&
-                 plans[b]->precision == MARIE_MIXED;
+                 !plans[b]->profile && plans[b]->precision == MARIE_MIXED;
   if (one_launch) {
     int dev = 0;
     cudaGetDevice(&dev);

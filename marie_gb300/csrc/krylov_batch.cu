@@ -1003,6 +1003,8 @@ int gmres_batch(marie_plan* p, const BatchOp& A, const BatchOp* L1, const BatchO
   // the relative tolerance of system s
   auto tol_of = [&](int s) { return tol_s ? (*tol_s)[s] : tol; };
   if (S < 1) return set_error(MARIE_EINVAL, "need at least one system");
+  // timed products wait for their events, which a capture cannot hold
+  if (p->profile) use_graph = false;
   cudaStream_t st = p->stream;
   BatchWork W;
   if (fp32_basis && (!A.apply32 || (L1 && !L1->apply32) || (R1 && !R1->apply32)))

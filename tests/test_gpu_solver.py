@@ -376,3 +376,37 @@ def test_mie_sphere_c1_and_refinement():
     e25 = mie_error(64, 2.5e-3, 0.075, precision="mixed")
     assert e5 < 0.35, e5
     assert e25 < 0.65 * e5, (e5, e25)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_solves_while_their_passes_are_timed(precision):
+    """With marie_plan_profile on, a solve of several restart cycles (the graph
+    forms otherwise), a batch and two bodies together run their products one by
+    one: the same bits, and every product counted."""
+    import ctypes as C
+
+    import marie_gb300 as mg
+
+    L, dx = 16, 5e-3
+    r, er, E = sphere_problem(L, dx, 0.035)
+    E2 = np.asfortranarray(np.stack([E, 2j * E], axis=4))
+    ops = [mg.Operator.assemble(L, L, L, dx, FREQ, precision=precision, nrhs_max=2) for _ in range(2)]
+    op = ops[0]
+
+    def calls():
+        one = mg.JVIE_Solver(E, er, r, FREQ, op, tol=1e-8, inner_it=5, solver="G")
+        two = mg.JVIE_Solver_batch(E2, er, r, FREQ, op, tol=1e-8, inner_it=5)
+        both = mg.JVIE_Solver_bodies([(E2, er, r, o) for o in ops], FREQ, tol=1e-8, inner_it=5)[0]
+        return one[0], one[3], two[0], list(map(list, two[3])), both[0][0], both[1][0]
+
+    ref = calls()
+    ms, n = (C.c_double * 5)(), C.c_int64()
+    timed = lambda on: op.lib.marie_plan_profile(op.plan, on, ms, C.byref(n))
+    timed(1)
+    out = calls()
+    timed(0)
+    for a, b in zip(out, ref):
+        np.testing.assert_array_equal(np.asarray(a), np.asarray(b))
+    assert n.value > 3 * 10 and min(ms) >= 0 and ms[2] > 0
+    for o in ops:
+        o.close()
