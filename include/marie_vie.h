@@ -61,6 +61,11 @@ int marie_plan_create(int64_t L, int64_t M, int64_t N, int precision, int64_t nr
 int marie_plan_destroy(marie_plan* plan);
 /* Device stream of the plan (a cudaStream_t). */
 void* marie_plan_stream(marie_plan* plan);
+/* Orders the plan's stream after the work that `stream` (a cudaStream_t of the
+ * current device, NULL: the default stream) holds now, for inputs and outputs
+ * that belong to it (no counterpart in the reference).  A stream that is idle or
+ * being captured needs no order and gets none. */
+int marie_plan_after_stream(marie_plan* plan, void* stream);
 
 /* Replaces getOPERATORS(r, f, op, type, singular)
  * (src_vie/src_operators/getOPERATORS.m:1-127) for op = 'N' (6 components)

@@ -19,7 +19,7 @@ import numpy as np
 
 from . import _lib
 from ._lib import check
-from .vie import EPS0, Operator, _in, _is_cuda, _out
+from .vie import EPS0, Operator, _in, _is_cuda, _out, _ready
 
 try:
     import torch
@@ -51,7 +51,7 @@ def adjoint_gradient(op: Operator, Einc, e_r, dx, freq, objective="power", E_tar
     F = C.c_double()
     flags = (C.c_int * 2)()
     iters = (C.c_int * 2)()
-    check(op.lib.marie_jvie_adjoint_grad(op.plan, ep, erp, float(dx), float(freq), _OBJ[objective], tp, float(tol),
+    check(op.lib.marie_jvie_adjoint_grad(_ready(op), ep, erp, float(dx), float(freq), _OBJ[objective], tp, float(tol),
                                          int(inner_it), int(outer_it), C.byref(F), gep, gsp, flags, iters))
     return F.value, ge, gs, (flags[0], flags[1]), (iters[0], iters[1])
 

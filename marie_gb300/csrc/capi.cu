@@ -865,6 +865,7 @@ int marie_plan_destroy(marie_plan* p) {
   release_cufft_state(p);
   free_bound(p);
   p->crop.reset();
+  if (p->after) cudaEventDestroy(p->after);
   if (p->wsB) cudaFreeAsync(p->wsB, p->stream);
   if (p->stream) cudaStreamSynchronize(p->stream);
   cudaFree(p->fN64);
@@ -886,6 +887,29 @@ int marie_plan_destroy(marie_plan* p) {
 }
 
 void* marie_plan_stream(marie_plan* p) { return p ? (void*)p->stream : nullptr; }
+
+int marie_plan_after_stream(marie_plan* p, void* stream) {
+  if (!p) return set_error(MARIE_EINVAL, "NULL plan");
+  cudaStream_t other = (cudaStream_t)stream;
+  if (other == p->stream) return MARIE_OK;
+  cudaStreamCaptureStatus capturing;
+  if (cudaStreamIsCapturing(other, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone ||
+      cudaStreamQuery(other) == cudaSuccess) {
+    cudaGetLastError();
+    return MARIE_OK;
+  }
+  cudaGetLastError();  // not ready
+  int dev = 0;
+  MARIE_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev != p->device) {  // an event belongs to one device
+    MARIE_CUDA_TRY(cudaStreamSynchronize(other));
+    return MARIE_OK;
+  }
+  if (!p->after) MARIE_CUDA_TRY(cudaEventCreateWithFlags(&p->after, cudaEventDisableTiming));
+  MARIE_CUDA_TRY(cudaEventRecord(p->after, other));
+  MARIE_CUDA_TRY(cudaStreamWaitEvent(p->stream, p->after, 0));
+  return MARIE_OK;
+}
 
 // A schedule is a choice on the grids that have fused passes.  Elsewhere there is
 // none to make, and the box that a product is cut to, which may have them where

@@ -59,6 +59,8 @@ struct marie_plan {
   void* arena = nullptr;
   bool whole_grid = false;  // no crop is made (a solve that ran out of memory beside one)
 
+  cudaEvent_t after = nullptr;  // marie_plan_after_stream's
+
   // Spectra workspace (3 x N x 2M x 2L per rhs).
   void* wsB = nullptr;
   size_t ws_bytes_B = 0;

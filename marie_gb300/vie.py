@@ -31,7 +31,8 @@ argument order, defaults and return tuples:
 Grid arrays are (L, M, N[, 3 or 6]) in column-major order, exactly the
 reference's MATLAB arrays: numpy arrays (host; copied to the device per call,
 like gpuArray/gather) or torch CUDA tensors with column-major strides (used in
-place).  idx vectors are 1-based.  All compute runs in libmarie_vie.so on the
+place, after what torch's current stream holds at the call; results are ready
+when it returns).  idx vectors are 1-based.  All compute runs in libmarie_vie.so on the
 GPU; there is no CPU path.
 """
 from __future__ import annotations
@@ -129,9 +130,20 @@ def _sync_stream(op):
     torch.cuda.ExternalStream(op.lib.marie_plan_stream(op.plan)).synchronize()
 
 
-def _sync():
-    if torch is not None and torch.cuda.is_available():
-        torch.cuda.current_stream().synchronize()
+def _ready(op):
+    """An Operator's plan for a call on arrays, its stream ordered after torch's
+    current one: CUDA inputs may still be computed there, and the memory of new
+    outputs may still be read."""
+    if torch is not None and torch.cuda.is_initialized():
+        check(op.lib.marie_plan_after_stream(op.plan, _current_stream(torch.cuda.current_device())))
+    return op.plan
+
+
+def _current_stream(device):
+    """The handle of torch's current stream (torch.cuda.current_stream builds an
+    object around it, 10 us of a call where this takes 1)."""
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return raw(device) if raw else torch.cuda.current_stream(device).cuda_stream
 
 
 # ---------------------------------------------------------------------------
@@ -164,7 +176,7 @@ class Operator:
             raise ValueError("fN must be 2L x 2M x 2N x 6")
         op = cls(Lf // 2, Mf // 2, Nf // 2, precision, nrhs_max)
         ptr, keep = _in(fN)
-        check(op.lib.marie_set_operator(op.plan, ptr, Lf, Mf, Nf))
+        check(op.lib.marie_set_operator(_ready(op), ptr, Lf, Mf, Nf))
         del keep
         return op
 
@@ -190,7 +202,7 @@ class Operator:
     def set_k(self, fK):
         """Upload the K operator into this plan (beside fN)."""
         ptr, keep = _in(fK)
-        check(self.lib.marie_set_operator_k(self.plan, ptr, 2 * self.L, 2 * self.M, 2 * self.N))
+        check(self.lib.marie_set_operator_k(_ready(self), ptr, 2 * self.L, 2 * self.M, 2 * self.N))
         del keep
         return self
 
@@ -233,7 +245,7 @@ class Operator:
         mcp, mck = _in(Mc)
         ip, ik = _in(idx, np.int64)
         n = int(np.asarray(idx).size) if not _is_cuda(idx) else int(idx.numel())
-        check(self.lib.marie_plan_bind_mv_AN(self.plan, mrp, mcp, float(Gram), 1 if transp_flag == "transp" else 0,
+        check(self.lib.marie_plan_bind_mv_AN(_ready(self), mrp, mcp, float(Gram), 1 if transp_flag == "transp" else 0,
                                              ip, n))
         return self
 
@@ -245,7 +257,7 @@ class Operator:
         nrhs = 1 if J.ndim == 1 else J.shape[1]
         jp, jk = _in(J)
         op_, out = _out(J.shape, cuda)
-        check(self.lib.marie_plan_apply_mv_AN(self.plan, jp, op_, nrhs, _PREC[precision]))
+        check(self.lib.marie_plan_apply_mv_AN(_ready(self), jp, op_, nrhs, _PREC[precision]))
         if cuda:
             _sync_stream(self)
         return out
@@ -385,7 +397,7 @@ def mv_AN(JIn0, fN, Mr, Mc, Gram, transp_flag, idx, GPU_flag=1, precision="fp64"
         mcp, mck = _in(Mc)
         ip, ik = _in(idx, np.int64)
         op_, out = _out(JIn0.shape, cuda)
-        check(opr.lib.marie_mv_AN(opr.plan, jp, mrp, mcp, float(Gram), 1 if transp_flag == "transp" else 0,
+        check(opr.lib.marie_mv_AN(_ready(opr), jp, mrp, mcp, float(Gram), 1 if transp_flag == "transp" else 0,
                                   ip, n, op_, nrhs, prec))
         return out
     finally:
@@ -404,7 +416,7 @@ def mv_L(JIn0, fN, r, Gram, idx, GPU_flag=1, precision="fp64"):
         jp, jk = _in(JIn0)
         ip, ik = _in(idx, np.int64)
         op_, out = _out(JIn0.shape, cuda)
-        check(opr.lib.marie_mv_L(opr.plan, jp, float(Gram), ip, n, op_, nrhs, prec))
+        check(opr.lib.marie_mv_L(_ready(opr), jp, float(Gram), ip, n, op_, nrhs, prec))
         return out
     finally:
         if tmp:
@@ -434,7 +446,7 @@ def mv_K(JIn0, fK, r, idx, GPU_flag=1, precision="fp64"):
         jp, jk = _in(JIn0)
         ip, ik = _in(idx, np.int64)
         op_, out = _out(JIn0.shape, cuda)
-        check(opr.lib.marie_mv_K(opr.plan, jp, ip, n, op_, nrhs, prec))
+        check(opr.lib.marie_mv_K(_ready(opr), jp, ip, n, op_, nrhs, prec))
         return out
     finally:
         if tmp:
@@ -450,7 +462,7 @@ def H_field_Kop(J, fK, Gram, Hinc=None, GPU_flag=1, precision="fp64"):
         jp, jk = _in(J)
         hp, hk = _in(Hinc) if Hinc is not None else (None, None)
         op_, out = _out(tuple(J.shape), _is_cuda(J))
-        check(opr.lib.marie_h_field_kop(opr.plan, jp, float(Gram), hp, op_, _PREC[precision]))
+        check(opr.lib.marie_h_field_kop(_ready(opr), jp, float(Gram), hp, op_, _PREC[precision]))
         return out
     finally:
         if tmp:
@@ -469,7 +481,7 @@ def E_field_Nop(J, fN, Gram, freq, Einc=None, GPU_flag=1, precision="fp64"):
         else:
             ep, ek = None, None
         op_, out = _out(tuple(J.shape), _is_cuda(J))
-        check(opr.lib.marie_e_field_nop(opr.plan, jp, float(Gram), float(freq), ep, op_, _PREC[precision]))
+        check(opr.lib.marie_e_field_nop(_ready(opr), jp, float(Gram), float(freq), ep, op_, _PREC[precision]))
         return out
     finally:
         if tmp:
@@ -561,7 +573,7 @@ def pgmres(A, b, restart=50, tol=1e-3, maxit=10, L1=None, L2=None, R1=None, R2=N
     cap = restart * maxit + 1
     resvec = np.zeros(cap)
     rlen = C.c_int64()
-    _call(opr.lib.marie_pgmres, opr.plan, cbs[0], None, bp, n, int(restart), float(tol), int(maxit),
+    _call(opr.lib.marie_pgmres, _ready(opr), cbs[0], None, bp, n, int(restart), float(tol), int(maxit),
           h[0], None, h[1], None, h[2], None, h[3], None, x0p, xp, C.byref(flag), C.byref(relres), it,
           resvec.ctypes.data_as(_lib._dp), cap, C.byref(rlen))
     return x, flag.value, relres.value, [it[0], it[1]], resvec[:rlen.value]
@@ -584,7 +596,7 @@ def pgmresDR(A, b, restart=50, tol=1e-3, maxit=10, ritz=None, L1=None, L2=None, 
     cap = restart * (maxit + 1) + 1
     resvec = np.zeros(cap)
     rlen = C.c_int64()
-    _call(opr.lib.marie_pgmres_dr, opr.plan, cbs[0], None, bp, n, int(restart), float(tol), int(maxit),
+    _call(opr.lib.marie_pgmres_dr, _ready(opr), cbs[0], None, bp, n, int(restart), float(tol), int(maxit),
           int(ritz) if ritz is not None else 0, h[0], None, h[1], None, h[2], None, h[3], None, x0p, xp,
           C.byref(flag), C.byref(relres), it, resvec.ctypes.data_as(_lib._dp), cap, C.byref(rlen))
     return x, flag.value, relres.value, [it[0], it[1]], resvec[:rlen.value]
@@ -607,7 +619,7 @@ def bicgstab(A, b, tol=1e-6, maxit=None, M1=None, M2=None, x0=None):
     cap = 2 * maxit + 1
     resvec = np.zeros(cap)
     rlen = C.c_int64()
-    _call(opr.lib.marie_bicgstab, opr.plan, cbs[0], None, bp, n, float(tol), int(maxit), h[0], None, h[1], None,
+    _call(opr.lib.marie_bicgstab, _ready(opr), cbs[0], None, bp, n, float(tol), int(maxit), h[0], None, h[1], None,
           x0p, xp, C.byref(flag), C.byref(relres), C.byref(it), resvec.ctypes.data_as(_lib._dp), cap,
           C.byref(rlen))
     return x, flag.value, relres.value, it.value, resvec[:rlen.value]
@@ -659,8 +671,8 @@ def JVIE_Solver(Einc, e_r, r, freq, fN, tol=None, form=None, solver=None, precon
         resvec = np.zeros(cap)
         rlen = C.c_int64()
         solvert = C.c_double()
-        check(opr.lib.marie_jvie_solve(opr.plan, ep, erp, dx, float(freq), float(tol), int(form), solver.encode(), pc,
-                                       int(max_it), int(inner_it), int(outer_it), int(ritz), jp, C.byref(flag),
+        check(opr.lib.marie_jvie_solve(_ready(opr), ep, erp, dx, float(freq), float(tol), int(form), solver.encode(),
+                                       pc, int(max_it), int(inner_it), int(outer_it), int(ritz), jp, C.byref(flag),
                                        C.byref(relres), it, resvec.ctypes.data_as(_lib._dp), cap, C.byref(rlen),
                                        C.byref(solvert)))
         iters = it[0] if solver == "B" else [int(it[0]), int(it[1])]
@@ -723,7 +735,7 @@ def Scat_Solver(Einc, Hinc, freq, r, epsilon_r, sigma_e, rho, tol=None, fN=None,
         opr = Operator(L, M, N, precision)
         if fN is not None:
             ptr, keep = _in(fN)
-            check(opr.lib.marie_set_operator(opr.plan, ptr, 2 * L, 2 * M, 2 * N))
+            check(opr.lib.marie_set_operator(_ready(opr), ptr, 2 * L, 2 * M, 2 * N))
         if fK is not None:
             opr.set_k(fK)
     cuda = _is_cuda(Einc)
@@ -737,7 +749,7 @@ def Scat_Solver(Einc, Hinc, freq, r, epsilon_r, sigma_e, rho, tol=None, fN=None,
     eo, Eout = _out((L, M, N, 3), cuda)
     bo, Bout = _out((L, M, N, 3), cuda)
     gsar, pabs = C.c_double(), C.c_double()
-    check(opr.lib.marie_scat_solver(opr.plan, ep, hp, dx, float(freq), epsp, sp_, rp_, float(tol), int(form),
+    check(opr.lib.marie_scat_solver(_ready(opr), ep, hp, dx, float(freq), epsp, sp_, rp_, float(tol), int(form),
                                     solver.encode(), pc, int(max_it), int(inner_it), int(outer_it), int(ritz), jp, spo,
                                     eo, bo, C.byref(gsar), C.byref(pabs)))
     solvelog.write_overall_log(logfile, time.perf_counter() - tstart)
@@ -768,7 +780,7 @@ def JVIE_Solver_batch(Einc, e_r, r, freq, fN, tol=None, form=None, precond=None,
         relres = np.zeros(nexc)
         it = np.zeros(2 * nexc, np.int32)
         solvert = C.c_double()
-        check(opr.lib.marie_jvie_solve_batch(opr.plan, ep, nexc, erp, dx, float(freq), int(form), pc, float(tol),
+        check(opr.lib.marie_jvie_solve_batch(_ready(opr), ep, nexc, erp, dx, float(freq), int(form), pc, float(tol),
                                              int(inner_it), int(outer_it), jp,
                                              flag.ctypes.data_as(_lib._ip), relres.ctypes.data_as(_lib._dp),
                                              it.ctypes.data_as(_lib._ip), C.byref(solvert)))
@@ -805,7 +817,7 @@ def JVIE_Solver_bodies(bodies, freq, tol=None, form=None, precond=None, inner_it
         Erp.append(erp.value)
         Jp.append(jp.value)
         outs.append(Je)
-        plans[b] = op.plan.value
+        plans[b] = _ready(op).value
     tot = int(nexc.sum())
     flag = np.zeros(tot, np.int32)
     relres = np.zeros(tot)
@@ -863,7 +875,7 @@ def jvie2solver(Vrhs, fN, idx, Mr, Mc, Gram, tol, Vini=None, max_it=1000):
         relres = C.c_double()
         it = C.c_double()
         solvert = C.c_double()
-        check(opr.lib.marie_jvie2solver(opr.plan, ip, n, mrp, mcp, float(Gram), bp, float(tol), int(max_it), xp, op_,
+        check(opr.lib.marie_jvie2solver(_ready(opr), ip, n, mrp, mcp, float(Gram), bp, float(tol), int(max_it), xp, op_,
                                         C.byref(flag), C.byref(relres), C.byref(it), C.byref(solvert)))
         return out, flag.value, relres.value, it.value, solvert.value
     finally:

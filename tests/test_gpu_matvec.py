@@ -266,3 +266,53 @@ def test_field_wrappers_refuse_a_current_that_requires_grad(cuda):
             f(J.clone().requires_grad_())
         assert f(torch.zeros_like(J)) is F
     op.close()
+
+
+@pytest.mark.parametrize("call", ["mv_AN", "bind", "apply", "e_field"])
+def test_inputs_still_being_computed_on_torchs_stream(cuda, call):
+    """CUDA inputs that torch's current stream has yet to write (behind a product
+    of 4096 x 4096 FP64 matrices) are waited for: the results are those of the
+    finished inputs, to the bit."""
+    import torch
+
+    import marie_gb300 as mg
+
+    shape, dx = (16, 12, 20), 5e-3
+    op = mg.Operator.assemble(*shape, dx, 298e6, precision="mixed")
+    V = int(np.prod(shape))
+    col = lambda s: torch.randn(*reversed(s), dtype=torch.complex128, device=cuda).permute(*reversed(range(len(s))))
+    final = {"J": torch.randn(3 * V, dtype=torch.complex128, device=cuda), "Mr": col(shape), "Mc": col(shape),
+             "idx": torch.randperm(3 * V, device=cuda) + 1, "field": col((*shape, 3)), "E": col((*shape, 3))}
+    big = torch.ones(4096, 4096, dtype=torch.float64, device=cuda)
+
+    def run(a, late):
+        def now(*names):
+            if late:
+                torch.cuda.synchronize()
+                torch.mm(big, big)
+                for n in names:
+                    a[n].copy_(final[n])
+            return [a[n] for n in names]
+
+        if call == "mv_AN":
+            J, Mr, Mc, idx = now("J", "Mr", "Mc", "idx")
+            return mg.mv_AN(J, op, Mr, Mc, dx**3, "notransp", idx, precision="fp32")
+        if call == "e_field":
+            J, = now("field")
+            return mg.E_field_Nop(J, op, dx**3, 298e6, None)
+        if call == "bind":
+            op.bind_mv_AN(*now("Mr", "Mc"), dx**3, "transp", *now("idx"))
+            return op.apply_mv_AN(final["J"], precision="fp64")
+        op.bind_mv_AN(final["Mr"], final["Mc"], dx**3, "notransp", final["idx"])
+        return op.apply_mv_AN(*now("J"), precision="fp32")
+
+    torch.cuda.synchronize()
+    ref = run({k: v.clone() for k, v in final.items()}, False)
+    torch.cuda.synchronize()
+    # valid but other inputs until the copies arrive
+    early = {k: v.clone() if k == "idx" else 2 * v for k, v in final.items()}
+    early["idx"] = final["idx"].flip(0).clone()
+    out = run(early, True)
+    torch.cuda.synchronize()
+    assert torch.equal(out, ref)
+    op.close()
