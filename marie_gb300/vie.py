@@ -77,6 +77,8 @@ def _is_cuda(a) -> bool:
 def _colmajor_cuda(t, dtype):
     """Column-major contiguous CUDA tensor of the same shape (no copy if already)."""
     t = t.to(dtype)
+    if t.is_conj() or t.is_neg():  # a view whose memory is not its value
+        t = t.resolve_conj().resolve_neg()
     if t.dim() <= 1:
         return t.contiguous()
     step, ordered = 1, True

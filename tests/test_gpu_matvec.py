@@ -316,3 +316,28 @@ def test_inputs_still_being_computed_on_torchs_stream(cuda, call):
     torch.cuda.synchronize()
     assert torch.equal(out, ref)
     op.close()
+
+
+def test_conjugate_and_negative_views_are_read_as_their_values(cuda):
+    """x.conj() and the imaginary part of one are views that torch resolves when
+    they are read: as inputs they give what their copies give."""
+    import torch
+
+    import marie_gb300 as mg
+
+    shape, dx = (8, 12, 16), 5e-3
+    op = mg.Operator.assemble(*shape, dx, 298e6)
+    V = int(np.prod(shape))
+    col = lambda s: torch.randn(*reversed(s), dtype=torch.complex128, device=cuda).permute(*reversed(range(len(s))))
+    J, Mr, Mc, F = torch.randn(3 * V, dtype=torch.complex128, device=cuda), col(shape), col(shape), col((*shape, 3))
+    idx = torch.arange(3 * V, device=cuda) + 1
+    negative = J.conj().imag
+    assert negative.is_neg()
+    for view in (J.conj(), negative):
+        out, ref = (mg.mv_AN(v, op, Mr.conj(), Mc, dx**3, "notransp", idx) for v in (view, view.resolve_conj().resolve_neg()))
+        assert torch.equal(out, ref)
+    own = mg.mv_AN(J.conj().resolve_conj(), op, Mr.conj().resolve_conj(), Mc, dx**3, "notransp", idx)
+    assert torch.equal(mg.mv_AN(J.conj(), op, Mr.conj(), Mc, dx**3, "notransp", idx), own)
+    E = [mg.E_field_Nop(f, op, dx**3, 298e6, F) for f in (F.conj(), F.conj().resolve_conj())]
+    assert torch.equal(*E)
+    op.close()
