@@ -66,6 +66,8 @@ void* marie_plan_stream(marie_plan* plan);
  * that belong to it (no counterpart in the reference).  A stream that is idle or
  * being captured needs no order and gets none. */
 int marie_plan_after_stream(marie_plan* plan, void* stream);
+/* Waits for the work queued on the plan's stream. */
+int marie_plan_synchronize(marie_plan* plan);
 
 /* Replaces getOPERATORS(r, f, op, type, singular)
  * (src_vie/src_operators/getOPERATORS.m:1-127) for op = 'N' (6 components)

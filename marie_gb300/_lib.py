@@ -41,6 +41,7 @@ SIGNATURES = {
     "marie_plan_destroy": (C.c_int, [_vp]),
     "marie_plan_stream": (_vp, [_vp]),
     "marie_plan_after_stream": (C.c_int, [_vp, _vp]),
+    "marie_plan_synchronize": (C.c_int, [_vp]),
     "marie_get_operators": (C.c_int, [_vp, C.c_int64, C.c_int64, C.c_int64, C.c_double, C.c_char, C.c_char,
                                       C.c_char, _vp, _vp]),
     "marie_singular_integrals": (C.c_int, [C.c_double, C.c_double, _vp]),

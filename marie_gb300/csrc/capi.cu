@@ -892,13 +892,15 @@ int marie_plan_after_stream(marie_plan* p, void* stream) {
   if (!p) return set_error(MARIE_EINVAL, "NULL plan");
   cudaStream_t other = (cudaStream_t)stream;
   if (other == p->stream) return MARIE_OK;
-  cudaStreamCaptureStatus capturing;
-  if (cudaStreamIsCapturing(other, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone ||
-      cudaStreamQuery(other) == cudaSuccess) {
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  if (other && (cudaStreamIsCapturing(other, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone)) {
     cudaGetLastError();
     return MARIE_OK;
   }
-  cudaGetLastError();  // not ready
+  const cudaError_t busy = cudaStreamQuery(other);
+  if (busy == cudaSuccess) return MARIE_OK;
+  cudaGetLastError();
+  if (busy != cudaErrorNotReady) return MARIE_OK;  // (the call itself meets an error that lasts)
   int dev = 0;
   MARIE_CUDA_TRY(cudaGetDevice(&dev));
   if (dev != p->device) {  // an event belongs to one device
@@ -908,6 +910,12 @@ int marie_plan_after_stream(marie_plan* p, void* stream) {
   if (!p->after) MARIE_CUDA_TRY(cudaEventCreateWithFlags(&p->after, cudaEventDisableTiming));
   MARIE_CUDA_TRY(cudaEventRecord(p->after, other));
   MARIE_CUDA_TRY(cudaStreamWaitEvent(p->stream, p->after, 0));
+  return MARIE_OK;
+}
+
+int marie_plan_synchronize(marie_plan* p) {
+  if (!p) return set_error(MARIE_EINVAL, "NULL plan");
+  MARIE_CUDA_TRY(cudaStreamSynchronize(p->stream));
   return MARIE_OK;
 }
 

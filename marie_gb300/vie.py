@@ -127,9 +127,9 @@ def release_cached_memory():
     check(_lib.load().marie_release_cached_memory())
 
 
-def _sync_stream(op):
-    """Waits for the work queued on an Operator's plan stream."""
-    torch.cuda.ExternalStream(op.lib.marie_plan_stream(op.plan)).synchronize()
+# torch's current stream as a handle: torch.cuda.current_stream builds an object
+# around it, 10 us of a call where this takes 1
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) if torch is not None else None
 
 
 def _ready(op):
@@ -137,15 +137,13 @@ def _ready(op):
     current one: CUDA inputs may still be computed there, and the memory of new
     outputs may still be read."""
     if torch is not None and torch.cuda.is_initialized():
-        check(op.lib.marie_plan_after_stream(op.plan, _current_stream(torch.cuda.current_device())))
+        if op._device is None:
+            op._device = torch.cuda.current_device()
+        stream = _raw_stream(op._device) if _raw_stream else torch.cuda.current_stream(op._device).cuda_stream
+        status = op.lib.marie_plan_after_stream(op._plan, stream)
+        if status:
+            check(status)
     return op.plan
-
-
-def _current_stream(device):
-    """The handle of torch's current stream (torch.cuda.current_stream builds an
-    object around it, 10 us of a call where this takes 1)."""
-    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-    return raw(device) if raw else torch.cuda.current_stream(device).cuda_stream
 
 
 # ---------------------------------------------------------------------------
@@ -162,6 +160,7 @@ class Operator:
         ph = C.c_void_p()
         check(self.lib.marie_plan_create(self.L, self.M, self.N, self.precision, int(nrhs_max), None, C.byref(ph)))
         self._plan = ph
+        self._device = None  # torch's index of the plan's device, from the first call on arrays
         self.dx = None
         self.freq = None
 
@@ -261,7 +260,7 @@ class Operator:
         op_, out = _out(J.shape, cuda)
         check(self.lib.marie_plan_apply_mv_AN(_ready(self), jp, op_, nrhs, _PREC[precision]))
         if cuda:
-            _sync_stream(self)
+            check(self.lib.marie_plan_synchronize(self.plan))
         return out
 
     def set_inner_restart(self, restart):
