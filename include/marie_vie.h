@@ -234,8 +234,9 @@ int marie_bicgstab(marie_plan* plan, marie_op_fn A, void* A_ctx, const double* b
  * bound mv_AN, run on the smallest transform grid that holds the body's box, if
  * that is at most 0.8 of the plan's.  The plan keeps that operator (FP64 plans or
  * MARIE_MIXED ones, at most 0.8 of its own) for the next body of the same box,
- * until its own changes, one of its calls finds no memory (the call then runs on
- * the whole grid) or marie_plan_destroy. */
+ * until its own changes, one of its solves, products or field calls finds no
+ * memory (the call, and the products of a bound mv_AN until it is bound again,
+ * then run on the whole grid) or marie_plan_destroy. */
 int marie_jvie_solve(marie_plan* plan, const double* Einc, const double* e_r, double dx,
                      double freq, double tol, int form, char solver, char precond, int max_it,
                      int inner_it, int outer_it, int ritz, double* Je, int* flag, double* relres,

@@ -97,29 +97,30 @@ using namespace marie;
 extern "C" int marie_jvie_adjoint_grad(marie_plan* p, const double* Einc, const double* e_r, double dx, double freq,
                                        int objective, const double* E_target, double tol, int inner_it, int outer_it,
                                        double* F, double* dF_deps, double* dF_dsigma, int* flags, int* iters) {
-  if (!p || !Einc || !e_r || !F || !dF_deps || !dF_dsigma) return set_error(MARIE_EINVAL, "NULL argument");
-  if (objective != 0 && objective != 1) return set_error(MARIE_EINVAL, "objective must be 0 (power) or 1 (misfit)");
-  if (objective == 1 && !E_target) return set_error(MARIE_EINVAL, "the misfit objective needs E_target");
-  if (!p->has_op) return set_error(MARIE_ENOOP, "plan has no operator");
-  if (tol < 1e-15 || tol >= 1) tol = 1e-3;
-  if (inner_it < 1) inner_it = 50;
-  if (outer_it < 1) outer_it = 200;
-  cudaStream_t st = p->stream;
-  const long long V = p->d.V;
-  DBuf tE, tER, tEt, tge, tgs;
-  const void *E_d, *er_d, *Et_d = nullptr;
-  void *ge_d, *gs_d;
-  MARIE_TRY(stage_in(Einc, 3 * V * sizeof(double2), st, tE, &E_d));
-  MARIE_TRY(stage_in(e_r, V * sizeof(double2), st, tER, &er_d));
-  if (E_target) MARIE_TRY(stage_in(E_target, 3 * V * sizeof(double2), st, tEt, &Et_d));
-  MARIE_TRY(stage_out(dF_deps, V * sizeof(double), st, tge, &ge_d));
-  MARIE_TRY(stage_out(dF_dsigma, V * sizeof(double), st, tgs, &gs_d));
-  MARIE_TRY(on_box_or_whole_grid(p, [&]() {
-    return jvie_adjoint_core(p, (const double2*)E_d, (const double2*)er_d, dx, freq, objective, (const double2*)Et_d,
-                             tol, inner_it, outer_it, F, (double*)ge_d, (double*)gs_d, flags, iters);
-  }));
-  MARIE_TRY(finish_out(dF_deps, ge_d, V * sizeof(double), st));
-  MARIE_TRY(finish_out(dF_dsigma, gs_d, V * sizeof(double), st));
-  MARIE_CUDA_TRY(cudaStreamSynchronize(st));
-  return check_kernel_status(p);
+  return on_box_or_whole_grid(p, [&]() -> int {
+    if (!p || !Einc || !e_r || !F || !dF_deps || !dF_dsigma) return set_error(MARIE_EINVAL, "NULL argument");
+    if (objective != 0 && objective != 1) return set_error(MARIE_EINVAL, "objective must be 0 (power) or 1 (misfit)");
+    if (objective == 1 && !E_target) return set_error(MARIE_EINVAL, "the misfit objective needs E_target");
+    if (!p->has_op) return set_error(MARIE_ENOOP, "plan has no operator");
+    if (tol < 1e-15 || tol >= 1) tol = 1e-3;
+    if (inner_it < 1) inner_it = 50;
+    if (outer_it < 1) outer_it = 200;
+    cudaStream_t st = p->stream;
+    const long long V = p->d.V;
+    DBuf tE, tER, tEt, tge, tgs;
+    const void *E_d, *er_d, *Et_d = nullptr;
+    void *ge_d, *gs_d;
+    MARIE_TRY(stage_in(Einc, 3 * V * sizeof(double2), st, tE, &E_d));
+    MARIE_TRY(stage_in(e_r, V * sizeof(double2), st, tER, &er_d));
+    if (E_target) MARIE_TRY(stage_in(E_target, 3 * V * sizeof(double2), st, tEt, &Et_d));
+    MARIE_TRY(stage_out(dF_deps, V * sizeof(double), st, tge, &ge_d));
+    MARIE_TRY(stage_out(dF_dsigma, V * sizeof(double), st, tgs, &gs_d));
+    MARIE_TRY(jvie_adjoint_core(p, (const double2*)E_d, (const double2*)er_d, dx, freq, objective,
+                                (const double2*)Et_d, tol, inner_it, outer_it, F, (double*)ge_d, (double*)gs_d, flags,
+                                iters));
+    MARIE_TRY(finish_out(dF_deps, ge_d, V * sizeof(double), st));
+    MARIE_TRY(finish_out(dF_dsigma, gs_d, V * sizeof(double), st));
+    MARIE_CUDA_TRY(cudaStreamSynchronize(st));
+    return check_kernel_status(p);
+  });
 }

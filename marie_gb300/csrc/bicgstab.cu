@@ -422,41 +422,43 @@ extern "C" int marie_bicgstab(marie_plan* p, marie_op_fn A, void* A_ctx, const d
                               int maxit, marie_op_fn M1, void* M1_ctx, marie_op_fn M2, void* M2_ctx, const double* x0,
                               double* x, int* flag, double* relres, double* iter, double* resvec, int64_t resvec_cap,
                               int64_t* resvec_len) {
-  if (!p || !b || !x || n < 1) return set_error(MARIE_EINVAL, "NULL argument or n < 1");
-  // user operators run outside the plan's stream: finish the plan's work first
-  auto wrap = [p](marie_op_fn f, void* ctx, long long nn) -> DevOp {
-    return [p, f, ctx, nn](const double2* xi, double2* yo) -> int {
-      MARIE_CUDA_TRY(cudaStreamSynchronize(p->stream));
-      const int s = f(ctx, reinterpret_cast<const double*>(xi), reinterpret_cast<double*>(yo), nn);
-      if (s != MARIE_OK) return set_error(s, "user operator returned status %d", s);
-      return MARIE_OK;
+  return on_box_or_whole_grid(p, [&]() -> int {
+    if (!p || !b || !x || n < 1) return set_error(MARIE_EINVAL, "NULL argument or n < 1");
+    // user operators run outside the plan's stream: finish the plan's work first
+    auto wrap = [p](marie_op_fn f, void* ctx, long long nn) -> DevOp {
+      return [p, f, ctx, nn](const double2* xi, double2* yo) -> int {
+        MARIE_CUDA_TRY(cudaStreamSynchronize(p->stream));
+        const int s = f(ctx, reinterpret_cast<const double*>(xi), reinterpret_cast<double*>(yo), nn);
+        if (s != MARIE_OK) return set_error(s, "user operator returned status %d", s);
+        return MARIE_OK;
+      };
     };
-  };
-  DevOp opA, oM1, oM2;
-  if (A)
-    opA = wrap(A, A_ctx, n);
-  else
-    MARIE_TRY(bound_operator(p, n, &opA));  // NULL A: the plan's bound mv_AN
-  if (M1) oM1 = wrap(M1, M1_ctx, n);
-  if (M2) oM2 = wrap(M2, M2_ctx, n);
-  const size_t bytes = (size_t)n * sizeof(double2);
-  DBuf tb, tx0, txo;
-  const void *b_d, *x0_d = nullptr;
-  void* x_d;
-  MARIE_TRY(stage_in(b, bytes, p->stream, tb, &b_d));
-  if (x0) MARIE_TRY(stage_in(x0, bytes, p->stream, tx0, &x0_d));
-  MARIE_TRY(stage_out(x, bytes, p->stream, txo, &x_d));
-  BicgResult res;
-  MARIE_TRY(bicgstab(p, opA, M1 ? &oM1 : nullptr, M2 ? &oM2 : nullptr, (const double2*)b_d, n, tol, maxit,
-                     (const double2*)x0_d, (double2*)x_d, res));
-  MARIE_TRY(finish_out(x, x_d, bytes, p->stream));
-  MARIE_CUDA_TRY(cudaStreamSynchronize(p->stream));
-  if (flag) *flag = res.flag;
-  if (relres) *relres = res.relres;
-  if (iter) *iter = res.iter;
-  const int64_t nr = (int64_t)res.resvec.size();
-  if (resvec_len) *resvec_len = nr;
-  if (resvec)
-    for (int64_t i = 0; i < nr && i < resvec_cap; ++i) resvec[i] = res.resvec[i];
-  return check_kernel_status(p);
+    DevOp opA, oM1, oM2;
+    if (A)
+      opA = wrap(A, A_ctx, n);
+    else
+      MARIE_TRY(bound_operator(p, n, &opA));  // NULL A: the plan's bound mv_AN
+    if (M1) oM1 = wrap(M1, M1_ctx, n);
+    if (M2) oM2 = wrap(M2, M2_ctx, n);
+    const size_t bytes = (size_t)n * sizeof(double2);
+    DBuf tb, tx0, txo;
+    const void *b_d, *x0_d = nullptr;
+    void* x_d;
+    MARIE_TRY(stage_in(b, bytes, p->stream, tb, &b_d));
+    if (x0) MARIE_TRY(stage_in(x0, bytes, p->stream, tx0, &x0_d));
+    MARIE_TRY(stage_out(x, bytes, p->stream, txo, &x_d));
+    BicgResult res;
+    MARIE_TRY(bicgstab(p, opA, M1 ? &oM1 : nullptr, M2 ? &oM2 : nullptr, (const double2*)b_d, n, tol, maxit,
+                       (const double2*)x0_d, (double2*)x_d, res));
+    MARIE_TRY(finish_out(x, x_d, bytes, p->stream));
+    MARIE_CUDA_TRY(cudaStreamSynchronize(p->stream));
+    if (flag) *flag = res.flag;
+    if (relres) *relres = res.relres;
+    if (iter) *iter = res.iter;
+    const int64_t nr = (int64_t)res.resvec.size();
+    if (resvec_len) *resvec_len = nr;
+    if (resvec)
+      for (int64_t i = 0; i < nr && i < resvec_cap; ++i) resvec[i] = res.resvec[i];
+    return check_kernel_status(p);
+  });
 }

@@ -1122,128 +1122,136 @@ static int check_prec(marie_plan* p, int precision) {
 
 int marie_mv_AN(marie_plan* p, const double* JIn0, const double* Mr, const double* Mc, double Gram, int transp,
                 const int64_t* idx, int64_t n_idx, double* JOut, int64_t nrhs, int precision) {
-  if (!p || !JIn0 || !Mr || !Mc || !JOut || (!idx && n_idx > 0)) return set_error(MARIE_EINVAL, "NULL argument");
-  if (nrhs < 1) return set_error(MARIE_EINVAL, "nrhs must be >= 1");
-  if (transp != 0 && transp != 1) return set_error(MARIE_EINVAL, "transp must be 0 ('notransp') or 1 ('transp')");
-  MARIE_TRY(check_prec(p, precision));
-  if (!p->has_op) return set_error(MARIE_ENOOP, "plan has no operator");
-  const long long V = p->d.V, n = n_idx;
-  DBuf tJ, tMr, tMc, tidx, tout, inv, ca, cb;
-  const void *J_d, *Mr_d, *Mc_d, *idx_d;
-  void* out_d;
-  MARIE_TRY(stage_in(JIn0, n * nrhs * sizeof(double2), p->stream, tJ, &J_d));
-  MARIE_TRY(stage_in(Mr, V * sizeof(double2), p->stream, tMr, &Mr_d));
-  MARIE_TRY(stage_in(Mc, V * sizeof(double2), p->stream, tMc, &Mc_d));
-  MARIE_TRY(stage_in(idx, n * sizeof(int64_t), p->stream, tidx, &idx_d));
-  MARIE_TRY(stage_out(JOut, n * nrhs * sizeof(double2), p->stream, tout, &out_d));
-  MARIE_TRY(inv.alloc(3 * V * sizeof(int), p->stream));
-  MARIE_TRY(ca.alloc(n * sizeof(double2), p->stream));
-  MARIE_TRY(cb.alloc(n * sizeof(double2), p->stream));
-  MARIE_TRY(build_inverse_index(p, (const int64_t*)idx_d, n, inv.as<int>()));
-  MARIE_TRY(build_coefficients(p, (const int64_t*)idx_d, n, (const double2*)Mr_d, (const double2*)Mc_d, Gram, transp,
-                               ca.as<double2>(), cb.as<double2>()));
-  Prologue pro{nullptr, 0};
-  Epilogue ep{};
-  if (transp == 0) {
-    ep.a = ca.as<double2>();
-    ep.b = cb.as<double2>();
-    ep.conjout = 0;
-  } else {
-    pro.pre = cb.as<double2>();
-    pro.conjin = 1;
-    ep.a = ca.as<double2>();
-    ep.conjout = 1;
-  }
-  if (n > 0)
-    MARIE_TRY(run_matvec(p, precision, (const double2*)J_d, (double2*)out_d, n, (int)nrhs, inv.as<int>(), pro, ep));
-  MARIE_TRY(finish_out(JOut, out_d, n * nrhs * sizeof(double2), p->stream));
-  return check_kernel_status(p);  // (synchronises)
+  return on_box_or_whole_grid(p, [&]() -> int {
+    if (!p || !JIn0 || !Mr || !Mc || !JOut || (!idx && n_idx > 0)) return set_error(MARIE_EINVAL, "NULL argument");
+    if (nrhs < 1) return set_error(MARIE_EINVAL, "nrhs must be >= 1");
+    if (transp != 0 && transp != 1) return set_error(MARIE_EINVAL, "transp must be 0 ('notransp') or 1 ('transp')");
+    MARIE_TRY(check_prec(p, precision));
+    if (!p->has_op) return set_error(MARIE_ENOOP, "plan has no operator");
+    const long long V = p->d.V, n = n_idx;
+    DBuf tJ, tMr, tMc, tidx, tout, inv, ca, cb;
+    const void *J_d, *Mr_d, *Mc_d, *idx_d;
+    void* out_d;
+    MARIE_TRY(stage_in(JIn0, n * nrhs * sizeof(double2), p->stream, tJ, &J_d));
+    MARIE_TRY(stage_in(Mr, V * sizeof(double2), p->stream, tMr, &Mr_d));
+    MARIE_TRY(stage_in(Mc, V * sizeof(double2), p->stream, tMc, &Mc_d));
+    MARIE_TRY(stage_in(idx, n * sizeof(int64_t), p->stream, tidx, &idx_d));
+    MARIE_TRY(stage_out(JOut, n * nrhs * sizeof(double2), p->stream, tout, &out_d));
+    MARIE_TRY(inv.alloc(3 * V * sizeof(int), p->stream));
+    MARIE_TRY(ca.alloc(n * sizeof(double2), p->stream));
+    MARIE_TRY(cb.alloc(n * sizeof(double2), p->stream));
+    MARIE_TRY(build_inverse_index(p, (const int64_t*)idx_d, n, inv.as<int>()));
+    MARIE_TRY(build_coefficients(p, (const int64_t*)idx_d, n, (const double2*)Mr_d, (const double2*)Mc_d, Gram, transp,
+                                 ca.as<double2>(), cb.as<double2>()));
+    Prologue pro{nullptr, 0};
+    Epilogue ep{};
+    if (transp == 0) {
+      ep.a = ca.as<double2>();
+      ep.b = cb.as<double2>();
+      ep.conjout = 0;
+    } else {
+      pro.pre = cb.as<double2>();
+      pro.conjin = 1;
+      ep.a = ca.as<double2>();
+      ep.conjout = 1;
+    }
+    if (n > 0)
+      MARIE_TRY(run_matvec(p, precision, (const double2*)J_d, (double2*)out_d, n, (int)nrhs, inv.as<int>(), pro, ep));
+    MARIE_TRY(finish_out(JOut, out_d, n * nrhs * sizeof(double2), p->stream));
+    return check_kernel_status(p);  // (synchronises)
+  });
 }
 
 int marie_plan_apply_mv_AN(marie_plan* p, const double* JIn0, double* JOut, int64_t nrhs, int precision) {
-  if (!p || !JIn0 || !JOut) return set_error(MARIE_EINVAL, "NULL argument");
-  if (nrhs < 1) return set_error(MARIE_EINVAL, "nrhs must be >= 1");
-  if (!p->bnd_n) return set_error(MARIE_EINVAL, "no mv_AN bound to the plan (marie_plan_bind_mv_AN)");
-  MARIE_TRY(check_prec(p, precision));
-  const long long n = p->bnd_n;
-  DBuf tJ, tout;
-  const void* J_d;
-  void* out_d;
-  MARIE_TRY(stage_in(JIn0, n * nrhs * sizeof(double2), p->stream, tJ, &J_d));
-  MARIE_TRY(stage_out(JOut, n * nrhs * sizeof(double2), p->stream, tout, &out_d));
-  Prologue pro{nullptr, 0};
-  Epilogue ep{};
-  ep.a = p->bnd_a;
-  if (p->bnd_transp == 0) {
-    ep.b = p->bnd_b;
-  } else {
-    pro.pre = p->bnd_b;
-    pro.conjin = 1;
-    ep.conjout = 1;
-  }
-  const int* inv;
-  marie_plan* q = bound_plan(p, &inv, &pro);
-  MARIE_TRY(run_matvec(q, precision, (const double2*)J_d, (double2*)out_d, n, (int)nrhs, inv, pro, ep));
-  if (out_d != JOut) {
-    MARIE_TRY(finish_out(JOut, out_d, n * nrhs * sizeof(double2), p->stream));
-    return check_kernel_status(p);
-  }
-  MARIE_CUDA_TRY(cudaGetLastError());
-  return MARIE_OK;
+  return on_box_or_whole_grid(p, [&]() -> int {
+    if (!p || !JIn0 || !JOut) return set_error(MARIE_EINVAL, "NULL argument");
+    if (nrhs < 1) return set_error(MARIE_EINVAL, "nrhs must be >= 1");
+    if (!p->bnd_n) return set_error(MARIE_EINVAL, "no mv_AN bound to the plan (marie_plan_bind_mv_AN)");
+    MARIE_TRY(check_prec(p, precision));
+    const long long n = p->bnd_n;
+    DBuf tJ, tout;
+    const void* J_d;
+    void* out_d;
+    MARIE_TRY(stage_in(JIn0, n * nrhs * sizeof(double2), p->stream, tJ, &J_d));
+    MARIE_TRY(stage_out(JOut, n * nrhs * sizeof(double2), p->stream, tout, &out_d));
+    Prologue pro{nullptr, 0};
+    Epilogue ep{};
+    ep.a = p->bnd_a;
+    if (p->bnd_transp == 0) {
+      ep.b = p->bnd_b;
+    } else {
+      pro.pre = p->bnd_b;
+      pro.conjin = 1;
+      ep.conjout = 1;
+    }
+    const int* inv;
+    marie_plan* q = bound_plan(p, &inv, &pro);
+    MARIE_TRY(run_matvec(q, precision, (const double2*)J_d, (double2*)out_d, n, (int)nrhs, inv, pro, ep));
+    if (out_d != JOut) {
+      MARIE_TRY(finish_out(JOut, out_d, n * nrhs * sizeof(double2), p->stream));
+      return check_kernel_status(p);
+    }
+    MARIE_CUDA_TRY(cudaGetLastError());
+    return MARIE_OK;
+  });
 }
 
 int marie_mv_L(marie_plan* p, const double* JIn0, double Gram, const int64_t* idx, int64_t n_idx, double* JOut,
                int64_t nrhs, int precision) {
-  if (!p || !JIn0 || !JOut || (!idx && n_idx > 0)) return set_error(MARIE_EINVAL, "NULL argument");
-  if (nrhs < 1) return set_error(MARIE_EINVAL, "nrhs must be >= 1");
-  MARIE_TRY(check_prec(p, precision));
-  if (!p->has_op) return set_error(MARIE_ENOOP, "plan has no operator");
-  const long long V = p->d.V, n = n_idx;
-  DBuf tJ, tidx, tout, inv;
-  const void *J_d, *idx_d;
-  void* out_d;
-  MARIE_TRY(stage_in(JIn0, n * nrhs * sizeof(double2), p->stream, tJ, &J_d));
-  MARIE_TRY(stage_in(idx, n * sizeof(int64_t), p->stream, tidx, &idx_d));
-  MARIE_TRY(stage_out(JOut, n * nrhs * sizeof(double2), p->stream, tout, &out_d));
-  MARIE_TRY(inv.alloc(3 * V * sizeof(int), p->stream));
-  MARIE_TRY(build_inverse_index(p, (const int64_t*)idx_d, n, inv.as<int>()));
-  Prologue pro{nullptr, 0};
-  Epilogue ep{};
-  ep.a_s = mk<double2>(-Gram, 0.0);
-  ep.b_s = mk<double2>(-1.0, 0.0);
-  if (n > 0)
-    MARIE_TRY(run_matvec(p, precision, (const double2*)J_d, (double2*)out_d, n, (int)nrhs, inv.as<int>(), pro, ep));
-  MARIE_TRY(finish_out(JOut, out_d, n * nrhs * sizeof(double2), p->stream));
-  return check_kernel_status(p);  // (synchronises)
+  return on_box_or_whole_grid(p, [&]() -> int {
+    if (!p || !JIn0 || !JOut || (!idx && n_idx > 0)) return set_error(MARIE_EINVAL, "NULL argument");
+    if (nrhs < 1) return set_error(MARIE_EINVAL, "nrhs must be >= 1");
+    MARIE_TRY(check_prec(p, precision));
+    if (!p->has_op) return set_error(MARIE_ENOOP, "plan has no operator");
+    const long long V = p->d.V, n = n_idx;
+    DBuf tJ, tidx, tout, inv;
+    const void *J_d, *idx_d;
+    void* out_d;
+    MARIE_TRY(stage_in(JIn0, n * nrhs * sizeof(double2), p->stream, tJ, &J_d));
+    MARIE_TRY(stage_in(idx, n * sizeof(int64_t), p->stream, tidx, &idx_d));
+    MARIE_TRY(stage_out(JOut, n * nrhs * sizeof(double2), p->stream, tout, &out_d));
+    MARIE_TRY(inv.alloc(3 * V * sizeof(int), p->stream));
+    MARIE_TRY(build_inverse_index(p, (const int64_t*)idx_d, n, inv.as<int>()));
+    Prologue pro{nullptr, 0};
+    Epilogue ep{};
+    ep.a_s = mk<double2>(-Gram, 0.0);
+    ep.b_s = mk<double2>(-1.0, 0.0);
+    if (n > 0)
+      MARIE_TRY(run_matvec(p, precision, (const double2*)J_d, (double2*)out_d, n, (int)nrhs, inv.as<int>(), pro, ep));
+    MARIE_TRY(finish_out(JOut, out_d, n * nrhs * sizeof(double2), p->stream));
+    return check_kernel_status(p);  // (synchronises)
+  });
 }
 
 int marie_mv_K(marie_plan* p, const double* JIn0, const int64_t* idx, int64_t n_idx, double* JOut, int64_t nrhs,
                int precision) {
-  if (!p || !JIn0 || !JOut || (!idx && n_idx > 0)) return set_error(MARIE_EINVAL, "NULL argument");
-  if (nrhs < 1) return set_error(MARIE_EINVAL, "nrhs must be >= 1");
-  if (precision != MARIE_FP64 && precision != MARIE_FP32)
-    return set_error(MARIE_EINVAL, "precision must be MARIE_FP64 or MARIE_FP32");
-  if (!p->has_opK) return set_error(MARIE_ENOOP, "plan has no K operator");
-  const long long V = p->d.V, n = n_idx;
-  DBuf tJ, tidx, tout, inv;
-  const void *J_d, *idx_d;
-  void* out_d;
-  MARIE_TRY(stage_in(JIn0, n * nrhs * sizeof(double2), p->stream, tJ, &J_d));
-  MARIE_TRY(stage_in(idx, n * sizeof(int64_t), p->stream, tidx, &idx_d));
-  MARIE_TRY(stage_out(JOut, n * nrhs * sizeof(double2), p->stream, tout, &out_d));
-  MARIE_TRY(inv.alloc(3 * V * sizeof(int), p->stream));
-  MARIE_TRY(build_inverse_index(p, (const int64_t*)idx_d, n, inv.as<int>()));
-  // out = crop(IFFT(fK x FFT(J))): no diagonal term
-  Prologue pro{nullptr, 0};
-  Epilogue ep{};
-  ep.a_s = mk<double2>(0.0, 0.0);
-  ep.b_s = mk<double2>(-1.0, 0.0);
-  if (n > 0)
-    MARIE_TRY(run_matvec(p, precision, (const double2*)J_d, n, (double2*)out_d, n, n, (int)nrhs, inv.as<int>(), pro,
-                         ep, nullptr, 0, 1));
-  MARIE_TRY(finish_out(JOut, out_d, n * nrhs * sizeof(double2), p->stream));
-  MARIE_CUDA_TRY(cudaStreamSynchronize(p->stream));
-  return MARIE_OK;
+  return on_box_or_whole_grid(p, [&]() -> int {
+    if (!p || !JIn0 || !JOut || (!idx && n_idx > 0)) return set_error(MARIE_EINVAL, "NULL argument");
+    if (nrhs < 1) return set_error(MARIE_EINVAL, "nrhs must be >= 1");
+    if (precision != MARIE_FP64 && precision != MARIE_FP32)
+      return set_error(MARIE_EINVAL, "precision must be MARIE_FP64 or MARIE_FP32");
+    if (!p->has_opK) return set_error(MARIE_ENOOP, "plan has no K operator");
+    const long long V = p->d.V, n = n_idx;
+    DBuf tJ, tidx, tout, inv;
+    const void *J_d, *idx_d;
+    void* out_d;
+    MARIE_TRY(stage_in(JIn0, n * nrhs * sizeof(double2), p->stream, tJ, &J_d));
+    MARIE_TRY(stage_in(idx, n * sizeof(int64_t), p->stream, tidx, &idx_d));
+    MARIE_TRY(stage_out(JOut, n * nrhs * sizeof(double2), p->stream, tout, &out_d));
+    MARIE_TRY(inv.alloc(3 * V * sizeof(int), p->stream));
+    MARIE_TRY(build_inverse_index(p, (const int64_t*)idx_d, n, inv.as<int>()));
+    // out = crop(IFFT(fK x FFT(J))): no diagonal term
+    Prologue pro{nullptr, 0};
+    Epilogue ep{};
+    ep.a_s = mk<double2>(0.0, 0.0);
+    ep.b_s = mk<double2>(-1.0, 0.0);
+    if (n > 0)
+      MARIE_TRY(run_matvec(p, precision, (const double2*)J_d, n, (double2*)out_d, n, n, (int)nrhs, inv.as<int>(), pro,
+                           ep, nullptr, 0, 1));
+    MARIE_TRY(finish_out(JOut, out_d, n * nrhs * sizeof(double2), p->stream));
+    MARIE_CUDA_TRY(cudaStreamSynchronize(p->stream));
+    return MARIE_OK;
+  });
 }
 
 }  // extern "C"

@@ -322,8 +322,11 @@ void crop_settings(const marie_plan* p, marie_plan* q) {
 }
 
 bool give_crop_back(marie_plan* p) {
-  if (!p->crop) return false;
+  if (!p->crop && !p->bnd_crop) return false;
   p->crop.reset();
+  p->bnd_crop.reset();  // (bnd_inv serves the whole grid)
+  cudaFree(p->bnd_inv_crop);
+  p->bnd_inv_crop = nullptr;
   trim_pool(p->stream);
   return true;
 }

@@ -1002,85 +1002,87 @@ int marie_scat_solver(marie_plan* p, const double* Einc, const double* Hinc, dou
                       const double* eps_r, const double* sigma_e, const double* rho, double tol, int form,
                       char solver, char precond, int max_it, int inner_it, int outer_it, int ritz, double* Jout,
                       double* Sout, double* Eout, double* Bout, double* Gsar, double* Pabs) {
-  if (!p || !Einc || !eps_r || !sigma_e || !rho || !Jout) return set_error(MARIE_EINVAL, "NULL argument");
-  if (!(dx > 0) || !(freq > 0)) return set_error(MARIE_EINVAL, "dx and freq must be positive");
-  MARIE_TRACE("Scat_Solver");
-  cudaStream_t st = p->stream;
-  const long long V = p->d.V;
-  const double Gram = dx * dx * dx;
-  // Scat_Solver.m:155-160: the operators when the plan has none
-  if (!p->has_op) MARIE_TRY(marie_plan_assemble(p, dx, freq, 'D', nullptr));
-  if ((Bout || Hinc) && !p->has_opK) MARIE_TRY(marie_plan_assemble_k(p, dx, freq));
-  DBuf tE, tH, teps, tsig, trho, tJ, tS, tEo, tB, er, part;
-  const void *E_d, *H_d = nullptr, *eps_d, *sig_d, *rho_d;
-  void *J_d, *S_d = nullptr, *Eo_d = nullptr, *B_d = nullptr;
-  MARIE_TRY(stage_in(Einc, 3 * V * sizeof(double2), st, tE, &E_d));
-  if (Hinc) MARIE_TRY(stage_in(Hinc, 3 * V * sizeof(double2), st, tH, &H_d));
-  MARIE_TRY(stage_in(eps_r, V * sizeof(double), st, teps, &eps_d));
-  MARIE_TRY(stage_in(sigma_e, V * sizeof(double), st, tsig, &sig_d));
-  MARIE_TRY(stage_in(rho, V * sizeof(double), st, trho, &rho_d));
-  MARIE_TRY(stage_out(Jout, 3 * V * sizeof(double2), st, tJ, &J_d));
-  // SAR and the powers need E even when the caller does not ask for it
-  MARIE_TRY(stage_out(Eout ? Eout : nullptr, 3 * V * sizeof(double2), st, tEo, &Eo_d));
-  if (Sout) MARIE_TRY(stage_out(Sout, V * sizeof(double), st, tS, &S_d));
-  if (Bout) MARIE_TRY(stage_out(Bout, 3 * V * sizeof(double2), st, tB, &B_d));
-  HostPrefault pfJ, pfE, pfS, pfB;
-  pfJ.start(Jout, 3 * V * sizeof(double2));
-  if (Eout) pfE.start(Eout, 3 * V * sizeof(double2));
-  if (Sout) pfS.start(Sout, V * sizeof(double));
-  if (Bout) pfB.start(Bout, 3 * V * sizeof(double2));
-  DBuf S_tmp;
-  if (!S_d) {
-    MARIE_TRY(S_tmp.alloc(V * sizeof(double), st));
-    S_d = S_tmp.p;
-  }
-  MARIE_TRY(er.alloc(V * sizeof(double2), st));
-  const double omega = 2.0 * M_PI * freq;
-  k_complex_permittivity<<<grid_n(V), 256, 0, st>>>((const double*)eps_d, (const double*)sig_d, eps0() * omega, V,
-                                                    er.as<double2>());
-  count_launch();
-  MARIE_CUDA_TRY(cudaGetLastError());
-  // the current (Scat_Solver.m:164)
-  double iter[2], relres;
-  int flag;
-  MARIE_TRY(marie_jvie_solve(p, (const double*)E_d, (const double*)er.p, dx, freq, tol, form, solver, precond,
-                             max_it, inner_it, outer_it, ritz, (double*)J_d, &flag, &relres, iter, nullptr, 0,
-                             nullptr, nullptr));
-  // total E (:181) and B = mu0 H (:186-187)
-  const int prec = p->fN64 ? MARIE_FP64 : MARIE_FP32;
-  MARIE_TRY(marie_e_field_nop(p, (const double*)J_d, Gram, freq, (const double*)E_d, (double*)Eo_d, prec));
-  if (Bout) {
-    const int precK = p->fK64 ? MARIE_FP64 : MARIE_FP32;
-    MARIE_TRY(marie_h_field_kop(p, (const double*)J_d, Gram, (const double*)H_d, (double*)B_d, precK));
-    k_scale_field<<<grid_n(3 * V), 256, 0, st>>>((double2*)B_d, 4.0 * M_PI * 1e-7, 3 * V);
+  return on_box_or_whole_grid(p, [&]() -> int {
+    if (!p || !Einc || !eps_r || !sigma_e || !rho || !Jout) return set_error(MARIE_EINVAL, "NULL argument");
+    if (!(dx > 0) || !(freq > 0)) return set_error(MARIE_EINVAL, "dx and freq must be positive");
+    MARIE_TRACE("Scat_Solver");
+    cudaStream_t st = p->stream;
+    const long long V = p->d.V;
+    const double Gram = dx * dx * dx;
+    // Scat_Solver.m:155-160: the operators when the plan has none
+    if (!p->has_op) MARIE_TRY(marie_plan_assemble(p, dx, freq, 'D', nullptr));
+    if ((Bout || Hinc) && !p->has_opK) MARIE_TRY(marie_plan_assemble_k(p, dx, freq));
+    DBuf tE, tH, teps, tsig, trho, tJ, tS, tEo, tB, er, part;
+    const void *E_d, *H_d = nullptr, *eps_d, *sig_d, *rho_d;
+    void *J_d, *S_d = nullptr, *Eo_d = nullptr, *B_d = nullptr;
+    MARIE_TRY(stage_in(Einc, 3 * V * sizeof(double2), st, tE, &E_d));
+    if (Hinc) MARIE_TRY(stage_in(Hinc, 3 * V * sizeof(double2), st, tH, &H_d));
+    MARIE_TRY(stage_in(eps_r, V * sizeof(double), st, teps, &eps_d));
+    MARIE_TRY(stage_in(sigma_e, V * sizeof(double), st, tsig, &sig_d));
+    MARIE_TRY(stage_in(rho, V * sizeof(double), st, trho, &rho_d));
+    MARIE_TRY(stage_out(Jout, 3 * V * sizeof(double2), st, tJ, &J_d));
+    // SAR and the powers need E even when the caller does not ask for it
+    MARIE_TRY(stage_out(Eout ? Eout : nullptr, 3 * V * sizeof(double2), st, tEo, &Eo_d));
+    if (Sout) MARIE_TRY(stage_out(Sout, V * sizeof(double), st, tS, &S_d));
+    if (Bout) MARIE_TRY(stage_out(Bout, 3 * V * sizeof(double2), st, tB, &B_d));
+    HostPrefault pfJ, pfE, pfS, pfB;
+    pfJ.start(Jout, 3 * V * sizeof(double2));
+    if (Eout) pfE.start(Eout, 3 * V * sizeof(double2));
+    if (Sout) pfS.start(Sout, V * sizeof(double));
+    if (Bout) pfB.start(Bout, 3 * V * sizeof(double2));
+    DBuf S_tmp;
+    if (!S_d) {
+      MARIE_TRY(S_tmp.alloc(V * sizeof(double), st));
+      S_d = S_tmp.p;
+    }
+    MARIE_TRY(er.alloc(V * sizeof(double2), st));
+    const double omega = 2.0 * M_PI * freq;
+    k_complex_permittivity<<<grid_n(V), 256, 0, st>>>((const double*)eps_d, (const double*)sig_d, eps0() * omega, V,
+                                                      er.as<double2>());
     count_launch();
-  }
-  // SAR (:170-178), Pabs and Gsar (:190-194)
-  const int G = 152 * 2;
-  MARIE_TRY(part.alloc(2 * G * sizeof(double), st));
-  k_sar_power<<<G, 256, 0, st>>>((const double2*)J_d, (const double2*)Eo_d, (const double*)sig_d,
-                                 (const double*)rho_d, V, (double*)S_d, part.as<double>());
-  count_launch();
-  MARIE_CUDA_TRY(cudaGetLastError());
-  std::vector<double> hp(2 * G);
-  MARIE_CUDA_TRY(cudaMemcpyAsync(hp.data(), part.p, 2 * G * sizeof(double), cudaMemcpyDeviceToHost, st));
-  pfJ.join();
-  pfE.join();
-  pfS.join();
-  pfB.join();
-  MARIE_TRY(finish_out(Jout, J_d, 3 * V * sizeof(double2), st));
-  if (Eout) MARIE_TRY(finish_out(Eout, Eo_d, 3 * V * sizeof(double2), st));
-  if (Sout) MARIE_TRY(finish_out(Sout, S_d, V * sizeof(double), st));
-  if (Bout) MARIE_TRY(finish_out(Bout, B_d, 3 * V * sizeof(double2), st));
-  MARIE_CUDA_TRY(cudaStreamSynchronize(st));
-  double ssum = 0, psum = 0;
-  for (int b = 0; b < G; ++b) {
-    ssum += hp[b];
-    psum += hp[G + b];
-  }
-  if (Gsar) *Gsar = ssum * Gram;
-  if (Pabs) *Pabs = 0.5 * psum * Gram;
-  return check_kernel_status(p);
+    MARIE_CUDA_TRY(cudaGetLastError());
+    // the current (Scat_Solver.m:164)
+    double iter[2], relres;
+    int flag;
+    MARIE_TRY(marie_jvie_solve(p, (const double*)E_d, (const double*)er.p, dx, freq, tol, form, solver, precond,
+                               max_it, inner_it, outer_it, ritz, (double*)J_d, &flag, &relres, iter, nullptr, 0,
+                               nullptr, nullptr));
+    // total E (:181) and B = mu0 H (:186-187)
+    const int prec = p->fN64 ? MARIE_FP64 : MARIE_FP32;
+    MARIE_TRY(marie_e_field_nop(p, (const double*)J_d, Gram, freq, (const double*)E_d, (double*)Eo_d, prec));
+    if (Bout) {
+      const int precK = p->fK64 ? MARIE_FP64 : MARIE_FP32;
+      MARIE_TRY(marie_h_field_kop(p, (const double*)J_d, Gram, (const double*)H_d, (double*)B_d, precK));
+      k_scale_field<<<grid_n(3 * V), 256, 0, st>>>((double2*)B_d, 4.0 * M_PI * 1e-7, 3 * V);
+      count_launch();
+    }
+    // SAR (:170-178), Pabs and Gsar (:190-194)
+    const int G = 152 * 2;
+    MARIE_TRY(part.alloc(2 * G * sizeof(double), st));
+    k_sar_power<<<G, 256, 0, st>>>((const double2*)J_d, (const double2*)Eo_d, (const double*)sig_d,
+                                   (const double*)rho_d, V, (double*)S_d, part.as<double>());
+    count_launch();
+    MARIE_CUDA_TRY(cudaGetLastError());
+    std::vector<double> hp(2 * G);
+    MARIE_CUDA_TRY(cudaMemcpyAsync(hp.data(), part.p, 2 * G * sizeof(double), cudaMemcpyDeviceToHost, st));
+    pfJ.join();
+    pfE.join();
+    pfS.join();
+    pfB.join();
+    MARIE_TRY(finish_out(Jout, J_d, 3 * V * sizeof(double2), st));
+    if (Eout) MARIE_TRY(finish_out(Eout, Eo_d, 3 * V * sizeof(double2), st));
+    if (Sout) MARIE_TRY(finish_out(Sout, S_d, V * sizeof(double), st));
+    if (Bout) MARIE_TRY(finish_out(Bout, B_d, 3 * V * sizeof(double2), st));
+    MARIE_CUDA_TRY(cudaStreamSynchronize(st));
+    double ssum = 0, psum = 0;
+    for (int b = 0; b < G; ++b) {
+      ssum += hp[b];
+      psum += hp[G + b];
+    }
+    if (Gsar) *Gsar = ssum * Gram;
+    if (Pabs) *Pabs = 0.5 * psum * Gram;
+    return check_kernel_status(p);
+  });
 }
 
 
@@ -1088,132 +1090,136 @@ int marie_jvie_solve(marie_plan* p, const double* Einc, const double* e_r, doubl
                      int form, char solver, char precond, int max_it, int inner_it, int outer_it, int ritz,
                      double* Je, int* flag, double* relres, double* iter, double* resvec, int64_t resvec_cap,
                      int64_t* resvec_len, double* solvert) {
-  if (!p || !Einc || !e_r || !Je) return set_error(MARIE_EINVAL, "NULL argument");
-  if (!p->has_op) return set_error(MARIE_ENOOP, "plan has no operator");
-  if (!(dx > 0) || !(freq > 0)) return set_error(MARIE_EINVAL, "dx and freq must be positive");
-  MARIE_TRY(clamp_args(tol, form, precond, inner_it, outer_it));
-  MARIE_TRACE("JVIE_Solver");
-  SolverArgs sa;
-  sa.solver = solver;
-  sa.max_it = max_it;
-  sa.ritz = ritz;
-  clamp_solver(sa, inner_it);
-  const auto t0 = std::chrono::steady_clock::now();
-  cudaStream_t st = p->stream;
-  const long long V = p->d.V;
-  DBuf tE, tER, tJe;
-  const void *E_d, *er_d;
-  void* Je_d;
-  MARIE_TRY(stage_in(Einc, 3 * V * sizeof(double2), st, tE, &E_d));
-  MARIE_TRY(stage_in(e_r, V * sizeof(double2), st, tER, &er_d));
-  MARIE_TRY(stage_out(Je, 3 * V * sizeof(double2), st, tJe, &Je_d));
-  HostPrefault pf;
-  pf.start(Je, 3 * V * sizeof(double2));
-  SolveOut so;
-  MARIE_TRY(jvie_solve_core(p, (const double2*)E_d, 3 * V, 1, (const double2*)er_d, dx, freq, form, precond, tol,
-                            inner_it, outer_it, (double2*)Je_d, 3 * V, so, sa));
-  pf.join();
-  MARIE_TRY(finish_out(Je, Je_d, 3 * V * sizeof(double2), st));
-  MARIE_CUDA_TRY(cudaStreamSynchronize(st));
-  const auto t1 = std::chrono::steady_clock::now();
-  const bool bi = sa.solver == 'B';
-  const GmresResult& R = so.r[0];
-  const std::vector<double>& rv = bi ? so.b.resvec : R.resvec;
-  if (flag) *flag = bi ? so.b.flag : R.flag;
-  if (relres) *relres = bi ? so.b.relres : R.relres;
-  if (iter) {
-    iter[0] = bi ? so.b.iter : R.iter[0];
-    iter[1] = bi ? 0.0 : R.iter[1];
-  }
-  if (resvec_len) *resvec_len = (int64_t)rv.size();
-  if (resvec)
-    for (int64_t i = 0; i < (int64_t)rv.size() && i < resvec_cap; ++i) resvec[i] = rv[i];
-  if (solvert) *solvert = std::chrono::duration<double>(t1 - t0).count();
-  return check_kernel_status(p);
+  return on_box_or_whole_grid(p, [&]() -> int {
+    if (!p || !Einc || !e_r || !Je) return set_error(MARIE_EINVAL, "NULL argument");
+    if (!p->has_op) return set_error(MARIE_ENOOP, "plan has no operator");
+    if (!(dx > 0) || !(freq > 0)) return set_error(MARIE_EINVAL, "dx and freq must be positive");
+    MARIE_TRY(clamp_args(tol, form, precond, inner_it, outer_it));
+    MARIE_TRACE("JVIE_Solver");
+    SolverArgs sa;
+    sa.solver = solver;
+    sa.max_it = max_it;
+    sa.ritz = ritz;
+    clamp_solver(sa, inner_it);
+    const auto t0 = std::chrono::steady_clock::now();
+    cudaStream_t st = p->stream;
+    const long long V = p->d.V;
+    DBuf tE, tER, tJe;
+    const void *E_d, *er_d;
+    void* Je_d;
+    MARIE_TRY(stage_in(Einc, 3 * V * sizeof(double2), st, tE, &E_d));
+    MARIE_TRY(stage_in(e_r, V * sizeof(double2), st, tER, &er_d));
+    MARIE_TRY(stage_out(Je, 3 * V * sizeof(double2), st, tJe, &Je_d));
+    HostPrefault pf;
+    pf.start(Je, 3 * V * sizeof(double2));
+    SolveOut so;
+    MARIE_TRY(jvie_solve_core(p, (const double2*)E_d, 3 * V, 1, (const double2*)er_d, dx, freq, form, precond, tol,
+                              inner_it, outer_it, (double2*)Je_d, 3 * V, so, sa));
+    pf.join();
+    MARIE_TRY(finish_out(Je, Je_d, 3 * V * sizeof(double2), st));
+    MARIE_CUDA_TRY(cudaStreamSynchronize(st));
+    const auto t1 = std::chrono::steady_clock::now();
+    const bool bi = sa.solver == 'B';
+    const GmresResult& R = so.r[0];
+    const std::vector<double>& rv = bi ? so.b.resvec : R.resvec;
+    if (flag) *flag = bi ? so.b.flag : R.flag;
+    if (relres) *relres = bi ? so.b.relres : R.relres;
+    if (iter) {
+      iter[0] = bi ? so.b.iter : R.iter[0];
+      iter[1] = bi ? 0.0 : R.iter[1];
+    }
+    if (resvec_len) *resvec_len = (int64_t)rv.size();
+    if (resvec)
+      for (int64_t i = 0; i < (int64_t)rv.size() && i < resvec_cap; ++i) resvec[i] = rv[i];
+    if (solvert) *solvert = std::chrono::duration<double>(t1 - t0).count();
+    return check_kernel_status(p);
+  });
 }
 
 int marie_jvie2solver(marie_plan* p, const int64_t* idx, int64_t n_idx, const double* Mr, const double* Mc,
                       double Gram, const double* Vrhs, double tol, int max_it, const double* Vini, double* Vsol,
                       int* flag, double* relres, double* iter, double* solvert) {
-  if (!p || !idx || !Mr || !Mc || !Vrhs || !Vsol || n_idx < 1) return set_error(MARIE_EINVAL, "NULL argument");
-  if (!p->has_op) return set_error(MARIE_ENOOP, "plan has no operator");
-  if (!(tol > 0)) return set_error(MARIE_EINVAL, "tol must be positive");
-  if (max_it < 1) return set_error(MARIE_EINVAL, "max_it must be >= 1");
-  MARIE_TRACE("jvie2solver");
-  const auto t0 = std::chrono::steady_clock::now();
-  cudaStream_t st = p->stream;
-  const long long V = p->d.V, n = n_idx;
-  DBuf tidx, tMr, tMc, tb, tx0, tx;
-  const void *idx_d, *Mr_d, *Mc_d, *b_d, *x0_d = nullptr;
-  void* x_d;
-  MARIE_TRY(stage_in(idx, n * sizeof(int64_t), st, tidx, &idx_d));
-  MARIE_TRY(stage_in(Mr, V * sizeof(double2), st, tMr, &Mr_d));
-  MARIE_TRY(stage_in(Mc, V * sizeof(double2), st, tMc, &Mc_d));
-  MARIE_TRY(stage_in(Vrhs, n * sizeof(double2), st, tb, &b_d));
-  if (Vini) MARIE_TRY(stage_in(Vini, n * sizeof(double2), st, tx0, &x0_d));
-  MARIE_TRY(stage_out(Vsol, n * sizeof(double2), st, tx, &x_d));
-  HostPrefault pf;
-  pf.start(Vsol, n * sizeof(double2));
-  if (flag) *flag = 0;
-  if (relres) *relres = 0;
-  if (iter) *iter = 0;
-  // jvie2solver.m:35-38: an all-zero right-hand side is returned as the solution
-  bool nz = true;
-  MARIE_TRY(any_nonzero(p, (const double2*)b_d, n, &nz));
-  if (!nz) {
-    MARIE_CUDA_TRY(cudaMemcpyAsync(x_d, b_d, n * sizeof(double2), cudaMemcpyDeviceToDevice, st));
-  } else {
-    SolveOut so;
-    MARIE_TRY(on_box_or_whole_grid(p, [&]() {
-      return jvie2_solve(p, (const int64_t*)idx_d, n, (const double2*)Mr_d, (const double2*)Mc_d, Gram,
-                         (const double2*)b_d, tol, max_it, (const double2*)x0_d, (double2*)x_d, so);
-    }));
-    if (flag) *flag = so.b.flag;
-    if (relres) *relres = so.b.relres;
-    if (iter) *iter = so.b.iter;
-  }
-  pf.join();
-  MARIE_TRY(finish_out(Vsol, x_d, n * sizeof(double2), st));
-  MARIE_CUDA_TRY(cudaStreamSynchronize(st));
-  if (solvert) *solvert = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-  return check_kernel_status(p);
+  return on_box_or_whole_grid(p, [&]() -> int {
+    if (!p || !idx || !Mr || !Mc || !Vrhs || !Vsol || n_idx < 1) return set_error(MARIE_EINVAL, "NULL argument");
+    if (!p->has_op) return set_error(MARIE_ENOOP, "plan has no operator");
+    if (!(tol > 0)) return set_error(MARIE_EINVAL, "tol must be positive");
+    if (max_it < 1) return set_error(MARIE_EINVAL, "max_it must be >= 1");
+    MARIE_TRACE("jvie2solver");
+    const auto t0 = std::chrono::steady_clock::now();
+    cudaStream_t st = p->stream;
+    const long long V = p->d.V, n = n_idx;
+    DBuf tidx, tMr, tMc, tb, tx0, tx;
+    const void *idx_d, *Mr_d, *Mc_d, *b_d, *x0_d = nullptr;
+    void* x_d;
+    MARIE_TRY(stage_in(idx, n * sizeof(int64_t), st, tidx, &idx_d));
+    MARIE_TRY(stage_in(Mr, V * sizeof(double2), st, tMr, &Mr_d));
+    MARIE_TRY(stage_in(Mc, V * sizeof(double2), st, tMc, &Mc_d));
+    MARIE_TRY(stage_in(Vrhs, n * sizeof(double2), st, tb, &b_d));
+    if (Vini) MARIE_TRY(stage_in(Vini, n * sizeof(double2), st, tx0, &x0_d));
+    MARIE_TRY(stage_out(Vsol, n * sizeof(double2), st, tx, &x_d));
+    HostPrefault pf;
+    pf.start(Vsol, n * sizeof(double2));
+    if (flag) *flag = 0;
+    if (relres) *relres = 0;
+    if (iter) *iter = 0;
+    // jvie2solver.m:35-38: an all-zero right-hand side is returned as the solution
+    bool nz = true;
+    MARIE_TRY(any_nonzero(p, (const double2*)b_d, n, &nz));
+    if (!nz) {
+      MARIE_CUDA_TRY(cudaMemcpyAsync(x_d, b_d, n * sizeof(double2), cudaMemcpyDeviceToDevice, st));
+    } else {
+      SolveOut so;
+      MARIE_TRY(jvie2_solve(p, (const int64_t*)idx_d, n, (const double2*)Mr_d, (const double2*)Mc_d, Gram,
+                            (const double2*)b_d, tol, max_it, (const double2*)x0_d, (double2*)x_d, so));
+      if (flag) *flag = so.b.flag;
+      if (relres) *relres = so.b.relres;
+      if (iter) *iter = so.b.iter;
+    }
+    pf.join();
+    MARIE_TRY(finish_out(Vsol, x_d, n * sizeof(double2), st));
+    MARIE_CUDA_TRY(cudaStreamSynchronize(st));
+    if (solvert) *solvert = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+    return check_kernel_status(p);
+  });
 }
 
 int marie_jvie_solve_batch(marie_plan* p, const double* Einc, int64_t nexc, const double* e_r, double dx, double freq,
                            int form, char precond, double tol, int inner_it, int outer_it, double* Je, int* flag,
                            double* relres, int* iter, double* solvert) {
-  if (!p || !Einc || !e_r || !Je || nexc < 1) return set_error(MARIE_EINVAL, "NULL argument or nexc < 1");
-  if (!p->has_op) return set_error(MARIE_ENOOP, "plan has no operator");
-  if (!(dx > 0) || !(freq > 0)) return set_error(MARIE_EINVAL, "dx and freq must be positive");
-  MARIE_TRY(clamp_args(tol, form, precond, inner_it, outer_it));
-  const auto t0 = std::chrono::steady_clock::now();
-  cudaStream_t st = p->stream;
-  const long long V = p->d.V;
-  DBuf tE, tER, tJe;
-  const void *E_d, *er_d;
-  void* Je_d;
-  MARIE_TRY(stage_in(Einc, (size_t)nexc * 3 * V * sizeof(double2), st, tE, &E_d));
-  MARIE_TRY(stage_in(e_r, V * sizeof(double2), st, tER, &er_d));
-  MARIE_TRY(stage_out(Je, (size_t)nexc * 3 * V * sizeof(double2), st, tJe, &Je_d));
-  HostPrefault pf;
-  pf.start(Je, (size_t)nexc * 3 * V * sizeof(double2));
-  SolveOut so;
-  MARIE_TRY(jvie_solve_core(p, (const double2*)E_d, 3 * V, (int)nexc, (const double2*)er_d, dx, freq, form, precond,
-                            tol, inner_it, outer_it, (double2*)Je_d, 3 * V, so));
-  pf.join();
-  MARIE_TRY(finish_out(Je, Je_d, (size_t)nexc * 3 * V * sizeof(double2), st));
-  MARIE_CUDA_TRY(cudaStreamSynchronize(st));
-  const auto t1 = std::chrono::steady_clock::now();
-  for (int64_t e = 0; e < nexc; ++e) {
-    if (flag) flag[e] = so.r[e].flag;
-    if (relres) relres[e] = so.r[e].relres;
-    if (iter) {
-      iter[2 * e] = so.r[e].iter[0];
-      iter[2 * e + 1] = so.r[e].iter[1];
+  return on_box_or_whole_grid(p, [&]() -> int {
+    if (!p || !Einc || !e_r || !Je || nexc < 1) return set_error(MARIE_EINVAL, "NULL argument or nexc < 1");
+    if (!p->has_op) return set_error(MARIE_ENOOP, "plan has no operator");
+    if (!(dx > 0) || !(freq > 0)) return set_error(MARIE_EINVAL, "dx and freq must be positive");
+    MARIE_TRY(clamp_args(tol, form, precond, inner_it, outer_it));
+    const auto t0 = std::chrono::steady_clock::now();
+    cudaStream_t st = p->stream;
+    const long long V = p->d.V;
+    DBuf tE, tER, tJe;
+    const void *E_d, *er_d;
+    void* Je_d;
+    MARIE_TRY(stage_in(Einc, (size_t)nexc * 3 * V * sizeof(double2), st, tE, &E_d));
+    MARIE_TRY(stage_in(e_r, V * sizeof(double2), st, tER, &er_d));
+    MARIE_TRY(stage_out(Je, (size_t)nexc * 3 * V * sizeof(double2), st, tJe, &Je_d));
+    HostPrefault pf;
+    pf.start(Je, (size_t)nexc * 3 * V * sizeof(double2));
+    SolveOut so;
+    MARIE_TRY(jvie_solve_core(p, (const double2*)E_d, 3 * V, (int)nexc, (const double2*)er_d, dx, freq, form, precond,
+                              tol, inner_it, outer_it, (double2*)Je_d, 3 * V, so));
+    pf.join();
+    MARIE_TRY(finish_out(Je, Je_d, (size_t)nexc * 3 * V * sizeof(double2), st));
+    MARIE_CUDA_TRY(cudaStreamSynchronize(st));
+    const auto t1 = std::chrono::steady_clock::now();
+    for (int64_t e = 0; e < nexc; ++e) {
+      if (flag) flag[e] = so.r[e].flag;
+      if (relres) relres[e] = so.r[e].relres;
+      if (iter) {
+        iter[2 * e] = so.r[e].iter[0];
+        iter[2 * e + 1] = so.r[e].iter[1];
+      }
     }
-  }
-  if (solvert) *solvert = std::chrono::duration<double>(t1 - t0).count();
-  return check_kernel_status(p);
+    if (solvert) *solvert = std::chrono::duration<double>(t1 - t0).count();
+    return check_kernel_status(p);
+  });
 }
 
 int marie_jvie_solve_bodies(int nbody, marie_plan* const* plans, const double* const* Einc, const int64_t* nexc,

@@ -437,49 +437,51 @@ extern "C" int marie_pgmres(marie_plan* p, marie_op_fn A, void* A_ctx, const dou
                             marie_op_fn R1, void* R1_ctx, marie_op_fn R2, void* R2_ctx, const double* x0, double* x,
                             int* flag, double* relres, int* iter, double* resvec, int64_t resvec_cap,
                             int64_t* resvec_len) {
-  if (!p || !b || !x || n < 1) return set_error(MARIE_EINVAL, "NULL argument or n < 1");
-  MARIE_TRACE("pgmres");
-  // User operators run outside the plan's stream: finish the plan's work
-  // before handing them x; they return with y complete.
-  auto wrap = [p](marie_op_fn f, void* ctx, long long nn) -> DevOp {
-    return [p, f, ctx, nn](const double2* xi, double2* yo) -> int {
-      MARIE_CUDA_TRY(cudaStreamSynchronize(p->stream));
-      const int s = f(ctx, reinterpret_cast<const double*>(xi), reinterpret_cast<double*>(yo), nn);
-      if (s != MARIE_OK) return set_error(s, "user operator returned status %d", s);
-      return MARIE_OK;
+  return on_box_or_whole_grid(p, [&]() -> int {
+    if (!p || !b || !x || n < 1) return set_error(MARIE_EINVAL, "NULL argument or n < 1");
+    MARIE_TRACE("pgmres");
+    // User operators run outside the plan's stream: finish the plan's work
+    // before handing them x; they return with y complete.
+    auto wrap = [p](marie_op_fn f, void* ctx, long long nn) -> DevOp {
+      return [p, f, ctx, nn](const double2* xi, double2* yo) -> int {
+        MARIE_CUDA_TRY(cudaStreamSynchronize(p->stream));
+        const int s = f(ctx, reinterpret_cast<const double*>(xi), reinterpret_cast<double*>(yo), nn);
+        if (s != MARIE_OK) return set_error(s, "user operator returned status %d", s);
+        return MARIE_OK;
+      };
     };
-  };
-  DevOp opA;
-  if (A)
-    opA = wrap(A, A_ctx, n);
-  else
-    MARIE_TRY(bound_operator(p, n, &opA));  // NULL A: the plan's bound mv_AN
-  DevOp oL1, oL2, oR1, oR2;
-  if (L1) oL1 = wrap(L1, L1_ctx, n);
-  if (L2) oL2 = wrap(L2, L2_ctx, n);
-  if (R1) oR1 = wrap(R1, R1_ctx, n);
-  if (R2) oR2 = wrap(R2, R2_ctx, n);
-  const size_t bytes = (size_t)n * sizeof(double2);
-  DBuf tb, tx0, txo;
-  const void *b_d, *x0_d = nullptr;
-  void* x_d;
-  MARIE_TRY(stage_in(b, bytes, p->stream, tb, &b_d));
-  if (x0) MARIE_TRY(stage_in(x0, bytes, p->stream, tx0, &x0_d));
-  MARIE_TRY(stage_out(x, bytes, p->stream, txo, &x_d));
-  GmresResult res;
-  MARIE_TRY(gmres(p, opA, L1 ? &oL1 : nullptr, L2 ? &oL2 : nullptr, R1 ? &oR1 : nullptr, R2 ? &oR2 : nullptr,
-                  (const double2*)b_d, n, restart, tol, maxit, (const double2*)x0_d, (double2*)x_d, res));
-  MARIE_TRY(finish_out(x, x_d, bytes, p->stream));
-  MARIE_CUDA_TRY(cudaStreamSynchronize(p->stream));
-  if (flag) *flag = res.flag;
-  if (relres) *relres = res.relres;
-  if (iter) {
-    iter[0] = res.iter[0];
-    iter[1] = res.iter[1];
-  }
-  const int64_t nr = (int64_t)res.resvec.size();
-  if (resvec_len) *resvec_len = nr;
-  if (resvec)
-    for (int64_t i = 0; i < nr && i < resvec_cap; ++i) resvec[i] = res.resvec[i];
-  return check_kernel_status(p);
+    DevOp opA;
+    if (A)
+      opA = wrap(A, A_ctx, n);
+    else
+      MARIE_TRY(bound_operator(p, n, &opA));  // NULL A: the plan's bound mv_AN
+    DevOp oL1, oL2, oR1, oR2;
+    if (L1) oL1 = wrap(L1, L1_ctx, n);
+    if (L2) oL2 = wrap(L2, L2_ctx, n);
+    if (R1) oR1 = wrap(R1, R1_ctx, n);
+    if (R2) oR2 = wrap(R2, R2_ctx, n);
+    const size_t bytes = (size_t)n * sizeof(double2);
+    DBuf tb, tx0, txo;
+    const void *b_d, *x0_d = nullptr;
+    void* x_d;
+    MARIE_TRY(stage_in(b, bytes, p->stream, tb, &b_d));
+    if (x0) MARIE_TRY(stage_in(x0, bytes, p->stream, tx0, &x0_d));
+    MARIE_TRY(stage_out(x, bytes, p->stream, txo, &x_d));
+    GmresResult res;
+    MARIE_TRY(gmres(p, opA, L1 ? &oL1 : nullptr, L2 ? &oL2 : nullptr, R1 ? &oR1 : nullptr, R2 ? &oR2 : nullptr,
+                    (const double2*)b_d, n, restart, tol, maxit, (const double2*)x0_d, (double2*)x_d, res));
+    MARIE_TRY(finish_out(x, x_d, bytes, p->stream));
+    MARIE_CUDA_TRY(cudaStreamSynchronize(p->stream));
+    if (flag) *flag = res.flag;
+    if (relres) *relres = res.relres;
+    if (iter) {
+      iter[0] = res.iter[0];
+      iter[1] = res.iter[1];
+    }
+    const int64_t nr = (int64_t)res.resvec.size();
+    if (resvec_len) *resvec_len = nr;
+    if (resvec)
+      for (int64_t i = 0; i < nr && i < resvec_cap; ++i) resvec[i] = res.resvec[i];
+    return check_kernel_status(p);
+  });
 }

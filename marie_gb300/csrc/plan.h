@@ -186,17 +186,18 @@ bool crop_possible(const marie_plan* p);
 int dof_box(marie_plan* p, const int64_t* idx_dev, long long n, int box[6]);
 std::shared_ptr<marie_plan> crop_plan(marie_plan* p, const int box[6], int origin[3]);
 void crop_settings(const marie_plan* p, marie_plan* q);
-// For a call that finds no memory: gives the plan's crop and the pool's cached
-// blocks back.  False when the plan holds no crop.
+// For a call that finds no memory: gives the plan's crop, a bound mv_AN's
+// included, and the pool's cached blocks back.  False when the plan holds none.
 bool give_crop_back(marie_plan* p);
 // Runs call(); when it finds no memory while the plan holds a crop, gives that
 // back and runs it again on the whole grid, as if no crop had been made.
 template <typename F> int on_box_or_whole_grid(marie_plan* p, F&& call) {
   int s = call();
   if (s != MARIE_ENOMEM || !give_crop_back(p)) return s;
+  const bool outer = p->whole_grid;
   p->whole_grid = true;
   s = call();
-  p->whole_grid = false;
+  p->whole_grid = outer;
   return s;
 }
 Extent box_extent(const marie_plan* q, const int box[6]);

@@ -391,3 +391,92 @@ def test_bodies_on_their_boxes_in_one_launch(cuda):
         assert list(flag) == [0, 0] and np.all(relres <= 1e-7)
     for b in bodies:
         b[3].close()
+
+
+@pytest.mark.parametrize("name", ["apply", "mv_AN", "mv_L", "E_field", "mv_K", "H_field", "pgmres", "pgmresDR",
+                                  "bicgstab", "solve", "batch", "inner", "gradient", "scat"])
+def test_calls_beside_a_boxs_operator_without_memory(cuda, name):
+    """Beside the operator of a box, which a bound mv_AN or a solve left on the
+    plan, the nth allocation of a call fails: the plan gives that operator back
+    and the call runs as it does without one.  Host arrays, so the calls' own
+    buffers are among the allocations.  Products and fields on either grid agree
+    to 1e-13, solves to their tolerance times a condition of up to 1e3."""
+    import marie_gb300 as mg
+    from marie_gb300.autograd import adjoint_gradient
+
+    shape, lo, size = CROPS[0]
+    dx = 4e-3
+    r, er = _off_centre_body(shape, lo, size)
+    op = mg.Operator.assemble(*shape, dx, FREQ, precision="fp64", nrhs_max=2).assemble_k(dx, FREQ)
+    em = vo.EMconstants(FREQ)
+    E = np.asfortranarray(vo.PlaneWave_Excitation(r, [0, 0, em["ko"]], em["omega_mu"], [1, 0, 0])[0])
+    idxS = np.flatnonzero(np.abs(er.reshape(-1, order="F") - 1) > 1e-12) + 1
+    idx = np.concatenate([idxS, er.size + idxS, 2 * er.size + idxS]).astype(np.int64)
+    Mr, Mc = np.asfortranarray(er / er), np.asfortranarray((er - 1) / er)
+    rng = np.random.default_rng(8)
+    J = rng.standard_normal(idx.size) + 1j * rng.standard_normal(idx.size)
+    F = np.asfortranarray(rng.standard_normal(E.shape) + 1j * rng.standard_normal(E.shape))
+    b = E.reshape(-1, order="F")[idx - 1] * dx**3
+    E2 = np.asfortranarray(np.stack([E, 1j * E], axis=4))
+    eps, sig = np.asfortranarray(er.real), np.asfortranarray(-er.imag * 2 * np.pi * FREQ * 8.854e-12)
+    calls = {
+        "apply": lambda: op.apply_mv_AN(J, "fp64"),
+        "mv_AN": lambda: mg.mv_AN(J, op, Mr, Mc, dx**3, "notransp", idx),
+        "mv_L": lambda: mg.mv_L(J, op, r, dx**3, idx),
+        "E_field": lambda: mg.E_field_Nop(F, op, dx**3, FREQ, E),
+        "mv_K": lambda: mg.mv_K(J, op, r, idx),
+        "H_field": lambda: mg.H_field_Kop(F, op, dx**3, E),
+        "pgmres": lambda: mg.pgmres(op, b, 30, 1e-8, 20)[0],
+        "pgmresDR": lambda: mg.pgmresDR(op, b, 30, 1e-8, 20, 4)[0],
+        "bicgstab": lambda: mg.bicgstab(op, b, 1e-8, 400)[0],
+        "solve": lambda: mg.JVIE_Solver(E, er, r, FREQ, op, tol=1e-8)[0],
+        "batch": lambda: mg.JVIE_Solver_batch(E2, er, r, FREQ, op, tol=1e-8)[0],
+        "inner": lambda: mg.jvie2solver(b, op, idx, Mr, Mc, dx**3, 1e-8)[0],
+        "gradient": lambda: adjoint_gradient(op, E, er, dx, FREQ, "power", tol=1e-8)[1],
+        "scat": lambda: mg.Scat_Solver(E, None, FREQ, r, eps, sig, np.ones(shape, order="F"), tol=1e-8, fN=op)[0],
+    }
+    call = calls[name]
+    bind = lambda: op.bind_mv_AN(Mr, Mc, dx**3, "notransp", idx)
+    bind()
+    ref = np.asarray(call())
+    tol = 1e-13 if name in ("apply", "mv_AN", "mv_L", "E_field", "mv_K", "H_field") else 1e-5
+    for nth in (1, 2, 3, 5, 8):
+        bind()
+        op.lib.marie_inject_alloc_failure(nth)
+        try:
+            out = np.asarray(call())
+        finally:
+            op.lib.marie_inject_alloc_failure(0)
+        assert np.max(np.abs(out - ref)) <= tol * np.max(np.abs(ref))
+    op.close()
+
+
+def test_a_bound_box_given_back_leaves_the_whole_grids_product(cuda):
+    """After a solve that found no memory the bound product runs on the whole grid
+    (bit for bit the product that per-pass timing runs there) until it is bound
+    again."""
+    import marie_gb300 as mg
+
+    shape, lo, size = CROPS[0]
+    op, er, idx = _bound_operator(shape, "fp64", box=(lo, size))
+    bind = lambda: op.bind_mv_AN(np.asfortranarray(er / er), np.asfortranarray((er - 1) / er), 4e-3**3, "notransp", idx)
+    bind()
+    rng = np.random.default_rng(6)
+    J = rng.standard_normal(idx.size) + 1j * rng.standard_normal(idx.size)
+    on_box = op.apply_mv_AN(J, "fp64")
+    op.lib.marie_plan_profile(op.plan, 1, None, None)
+    whole = op.apply_mv_AN(J, "fp64")
+    op.lib.marie_plan_profile(op.plan, 0, None, None)
+    assert np.any(on_box != whole)
+    r = vo.grid(*shape, 4e-3)
+    em = vo.EMconstants(FREQ)
+    E = np.asfortranarray(vo.PlaneWave_Excitation(r, [0, 0, em["ko"]], em["omega_mu"], [1, 0, 0])[0])
+    op.lib.marie_inject_alloc_failure(6)
+    try:
+        assert mg.JVIE_Solver(E, er, r, FREQ, op, tol=1e-6)[1] == 0
+    finally:
+        op.lib.marie_inject_alloc_failure(0)
+    np.testing.assert_array_equal(op.apply_mv_AN(J, "fp64"), whole)
+    bind()
+    np.testing.assert_array_equal(op.apply_mv_AN(J, "fp64"), on_box)
+    op.close()
