@@ -51,8 +51,9 @@ def adjoint_gradient(op: Operator, Einc, e_r, dx, freq, objective="power", E_tar
     F = C.c_double()
     flags = (C.c_int * 2)()
     iters = (C.c_int * 2)()
-    check(op.lib.marie_jvie_adjoint_grad(_ready(op), ep, erp, float(dx), float(freq), _OBJ[objective], tp, float(tol),
-                                         int(inner_it), int(outer_it), C.byref(F), gep, gsp, flags, iters))
+    check(op.lib.marie_jvie_adjoint_grad(_ready(op, Einc, e_r, E_target), ep, erp, float(dx), float(freq),
+                                         _OBJ[objective], tp, float(tol), int(inner_it), int(outer_it), C.byref(F),
+                                         gep, gsp, flags, iters))
     return F.value, ge, gs, (flags[0], flags[1]), (iters[0], iters[1])
 
 

@@ -132,11 +132,12 @@ def release_cached_memory():
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) if torch is not None else None
 
 
-def _ready(op):
-    """An Operator's plan for a call on arrays, its stream ordered after torch's
-    current one: CUDA inputs may still be computed there, and the memory of new
-    outputs may still be read."""
-    if torch is not None and torch.cuda.is_initialized():
+def _ready(op, *arrays):
+    """An Operator's plan for a call on arrays.  With a CUDA tensor among them its
+    stream is ordered after torch's current one: inputs may still be computed
+    there, and the memory of new outputs may still be read.  A call on numpy arrays
+    runs beside what torch computes."""
+    if any(map(_is_cuda, arrays)):
         if op._device is None:
             op._device = torch.cuda.current_device()
         stream = _raw_stream(op._device) if _raw_stream else torch.cuda.current_stream(op._device).cuda_stream
@@ -177,7 +178,7 @@ class Operator:
             raise ValueError("fN must be 2L x 2M x 2N x 6")
         op = cls(Lf // 2, Mf // 2, Nf // 2, precision, nrhs_max)
         ptr, keep = _in(fN)
-        check(op.lib.marie_set_operator(_ready(op), ptr, Lf, Mf, Nf))
+        check(op.lib.marie_set_operator(_ready(op, fN), ptr, Lf, Mf, Nf))
         del keep
         return op
 
@@ -203,7 +204,7 @@ class Operator:
     def set_k(self, fK):
         """Upload the K operator into this plan (beside fN)."""
         ptr, keep = _in(fK)
-        check(self.lib.marie_set_operator_k(_ready(self), ptr, 2 * self.L, 2 * self.M, 2 * self.N))
+        check(self.lib.marie_set_operator_k(_ready(self, fK), ptr, 2 * self.L, 2 * self.M, 2 * self.N))
         del keep
         return self
 
@@ -246,8 +247,8 @@ class Operator:
         mcp, mck = _in(Mc)
         ip, ik = _in(idx, np.int64)
         n = int(np.asarray(idx).size) if not _is_cuda(idx) else int(idx.numel())
-        check(self.lib.marie_plan_bind_mv_AN(_ready(self), mrp, mcp, float(Gram), 1 if transp_flag == "transp" else 0,
-                                             ip, n))
+        check(self.lib.marie_plan_bind_mv_AN(_ready(self, Mr, Mc, idx), mrp, mcp, float(Gram),
+                                             1 if transp_flag == "transp" else 0, ip, n))
         return self
 
     def apply_mv_AN(self, J, precision="fp64"):
@@ -258,7 +259,7 @@ class Operator:
         nrhs = 1 if J.ndim == 1 else J.shape[1]
         jp, jk = _in(J)
         op_, out = _out(J.shape, cuda)
-        check(self.lib.marie_plan_apply_mv_AN(_ready(self), jp, op_, nrhs, _PREC[precision]))
+        check(self.lib.marie_plan_apply_mv_AN(_ready(self, J), jp, op_, nrhs, _PREC[precision]))
         if cuda:
             check(self.lib.marie_plan_synchronize(self.plan))
         return out
@@ -398,8 +399,8 @@ def mv_AN(JIn0, fN, Mr, Mc, Gram, transp_flag, idx, GPU_flag=1, precision="fp64"
         mcp, mck = _in(Mc)
         ip, ik = _in(idx, np.int64)
         op_, out = _out(JIn0.shape, cuda)
-        check(opr.lib.marie_mv_AN(_ready(opr), jp, mrp, mcp, float(Gram), 1 if transp_flag == "transp" else 0,
-                                  ip, n, op_, nrhs, prec))
+        check(opr.lib.marie_mv_AN(_ready(opr, JIn0, Mr, Mc, idx), jp, mrp, mcp, float(Gram),
+                                  1 if transp_flag == "transp" else 0, ip, n, op_, nrhs, prec))
         return out
     finally:
         if tmp:
@@ -417,7 +418,7 @@ def mv_L(JIn0, fN, r, Gram, idx, GPU_flag=1, precision="fp64"):
         jp, jk = _in(JIn0)
         ip, ik = _in(idx, np.int64)
         op_, out = _out(JIn0.shape, cuda)
-        check(opr.lib.marie_mv_L(_ready(opr), jp, float(Gram), ip, n, op_, nrhs, prec))
+        check(opr.lib.marie_mv_L(_ready(opr, JIn0, idx), jp, float(Gram), ip, n, op_, nrhs, prec))
         return out
     finally:
         if tmp:
@@ -447,7 +448,7 @@ def mv_K(JIn0, fK, r, idx, GPU_flag=1, precision="fp64"):
         jp, jk = _in(JIn0)
         ip, ik = _in(idx, np.int64)
         op_, out = _out(JIn0.shape, cuda)
-        check(opr.lib.marie_mv_K(_ready(opr), jp, ip, n, op_, nrhs, prec))
+        check(opr.lib.marie_mv_K(_ready(opr, JIn0, idx), jp, ip, n, op_, nrhs, prec))
         return out
     finally:
         if tmp:
@@ -463,7 +464,7 @@ def H_field_Kop(J, fK, Gram, Hinc=None, GPU_flag=1, precision="fp64"):
         jp, jk = _in(J)
         hp, hk = _in(Hinc) if Hinc is not None else (None, None)
         op_, out = _out(tuple(J.shape), _is_cuda(J))
-        check(opr.lib.marie_h_field_kop(_ready(opr), jp, float(Gram), hp, op_, _PREC[precision]))
+        check(opr.lib.marie_h_field_kop(_ready(opr, J, Hinc), jp, float(Gram), hp, op_, _PREC[precision]))
         return out
     finally:
         if tmp:
@@ -482,7 +483,8 @@ def E_field_Nop(J, fN, Gram, freq, Einc=None, GPU_flag=1, precision="fp64"):
         else:
             ep, ek = None, None
         op_, out = _out(tuple(J.shape), _is_cuda(J))
-        check(opr.lib.marie_e_field_nop(_ready(opr), jp, float(Gram), float(freq), ep, op_, _PREC[precision]))
+        check(opr.lib.marie_e_field_nop(_ready(opr, J, Einc), jp, float(Gram), float(freq), ep, op_,
+                                        _PREC[precision]))
         return out
     finally:
         if tmp:
@@ -574,7 +576,7 @@ def pgmres(A, b, restart=50, tol=1e-3, maxit=10, L1=None, L2=None, R1=None, R2=N
     cap = restart * maxit + 1
     resvec = np.zeros(cap)
     rlen = C.c_int64()
-    _call(opr.lib.marie_pgmres, _ready(opr), cbs[0], None, bp, n, int(restart), float(tol), int(maxit),
+    _call(opr.lib.marie_pgmres, _ready(opr, b, x0), cbs[0], None, bp, n, int(restart), float(tol), int(maxit),
           h[0], None, h[1], None, h[2], None, h[3], None, x0p, xp, C.byref(flag), C.byref(relres), it,
           resvec.ctypes.data_as(_lib._dp), cap, C.byref(rlen))
     return x, flag.value, relres.value, [it[0], it[1]], resvec[:rlen.value]
@@ -597,7 +599,7 @@ def pgmresDR(A, b, restart=50, tol=1e-3, maxit=10, ritz=None, L1=None, L2=None, 
     cap = restart * (maxit + 1) + 1
     resvec = np.zeros(cap)
     rlen = C.c_int64()
-    _call(opr.lib.marie_pgmres_dr, _ready(opr), cbs[0], None, bp, n, int(restart), float(tol), int(maxit),
+    _call(opr.lib.marie_pgmres_dr, _ready(opr, b, x0), cbs[0], None, bp, n, int(restart), float(tol), int(maxit),
           int(ritz) if ritz is not None else 0, h[0], None, h[1], None, h[2], None, h[3], None, x0p, xp,
           C.byref(flag), C.byref(relres), it, resvec.ctypes.data_as(_lib._dp), cap, C.byref(rlen))
     return x, flag.value, relres.value, [it[0], it[1]], resvec[:rlen.value]
@@ -620,8 +622,8 @@ def bicgstab(A, b, tol=1e-6, maxit=None, M1=None, M2=None, x0=None):
     cap = 2 * maxit + 1
     resvec = np.zeros(cap)
     rlen = C.c_int64()
-    _call(opr.lib.marie_bicgstab, _ready(opr), cbs[0], None, bp, n, float(tol), int(maxit), h[0], None, h[1], None,
-          x0p, xp, C.byref(flag), C.byref(relres), C.byref(it), resvec.ctypes.data_as(_lib._dp), cap,
+    _call(opr.lib.marie_bicgstab, _ready(opr, b, x0), cbs[0], None, bp, n, float(tol), int(maxit), h[0], None, h[1],
+          None, x0p, xp, C.byref(flag), C.byref(relres), C.byref(it), resvec.ctypes.data_as(_lib._dp), cap,
           C.byref(rlen))
     return x, flag.value, relres.value, it.value, resvec[:rlen.value]
 
@@ -672,10 +674,10 @@ def JVIE_Solver(Einc, e_r, r, freq, fN, tol=None, form=None, solver=None, precon
         resvec = np.zeros(cap)
         rlen = C.c_int64()
         solvert = C.c_double()
-        check(opr.lib.marie_jvie_solve(_ready(opr), ep, erp, dx, float(freq), float(tol), int(form), solver.encode(),
-                                       pc, int(max_it), int(inner_it), int(outer_it), int(ritz), jp, C.byref(flag),
-                                       C.byref(relres), it, resvec.ctypes.data_as(_lib._dp), cap, C.byref(rlen),
-                                       C.byref(solvert)))
+        check(opr.lib.marie_jvie_solve(_ready(opr, Einc, e_r), ep, erp, dx, float(freq), float(tol), int(form),
+                                       solver.encode(), pc, int(max_it), int(inner_it), int(outer_it), int(ritz), jp,
+                                       C.byref(flag), C.byref(relres), it, resvec.ctypes.data_as(_lib._dp), cap,
+                                       C.byref(rlen), C.byref(solvert)))
         iters = it[0] if solver == "B" else [int(it[0]), int(it[1])]
         resvec = resvec[:min(rlen.value, cap)]
         if logfile is not None or runlog is not None:
@@ -736,7 +738,7 @@ def Scat_Solver(Einc, Hinc, freq, r, epsilon_r, sigma_e, rho, tol=None, fN=None,
         opr = Operator(L, M, N, precision)
         if fN is not None:
             ptr, keep = _in(fN)
-            check(opr.lib.marie_set_operator(_ready(opr), ptr, 2 * L, 2 * M, 2 * N))
+            check(opr.lib.marie_set_operator(_ready(opr, fN), ptr, 2 * L, 2 * M, 2 * N))
         if fK is not None:
             opr.set_k(fK)
     cuda = _is_cuda(Einc)
@@ -750,9 +752,9 @@ def Scat_Solver(Einc, Hinc, freq, r, epsilon_r, sigma_e, rho, tol=None, fN=None,
     eo, Eout = _out((L, M, N, 3), cuda)
     bo, Bout = _out((L, M, N, 3), cuda)
     gsar, pabs = C.c_double(), C.c_double()
-    check(opr.lib.marie_scat_solver(_ready(opr), ep, hp, dx, float(freq), epsp, sp_, rp_, float(tol), int(form),
-                                    solver.encode(), pc, int(max_it), int(inner_it), int(outer_it), int(ritz), jp, spo,
-                                    eo, bo, C.byref(gsar), C.byref(pabs)))
+    check(opr.lib.marie_scat_solver(_ready(opr, Einc, Hinc, epsilon_r, sigma_e, rho), ep, hp, dx, float(freq), epsp,
+                                    sp_, rp_, float(tol), int(form), solver.encode(), pc, int(max_it), int(inner_it),
+                                    int(outer_it), int(ritz), jp, spo, eo, bo, C.byref(gsar), C.byref(pabs)))
     solvelog.write_overall_log(logfile, time.perf_counter() - tstart)
     return Jout, Sout, Eout, Bout, gsar.value, pabs.value, opr
 
@@ -781,8 +783,8 @@ def JVIE_Solver_batch(Einc, e_r, r, freq, fN, tol=None, form=None, precond=None,
         relres = np.zeros(nexc)
         it = np.zeros(2 * nexc, np.int32)
         solvert = C.c_double()
-        check(opr.lib.marie_jvie_solve_batch(_ready(opr), ep, nexc, erp, dx, float(freq), int(form), pc, float(tol),
-                                             int(inner_it), int(outer_it), jp,
+        check(opr.lib.marie_jvie_solve_batch(_ready(opr, Einc, e_r), ep, nexc, erp, dx, float(freq), int(form), pc,
+                                             float(tol), int(inner_it), int(outer_it), jp,
                                              flag.ctypes.data_as(_lib._ip), relres.ctypes.data_as(_lib._dp),
                                              it.ctypes.data_as(_lib._ip), C.byref(solvert)))
         return Je, flag, relres, it.reshape(nexc, 2), solvert.value
@@ -818,7 +820,7 @@ def JVIE_Solver_bodies(bodies, freq, tol=None, form=None, precond=None, inner_it
         Erp.append(erp.value)
         Jp.append(jp.value)
         outs.append(Je)
-        plans[b] = _ready(op).value
+        plans[b] = _ready(op, Einc, e_r).value
     tot = int(nexc.sum())
     flag = np.zeros(tot, np.int32)
     relres = np.zeros(tot)
@@ -876,8 +878,9 @@ def jvie2solver(Vrhs, fN, idx, Mr, Mc, Gram, tol, Vini=None, max_it=1000):
         relres = C.c_double()
         it = C.c_double()
         solvert = C.c_double()
-        check(opr.lib.marie_jvie2solver(_ready(opr), ip, n, mrp, mcp, float(Gram), bp, float(tol), int(max_it), xp, op_,
-                                        C.byref(flag), C.byref(relres), C.byref(it), C.byref(solvert)))
+        check(opr.lib.marie_jvie2solver(_ready(opr, idx, Mr, Mc, Vrhs, Vini), ip, n, mrp, mcp, float(Gram), bp,
+                                        float(tol), int(max_it), xp, op_, C.byref(flag), C.byref(relres), C.byref(it),
+                                        C.byref(solvert)))
         return out, flag.value, relres.value, it.value, solvert.value
     finally:
         if tmp:

@@ -341,3 +341,32 @@ def test_conjugate_and_negative_views_are_read_as_their_values(cuda):
     E = [mg.E_field_Nop(f, op, dx**3, 298e6, F) for f in (F.conj(), F.conj().resolve_conj())]
     assert torch.equal(*E)
     op.close()
+
+
+def test_calls_on_numpy_arrays_run_beside_torchs_stream(cuda):
+    """Host arrays have nothing to wait for: a product returns while a second of
+    work is still queued on torch's current stream."""
+    import torch
+
+    import marie_gb300 as mg
+
+    shape, dx = (16, 12, 20), 5e-3
+    op = mg.Operator.assemble(*shape, dx, 298e6)
+    n = 3 * int(np.prod(shape))
+    rng = np.random.default_rng(1)
+    idx = np.arange(1, n + 1)
+    er = np.asfortranarray(rng.uniform(2, 40, shape) - 10j)
+    op.bind_mv_AN(er / er, (er - 1) / er, dx**3, "notransp", idx)
+    J = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    ref = op.apply_mv_AN(J)
+    big = torch.ones(4096, 4096, dtype=torch.float64, device=cuda)
+    out = torch.mm(big, big)
+    torch.cuda.synchronize()
+    for _ in range(10):  # 0.11 s each at the FP64 pipe's rate
+        torch.mm(big, big, out=out)
+    x = op.apply_mv_AN(J)
+    busy = not torch.cuda.current_stream().query()
+    torch.cuda.synchronize()
+    assert busy
+    np.testing.assert_array_equal(x, ref)
+    op.close()
