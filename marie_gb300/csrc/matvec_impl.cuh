@@ -40,14 +40,14 @@ template <typename T> struct MatvecImpl {
       return launch_pass(k_xfwd_rows<NL, THR, IO>, grid, RowCfg<V, NL, THR>::THREADS, X::bytes, st, J, js, inv, pro, A,
                          as, d, tw);
     } else {
-    constexpr int S = RowCfg<cplx<T>, NL, THR>::S;
-    const size_t smem = (size_t)(NL + NL * (S + 1)) * sizeof(V);
-    cudaError_t e = opt_in_smem(k_xfwd<T, NL, THR, IO>, smem);
-    if (e != cudaSuccess) return e;
-    const int rows = d.M * d.N * 3;
-    dim3 grid((rows + S - 1) / S, nrhs);
-    return launch_pass(k_xfwd<T, NL, THR, IO>, grid, RowCfg<cplx<T>, NL, THR>::THREADS, smem, st, J, js, inv, pro, A, as,
-                       d, tw);
+      constexpr int S = RowCfg<cplx<T>, NL, THR>::S;
+      const size_t smem = (size_t)(NL + NL * (S + 1)) * sizeof(V);
+      cudaError_t e = opt_in_smem(k_xfwd<T, NL, THR, IO>, smem);
+      if (e != cudaSuccess) return e;
+      const int rows = d.M * d.N * 3;
+      dim3 grid((rows + S - 1) / S, nrhs);
+      return launch_pass(k_xfwd<T, NL, THR, IO>, grid, RowCfg<cplx<T>, NL, THR>::THREADS, smem, st, J, js, inv, pro, A, as,
+                         d, tw);
     }
   }
   template <int NL, int THR, typename IO>
@@ -61,14 +61,14 @@ template <typename T> struct MatvecImpl {
       return launch_pass(k_xinv_rows<NL, THR, IO>, grid, RowCfg<V, NL, THR>::THREADS, X::bytes, st, A, as, J, js, inv,
                          ep, out, os, d, tw);
     } else {
-    constexpr int S = RowCfg<cplx<T>, NL, THR>::S;
-    const size_t smem = (size_t)(NL + NL * (S + 1)) * sizeof(V);
-    cudaError_t e = opt_in_smem(k_xinv<T, NL, THR, IO>, smem);
-    if (e != cudaSuccess) return e;
-    const int rows = d.M * d.N * 3;
-    dim3 grid((rows + S - 1) / S, nrhs);
-    return launch_pass(k_xinv<T, NL, THR, IO>, grid, RowCfg<cplx<T>, NL, THR>::THREADS, smem, st, A, as, J, js, inv, ep,
-                       out, os, d, tw);
+      constexpr int S = RowCfg<cplx<T>, NL, THR>::S;
+      const size_t smem = (size_t)(NL + NL * (S + 1)) * sizeof(V);
+      cudaError_t e = opt_in_smem(k_xinv<T, NL, THR, IO>, smem);
+      if (e != cudaSuccess) return e;
+      const int rows = d.M * d.N * 3;
+      dim3 grid((rows + S - 1) / S, nrhs);
+      return launch_pass(k_xinv<T, NL, THR, IO>, grid, RowCfg<cplx<T>, NL, THR>::THREADS, smem, st, A, as, J, js, inv, ep,
+                         out, os, d, tw);
     }
   }
   // An x pass of 256-thread CTAs is taken when it fills the chip four times over;
@@ -77,7 +77,7 @@ template <typename T> struct MatvecImpl {
   // x 20 grid, two CTAs before, 34 -> 15 and 47 -> 18 us.
   template <int NL> static bool many_rows(const Dims& d, int nrhs) {
     constexpr int S = RowCfg<cplx<T>, NL>::S;
-    return ((long long)d.M * d.N * 3 + S - 1) / S * nrhs >= 4 * 152;
+    return ((long long)d.M * d.N * 3 + S - 1) / S * nrhs >= 4LL * sm_count();
   }
   template <int NL, typename IO>
   static cudaError_t xfwd_n(const IO* J, long long js, const int* inv, Prologue pro, V* A, long long as,
@@ -164,12 +164,12 @@ template <typename T> struct MatvecImpl {
 #undef MARIE_CASE
       }
     } else {
-      switch (NC) {
+        switch (NC) {
 #define MARIE_CASE(n_) \
   case n_: return cols_n<n_, false>(in, in_w, in_rhs, n_in, out, out_w, out_rhs, n_out, Lp, nw, tw, nrhs, st, stop, step);
-        MARIE_FFT_LENGTHS(MARIE_CASE)
+          MARIE_FFT_LENGTHS(MARIE_CASE)
 #undef MARIE_CASE
-      }
+        }
     }
     return cudaErrorInvalidValue;
   }
@@ -228,7 +228,7 @@ template <typename T> struct FusedImpl {
                       (void*)&twx, (void*)&twy};
       return launch(k_xyfwd<T, NL, NM, CS, IO>, CS, CS * 3 * d.N, nrhs, XYCfg<T, NL, NM, CS>::fwd_smem, st, args);
     } else {
-      return cudaErrorNotSupported;
+        return cudaErrorNotSupported;
     }
   }
   template <int NL, int NM, int CS, typename IO>
@@ -240,7 +240,7 @@ template <typename T> struct FusedImpl {
                       (void*)&os, (void*)&d, (void*)&twx, (void*)&twy};
       return launch(k_yxinv<T, NL, NM, CS, IO>, CS, CS * 3 * d.N, nrhs, XYCfg<T, NL, NM, CS>::inv_smem, st, args);
     } else {
-      return cudaErrorNotSupported;
+        return cudaErrorNotSupported;
     }
   }
 };
