@@ -537,8 +537,9 @@ static EncodeTiledFn encode_tiled() {
 }
 
 // The z pass's bulk tile source of an FP32 octant N operator: fN32x and its
-// tensor map (boxes of 8 columns) over (2L, M+1, N+1, 6) 8-byte elements.  Without the driver entry point, or with N + 1 > 256 (beyond the
-// box limit), the plan keeps the per-thread tile copies.
+// tensor map (boxes of 8 columns) over (2L, M+1, N+1, 6) 8-byte elements.
+// Without the driver entry point, or with N + 1 > 256 (beyond the box limit), the
+// plan keeps the per-thread tile copies.
 size_t fullx_elems(const Dims& d) { return (size_t)6 * d.Lp * (d.M + 1) * (d.N + 1); }
 
 // Fills p->fN32x from the operator (full or octant, scaled by s here) and

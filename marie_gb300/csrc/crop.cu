@@ -19,8 +19,15 @@
 // matrices are at most 257 square and run at the FP64 pipe's rate).
 // Measured with ellipsoid phantoms (whole grid -> box): FP64 product of a 96 x
 // 80 x 64 grid 2.24 -> 0.61 ms, FP32 product of 256 x 192 x 160 3.15 -> 0.41 ms,
-// BiCGSTAB solve of 48^3 in FP64 217 -> 138 ms; the first solve or product of a
-// new plan, the new spectrum included, gains as well.
+// BiCGSTAB solve of 48^3 in FP64 217 -> 138 ms.
+//
+// The maps are FP64 work (31 GFLOP from 256 x 192 x 160 to 128 x 80 x 128): a
+// plan's first solve or bind on a box, and every one after a body of another box,
+// takes 30 ms more there, 4.3 ms more for 128^3 (to 128 x 80 x 128) and 1.0 ms
+// more for 96 x 80 x 64; a bind on the box that the plan holds takes 0.5 to 0.7
+// ms in all.  A solve's first use pays for it; a bound FP32 product does after 11
+// applications at 256 x 192 x 160 and about 24 at 128^3, an FP64 one of 96 x 80 x
+// 64 after one.
 #include <algorithm>
 #include <cstring>
 #include <vector>

@@ -25,12 +25,15 @@
 namespace marie {
 
 // Restart length of the inner GMRES of mixed-precision refinement with an FP64
-// Krylov basis (when the plan sets none).  Its Gram-Schmidt costs ~0.016 ms
-// per basis vector per step at 128^3 on the FP64 pipe, so shorter cycles win
-// although they take more matvecs: measured on the 128^3 phantom, restart
-// 12 / 20 / 30 / 50 gave 224 / 224 / 241 / 262 ms per solve (303 / 273 / 261 /
-// 236 matvecs) with products of 0.455 ms (0.25 ms since; 20 takes 156 ms).  With the FP32 basis the time is flat in the restart and the
-// caller's inner_it is kept.
+// Krylov basis (when the plan sets none).  Its Gram-Schmidt costs ~0.01 ms per
+// basis vector per step at 128^3 on the FP64 pipe, so shorter cycles win although
+// they take more matvecs.  Measured on three ellipsoid phantoms, restart 8 / 12 /
+// 16 / 20 / 24 / 30 / 50: one excitation of 128^3 198 / 176 / 189 / 188 / 200 /
+// 210 / 240 ms, eight of 64^3 121 / 101 / 102 / 105 / 110 / 116 / 143 ms, the
+// gradient of 64^3 76 / 62 / 62 / 63 / 65 / 68 / 82 ms: flat from 12 to 20 but for
+// the first, whose 12 may be that body's.  20 was chosen when products cost
+// almost twice as much.  With the FP32 basis the time is flat in the restart and
+// the caller's inner_it is kept.
 constexpr int kInnerRestart64 = 20;
 
 // EMconstants.m:13-20

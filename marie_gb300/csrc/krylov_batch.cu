@@ -511,7 +511,8 @@ __device__ void givens_warp(const GState& G, int m, int k, const double2* __rest
   if (lane == 0) G.stop[s] = k;
 }
 // w_s -= V_s(:,0:k) h_s with w_s = V_s(:,k) ; partial norms of the new w_s,
-// then the Givens step of the system (givens_warp) by the last block
+// then the Givens step of the system (givens_warp) by the last block.
+//
 // FP64-pipe bound at large n (4 FMAs per element and column); at 40k to 170k
 // rows the step's end counts as much, hence givens_warp's short chains: 42k
 // rows and 19 columns 25.8 -> 18.6 us, 170k rows and 40 columns 84 -> 68 us.

@@ -45,8 +45,8 @@ __device__ __forceinline__ bool rhs_skipped(const Dims& d, int rhs) { return d.s
 // operator tile and twiddles), then waits for it to complete (pdl_wait; a
 // no-op when launched without the attribute) before reading anything else.
 // The skip mask read at the top of the passes after the first is written by
-// the Givens step at least two kernels earlier, and the first pass has waited.  A pass signals with pdl_trigger,
-// in its last phase, that the next one may start.
+// the Givens step at least two kernels earlier, and the first pass has waited.
+// A pass signals with pdl_trigger, in its last phase, that the next one may start.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -74,13 +74,13 @@ struct Epilogue {
   const float2* af;
   const float2* bf;
 };
-// Prologue: x_in[k] = (pre ? pre[k] : 1) * (conjin ? conj(J[k]) : J[k])
 // Rows (y) and planes (z) of a DOF map that starts at its body's box, 0: the
 // whole grid's.
 struct Extent {
   int M = 0, N = 0;
 };
 
+// Prologue: x_in[k] = (pre ? pre[k] : 1) * (conjin ? conj(J[k]) : J[k])
 struct Prologue {
   const double2* pre;
   int conjin;
@@ -256,12 +256,16 @@ template <typename V> __device__ __forceinline__ V cfma(V a, V b, V c) {
 
 // out[kk] = A J - B v of one row sweep: reg[i] is the circulant term at DOF
 // kk[i] (-1: none).  In the vectors' precision: the diagonal term of FP64 vectors
-// is FP64's whatever the transforms' is (for bodies of low contrast it is most of
-// the result: with a relative permittivity of 1.2 the FP32 product of 96 x 80 x
-// 64 is off by 2e-8, with an FP32 epilogue by 6e-8).  Its ten FP64 instructions
-// per DOF cost 22 us of a 128^3 product's 344 (322 with an FP32 epilogue).
-// Per-DOF loads in groups of EPI (bounded registers): groups of 4 took 345 us
-// where groups of 2 took 348.
+// is FP64's whatever the transforms' is.  For bodies of low contrast it is most of
+// the result (relative permittivity 1.2, 96 x 80 x 64: the FP32 product is off by
+// 2e-8, with an FP32 epilogue by 6e-8).  Where the circulant term is as large, its
+// own 2e-7 covers the difference, and which form is nearer depends on how Gram
+// rounds to FP32: random vectors on tissue, FP32 and FP64 epilogue, 2.4e-7 and
+// 2.7e-7 (128^3 at 2 mm), 2.6e-7 and 2.2e-7 (at 3 mm), 1.9e-7 and 2.1e-7 (96 x 80
+// x 64 at 2 mm), 2.4e-7 and 2.1e-7 (64^3 at 3 mm).  The ten FP64 instructions per
+// DOF cost 22 us of a 128^3 product's 344 (322 with an FP32 epilogue).  Per-DOF
+// loads in groups of EPI (bounded registers): groups of 4 took 345 us where groups
+// of 2 took 348.
 template <typename IO, typename V, int E, int EPI>
 __device__ __forceinline__ void epilogue_dofs(const V* reg, const int* kk, const IO* Jr, const Epilogue& ep, IO* outr) {
 #pragma unroll
@@ -296,8 +300,9 @@ __device__ __forceinline__ void epilogue_dofs(const V* reg, const int* kk, const
 // spectrum go straight between global memory and the transform's registers
 // (16-value schedules: whole 128-byte segments per access); only the exchange
 // between its passes uses shared memory.  Staging the rows through shared
-// memory first, as the FP64 passes do (whose time is the FP64 pipe's), cost
-// two more shared round trips and three barriers per row.  Measured with every
+// memory first, as the FP64 passes do (30 and 48 us on a 48^3 body's box, where
+// the FP64 pipe needs 8: few warps per SM and a division per staged element),
+// cost two more shared round trips and three barriers per row.  Measured with every
 // voxel a DOF: first pass of a 64^3 grid 21 -> 13 us, of 96^3 60 -> 38 us; of
 // 128^3, where the vectors' own 20 bytes per DOF bound it, 96 -> 93 us.
 template <int NL, int THR> struct XRow {
