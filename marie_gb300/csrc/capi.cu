@@ -909,7 +909,11 @@ int marie_plan_after_stream(marie_plan* p, void* stream) {
     return MARIE_OK;
   }
   if (!p->after) MARIE_CUDA_TRY(cudaEventCreateWithFlags(&p->after, cudaEventDisableTiming));
-  MARIE_CUDA_TRY(cudaEventRecord(p->after, other));
+  if (cudaEventRecord(p->after, other) != cudaSuccess) {  // a stream of another device
+    cudaGetLastError();
+    MARIE_CUDA_TRY(cudaStreamSynchronize(other));
+    return MARIE_OK;
+  }
   MARIE_CUDA_TRY(cudaStreamWaitEvent(p->stream, p->after, 0));
   return MARIE_OK;
 }

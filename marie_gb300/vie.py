@@ -137,13 +137,14 @@ def _ready(op, *arrays):
     stream is ordered after torch's current one: inputs may still be computed
     there, and the memory of new outputs may still be read.  A call on numpy arrays
     runs beside what torch computes."""
-    if any(map(_is_cuda, arrays)):
-        if op._device is None:
-            op._device = torch.cuda.current_device()
-        stream = _raw_stream(op._device) if _raw_stream else torch.cuda.current_stream(op._device).cuda_stream
-        status = op.lib.marie_plan_after_stream(op._plan, stream)
-        if status:
-            check(status)
+    for a in arrays:
+        if _is_cuda(a):
+            dev = a.get_device()
+            stream = _raw_stream(dev) if _raw_stream else torch.cuda.current_stream(dev).cuda_stream
+            status = op.lib.marie_plan_after_stream(op._plan, stream)
+            if status:
+                check(status)
+            break
     return op.plan
 
 
@@ -161,7 +162,6 @@ class Operator:
         ph = C.c_void_p()
         check(self.lib.marie_plan_create(self.L, self.M, self.N, self.precision, int(nrhs_max), None, C.byref(ph)))
         self._plan = ph
-        self._device = None  # torch's index of the plan's device, from the first call on arrays
         self.dx = None
         self.freq = None
 
