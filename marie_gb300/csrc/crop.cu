@@ -328,6 +328,13 @@ void crop_settings(const marie_plan* p, marie_plan* q) {
   q->graph_refine = p->graph_refine;
 }
 
+void drain(cudaStream_t st) {
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusActive;
+  if (cudaStreamIsCapturing(st, &capturing) == cudaSuccess && capturing == cudaStreamCaptureStatusNone)
+    cudaStreamSynchronize(st);
+  cudaGetLastError();
+}
+
 bool give_crop_back(marie_plan* p) {
   if (!p->crop && !p->bnd_crop) return false;
   p->crop.reset();

@@ -189,15 +189,20 @@ void crop_settings(const marie_plan* p, marie_plan* q);
 // For a call that finds no memory: gives the plan's crop, a bound mv_AN's
 // included, and the pool's cached blocks back.  False when the plan holds none.
 bool give_crop_back(marie_plan* p);
+void drain(cudaStream_t st);  // waits for a stream that is not being captured
 // Runs call(); when it finds no memory while the plan holds a crop, gives that
-// back and runs it again on the whole grid, as if no crop had been made.
+// back and runs it again on the whole grid, as if no crop had been made.  A call
+// that fails returns when the plan's stream is done: its caller may free or reuse
+// the arrays at once.
 template <typename F> int on_box_or_whole_grid(marie_plan* p, F&& call) {
   int s = call();
-  if (s != MARIE_ENOMEM || !give_crop_back(p)) return s;
-  const bool outer = p->whole_grid;
-  p->whole_grid = true;
-  s = call();
-  p->whole_grid = outer;
+  if (s == MARIE_ENOMEM && give_crop_back(p)) {
+    const bool outer = p->whole_grid;
+    p->whole_grid = true;
+    s = call();
+    p->whole_grid = outer;
+  }
+  if (s != MARIE_OK && p) drain(p->stream);
   return s;
 }
 Extent box_extent(const marie_plan* q, const int box[6]);

@@ -370,3 +370,34 @@ def test_calls_on_numpy_arrays_run_beside_torchs_stream(cuda):
     assert busy
     np.testing.assert_array_equal(x, ref)
     op.close()
+
+
+def test_a_call_that_fails_leaves_nothing_on_its_stream(cuda):
+    """A product that finds no memory behind work it waits for returns when the
+    plan's stream is idle, so its arrays may be freed at once."""
+    import torch
+
+    import marie_gb300 as mg
+
+    shape, dx = (16, 12, 20), 5e-3
+    op = mg.Operator.assemble(*shape, dx, 298e6)
+    n = 3 * int(np.prod(shape))
+    M = torch.ones(tuple(reversed(shape)), dtype=torch.complex128, device=cuda).permute(2, 1, 0)
+    J = torch.randn(n, dtype=torch.complex128, device=cuda)
+    idx = torch.arange(n, device=cuda) + 1
+    ref = mg.mv_AN(J, op, M, 0.5 * M, dx**3, "notransp", idx)
+    Mc = 0.5 * M
+    big = torch.ones(4096, 4096, dtype=torch.float64, device=cuda)
+    out = torch.mm(big, big)
+    stream = torch.cuda.ExternalStream(op.lib.marie_plan_stream(op.plan))
+    torch.cuda.synchronize()
+    torch.mm(big, big, out=out)
+    op.lib.marie_inject_alloc_failure(2)
+    try:
+        with pytest.raises(mg.MarieError):
+            mg.mv_AN(J, op, M, Mc, dx**3, "notransp", idx)
+        assert stream.query()
+    finally:
+        op.lib.marie_inject_alloc_failure(0)
+    assert torch.equal(mg.mv_AN(J, op, M, Mc, dx**3, "notransp", idx), ref)
+    op.close()
